@@ -72,6 +72,7 @@ bool derive_params(const SceneConfig& c, DevParams& d, std::string* err) {
     d.gamma = c.gamma;
     const float inv_gamma = (c.gamma == 0.0f) ? 1.0f : 1.0f / c.gamma;
     d.eos_k = c.gas_constant * c.rest_density * inv_gamma;
+    d.cs_k = c.gas_constant / d.inv_rest_density;
     d.mass = c.mass;
     d.two_mass = 2.0f * c.mass;
     d.particle_size = c.particle_size;
@@ -101,7 +102,9 @@ bool derive_params(const SceneConfig& c, DevParams& d, std::string* err) {
     return true;
 }
 
-uint64_t Engine::bytes_per_particle() { return 10 * 16 + 5 * 4 + SPH_MASK_ROWS * 4; }
+// eight float4 arrays and the 32-byte records; key, slot, perm, okey and rho
+// (the sort's scatter list shares the mask words)
+uint64_t Engine::bytes_per_particle() { return 8 * 16 + 32 + 5 * 4 + SPH_MASK_ROWS * 4; }
 uint64_t Engine::bytes_per_cell() { return 2 * 4 + 1; }
 const char* Engine::pass_name(int i) { return (i >= 0 && i < kPasses) ? kPassNames[i] : "?"; }
 
@@ -163,9 +166,11 @@ int Engine::cuda_fail(cudaError_t e, const char* what) {
     } while (0)
 
 void Engine::free_all() {
-    float4** f4[] = {&P0_, &P1_, &V0_, &V1_, &V2_, &A0_, &A1_, &S_, &N_, &Vc_, &dbg_forces_};
+    float4** f4[] = {&P0_, &P1_, &V0_, &V1_, &V2_, &A0_, &A1_, &N_, &R_, &dbg_forces_};
     for (auto p : f4) { if (*p) cudaFree(*p); *p = nullptr; }
-    uint32_t** u[] = {&key_, &slot_, &tmp_, &perm_, &count_, &start_, &scan_sums_, &dbg_nbr_, &mask_,
+    if (rho_) cudaFree(rho_);
+    rho_ = nullptr;
+    uint32_t** u[] = {&key_, &slot_, &perm_, &count_, &start_, &scan_sums_, &dbg_nbr_, &mask_,
                       &okey_, &pend_};
     for (auto p : u) { if (*p) cudaFree(*p); *p = nullptr; }
     if (stage_) cudaFree(stage_);
@@ -191,31 +196,25 @@ int Engine::ensure_capacity(uint64_t parts, uint64_t cells) {
     if (plan.parts > pcap_) {
         const uint64_t np = plan.parts;
         if (np >= (1ull << 31)) return fail(ENG_ENOMEM, "particle capacity exceeds 2^31");
-        // state between substeps: P0, V0, A0, S, and for scenes with a
-        // pending XSPH update their post-integration velocities V2 and cells
-        float4** state[] = {&P0_, &V0_, &A0_, &S_, &V2_};
-        float4** scratch[] = {&P1_, &V1_, &A1_, &N_, &Vc_};
-        for (auto p : state) {
-            float4* q = nullptr;
-            cudaError_t e = cudaMalloc((void**)&q, np * sizeof(float4));
+        // state between substeps: P0, V0, A0, and for scenes with a pending
+        // XSPH update their post-integration velocities V2 and cells; and the
+        // fields of the last substep that the debug taps read (rho, R)
+        struct Kept { void** p; size_t entry; };
+        const Kept state[] = {{(void**)&P0_, sizeof(float4)}, {(void**)&V0_, sizeof(float4)},
+                              {(void**)&A0_, sizeof(float4)}, {(void**)&V2_, sizeof(float4)},
+                              {(void**)&R_, 2 * sizeof(float4)}, {(void**)&rho_, sizeof(float)},
+                              {(void**)&okey_, sizeof(uint32_t)}};
+        float4** scratch[] = {&P1_, &V1_, &A1_, &N_};
+        for (const Kept& k : state) {
+            void* q = nullptr;
+            cudaError_t e = cudaMalloc(&q, np * k.entry);
             if (e != cudaSuccess) return fail(ENG_ENOMEM, std::string("device allocation failed: ") + cudaGetErrorString(e));
-            if (*p) {
-                ENG_CK(cudaMemcpyAsync(q, *p, pcap_ * sizeof(float4), cudaMemcpyDeviceToDevice, stream_), "grow copy");
+            if (*k.p) {
+                ENG_CK(cudaMemcpyAsync(q, *k.p, pcap_ * k.entry, cudaMemcpyDeviceToDevice, stream_), "grow copy");
                 ENG_CK(cudaStreamSynchronize(stream_), "grow sync");
-                cudaFree(*p);
+                cudaFree(*k.p);
             }
-            *p = q;
-        }
-        {
-            uint32_t* q = nullptr;
-            cudaError_t e = cudaMalloc((void**)&q, np * sizeof(uint32_t));
-            if (e != cudaSuccess) return fail(ENG_ENOMEM, std::string("device allocation failed: ") + cudaGetErrorString(e));
-            if (okey_) {
-                ENG_CK(cudaMemcpyAsync(q, okey_, pcap_ * sizeof(uint32_t), cudaMemcpyDeviceToDevice, stream_), "grow copy");
-                ENG_CK(cudaStreamSynchronize(stream_), "grow sync");
-                cudaFree(okey_);
-            }
-            okey_ = q;
+            *k.p = q;
         }
         prefix_valid_ = false;
         for (auto p : scratch) {
@@ -224,7 +223,7 @@ int Engine::ensure_capacity(uint64_t parts, uint64_t cells) {
             cudaError_t e = cudaMalloc((void**)p, np * sizeof(float4));
             if (e != cudaSuccess) return fail(ENG_ENOMEM, std::string("device allocation failed: ") + cudaGetErrorString(e));
         }
-        uint32_t** u[] = {&key_, &slot_, &tmp_, &perm_};
+        uint32_t** u[] = {&key_, &slot_, &perm_};
         for (auto p : u) {
             if (*p) cudaFree(*p);
             *p = nullptr;
@@ -514,15 +513,15 @@ StepArgs Engine::args() const {
     a.total_cells = total_cells_;
     a.P0 = P0_; a.V0 = V0_; a.A0 = A0_;
     a.P1 = P1_; a.V1 = V1_; a.A1 = A1_;
-    a.V2 = V2_; a.S = S_; a.N = N_;
-    a.Vc = Vc_; a.okey = okey_; a.pend = pend_;
+    a.V2 = V2_; a.rho = rho_; a.N = N_;
+    a.R = R_; a.okey = okey_; a.pend = pend_;
     a.count = count_; a.start = start_; a.scan_sums = scan_sums_;
     a.scan_first = 0u;
     a.scan_cells = 0u;   // all cells
     a.scan_zeroes_counts = 1u;
     a.scan_spin_limit = scan_spin_limit_;
     a.scan_withhold = scan_withhold_ ? 1u : 0u;
-    a.key = key_; a.slot = slot_; a.tmp = tmp_; a.perm = perm_;
+    a.key = key_; a.slot = slot_; a.tmp = mask_; a.perm = perm_;
     a.status = status_;
     a.mask = mask_;
     a.mask_stride = pcap_;
@@ -769,7 +768,7 @@ int Engine::step(uint32_t substeps, bool sync) {
 }
 
 // Run the next substep's prefix once, for reads of scenes whose XSPH update
-// is pending: its density pass computes the updated velocities (Vc); the next
+// is pending: its density pass computes the updated velocities (in R); the next
 // step() starts from the suffix, so the work is not repeated.  With
 // wait = false the caller reads the status word (read_status) afterwards and
 // clears prefix_valid_ if it reports an error.
@@ -928,7 +927,7 @@ int Engine::set_state(int id, const float* pos, const float* vel, uint32_t n, bo
         }
     }
     clear_pending(*s);
-    ENG_CK(launch_unpack(dpos, dvel, n, s->part_base, P0_, V0_, A0_, S_, stream_), "unpack");
+    ENG_CK(launch_unpack(dpos, dvel, n, s->part_base, P0_, V0_, A0_, rho_, stream_), "unpack");
     ENG_CK(cudaStreamSynchronize(stream_), "upload sync");
     return ENG_OK;
 }
@@ -964,7 +963,7 @@ int Engine::generate_lattice(int id, const LatticeSpec& spec, uint32_t first) {
     if (s->pending) { int rc = materialize(*s); if (rc) return rc; }
     prefix_valid_ = false;
     hashed_ = false;
-    ENG_CK(launch_lattice(spec, s->part_base + first, P0_, V0_, A0_, S_, stream_), "lattice");
+    ENG_CK(launch_lattice(spec, s->part_base + first, P0_, V0_, A0_, rho_, stream_), "lattice");
     return ENG_OK;
 }
 
@@ -1127,7 +1126,7 @@ int Engine::load_state(int id, const float4* host, uint32_t n) {
     ENG_CK(cudaMemcpyAsync(V0_ + s->part_base, host + n, bytes, cudaMemcpyHostToDevice, stream_), "restore");
     ENG_CK(cudaMemcpyAsync(A0_ + s->part_base, host + 2 * (size_t)n, bytes, cudaMemcpyHostToDevice, stream_),
            "restore");
-    ENG_CK(cudaMemsetAsync(S_ + s->part_base, 0, bytes, stream_), "restore");
+    ENG_CK(cudaMemsetAsync(rho_ + s->part_base, 0, n * sizeof(float), stream_), "restore");
     ENG_CK(cudaStreamSynchronize(stream_), "restore sync");
     return ENG_OK;
 }
@@ -1196,11 +1195,22 @@ int Engine::debug_get(int id, int field, void* host, uint64_t count) {
         case F_PRESSURE:
         case F_SOUNDSPEED: {
             if (!need(n)) return fail(ENG_EINVAL, "buffer too small");
-            std::vector<float4> v(n);
-            ENG_CK(cudaMemcpy(v.data(), S_ + pb, n * sizeof(float4), cudaMemcpyDeviceToHost), "debug copy");
             float* out = (float*)host;
-            for (uint32_t i = 0; i < n; ++i)
-                out[i] = field == F_DENSITY ? v[i].x : field == F_PRESSURE ? v[i].y : v[i].z;
+            ENG_CK(cudaMemcpy(out, rho_ + pb, n * sizeof(float), cudaMemcpyDeviceToHost), "debug copy");
+            if (field == F_DENSITY) return ENG_OK;
+            // pressure and squared sound speed from the record's (rho/rho0)^gamma;
+            // both are zero outside the grid (rho 0) and where the summed
+            // density is zero (-0 in the record)
+            std::vector<float4> v((size_t)n * 2);
+            ENG_CK(cudaMemcpy(v.data(), R_ + 2 * (size_t)pb, (size_t)n * 2 * sizeof(float4), cudaMemcpyDeviceToHost),
+                   "debug copy");
+            const DevParams& d = s->dp;
+            for (uint32_t i = 0; i < n; ++i) {
+                const float e = v[2 * (size_t)i + 1].w;
+                const bool none = out[i] == 0.0f || (e == 0.0f && std::signbit(e));
+                if (field == F_PRESSURE) out[i] = none ? 0.0f : d.eos_k * (e - 1.0f);
+                else out[i] = none ? 0.0f : d.gas_constant * std::pow(std::fabs(e), (d.gamma - 1.0f) / d.gamma);
+            }
             return ENG_OK;
         }
         case F_FPRESSURE:

@@ -222,10 +222,11 @@ private:
     uint64_t pcap_ = 0, ccap_ = 0, slots_end_ = 0;
     // device arenas
     float4 *P0_ = nullptr, *P1_ = nullptr, *V0_ = nullptr, *V1_ = nullptr, *V2_ = nullptr, *A0_ = nullptr,
-           *A1_ = nullptr, *S_ = nullptr, *N_ = nullptr, *Vc_ = nullptr;
+           *A1_ = nullptr, *N_ = nullptr, *R_ = nullptr;   // R_: two per slot
+    float* rho_ = nullptr;
     uint32_t *okey_ = nullptr;         // packed cells of the last substep (state order)
     uint32_t *pend_ = nullptr;                      // per scene-table entry: XSPH update pending
-    uint32_t *key_ = nullptr, *slot_ = nullptr, *tmp_ = nullptr, *perm_ = nullptr;
+    uint32_t *key_ = nullptr, *slot_ = nullptr, *perm_ = nullptr;
     uint32_t *count_ = nullptr, *start_ = nullptr, *scan_sums_ = nullptr, *status_ = nullptr;
     uint32_t *gate_ = nullptr;        // status word of the passes an export ran ahead (status_ + 1)
     uint32_t *mask_ = nullptr;        // SPH_MASK_ROWS neighbour-mask words per slot

@@ -14,8 +14,10 @@
 //             scene whose XSPH update is pending (pend[scene] != 0)
 //   P1,V1,A1  state gathered into cell order (with a pending update, V1.w
 //             holds the gathered okey bits)
-//   S         (rho, p, c^2, 1/rho^2) per sorted slot
-//   Vc        cell-ordered velocities with the pending XSPH update applied
+//   rho       density per sorted slot
+//   R         neighbour record per sorted slot, 32 bytes, written by the
+//             density pass: (x, y, z, 1/rho) and (velocity with the pending
+//             XSPH update applied, (rho/rho0)^gamma); see density_record
 //   N         surface normals (only when a scene has surface tension)
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -423,18 +425,21 @@ __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevScene* __rest
 // lists were those of the previous sort); every such pair is within h now, so
 // phase 2 meets all of them, and the previous-cell test keeps exactly the
 // reference's pairs.  The poly6 weight is the one the density sum uses.  The
-// corrected velocity goes to Vc, which the force pass reads; without a
-// pending update Vc = V1.
+// corrected velocity goes to the record R, which the force pass reads; without
+// a pending update it is V1's.
+//
+// The record.  All that a later pass needs of a neighbour sits in 32 bytes,
+// one sector, fetched by one 256-bit load: position, velocity, q = 1/rho and
+// e = (rho/rho0)^gamma.  Pressure, squared sound speed and 1/rho^2 follow as
+// eos_k (e - 1), cs_k e q and q^2 (a few multiplications per pair against a
+// third and half of a second gather).  e is stored instead of the pressure
+// because the sound speed of a thin spray ((rho/rho0)^7 near 0) would cancel
+// in p + eos_k.
+// Measured against separate gathers of position, (rho, p, c^2, 1/rho^2) and
+// velocity (48 bytes in three requests): force pass 230 -> 196 us on the 1M
+// dam break, 2.19 -> 1.86 ms on the 8M tension scene, whose normal pass (one
+// 16-byte gather instead of two) went from 1.16 to 1.09 ms.
 // ---------------------------------------------------------------------------
-// Two consecutive cell-ordered positions in one 256-bit load: the slot must
-// be even (32-byte aligned from the 256-byte aligned arena).  The positions
-// are not written during the pass that reads them.
-__device__ __forceinline__ void ld_pos_pair(const float4* p, float4& a, float4& b) {
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-        : "l"(p));
-}
-
 #ifndef DENSITY_MINB
 #define DENSITY_MINB 4
 #endif
@@ -450,10 +455,10 @@ k_density(const DevParams* __restrict__ params,
                                                       const DevScene* __restrict__ scenes,
                                                       const uint4* __restrict__ tiles,
                                                       const uint32_t* __restrict__ start,
-                                                      const float4* __restrict__ P1, float4* __restrict__ S,
+                                                      const float4* __restrict__ P1, float* __restrict__ rho_out,
                                                       uint32_t* __restrict__ mask, size_t mask_stride,
                                                       const float4* __restrict__ V1,
-                                                      const uint32_t* __restrict__ pend, float4* __restrict__ Vc,
+                                                      const uint32_t* __restrict__ pend, float4* __restrict__ R,
                                                       uint32_t* __restrict__ nbr_out, uint32_t ntiles,
                                                       uint32_t* __restrict__ tile_ctr,
                                                       const uint32_t* __restrict__ status) {
@@ -480,8 +485,8 @@ k_density(const DevParams* __restrict__ params,
     const bool work = act && grid_inside(pp, g);
     if (act && !work) {
         if (part == 0u) {
-            S[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            Vc[k] = make_float4(vi.x, vi.y, vi.z, 0.f);
+            rho_out[k] = 0.f;
+            st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, 0.f), make_float4(vi.x, vi.y, vi.z, 0.f));
             if (nbr_out) nbr_out[k] = 0;
         }
         if (!SPLIT) return;
@@ -571,15 +576,15 @@ k_density(const DevParams* __restrict__ params,
                 }
                 for (; jj + 4u <= ce; jj += 4u) {
                     float4 q0, q1, q2, q3;
-                    ld_pos_pair(P1 + jj, q0, q1);
-                    ld_pos_pair(P1 + jj + 2u, q2, q3);
+                    ld_float4_pair(P1 + jj, q0, q1);
+                    ld_float4_pair(P1 + jj + 2u, q2, q3);
                     visit2(q0, q1, bit, dm, sm);
                     visit2(q2, q3, bit << 2, dm, sm);
                     bit <<= 4;
                 }
                 if (jj + 2u <= ce) {
                     float4 q0, q1;
-                    ld_pos_pair(P1 + jj, q0, q1);
+                    ld_float4_pair(P1 + jj, q0, q1);
                     visit2(q0, q1, bit, dm, sm);
                     bit <<= 2;
                     jj += 2u;
@@ -689,12 +694,17 @@ k_density(const DevParams* __restrict__ params,
     if (d < pp.h) corr = fmaf(pp.rest_density, 1.0f - boundary_density(pp, d), corr);
     const float rho = (sum == 0.0f) ? pp.rest_density : corr;
     const float ratio = corr * pp.inv_rest_density;
-    const float prs = (corr == 0.0f) ? 0.0f : pp.eos_k * (powf(ratio, pp.gamma) - 1.0f);
-    const float cs = pp.gas_constant * powf(ratio, pp.gamma - 1.0f);
-    // w = 1/rho^2, used by the force pass for p_j/rho_i^2 + p_i/rho_j^2
-    S[k] = make_float4(rho, prs, cs, 1.0f / (rho * rho));
-    Vc[k] = xs ? make_float4(fmaf(pp.xsph, axy.x, vi.x), fmaf(pp.xsph, axy.y, vi.y), fmaf(pp.xsph, az, vi.z), 0.f)
-               : make_float4(vi.x, vi.y, vi.z, 0.f);
+    // no density at all (corr 0) has pressure 0: marked by -0
+    const float e = (corr == 0.0f) ? -0.0f : powf(ratio, pp.gamma) + 0.0f;
+    rho_out[k] = rho;
+    if (xs) {
+        vi.x = fmaf(pp.xsph, axy.x, vi.x);
+        vi.y = fmaf(pp.xsph, axy.y, vi.y);
+        vi.z = fmaf(pp.xsph, az, vi.z);
+    }
+    // a density the later passes skip as a neighbour's (rho <= eps) is marked by 0
+    st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, rho > eps ? 1.0f / rho : 0.0f),
+                   make_float4(vi.x, vi.y, vi.z, e));
     if (nbr_out) nbr_out[k] = cnt;
   });
 }
@@ -710,8 +720,7 @@ __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restric
                                                       const DevScene* __restrict__ scenes,
                                                       const uint4* __restrict__ tiles,
                                                       const uint32_t* __restrict__ start,
-                                                      const float4* __restrict__ P1,
-                                                      const float4* __restrict__ S,
+                                                      const float4* __restrict__ R,
                                                       const uint32_t* __restrict__ mask, size_t mask_stride,
                                                       float4* __restrict__ N, uint32_t ntiles,
                                                       uint32_t* __restrict__ tile_ctr,
@@ -723,7 +732,7 @@ __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restric
     if (threadIdx.x >= t.z) return;
     const uint32_t k = t.y + threadIdx.x;
     const DevScene sc = scenes[t.x];
-    const float4 p = P1[k];
+    const float4 p = R[2 * (size_t)k];
     const int3 g = grid_of(pp, p.x, p.y, p.z);
     if (!grid_inside(pp, g)) {
         N[k] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -742,15 +751,14 @@ __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restric
     auto run = [&](auto& walk) {
         uint32_t j;
         while (walk.next(j)) {
-            const float4 q = __ldg(P1 + j);
-            const float rhoj = __ldg(&S[j].x);
+            const float4 q = __ldg(R + 2 * (size_t)j);   // w = 1/rho_j, 0 where rho_j <= eps
             const float2 rxy = __fadd2_rn(pxy, make_float2(-q.x, -q.y));
             const float rx = rxy.x, ry = rxy.y, rz = p.z - q.z;
             const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-            if (r2 <= h2 && r2 > eps && j != k && rhoj > eps) {
+            if (r2 <= h2 && r2 > eps && j != k && q.w > 0.0f) {
                 const float r = sqrtf(r2);
                 const float x = fmaf(-r, r, h2);
-                const float s = (r >= h) ? 0.0f : __fdividef(mc * (x * x), rhoj);
+                const float s = (r >= h) ? 0.0f : mc * (x * x) * q.w;
                 sxy = __ffma2_rn(make_float2(s, s), rxy, sxy);
                 sz = fmaf(s, rz, sz);
             }
@@ -775,9 +783,9 @@ __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restric
 // ---------------------------------------------------------------------------
 // Forces (computeAllForces, fluidphysics.cu:215-352) fused with the leapfrog
 // integrator and box boundary (LeapfrogIntegratorOperator,
-// fluidintegrator.cu:11-70).  Reads cell-order state (P1, the velocities Vc
-// of the density pass (V1 with any pending XSPH update applied) through the
-// V1 argument, A1, S, N), writes the integrated state to P0 (w = density), V2,
+// fluidintegrator.cu:11-70).  Reads cell-order state (the density pass's
+// records R and densities, A1, N), writes the integrated state to P0 (w =
+// density), V2,
 // A0, each particle's cell to okey, and the next substep's hash of the new
 // positions (key, slot, cell counts), so that substep needs no hash pass.
 // The integrator sums the
@@ -795,10 +803,9 @@ k_force_integrate(const DevParams* __restrict__ params,
                                                               const DevScene* __restrict__ scenes,
                                                               const uint4* __restrict__ tiles,
                                                               const uint32_t* __restrict__ start,
-                                                              const float4* __restrict__ P1,
-                                                              const float4* __restrict__ V1,
+                                                              const float4* __restrict__ R,
+                                                              const float* __restrict__ rho,
                                                               const float4* __restrict__ A1,
-                                                              const float4* __restrict__ S,
                                                               const float4* __restrict__ N,
                                                               const uint32_t* __restrict__ mask, size_t mask_stride,
                                                               float4* __restrict__ P0, float4* __restrict__ V2,
@@ -819,9 +826,9 @@ k_force_integrate(const DevParams* __restrict__ params,
     // the scene's XSPH update is now pending (applied by the next density
     // pass, or by k_xsph right after this pass)
     if (threadIdx.x == 0) pend[t.x] = 1u;
-    const float4 pi = P1[k];
-    const float4 vi = V1[k];
-    const float4 si = S[k];
+    float4 pi, vi;
+    ld_float4_pair(R + 2 * (size_t)k, pi, vi);
+    const float ri = rho[k];
     const int3 g = grid_of(pp, pi.x, pi.y, pi.z);
     const bool tension = TENSION && (pp.flags & 1u) != 0u;
     const bool inside = grid_inside(pp, g);
@@ -830,22 +837,22 @@ k_force_integrate(const DevParams* __restrict__ params,
     float ftx = 0.f, fty = 0.f, ftz = 0.f;   // tension
     float fax = 0.f, fay = 0.f, faz = 0.f;   // adhesion
     const uint32_t delta = sc.part_base - __ldg(start + sc.cell_base);
-    const float ri = si.x, pri = si.y, csi = si.z;
+    const float pri = pp.eos_k * (vi.w - 1.0f), csi = pp.cs_k * (vi.w * pi.w);
     float4 ni = make_float4(0.f, 0.f, 0.f, 0.f);
     if (tension && inside) ni = N[k];
-    const float h2 = pp.h2, eps = pp.eps, inv_ri2 = si.w;
+    const float h2 = pp.h2, eps = pp.eps, inv_ri2 = 1.0f / (ri * ri);
     // 2 rho0 / (rho_i + rho_i) of the tension sum (fluidphysics.cu:293), once per particle
     const float tden = (2.0f * pp.rest_density) / (ri + ri);
     const float sm = -pp.surface_tension * pp.mass;
     const float coh_m = -pp.mass * pp.mass;
     // per-scene constants of the pair loop, held in registers
     const float visc = pp.viscosity, hh = pp.h, visc_eps = pp.visc_eps, mass = pp.mass, gsp = pp.grad_spiky;
-    // One pair: neighbour j with its position, (rho, p, c^2, 1/rho^2),
-    // velocity and normal.
-    auto pair = [&](uint32_t j, const float4& pj, const float4& sj, const float4& vj, const float4& nj) {
+    const float eos_k = pp.eos_k, cs_k = pp.cs_k;
+    // One pair: neighbour j with its record and normal.
+    auto pair = [&](uint32_t j, const float4& pj, const float4& vj, const float4& nj) {
         const float rx = pj.x - pi.x, ry = pj.y - pi.y, rz = pj.z - pi.z;
         const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-        if (r2 <= h2 && r2 > eps && j != k && sj.x > eps) {
+        if (r2 <= h2 && r2 > eps && j != k && pj.w > 0.0f) {
             // r is the correctly rounded root: h - r below cancels, and pairs at
             // r ~ h must see the reference's r; 1/r only scales (approximate)
             const float r = sqrtf(r2);
@@ -854,10 +861,12 @@ k_force_integrate(const DevParams* __restrict__ params,
             // artificial viscosity -visc (cs_i + cs_j) mu / (rho_i + rho_j),
             // mu = h ux / (r^2 + 0.01 h^2), only for approaching pairs;
             // evaluated without a branch (finite for every pair) and selected
-            const float Pv = __fdividef(-visc * (csi + sj.z) * (hh * ux), (r2 + visc_eps) * (ri + sj.x));
+            // (1/(rho_i + rho_j) = q_j / (rho_i q_j + 1))
+            const float cs = fmaf(cs_k, vj.w * pj.w, csi);
+            const float Pv = __fdividef(-visc * cs * (hh * ux) * pj.w, (r2 + visc_eps) * fmaf(ri, pj.w, 1.0f));
             const float Pi = (ux < 0.0f) ? Pv : 0.0f;
             // p_j/rho_i^2 + p_i/rho_j^2 with the reciprocals from the density pass
-            const float mid = sj.y * inv_ri2 + pri * sj.w;
+            const float mid = eos_k * (vj.w - 1.0f) * inv_ri2 + pri * (pj.w * pj.w);
             const float gspk = (r >= hh) ? 0.0f : gsp * (hh - r) * (hh - r);   // grad_spiky
             const float sr = (mass * gspk) * inv_r;
             const float cx = sr * rx, cy = sr * ry, cz = sr * rz;
@@ -881,10 +890,10 @@ k_force_integrate(const DevParams* __restrict__ params,
     // their latencies overlap (the masks hold exact neighbours: nearly every
     // j is used).
     auto gathered = [&](uint32_t j) {
-        const float4 pj = __ldg(P1 + j), sj = __ldg(S + j), vj = __ldg(V1 + j);
-        float4 nj = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 pj, vj, nj = make_float4(0.f, 0.f, 0.f, 0.f);
+        ld_float4_pair(R + 2 * (size_t)j, pj, vj);
         if (tension) nj = __ldg(N + j);
-        pair(j, pj, sj, vj, nj);
+        pair(j, pj, vj, nj);
     };
     // exact neighbours recorded by the density pass (SPH_MASK_EXACT words)
     if (inside) {
@@ -949,7 +958,7 @@ k_force_integrate(const DevParams* __restrict__ params,
         const float kk = (1.0f + pp.vdamp) * dot3(nb.x, nb.y, nb.z, vx, vy, vz);
         vx = fmaf(-kk, nb.x, vx); vy = fmaf(-kk, nb.y, vy); vz = fmaf(-kk, nb.z, vz);
     }
-    P0[k] = make_float4(px, py, pz, si.x);
+    P0[k] = make_float4(px, py, pz, ri);
     V2[k] = make_float4(vx, vy, vz, 0.f);
     A0[k] = make_float4(anx, any, anz, 0.f);
     // The next substep's hash (k_hash's work, on the position just written):
@@ -1070,14 +1079,14 @@ __global__ void k_xsph(const DevParams* __restrict__ params,
 }
 
 // ---------------------------------------------------------------------------
-// The velocities of a density pass (Vc, cell order) back in the state order
+// The velocities of a density pass (in R, cell order) back in the state order
 // of the substep before it (slot perm[f]): the export of a scene whose XSPH
 // update was pending (packed xyz into `out`, particle perm[f] - base), and its
 // materialisation into the state (V0, clearing the scene's pending flag).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(SPH_TILE) k_unsort_vel(const uint4* __restrict__ tiles,
                                                          const uint32_t* __restrict__ perm,
-                                                         const float4* __restrict__ Vc, uint32_t base,
+                                                         const float4* __restrict__ R, uint32_t base,
                                                          float* __restrict__ out, float4* __restrict__ V0,
                                                          uint32_t* __restrict__ pend,
                                                          const uint32_t* __restrict__ status,
@@ -1093,7 +1102,8 @@ __global__ void __launch_bounds__(SPH_TILE) k_unsort_vel(const uint4* __restrict
     const uint32_t f = t.y + threadIdx.x;
     const uint32_t i = __ldg(perm + f);
     if (i - base >= n) return;   // every slot of the scene, once, after a complete prefix
-    const float4 v = Vc[f];
+    const float4 r = R[2 * (size_t)f + 1];
+    const float4 v = make_float4(r.x, r.y, r.z, 0.f);
     if (out) {
         const size_t o = 3 * (size_t)(i - base);
         out[o] = v.x;
@@ -1133,14 +1143,14 @@ __global__ void __launch_bounds__(SPH_TILE) k_undo_ahead(const uint4* __restrict
 // ---------------------------------------------------------------------------
 __global__ void k_unpack_state(const float* __restrict__ pos, const float* __restrict__ vel, uint32_t n,
                                uint32_t base, float4* __restrict__ P0, float4* __restrict__ V0,
-                               float4* __restrict__ A0, float4* __restrict__ S) {
+                               float4* __restrict__ A0, float* __restrict__ rho) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t s = base + i;
     P0[s] = make_float4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], 0.f);
     V0[s] = vel ? make_float4(vel[3 * i], vel[3 * i + 1], vel[3 * i + 2], 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
     A0[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-    S[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+    rho[s] = 0.f;
 }
 
 // Overwrite positions of slots [base, base+n) keeping the rest of the state
@@ -1175,7 +1185,7 @@ __global__ void k_pack_state(const float4* __restrict__ P0, const float4* __rest
 // Lattice block with seeded jitter; site (ix,iy,iz) -> particle
 // (ix*ny + iy)*nz + iz.  Coordinate: lo + (i + 0.5)*spacing + (2u-1)*jitter.
 __global__ void k_lattice(LatticeSpec spec, uint32_t base, float4* __restrict__ P0, float4* __restrict__ V0,
-                          float4* __restrict__ A0, float4* __restrict__ S) {
+                          float4* __restrict__ A0, float* __restrict__ rho) {
     const uint32_t n = spec.nx * spec.ny * spec.nz;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -1192,7 +1202,7 @@ __global__ void k_lattice(LatticeSpec spec, uint32_t base, float4* __restrict__ 
     P0[s] = make_float4(c[0], c[1], c[2], 0.f);
     V0[s] = make_float4(spec.vel[0], spec.vel[1], spec.vel[2], 0.f);
     A0[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-    S[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+    rho[s] = 0.f;
 }
 
 // Sorted hash for the debug tap: key of the particle now at each slot, with
@@ -1312,21 +1322,21 @@ cudaError_t launch_density(const StepArgs& a, cudaStream_t st) {
     const size_t smem = (size_t)SPH_ROW_TABLE_WORDS * a.block * sizeof(uint32_t);   // the row table
     if (density_split(a)) {
         k_density<1, false, true><<<a.ntiles, 3u * a.block, smem, st>>>(
-            a.params, a.scenes, a.tiles, a.start, a.P1, a.S, a.mask, a.mask_stride, a.V1, a.pend, a.Vc, a.dbg_nbr,
+            a.params, a.scenes, a.tiles, a.start, a.P1, a.rho, a.mask, a.mask_stride, a.V1, a.pend, a.R, a.dbg_nbr,
             a.ntiles, nullptr, a.status);
         return cudaGetLastError();
     }
     const bool rows = (a.variant & SPH_VARIANT_DENSITY_ROWS) != 0u;
     auto kern = a.skin_masks ? (rows ? k_density<1, true> : k_density<0, true>)
                              : (rows ? k_density<1, false> : k_density<0, false>);
-    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.P1, a.S, a.mask, a.mask_stride,
-                                            a.V1, a.pend, a.Vc, a.dbg_nbr, a.ntiles, ctr(a, 0), a.status);
+    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.P1, a.rho, a.mask, a.mask_stride,
+                                            a.V1, a.pend, a.R, a.dbg_nbr, a.ntiles, ctr(a, 0), a.status);
     return cudaGetLastError();
 }
 cudaError_t launch_unsort_vel(const StepArgs& a, uint32_t first_tile, uint32_t ntiles, uint32_t base, uint32_t n,
                               float* out, float4* V0, bool clear_pending, cudaStream_t st, uint32_t* gate) {
     if (ntiles == 0) return cudaSuccess;
-    k_unsort_vel<<<ntiles, a.block, 0, st>>>(a.tiles + first_tile, a.perm, a.Vc, base, out, V0,
+    k_unsort_vel<<<ntiles, a.block, 0, st>>>(a.tiles + first_tile, a.perm, a.R, base, out, V0,
                                              clear_pending ? a.pend : nullptr, a.status, gate, n);
     return cudaGetLastError();
 }
@@ -1340,7 +1350,7 @@ cudaError_t launch_normals(const StepArgs& a, cudaStream_t st) {
     const bool table = (a.variant & SPH_VARIANT_NORMALS_TABLE) != 0u;
     auto kern = table ? k_normals<true> : k_normals<false>;
     const size_t smem = table ? (size_t)SPH_ROW_TABLE_WORDS * a.block * sizeof(uint32_t) : 0;
-    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.P1, a.S, a.mask, a.mask_stride,
+    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.mask, a.mask_stride,
                                             a.N, a.ntiles, ctr(a, 1), a.status);
     return cudaGetLastError();
 }
@@ -1353,7 +1363,7 @@ cudaError_t launch_force(const StepArgs& a, cudaStream_t st) {
                     : (table ? (occ ? k_force_integrate<false, 4, true> : k_force_integrate<false, 3, true>)
                              : (occ ? k_force_integrate<false, 4, false> : k_force_integrate<false, 3, false>));
     const size_t smem = table ? (size_t)SPH_ROW_TABLE_WORDS * a.block * sizeof(uint32_t) : 0;
-    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.P1, a.Vc, a.A1, a.S, a.N, a.mask,
+    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.rho, a.A1, a.N, a.mask,
                                             a.mask_stride, a.P0, a.V2, a.A0, a.skin_masks ? a.maxdisp : nullptr,
                                             a.okey, a.pend, a.count, a.key, a.slot, a.status, a.dbg_forces,
                                             a.ntiles, ctr(a, 2));
@@ -1366,9 +1376,9 @@ cudaError_t launch_xsph(const StepArgs& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 cudaError_t launch_unpack(const float* pos, const float* vel, uint32_t n, uint32_t base, float4* P0, float4* V0,
-                          float4* A0, float4* S, cudaStream_t st) {
+                          float4* A0, float* rho, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    k_unpack_state<<<(n + 255) / 256, 256, 0, st>>>(pos, vel, n, base, P0, V0, A0, S);
+    k_unpack_state<<<(n + 255) / 256, 256, 0, st>>>(pos, vel, n, base, P0, V0, A0, rho);
     return cudaGetLastError();
 }
 cudaError_t launch_set_positions(const float* pos, uint32_t n, uint32_t base, float4* P0, cudaStream_t st) {
@@ -1382,11 +1392,11 @@ cudaError_t launch_pack(const float4* P0, const float4* V0, uint32_t n, uint32_t
     k_pack_state<<<(n + 255) / 256, 256, 0, st>>>(P0, V0, n, base, inv_rest_density, pos, colour, vel);
     return cudaGetLastError();
 }
-cudaError_t launch_lattice(const LatticeSpec& spec, uint32_t base, float4* P0, float4* V0, float4* A0, float4* S,
+cudaError_t launch_lattice(const LatticeSpec& spec, uint32_t base, float4* P0, float4* V0, float4* A0, float* rho,
                            cudaStream_t st) {
     const uint32_t n = spec.nx * spec.ny * spec.nz;
     if (n == 0) return cudaSuccess;
-    k_lattice<<<(n + 255) / 256, 256, 0, st>>>(spec, base, P0, V0, A0, S);
+    k_lattice<<<(n + 255) / 256, 256, 0, st>>>(spec, base, P0, V0, A0, rho);
     return cudaGetLastError();
 }
 cudaError_t launch_sorted_keys(const DevParams* params, const float4* P1, uint32_t n, uint32_t base,

@@ -17,10 +17,11 @@ struct StepArgs {
     float4 *P0, *V0, *A0;      // state
     float4 *P1, *V1, *A1;      // cell-ordered state
     float4 *V2;                // post-integration velocity (before XSPH)
-    float4 *Vc;                // cell-ordered velocities with any pending XSPH update applied
+    float4 *R;                 // neighbour records, two per slot: (x, y, z, 1/rho), (velocity with any pending
+                               // XSPH update applied, (rho/rho0)^gamma)
     uint32_t *okey;            // each slot's cell in the last substep (packed; gathered into V1.w)
     uint32_t *pend;            // per scene: its last XSPH update is pending
-    float4 *S;                 // (rho, p, c^2, 0)
+    float *rho;                // density per sorted slot
     float4 *N;                 // normals
     uint32_t *count, *start, *scan_sums;
     uint32_t scan_first;           // the scan covers cells [scan_first, scan_first + scan_cells) (one scene's
@@ -28,7 +29,8 @@ struct StepArgs {
     uint32_t scan_zeroes_counts;   // nonzero: the scan leaves every count it read at zero for the next hash
     uint32_t scan_spin_limit;      // polls of one look-back wait before it gives up (SPH_STATUS_SCAN_TIMEOUT)
     uint32_t scan_withhold;        // test control: tile 0 is never handed out, so waits on it run out
-    uint32_t *key, *slot, *tmp, *perm;
+    uint32_t *key, *slot, *perm;
+    uint32_t *tmp;             // scatter list of the sort; shares the mask words, which the density pass writes later
     uint32_t *status;
     uint32_t *mask;            // SPH_MASK_ROWS neighbour-mask words per slot, word m at mask[m*mask_stride + slot]:
                                // SPH_MASK_SKIN skin radius (XSPH), SPH_MASK_EXACT exact neighbours (normals, forces)
@@ -76,7 +78,7 @@ bool density_split(const StepArgs& a);
 cudaError_t launch_normals(const StepArgs& a, cudaStream_t st);
 cudaError_t launch_force(const StepArgs& a, cudaStream_t st);
 cudaError_t launch_xsph(const StepArgs& a, cudaStream_t st);
-// Vc (cell order, over tiles [first_tile, first_tile + ntiles) of one scene
+// The velocities of R (cell order, over tiles [first_tile, first_tile + ntiles) of one scene
 // of n particles) back into state order: packed xyz into `out` (particle
 // slot - base) and/or into V0; optionally clears the scene's pending flag.
 // Does nothing after a failed prefix.  With `gate`, also
@@ -89,11 +91,11 @@ cudaError_t launch_unsort_vel(const StepArgs& a, uint32_t first_tile, uint32_t n
 cudaError_t launch_undo_ahead(const StepArgs& a, uint32_t first_tile, uint32_t ntiles, cudaStream_t st);
 
 cudaError_t launch_unpack(const float* pos, const float* vel, uint32_t n, uint32_t base, float4* P0, float4* V0,
-                          float4* A0, float4* S, cudaStream_t st);
+                          float4* A0, float* rho, cudaStream_t st);
 cudaError_t launch_set_positions(const float* pos, uint32_t n, uint32_t base, float4* P0, cudaStream_t st);
 cudaError_t launch_pack(const float4* P0, const float4* V0, uint32_t n, uint32_t base, float inv_rest_density,
                         float* pos, float* colour, float* vel, cudaStream_t st);
-cudaError_t launch_lattice(const LatticeSpec& spec, uint32_t base, float4* P0, float4* V0, float4* A0, float4* S,
+cudaError_t launch_lattice(const LatticeSpec& spec, uint32_t base, float4* P0, float4* V0, float4* A0, float* rho,
                            cudaStream_t st);
 cudaError_t launch_sorted_keys(const DevParams* params, const float4* P1, uint32_t n, uint32_t base,
                                uint32_t* out, cudaStream_t st);
