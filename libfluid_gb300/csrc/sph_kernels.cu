@@ -19,7 +19,9 @@
 //             density pass: (x, y, z, 1/rho) and (velocity with the pending
 //             XSPH update applied, (rho/rho0)^gamma); see density_record
 //   N         surface normals (only when a scene has surface tension)
+#include <cfloat>
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 #include "sph_types.h"
 #include "sph_device.cuh"
@@ -794,9 +796,9 @@ __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restric
 // ---------------------------------------------------------------------------
 // TENSION = false is the build for launches where no scene has surface
 // tension (the tension terms are then compiled out).  MINB is the register
-// budget as resident blocks of 256 threads per SM: 3 (85 registers; the
-// tension-free build needs 72, the tension build 80, no spills) or 4 (64
-// registers, more warps per SM, a few spilled values).
+// budget as resident blocks of 256 threads per SM: 3 (80 registers, no
+// spills) or 4 (64 registers, more warps per SM, a few spilled values in the
+// tension build).
 template <bool TENSION, int MINB, bool TABLE>
 __global__ void __launch_bounds__(SPH_TILE, MINB)
 k_force_integrate(const DevParams* __restrict__ params,
@@ -833,56 +835,56 @@ k_force_integrate(const DevParams* __restrict__ params,
     const bool tension = TENSION && (pp.flags & 1u) != 0u;
     const bool inside = grid_inside(pp, g);
     float fpx = 0.f, fpy = 0.f, fpz = 0.f;   // pressure
-    float fvx = 0.f, fvy = 0.f, fvz = 0.f;   // "viscosity" (pressure re-added)
+    float fvx = 0.f, fvy = 0.f, fvz = 0.f;   // viscosity (the pressure is added after the sums)
     float ftx = 0.f, fty = 0.f, ftz = 0.f;   // tension
     float fax = 0.f, fay = 0.f, faz = 0.f;   // adhesion
     const uint32_t delta = sc.part_base - __ldg(start + sc.cell_base);
-    const float pri = pp.eos_k * (vi.w - 1.0f), csi = pp.cs_k * (vi.w * pi.w);
     float4 ni = make_float4(0.f, 0.f, 0.f, 0.f);
     if (tension && inside) ni = N[k];
-    const float h2 = pp.h2, eps = pp.eps, inv_ri2 = 1.0f / (ri * ri);
-    // 2 rho0 / (rho_i + rho_i) of the tension sum (fluidphysics.cu:293), once per particle
-    const float tden = (2.0f * pp.rest_density) / (ri + ri);
-    const float sm = -pp.surface_tension * pp.mass;
-    const float coh_m = -pp.mass * pp.mass;
-    // per-scene constants of the pair loop, held in registers
-    const float visc = pp.viscosity, hh = pp.h, visc_eps = pp.visc_eps, mass = pp.mass, gsp = pp.grad_spiky;
-    const float eos_k = pp.eos_k, cs_k = pp.cs_k;
-    // One pair: neighbour j with its record and normal.
-    auto pair = [&](uint32_t j, const float4& pj, const float4& vj, const float4& nj) {
+    const float h2 = pp.h2, hh = pp.h, visc_eps = pp.visc_eps;
+    const float inv_ri2 = 1.0f / (ri * ri), eos_k = pp.eos_k, pri = eos_k * (vi.w - 1.0f), eqi = vi.w * pi.w;
+    // r > rsel selects the cohesion branch (never, were the coefficient 0)
+    const float coh = pp.mass / pp.surface_tension, rsel = pp.cohesion != 0.0f ? pp.halfh : INFINITY;
+    const float coh_near = pp.h6 * 0.0156f;
+    // One pair: neighbour j with its record and normal.  Every factor that is
+    // the same for all pairs is left to the end of the sums (it would cost an
+    // instruction per pair and a register), and each scalar is formed once:
+    // with s = (h - r)^2 / r (the spiky gradient over r without its
+    // coefficient), the pressure sum takes s mid rvec and the viscosity sum,
+    // which has the pressure in it again, only s Pi rvec (the pressure sum is
+    // added at the end).  j == k has r^2 = 0 and drops out with the coincident
+    // pairs.  Against one division, rounded root and pair of weighted vectors
+    // per term this took 18 of 145 M warp instructions from the pass: 196 -> 189
+    // us on the 1M dam break, 1.86 -> 1.69 ms on the 8M tension scene.
+    auto pair = [&](const float4& pj, const float4& vj, const float4& nj) {
         const float rx = pj.x - pi.x, ry = pj.y - pi.y, rz = pj.z - pi.z;
         const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-        if (r2 <= h2 && r2 > eps && j != k && pj.w > 0.0f) {
-            // r is the correctly rounded root: h - r below cancels, and pairs at
-            // r ~ h must see the reference's r; 1/r only scales (approximate)
-            const float r = sqrtf(r2);
-            const float inv_r = rsqrtf(r2);
-            const float ux = dot3(vi.x - vj.x, vi.y - vj.y, vi.z - vj.z, -rx, -ry, -rz);
+        if (r2 <= h2 && r2 > FLT_MIN && pj.w > 0.0f) {
+            const float inv_r = rsqrt_approx(r2), r = r2 * inv_r;
+            const float hr = h_minus_r(r2, r, hh, h2);
             // artificial viscosity -visc (cs_i + cs_j) mu / (rho_i + rho_j),
-            // mu = h ux / (r^2 + 0.01 h^2), only for approaching pairs;
-            // evaluated without a branch (finite for every pair) and selected
-            // (1/(rho_i + rho_j) = q_j / (rho_i q_j + 1))
-            const float cs = fmaf(cs_k, vj.w * pj.w, csi);
-            const float Pv = __fdividef(-visc * cs * (hh * ux) * pj.w, (r2 + visc_eps) * fmaf(ri, pj.w, 1.0f));
-            const float Pi = (ux < 0.0f) ? Pv : 0.0f;
-            // p_j/rho_i^2 + p_i/rho_j^2 with the reciprocals from the density pass
-            const float mid = eos_k * (vj.w - 1.0f) * inv_ri2 + pri * (pj.w * pj.w);
-            const float gspk = (r >= hh) ? 0.0f : gsp * (hh - r) * (hh - r);   // grad_spiky
-            const float sr = (mass * gspk) * inv_r;
-            const float cx = sr * rx, cy = sr * ry, cz = sr * rz;
-            fpx = fmaf(cx, mid, fpx); fpy = fmaf(cy, mid, fpy); fpz = fmaf(cz, mid, fpz);
-            const float mp = mid + Pi;
-            fvx = fmaf(cx, mp, fvx); fvy = fmaf(cy, mp, fvy); fvz = fmaf(cz, mp, fvz);
+            // mu = h ux / (r^2 + 0.01 h^2), only for approaching pairs (ux < 0),
+            // over -visc h cs_k; 1/(rho_i + rho_j) = q_j / (rho_i q_j + 1)
+            const float ux = dot3(vj.x - vi.x, vj.y - vi.y, vj.z - vi.z, rx, ry, rz);
+            const float den = pj.w * rcp_approx((r2 + visc_eps) * fmaf(ri, pj.w, 1.0f));
+            const float Pi = fminf(ux, 0.0f) * fmaf(vj.w, pj.w, eqi) * den;
+            // p_j/rho_i^2 + p_i/rho_j^2, p_j formed first: where rho is next to
+            // nothing, the terms overflow exactly where the reference's do
+            const float mid = fmaf(pri, pj.w * pj.w, eos_k * (vj.w - 1.0f) * inv_ri2);
+            const float hr2 = hr * hr;
+            const float sr = hr2 * inv_r;
+            const float sp = sr * mid, sv = sr * Pi;
+            fpx = fmaf(sp, rx, fpx); fpy = fmaf(sp, ry, fpy); fpz = fmaf(sp, rz, fpz);
+            fvx = fmaf(sv, rx, fvx); fvy = fmaf(sv, ry, fvy); fvz = fmaf(sv, rz, fvz);
             if (tension) {
-                // Akinci cohesion + curvature (fluidphysics.cu:291-293).  With
-                // sigma == 0 the tension force is sigma * (finite sum) = 0, so
-                // the term is skipped.
-                const float sc2 = coh_m * cohesion_k(pp, r) * inv_r;
-                const float hx = sc2 * rx, hy = sc2 * ry, hz = sc2 * rz;
-                const float kx = sm * (ni.x - nj.x), ky = sm * (ni.y - nj.y), kz = sm * (ni.z - nj.z);
-                ftx = fmaf(tden, hx + kx, ftx);
-                fty = fmaf(tden, hy + ky, fty);
-                ftz = fmaf(tden, hz + kz, ftz);
+                // Akinci cohesion + curvature (fluidphysics.cu:291-293), cohesion
+                // times 1/r, both over -sigma m.  With sigma == 0 the tension
+                // force is sigma * (finite sum) = 0, so the term is skipped.
+                const float t = hr2 * hr * r2;
+                const float c = coh * ((r > rsel) ? t : fmaf(2.0f, t, -(coh_near * inv_r)));
+                ftx = fmaf(c, rx, ftx) + (ni.x - nj.x);
+                fty = fmaf(c, ry, fty) + (ni.y - nj.y);
+                ftz = fmaf(c, rz, ftz) + (ni.z - nj.z);
             }
         }
     };
@@ -893,7 +895,7 @@ k_force_integrate(const DevParams* __restrict__ params,
         float4 pj, vj, nj = make_float4(0.f, 0.f, 0.f, 0.f);
         ld_float4_pair(R + 2 * (size_t)j, pj, vj);
         if (tension) nj = __ldg(N + j);
-        pair(j, pj, vj, nj);
+        pair(pj, vj, nj);
     };
     // exact neighbours recorded by the density pass (SPH_MASK_EXACT words)
     if (inside) {
@@ -912,8 +914,18 @@ k_force_integrate(const DevParams* __restrict__ params,
         }
     }
     if (inside) {
-        fvx = pp.viscosity * fvx; fvy = pp.viscosity * fvy; fvz = pp.viscosity * fvz;
-        ftx = pp.surface_tension * ftx; fty = pp.surface_tension * fty; ftz = pp.surface_tension * ftz;
+        // the factors left out of the sums
+        const float sp = pp.mass * pp.grad_spiky, sv = -pp.viscosity * hh * pp.cs_k * sp;
+        fpx = sp * fpx; fpy = sp * fpy; fpz = sp * fpz;
+        fvx = pp.viscosity * fmaf(sv, fvx, fpx);
+        fvy = pp.viscosity * fmaf(sv, fvy, fpy);
+        fvz = pp.viscosity * fmaf(sv, fvz, fpz);
+        if (tension) {
+            // sigma, -sigma m, and 2 rho0 / (rho_i + rho_i) of the tension sum (fluidphysics.cu:293)
+            const float st = pp.surface_tension * ((2.0f * pp.rest_density) / (ri + ri)) *
+                             (-pp.surface_tension * pp.mass);
+            ftx = st * ftx; fty = st * fty; ftz = st * ftz;
+        }
         const float z = -fminf(sdf(pp, pi.x, pi.y, pi.z), 0.0f) * 0.25f * pp.inv_particle_size;
         if (z < 1.0f) {
             const float3 nb = sdf_normal(pp, pi.x, pi.y, pi.z);
