@@ -397,26 +397,21 @@ __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevScene* __rest
 // ---------------------------------------------------------------------------
 // Density + Tait EOS (computeDensity, fluidphysics.cu:8-84), in two phases.
 //
-// Phase 1 scans the candidates of the 27 cells, 32 at a time, with the
-// distance test alone and records a bit per candidate within h (density
-// pairs, j != i) and, with SKIN, within the skin radius.  The words go to the
-// neighbour masks of the later passes (SPH_MASK_SKIN rows for rows of up to
-// 32 candidates; SPH_MASK_EXACT rows, two words per row of up to 64) and to a
-// row table in shared memory (build_row_table's layout).  Coincident pairs
-// (r^2 <= eps) stay in the words: the density sum and XSPH take them, and the
-// normal and force passes drop them with their own r^2 > eps test.  Phase 2
-// walks that table and does the kernel arithmetic for the density pairs only
-// (about one candidate in six), so a warp no longer runs the neighbour path
-// on every candidate that any of its lanes accepts.  Rows longer than 64
-// candidates are not scanned in phase 1; phase 2 walks them in full with the
-// test.  Both phases visit candidates in the same order (rows z outer, then
-// y, then slots, the row's cells x ascending), so the sum follows phase 1's
-// candidate order; the reference's loop runs the cells x outer and z inner
-// (fluidphysics.cu:29-33), the same terms in another order.  WALK selects
-// phase 1's loop: flattened across the
-// rows (0) or one loop per row with four candidates in flight, two per
-// 256-bit load (1); the words are
-// the same.
+// Phase 1 scans the candidates of the 27 cells with the distance test alone,
+// 32 at a time, and appends those within h (j != i) to the particle's
+// neighbour list in shared memory (NbrList).  Phase 2 walks that list, does
+// the kernel arithmetic for the pairs (about one candidate in six), so a warp
+// does not run it on every candidate that any of its lanes accepts, and
+// stores the list for the normal and force passes.  Coincident pairs
+// (r^2 <= eps) stay in the list: the density sum and XSPH take them, the other
+// passes drop them with their own r^2 > eps test.  Neighbours past the list's
+// end are found again by testing the remaining candidates (walk_tail).  Both
+// forms visit neighbours in the same order (rows z outer, then y, then slots,
+// the row's cells x ascending); the reference's loop runs the cells x outer
+// and z inner (fluidphysics.cu:29-33), the same terms in another order.
+//
+// With SKIN, phase 1 also records the candidates within the skin radius, one
+// word per row of up to 32 candidates (SPH_MASK_SKIN).
 //
 // Deferred XSPH.  For a scene whose previous substep ended without its XSPH
 // update (pend[scene] != 0), P1 holds that substep's post-integration
@@ -445,13 +440,18 @@ __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevScene* __rest
 #ifndef DENSITY_MINB
 #define DENSITY_MINB 4
 #endif
-// SPLIT (with WALK == 1, no SKIN, one block per tile): three threads per
-// particle share phase 1, thread q of the particle taking rows 3q..3q+2; its
-// words and row-table entries are per row, so phase 1 writes exactly what
-// one thread would.  After a barrier the first thread runs phase 2 over the
-// whole table.  A small scene's pass lasts as long as one thread's walk, and
-// the split shortens the candidate scan's share of it threefold.
-template <int WALK, bool SKIN, bool SPLIT = false>
+// Neighbour loads in flight per list step: two where the registers hold them
+// (density 239.5 against 246.5 us on the 1M dam break, normals 26.7 against 30.7
+// us at 250k), one in the force pass (two measured the same at 64 registers,
+// where they spill, and 5% slower at 80).
+constexpr int kDensityDepth = 2, kNormalsDepth = 2, kForceDepth = 1;
+// SPLIT (no SKIN, one block per tile): three threads per particle share phase
+// 1, thread q of the particle taking rows 3q..3q+2 and a list of its own;
+// after a barrier the first thread appends the others' lists to its own, which
+// gives the list one thread would have made, and runs phase 2.  A small
+// scene's pass lasts as long as one thread's walk, and the split shortens the
+// candidate scan's share of it threefold.
+template <bool SKIN, bool SPLIT = false>
 __global__ void __launch_bounds__(SPLIT ? 3 * SPH_TILE : SPH_TILE, SPLIT ? 1 : DENSITY_MINB)
 k_density(const DevParams* __restrict__ params,
                                                       const DevScene* __restrict__ scenes,
@@ -464,8 +464,8 @@ k_density(const DevParams* __restrict__ params,
                                                       uint32_t* __restrict__ nbr_out, uint32_t ntiles,
                                                       uint32_t* __restrict__ tile_ctr,
                                                       const uint32_t* __restrict__ status) {
-  static_assert(!SPLIT || (WALK == 1 && !SKIN), "the split scan is the per-row scan without skin words");
-  extern __shared__ uint32_t s_rows[];
+  static_assert(!SPLIT || !SKIN, "the split scan writes no skin words");
+  extern __shared__ uint32_t s_list[];
   if (step_failed(status)) return;
   for_each_tile(tiles, ntiles, tile_ctr, [&](const uint4 t) {
     // particle li of the tile; with SPLIT, part q of its phase 1.  Every
@@ -496,159 +496,148 @@ k_density(const DevParams* __restrict__ params,
     const uint32_t delta = sc.part_base - __ldg(start + sc.cell_base);
     // the skin-radius words serve only the per-substep XSPH pass
     const float h2 = pp.h2, skin2 = SKIN ? pp.skin2 : pp.h2, eps = pp.eps;
-    uint32_t* tab = s_rows + li;
-    uint32_t live = 0u, full = 0u;
-    // rows of this thread's phase 1
-    constexpr int kRows = SPLIT ? 3 : 9;
-    const int r0 = SPLIT ? 3 * (int)part : 0;
+    // row starts in a column per thread, list words in a row per thread; a
+    // split block has one set per thread
+    uint32_t* rows = s_list + threadIdx.x;
+    const uint32_t rs = blockDim.x;
+    uint8_t* list = reinterpret_cast<uint8_t*>(s_list + SPH_NBR_ROWS * rs + threadIdx.x * SPH_NBR_LIST_WORDS);
+    NbrHeader hd;
 
     // ---- phase 1: distance test of every candidate ----
-    auto visit = [&](const float4& q, uint32_t bit, uint32_t& dm, uint32_t& sm) {
+    // A candidate's bit is the sign of h^2 - r^2 (set outside; the sign of a
+    // rounded difference is that of the exact one, so the test is r^2 <= h^2
+    // to the bit), shifted into the word: the first candidate of a chunk ends
+    // in its highest bit.
+    auto visit = [&](const float4& q, uint32_t& dm, uint32_t& sm) {
         const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
         const float rr = dot3(dx, dy, dz, dx, dy, dz);
-        if (rr <= h2) dm |= bit;
-        if (SKIN && rr <= skin2) sm |= bit;
+        dm = __funnelshift_l(__float_as_uint(h2 - rr), dm, 1);
+        if (SKIN) sm = __funnelshift_l(__float_as_uint(skin2 - rr), sm, 1);
     };
     // Two candidates at once with the packed FP32 instructions of sm_100-class
     // GPUs (add/mul/fma.rn.f32x2): each component is rounded exactly as the
     // scalar operation, so r^2 (dot3's fusion order) is the same to the bit.
     const float2 px2 = make_float2(p.x, p.x), py2 = make_float2(p.y, p.y), pz2 = make_float2(p.z, p.z);
-    auto visit2 = [&](const float4& q0, const float4& q1, uint32_t bit, uint32_t& dm, uint32_t& sm) {
+    const float2 h22 = make_float2(h2, h2);
+    auto visit2 = [&](const float4& q0, const float4& q1, uint32_t& dm, uint32_t& sm) {
         const float2 dx = __fadd2_rn(px2, make_float2(-q0.x, -q1.x));
         const float2 dy = __fadd2_rn(py2, make_float2(-q0.y, -q1.y));
         const float2 dz = __fadd2_rn(pz2, make_float2(-q0.z, -q1.z));
         const float2 rr = __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
-        if (rr.x <= h2) dm |= bit;
-        if (rr.y <= h2) dm |= bit << 1;
-        if (SKIN && rr.x <= skin2) sm |= bit;
-        if (SKIN && rr.y <= skin2) sm |= bit << 1;
+        const float2 x = __fadd2_rn(h22, make_float2(-rr.x, -rr.y));
+        dm = __funnelshift_l(__float_as_uint(x.x), dm, 1);
+        dm = __funnelshift_l(__float_as_uint(x.y), dm, 1);
+        if (SKIN) {
+            sm = __funnelshift_l(__float_as_uint(skin2 - rr.x), sm, 1);
+            sm = __funnelshift_l(__float_as_uint(skin2 - rr.y), sm, 1);
+        }
     };
-    // The words of chunk c of row r (bit b = candidate jb0 + 32c + b) minus
-    // the particle itself, stored to the masks and the row table.
-    auto close_chunk = [&](int r, uint32_t c, uint32_t jb0, uint32_t len, uint32_t dm, uint32_t sm) {
-        const uint32_t so = k - (jb0 + 32u * c);
-        const uint32_t notself = (so < 32u) ? ~(1u << so) : ~0u;
-        dm &= notself;
-        if (SKIN && len <= 32u) mask[(size_t)(SPH_MASK_SKIN + r) * mask_stride + k] = sm & notself;
-        mask[(size_t)(SPH_MASK_EXACT + 2 * r + c) * mask_stride + k] = dm;
-        if (c == 0u) tab[r * ts] = jb0;
-        tab[(9 + 2 * r + c) * ts] = dm;
-        if (dm) live |= 1u << (2 * r + c);
-    };
-    // A row longer than 64 candidates: no words, phase 2 tests every candidate.
-    auto long_row = [&](int r, uint32_t jb0, uint32_t len) {
-        tab[r * ts] = jb0;
-        tab[(9 + 2 * r) * ts] = len;
-        full |= 1u << (2 * r);
-        live |= 1u << (2 * r);
-    };
-    // The 9 row ranges, loaded together (18 independent loads) into the row
-    // table; a row's end sits in its first word's entry until the scan of
-    // the row replaces it.
-    uint32_t rows = 0u;
+    // The row ranges of this thread, loaded together (18 independent loads):
+    // starts into the row table, lengths (at most 255 kept: a longer row is
+    // cut short as any above 128 is) packed into bytes.
+    constexpr int kRows = SPLIT ? 3 : 9;
+    const int r0 = SPLIT ? 3 * (int)part : 0;
+    uint32_t lens[(kRows + 3) / 4] = {};
 #pragma unroll
     for (int rr = 0; rr < kRows; ++rr) {
-        const int r = r0 + rr;
         uint32_t jb0, je0;
-        if ((!SPLIT || work) && row_range(pp, start, sc.cell_base, delta, g, r, jb0, je0)) {
-            rows |= 1u << r;
-            tab[r * ts] = jb0;
-            tab[(9 + 2 * r) * ts] = je0;
+        if ((!SPLIT || work) && row_range(pp, start, sc.cell_base, delta, g, r0 + rr, jb0, je0)) {
+            rows[rr * rs] = jb0;
+            lens[rr / 4] |= min(je0 - jb0, 255u) << (8 * (rr % 4));
         }
     }
-    if (WALK == 1) {
+    uint32_t nrows = 0u;   // rows with a neighbour so far: their starts move to the front of the table
 #pragma unroll 1
-        for (int rr = 0; rr < kRows; ++rr) {
-            const int r = r0 + rr;
-            if (!((rows >> r) & 1u)) continue;
-            const uint32_t jb0 = tab[r * ts], je0 = tab[(9 + 2 * r) * ts];
-            const uint32_t len = je0 - jb0;
-            if (len > SPH_WIDE_ROW) { long_row(r, jb0, len); continue; }
-            uint32_t cb = jb0, c = 0u;
-            do {
-                const uint32_t ce = min(cb + 32u, je0);
-                uint32_t dm = 0u, sm = 0u, bit = 1u;
-                uint32_t jj = cb;
-                // from an even slot on, two candidates per 256-bit load (an
-                // empty row runs this body once, with cb == ce: no candidate)
-                if (jj < ce && (jj & 1u) != 0u) {
-                    visit(__ldg(P1 + jj), bit, dm, sm);
-                    bit <<= 1;
-                    ++jj;
-                }
-                for (; jj + 4u <= ce; jj += 4u) {
-                    float4 q0, q1, q2, q3;
-                    ld_float4_pair(P1 + jj, q0, q1);
-                    ld_float4_pair(P1 + jj + 2u, q2, q3);
-                    visit2(q0, q1, bit, dm, sm);
-                    visit2(q2, q3, bit << 2, dm, sm);
-                    bit <<= 4;
-                }
-                if (jj + 2u <= ce) {
-                    float4 q0, q1;
-                    ld_float4_pair(P1 + jj, q0, q1);
-                    visit2(q0, q1, bit, dm, sm);
-                    bit <<= 2;
-                    jj += 2u;
-                }
-                if (jj < ce) visit(__ldg(P1 + jj), bit, dm, sm);
-                close_chunk(r, c, jb0, len, dm, sm);
-                cb += 32u;
-                ++c;
-            } while (cb < je0);
+    for (int rr = 0; rr < kRows; ++rr) {
+        const uint32_t len = (lens[0] & 255u);
+#pragma unroll
+        for (int q = 0; q < (kRows + 3) / 4; ++q)
+            lens[q] = (lens[q] >> 8) | (q + 1 < (kRows + 3) / 4 ? lens[q + 1] << 24 : 0u);
+        if (len == 0u) continue;
+        const uint32_t jb0 = rows[rr * rs];
+        if (len > SPH_NBR_MAX_ROW) {   // its offsets do not fit: the list ends here
+            hd.over = true;
+            if (SKIN) continue;   // later rows still get their skin words
+            break;
         }
-    } else {
-        // one loop across all 9 rows and their chunks, so lanes do not wait at
-        // row ends
-        int r = -1;
-        uint32_t jb = 0, je = 0, j = 0, cend = 0, c = 0, len = 0, dm = 0u, sm = 0u, bit = 0u;
-        bool valid = false;
-        for (;;) {
-            if (j >= cend) {
-                if (valid) {
-                    close_chunk(r, c, jb, len, dm, sm);
-                    if (j < je) {   // the row's second chunk
-                        ++c;
-                        cend = min(j + 32u, je);
-                        dm = sm = 0u;
-                        bit = 1u;
-                        continue;
-                    }
-                }
-                if (++r >= 9) break;
-                valid = ((rows >> r) & 1u) != 0u;
-                jb = valid ? tab[r * ts] : 0u;
-                je = valid ? tab[(9 + 2 * r) * ts] : 0u;
-                len = je - jb;
-                if (valid && len > SPH_WIDE_ROW) {
-                    long_row(r, jb, len);
-                    valid = false;
-                    j = cend = 0;
-                    continue;
-                }
-                c = 0u;
-                j = jb;
-                cend = min(jb + 32u, je);
-                dm = sm = 0u;
-                bit = 1u;
-                continue;
+        bool first = true;
+        uint32_t c0 = 0u;   // offset of the chunk in the row
+        do {
+            const uint32_t cb = jb0 + c0, clen = min(len - c0, 32u), ce = cb + clen;
+            uint32_t dm = 0u, sm = 0u;
+            uint32_t jj = cb;
+            // from an even slot on, two candidates per 256-bit load
+            if ((jj & 1u) != 0u) {
+                visit(__ldg(P1 + jj), dm, sm);
+                ++jj;
             }
-            visit(__ldg(P1 + j), bit, dm, sm);
-            bit <<= 1;
-            ++j;
-        }
+            for (; jj + 4u <= ce; jj += 4u) {
+                float4 q0, q1, q2, q3;
+                ld_float4_pair(P1 + jj, q0, q1);
+                ld_float4_pair(P1 + jj + 2u, q2, q3);
+                visit2(q0, q1, dm, sm);
+                visit2(q2, q3, dm, sm);
+            }
+            if (jj + 2u <= ce) {
+                float4 q0, q1;
+                ld_float4_pair(P1 + jj, q0, q1);
+                visit2(q0, q1, dm, sm);
+                jj += 2u;
+            }
+            if (jj < ce) visit(__ldg(P1 + jj), dm, sm);
+            // candidate cb + b in bit 31 - b, the particle itself left out
+            const uint32_t so = k - cb;
+            const uint32_t notself = (so < 32u) ? ~(0x80000000u >> so) : ~0u;
+            uint32_t bits = (~dm << (32u - clen)) & notself;
+            if (SKIN && len <= 32u)
+                mask[(size_t)(SPH_MASK_SKIN + rr) * mask_stride + k] = __brev((~sm << (32u - clen)) & notself);
+            if (hd.n + (uint32_t)__popc(bits) > SPH_NBR_CAP) hd.over = true;
+            if (bits && !hd.over) {
+                int b = __clz(bits);
+                if (first) {
+                    first = false;
+                    rows[nrows++ * rs] = jb0;
+                    hd.live |= 1u << (r0 + rr);
+                    bits &= ~(0x80000000u >> b);
+                    list[hd.n++] = (uint8_t)(c0 + b + SPH_NBR_NEW_ROW);
+                }
+                while (bits) {
+                    b = __clz(bits);
+                    bits &= ~(0x80000000u >> b);
+                    list[hd.n++] = (uint8_t)(c0 + b);
+                }
+            }
+            c0 += 32u;
+        } while (c0 < len && (SKIN || !hd.over));
+        if (!SKIN && hd.over) break;
     }
 
     if constexpr (SPLIT) {
-        // the parts' row bits are disjoint: the first thread takes their union
-        __shared__ uint32_t s_bits[2 * 3 * SPH_TILE];
-        s_bits[2 * threadIdx.x] = live;
-        s_bits[2 * threadIdx.x + 1] = full;
+        // the first thread appends the lists of the other two
+        __shared__ uint32_t s_hd[3 * SPH_TILE];
+        s_hd[threadIdx.x] = hd.pack() | (nrows << 9);
         __syncthreads();
         if (part != 0u || !work) return;
-        live = s_bits[2 * li] | s_bits[2 * (ts + li)] | s_bits[2 * (2 * ts + li)];
-        full = s_bits[2 * li + 1] | s_bits[2 * (ts + li) + 1] | s_bits[2 * (2 * ts + li) + 1];
+        for (uint32_t q = 1; q < 3u && !hd.over; ++q) {
+            const uint32_t o = q * ts;
+            const uint32_t w = s_hd[li + o];
+            const NbrHeader ho(w & ~(15u << 9));
+            const uint8_t* from = reinterpret_cast<const uint8_t*>(
+                s_list + SPH_NBR_ROWS * rs + (li + o) * SPH_NBR_LIST_WORDS);
+            if (hd.n + ho.n > SPH_NBR_CAP) {
+                hd.over = true;
+                break;
+            }
+            for (uint32_t m = 0; m < ho.n; ++m) list[hd.n + m] = from[m];
+            for (uint32_t r = 0; r < ((w >> 9) & 15u); ++r) rows[nrows++ * rs] = rows[r * rs + o];
+            hd.n += ho.n;
+            hd.live |= ho.live;
+            hd.over = ho.over;
+        }
     }
+    // the last word's padding: offset 0 of the current row (read, not used)
+    for (uint32_t m = hd.n; m & 3u; ++m) list[m] = 0;
+    mask[k] = hd.pack();
 
     // ---- phase 2: the density pairs, in candidate order ----
     const float h = pp.h, mass = pp.mass, c6 = pp.poly6, two_m = pp.two_mass;
@@ -661,21 +650,24 @@ k_density(const DevParams* __restrict__ params,
     float2 axy = make_float2(0.f, 0.f);
     float az = 0.f;
     const float2 mvixy = make_float2(-vi.x, -vi.y);
-    TableWalk walk(tab, ts, live, full);
-    uint32_t j;
-    while (walk.next(j)) {
-        // the pair's XSPH operands (velocity, and its last cell in the w
-        // lane) are loaded with its position, before any test, so that the
-        // two latencies overlap
-        const float4 q = __ldg(P1 + j);
-        float4 vj = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (xs) vj = __ldg(V1 + j);
+    // the pair's XSPH operands (velocity, and its last cell in the w lane) are
+    // loaded with its position, before any test, so that the latencies overlap
+    struct Nbr { float4 q, v; };
+    auto load = [&](uint32_t j) {
+        Nbr n;
+        n.q = __ldg(P1 + j);
+        n.v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (xs) n.v = __ldg(V1 + j);
+        return n;
+    };
+    auto use = [&](const Nbr& n) {
+        const float4 q = n.q, vj = n.v;
         const uint32_t oj = __float_as_uint(vj.w);
         const float2 dxy = __fadd2_rn(make_float2(p.x, p.y), make_float2(-q.x, -q.y));
         const float dx = dxy.x, dy = dxy.y, dz = p.z - q.z;
         const float rr = dot3(dx, dy, dz, dx, dy, dz);
-        // true for every recorded bit; the test matters in rows walked in full
-        if (rr <= h2 && j != k) {
+        // true for every listed neighbour of finite position; the test matters in the tail
+        if (rr <= h2) {
             const float rd = sqrtf(rr);
             const float x = fmaf(-rd, rd, h2);
             const float w = (rd >= h) ? 0.0f : c6 * (x * x * x);
@@ -690,7 +682,18 @@ k_density(const DevParams* __restrict__ params,
                 }
             }
         }
+    };
+    const uint32_t* words = reinterpret_cast<const uint32_t*>(list);
+    NbrRows table(rows, rs);
+    uint32_t last = 0u;
+    for (uint32_t m = 0; m < hd.n; m += 4u) {
+        const uint32_t w = words[m >> 2];
+        mask[(size_t)(SPH_NBR_LIST + (m >> 2)) * mask_stride + k] = w;
+        last = visit_word<kDensityDepth>(w, hd.n - m, table, load, use);
     }
+    if (hd.over)
+        walk_tail(pp, start, sc.cell_base, delta, g, hd.n ? last + 1u : 0u,
+                  [&](uint32_t j) { if (j != k) use(load(j)); });
     const float d = fabsf(sdf(pp, p.x, p.y, p.z));
     float corr = sum;
     if (d < pp.h) corr = fmaf(pp.rest_density, 1.0f - boundary_density(pp, d), corr);
@@ -714,10 +717,9 @@ k_density(const DevParams* __restrict__ params,
 // ---------------------------------------------------------------------------
 // Surface normals (computeNormals, fluidphysics.cu:154-210).  Only launched
 // for scenes with surface tension: with sigma == 0 the normals enter the
-// force only through sigma * (...), which is exactly zero.  TABLE walks a row
-// table in shared memory as the force pass does; same neighbours, same order.
+// force only through sigma * (...), which is exactly zero.  Neighbours come
+// from the density pass's list, as in the force pass.
 // ---------------------------------------------------------------------------
-template <bool TABLE>
 __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restrict__ params,
                                                       const DevScene* __restrict__ scenes,
                                                       const uint4* __restrict__ tiles,
@@ -750,34 +752,22 @@ __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restric
     // rounded root r as gradPoly6 forms it (it cancels near r = h)
     const float mc = pp.mass * pp.grad_poly6;
     const float h2 = pp.h2, eps = pp.eps, h = pp.h;
-    auto run = [&](auto& walk) {
-        uint32_t j;
-        while (walk.next(j)) {
-            const float4 q = __ldg(R + 2 * (size_t)j);   // w = 1/rho_j, 0 where rho_j <= eps
+    extern __shared__ uint32_t s_rows[];
+    walk_neighbours<kNormalsDepth>(
+        pp, start, sc.cell_base, delta, g, mask, mask_stride, k, s_rows + threadIdx.x, blockDim.x,
+        [&](uint32_t j) { return __ldg(R + 2 * (size_t)j); },   // w = 1/rho_j, 0 where rho_j <= eps
+        [&](const float4& q) {
             const float2 rxy = __fadd2_rn(pxy, make_float2(-q.x, -q.y));
             const float rx = rxy.x, ry = rxy.y, rz = p.z - q.z;
             const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-            if (r2 <= h2 && r2 > eps && j != k && q.w > 0.0f) {
+            if (r2 <= h2 && r2 > eps && q.w > 0.0f) {
                 const float r = sqrtf(r2);
                 const float x = fmaf(-r, r, h2);
                 const float s = (r >= h) ? 0.0f : mc * (x * x) * q.w;
                 sxy = __ffma2_rn(make_float2(s, s), rxy, sxy);
                 sz = fmaf(s, rz, sz);
             }
-        }
-    };
-    // exact neighbours recorded by the density pass (SPH_MASK_EXACT words)
-    if constexpr (TABLE) {
-        extern __shared__ uint32_t s_rows[];
-        uint32_t live, full;
-        build_row_table(pp, start, sc.cell_base, delta, g, mask + SPH_MASK_EXACT * mask_stride, mask_stride, k,
-                        s_rows + threadIdx.x, blockDim.x, live, full);
-        TableWalk walk(s_rows + threadIdx.x, blockDim.x, live, full);
-        run(walk);
-    } else {
-        WideMaskWalk walk(pp, start, sc.cell_base, delta, g, mask + SPH_MASK_EXACT * mask_stride, mask_stride, k);
-        run(walk);
-    }
+        });
     N[k] = make_float4(pp.h * sxy.x, pp.h * sxy.y, pp.h * sz, 0.f);
   });
 }
@@ -799,7 +789,7 @@ __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restric
 // budget as resident blocks of 256 threads per SM: 3 (80 registers, no
 // spills) or 4 (64 registers, more warps per SM, a few spilled values in the
 // tension build).
-template <bool TENSION, int MINB, bool TABLE>
+template <bool TENSION, int MINB>
 __global__ void __launch_bounds__(SPH_TILE, MINB)
 k_force_integrate(const DevParams* __restrict__ params,
                                                               const DevScene* __restrict__ scenes,
@@ -888,30 +878,19 @@ k_force_integrate(const DevParams* __restrict__ params,
             }
         }
     };
-    // The neighbour's loads are issued together, before any test, so that
-    // their latencies overlap (the masks hold exact neighbours: nearly every
-    // j is used).
-    auto gathered = [&](uint32_t j) {
-        float4 pj, vj, nj = make_float4(0.f, 0.f, 0.f, 0.f);
-        ld_float4_pair(R + 2 * (size_t)j, pj, vj);
-        if (tension) nj = __ldg(N + j);
-        pair(pj, vj, nj);
-    };
-    // exact neighbours recorded by the density pass (SPH_MASK_EXACT words)
+    struct Nbr { float4 p, v, n; };
     if (inside) {
-        if constexpr (TABLE) {
-            extern __shared__ uint32_t s_rows[];
-            uint32_t live, full;
-            build_row_table(pp, start, sc.cell_base, delta, g, mask + SPH_MASK_EXACT * mask_stride, mask_stride, k,
-                            s_rows + threadIdx.x, blockDim.x, live, full);
-            TableWalk walk(s_rows + threadIdx.x, blockDim.x, live, full);
-            uint32_t j;
-            while (walk.next(j)) gathered(j);
-        } else {
-            WideMaskWalk walk(pp, start, sc.cell_base, delta, g, mask + SPH_MASK_EXACT * mask_stride, mask_stride, k);
-            uint32_t j;
-            while (walk.next(j)) gathered(j);
-        }
+        extern __shared__ uint32_t s_rows[];
+        walk_neighbours<kForceDepth>(
+            pp, start, sc.cell_base, delta, g, mask, mask_stride, k, s_rows + threadIdx.x, blockDim.x,
+            [&](uint32_t j) {
+                Nbr r;
+                ld_float4_pair(R + 2 * (size_t)j, r.p, r.v);
+                r.n = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (tension) r.n = __ldg(N + j);
+                return r;
+            },
+            [&](const Nbr& r) { pair(r.p, r.v, r.n); });
     }
     if (inside) {
         // the factors left out of the sums
@@ -1075,12 +1054,13 @@ __global__ void k_xsph(const DevParams* __restrict__ params,
     // moved less than skin*h/2 each, which the force pass recorded.
     uint32_t j;
     const bool masked = __uint_as_float(__ldg(maxdisp)) <= pp.xsph_disp_limit2;
+    const uint32_t* skin = mask + SPH_MASK_SKIN * mask_stride;
     if (WALK == 1) {
         auto visit = [&](uint32_t jj) { xsph_pair(P0, V2, jj, k, pi, vi, h2, h, c6, two_m, eps, sx, sy, sz); };
-        if (masked) for_masked(pp, start, sc.cell_base, delta, g, mask, mask_stride, k, visit);   // skin words 0-8
+        if (masked) for_masked(pp, start, sc.cell_base, delta, g, skin, mask_stride, k, visit);
         else for_candidates(pp, start, sc.cell_base, delta, g, visit);
     } else if (masked) {
-        MaskWalk walk(pp, start, sc.cell_base, delta, g, mask, mask_stride, k);   // skin mask, words 0-8
+        MaskWalk walk(pp, start, sc.cell_base, delta, g, skin, mask_stride, k);
         while (walk.next(j)) xsph_pair(P0, V2, j, k, pi, vi, h2, h, c6, two_m, eps, sx, sy, sz);
     } else {
         RangeWalk walk(pp, start, sc.cell_base, delta, g);
@@ -1265,24 +1245,27 @@ cudaError_t launch_hash(const StepArgs& a, cudaStream_t st) {
 }
 static inline uint32_t* ctr(const StepArgs& a, int k) { return a.tile_ctr ? a.tile_ctr + k : nullptr; }
 
-// Kernels with a row table in shared memory need 72 B per thread of it; left
-// to itself the driver may give them the largest shared-memory carveout and
-// shrink L1, which holds the neighbour gathers.  Ask for the smallest carveout
-// that still fits 8 blocks of 128 threads (8 x 9 KB + per-block reserve).
+// Kernels with row starts or neighbour lists in shared memory: left to itself
+// the driver may give them the largest shared-memory carveout and shrink L1,
+// which holds the neighbour gathers.  Ask for the smallest carveout that still
+// fits the blocks that registers allow on an SM (SPH_*_CARVEOUT_PCT).
 cudaError_t init_kernel_attributes() {
-    const int pct = SPH_TABLE_CARVEOUT_PCT;
-    const void* fns[] = {
-        (const void*)k_force_integrate<true, 3, true>, (const void*)k_force_integrate<true, 4, true>,
-        (const void*)k_force_integrate<false, 3, true>, (const void*)k_force_integrate<false, 4, true>,
-        (const void*)k_normals<true>,
-        (const void*)k_density<0, false>, (const void*)k_density<0, true>,
-        (const void*)k_density<1, false>, (const void*)k_density<1, true>,
-        (const void*)k_density<1, false, true>};
-    for (const void* f : fns) {
-        const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+    struct { const void* f; int pct; } fns[] = {
+        {(const void*)k_force_integrate<true, 3>, SPH_ROWS_CARVEOUT_PCT},
+        {(const void*)k_force_integrate<true, 4>, SPH_ROWS_CARVEOUT_PCT},
+        {(const void*)k_force_integrate<false, 3>, SPH_ROWS_CARVEOUT_PCT},
+        {(const void*)k_force_integrate<false, 4>, SPH_ROWS_CARVEOUT_PCT},
+        {(const void*)k_normals, SPH_ROWS_CARVEOUT_PCT},
+        {(const void*)k_density<false>, SPH_LIST_CARVEOUT_PCT},
+        {(const void*)k_density<true>, SPH_LIST_CARVEOUT_PCT},
+        {(const void*)k_density<false, true>, SPH_LIST_CARVEOUT_PCT}};
+    for (const auto& x : fns) {
+        const cudaError_t e = cudaFuncSetAttribute(x.f, cudaFuncAttributePreferredSharedMemoryCarveout, x.pct);
         if (e != cudaSuccess) return e;
     }
-    return cudaSuccess;
+    // the split scan keeps three lists per particle: above 48 KB from 128-particle tiles on
+    return cudaFuncSetAttribute((const void*)k_density<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(3u * SPH_TILE * SPH_NBR_SMEM_WORDS * sizeof(uint32_t)));
 }
 
 // a.scan_sums holds at least nt + 2 64-bit words: the tile counter, then one
@@ -1331,16 +1314,14 @@ bool density_split(const StepArgs& a) {
            !a.skin_masks && a.tile_ctr == nullptr && a.particles <= SPH_DENSITY_SPLIT_MAX;
 }
 cudaError_t launch_density(const StepArgs& a, cudaStream_t st) {
-    const size_t smem = (size_t)SPH_ROW_TABLE_WORDS * a.block * sizeof(uint32_t);   // the row table
+    const size_t smem = (size_t)SPH_NBR_SMEM_WORDS * a.block * sizeof(uint32_t);
     if (density_split(a)) {
-        k_density<1, false, true><<<a.ntiles, 3u * a.block, smem, st>>>(
+        k_density<false, true><<<a.ntiles, 3u * a.block, 3u * smem, st>>>(
             a.params, a.scenes, a.tiles, a.start, a.P1, a.rho, a.mask, a.mask_stride, a.V1, a.pend, a.R, a.dbg_nbr,
             a.ntiles, nullptr, a.status);
         return cudaGetLastError();
     }
-    const bool rows = (a.variant & SPH_VARIANT_DENSITY_ROWS) != 0u;
-    auto kern = a.skin_masks ? (rows ? k_density<1, true> : k_density<0, true>)
-                             : (rows ? k_density<1, false> : k_density<0, false>);
+    auto kern = a.skin_masks ? k_density<true> : k_density<false>;
     kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.P1, a.rho, a.mask, a.mask_stride,
                                             a.V1, a.pend, a.R, a.dbg_nbr, a.ntiles, ctr(a, 0), a.status);
     return cudaGetLastError();
@@ -1358,27 +1339,20 @@ cudaError_t launch_undo_ahead(const StepArgs& a, uint32_t first_tile, uint32_t n
                                              a.okey);
     return cudaGetLastError();
 }
+static size_t rows_smem(const StepArgs& a) { return (size_t)SPH_NBR_ROWS * a.block * sizeof(uint32_t); }
 cudaError_t launch_normals(const StepArgs& a, cudaStream_t st) {
-    const bool table = (a.variant & SPH_VARIANT_NORMALS_TABLE) != 0u;
-    auto kern = table ? k_normals<true> : k_normals<false>;
-    const size_t smem = table ? (size_t)SPH_ROW_TABLE_WORDS * a.block * sizeof(uint32_t) : 0;
-    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.mask, a.mask_stride,
-                                            a.N, a.ntiles, ctr(a, 1), a.status);
+    k_normals<<<a.grid_nbr, a.block, rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.mask,
+                                                         a.mask_stride, a.N, a.ntiles, ctr(a, 1), a.status);
     return cudaGetLastError();
 }
 cudaError_t launch_force(const StepArgs& a, cudaStream_t st) {
     const bool occ = (a.variant & SPH_VARIANT_FORCE_OCC) != 0u;
-    const bool table = (a.variant & SPH_VARIANT_FORCE_TABLE) != 0u;
-    auto kern = a.any_tension
-                    ? (table ? (occ ? k_force_integrate<true, 4, true> : k_force_integrate<true, 3, true>)
-                             : (occ ? k_force_integrate<true, 4, false> : k_force_integrate<true, 3, false>))
-                    : (table ? (occ ? k_force_integrate<false, 4, true> : k_force_integrate<false, 3, true>)
-                             : (occ ? k_force_integrate<false, 4, false> : k_force_integrate<false, 3, false>));
-    const size_t smem = table ? (size_t)SPH_ROW_TABLE_WORDS * a.block * sizeof(uint32_t) : 0;
-    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.rho, a.A1, a.N, a.mask,
-                                            a.mask_stride, a.P0, a.V2, a.A0, a.skin_masks ? a.maxdisp : nullptr,
-                                            a.okey, a.pend, a.count, a.key, a.slot, a.status, a.dbg_forces,
-                                            a.ntiles, ctr(a, 2));
+    auto kern = a.any_tension ? (occ ? k_force_integrate<true, 4> : k_force_integrate<true, 3>)
+                              : (occ ? k_force_integrate<false, 4> : k_force_integrate<false, 3>);
+    kern<<<a.grid_nbr, a.block, rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.rho, a.A1, a.N,
+                                                    a.mask, a.mask_stride, a.P0, a.V2, a.A0,
+                                                    a.skin_masks ? a.maxdisp : nullptr, a.okey, a.pend, a.count,
+                                                    a.key, a.slot, a.status, a.dbg_forces, a.ntiles, ctr(a, 2));
     return cudaGetLastError();
 }
 cudaError_t launch_xsph(const StepArgs& a, cudaStream_t st) {

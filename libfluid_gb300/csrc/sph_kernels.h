@@ -32,8 +32,7 @@ struct StepArgs {
     uint32_t *key, *slot, *perm;
     uint32_t *tmp;             // scatter list of the sort; shares the mask words, which the density pass writes later
     uint32_t *status;
-    uint32_t *mask;            // SPH_MASK_ROWS neighbour-mask words per slot, word m at mask[m*mask_stride + slot]:
-                               // SPH_MASK_SKIN skin radius (XSPH), SPH_MASK_EXACT exact neighbours (normals, forces)
+    uint32_t *mask;            // SPH_MASK_ROWS neighbour words per slot, word m at mask[m*mask_stride + slot]
     size_t mask_stride;
     uint32_t *maxdisp;         // largest (displacement/h)^2 of the substep, float bits
     uint32_t block;            // threads per block = particles per tile
@@ -46,11 +45,16 @@ struct StepArgs {
     float4 *dbg_forces;        // optional: 4 force vectors per sorted slot
 };
 
-// Shared-memory carveout (percent of the SM's maximum) requested for the
-// kernels that keep a row table in shared memory: the smallest that holds
-// the tables of 8 blocks of 128 threads, so that L1 keeps the rest.
-#ifndef SPH_TABLE_CARVEOUT_PCT
-#define SPH_TABLE_CARVEOUT_PCT 50
+// Shared-memory carveouts (percent of the SM's maximum) requested for the
+// density pass (lists and row starts of 9 blocks of 128 threads) and for the
+// normal and force passes (row starts of 8), so that L1 keeps the rest.
+// Measured on the 1M dam break: 50 and 18 give 237.7 and 138.0 us, 58 and 25
+// 239.5 and 139.3, 44 and 10 237.9 and 191.8 (too few blocks fit).
+#ifndef SPH_LIST_CARVEOUT_PCT
+#define SPH_LIST_CARVEOUT_PCT 50
+#endif
+#ifndef SPH_ROWS_CARVEOUT_PCT
+#define SPH_ROWS_CARVEOUT_PCT 18
 #endif
 // One-time per-device kernel attributes (call before the first launch).
 cudaError_t init_kernel_attributes();

@@ -47,31 +47,33 @@ struct DevParams {
     uint32_t pad_;
 };
 
-// Neighbour masks are built with radius (1 + skin) h (default skin below).
+// The skin words are built with radius (1 + skin) h (default skin below).
 // XSPH, which runs on positions moved by the integrator, may use them only
 // while every particle moved less than skin*h/2 in the substep (checked on
 // the device; otherwise XSPH walks all candidates).
 #define SPH_SKIN_DEFAULT 0.1f
 
-// Neighbour-mask rows per slot (row m of slot k at mask[m * stride + k]).
-// Exact-neighbour words of a cell row: rows of up to 64 candidates carry two
-// words (word h: candidates jb + 32h .. jb + 32h + 31; the second is written
-// and read only for rows longer than 32); longer rows carry none and are
-// walked in full.  Words of row r sit at mask rows SPH_MASK_EXACT + 2r + h.
-#define SPH_MASK_SKIN   0u    // 9 rows: candidates within the skin radius (rows of <= 32)
-#define SPH_MASK_EXACT  9u    // 18 rows: neighbours r^2 <= h^2, j != i (readers test r^2 > eps)
-#define SPH_MASK_ROWS   27u
-#define SPH_WIDE_ROW    64u   // longest row with mask words
-#define SPH_ROW_TABLE_WORDS 27u   // per-thread row table: 9 row starts + 18 words
+// Neighbour words per slot (row m of slot k at mask[m * stride + k]): the
+// neighbour list's header, its words (four neighbours each), and the skin-radius
+// words, used only when some scene runs a per-substep XSPH pass.
+#define SPH_NBR_LIST       1u    // first list row; row 0 is the header
+#define SPH_NBR_LIST_WORDS 17u   // (odd: the threads' lists in shared memory start in different banks)
+#define SPH_MASK_SKIN      18u   // 9 rows: candidates within the skin radius (rows of <= 32)
+#define SPH_MASK_ROWS      27u
+#define SPH_NBR_CAP        68u   // listed neighbours: four to a word
+#define SPH_NBR_NEW_ROW    128u  // added to a row's first neighbour
+#define SPH_NBR_MAX_ROW    128u  // longest row whose offsets fit below that
+#define SPH_NBR_ROWS       10u   // row starts kept per thread: nine and one that is read ahead
+#define SPH_NBR_SMEM_WORDS (SPH_NBR_ROWS + SPH_NBR_LIST_WORDS)
 
 // Kernel variants (bits of the execution config's `variant`). All variants
 // visit neighbours in the same order and give identical results; they differ
 // only in how the walk is scheduled.
-#define SPH_VARIANT_DENSITY_ROWS  0x1u   // density: one loop per cell row, four candidates in flight (two 256-bit loads)
+#define SPH_VARIANT_DENSITY_ROWS  0x1u   // density: with DENSITY_SPLIT, the split scan (else no effect: one scan is left)
 #define SPH_VARIANT_XSPH_ROWS     0x2u   // XSPH: one loop per cell row instead of one flattened walk
 #define SPH_VARIANT_FORCE_OCC     0x4u   // force: 64-register build (more resident warps)
-#define SPH_VARIANT_FORCE_TABLE   0x8u   // force: walk over a per-thread row table in shared memory
-#define SPH_VARIANT_NORMALS_TABLE 0x10u  // normals: the same
+#define SPH_VARIANT_FORCE_TABLE   0x8u   // no effect: the force and normal passes walk the neighbour list
+#define SPH_VARIANT_NORMALS_TABLE 0x10u  // no effect
 #define SPH_VARIANT_DENSITY_SPLIT 0x20u  // density: three threads per particle share the candidate scan
                                          // (launches of at most SPH_DENSITY_SPLIT_MAX particles)
 #define SPH_VARIANT_MASK          0x3fu
