@@ -102,9 +102,9 @@ bool derive_params(const SceneConfig& c, DevParams& d, std::string* err) {
     return true;
 }
 
-// eight float4 arrays and the 32-byte records; key, slot, perm, okey and rho
+// six float4 arrays, the gathered state and the records of two each; key, slot, perm, okey and rho
 // (the sort's scatter list shares the mask words)
-uint64_t Engine::bytes_per_particle() { return 8 * 16 + 32 + 5 * 4 + SPH_MASK_ROWS * 4; }
+uint64_t Engine::bytes_per_particle() { return 6 * 16 + 2 * 32 + 5 * 4 + SPH_MASK_ROWS * 4; }
 uint64_t Engine::bytes_per_cell() { return 2 * 4 + 1; }
 const char* Engine::pass_name(int i) { return (i >= 0 && i < kPasses) ? kPassNames[i] : "?"; }
 
@@ -166,7 +166,7 @@ int Engine::cuda_fail(cudaError_t e, const char* what) {
     } while (0)
 
 void Engine::free_all() {
-    float4** f4[] = {&P0_, &P1_, &V0_, &V1_, &V2_, &A0_, &A1_, &N_, &R_, &dbg_forces_};
+    float4** f4[] = {&P0_, &G_, &V0_, &V2_, &A0_, &A1_, &N_, &R_, &dbg_forces_};
     for (auto p : f4) { if (*p) cudaFree(*p); *p = nullptr; }
     if (rho_) cudaFree(rho_);
     rho_ = nullptr;
@@ -204,7 +204,7 @@ int Engine::ensure_capacity(uint64_t parts, uint64_t cells) {
                               {(void**)&A0_, sizeof(float4)}, {(void**)&V2_, sizeof(float4)},
                               {(void**)&R_, 2 * sizeof(float4)}, {(void**)&rho_, sizeof(float)},
                               {(void**)&okey_, sizeof(uint32_t)}};
-        float4** scratch[] = {&P1_, &V1_, &A1_, &N_};
+        struct { float4** p; uint64_t per_slot; } scratch[] = {{&G_, 2}, {&A1_, 1}, {&N_, 1}};
         for (const Kept& k : state) {
             void* q = nullptr;
             cudaError_t e = cudaMalloc(&q, np * k.entry);
@@ -217,10 +217,10 @@ int Engine::ensure_capacity(uint64_t parts, uint64_t cells) {
             *k.p = q;
         }
         prefix_valid_ = false;
-        for (auto p : scratch) {
-            if (*p) cudaFree(*p);
-            *p = nullptr;
-            cudaError_t e = cudaMalloc((void**)p, np * sizeof(float4));
+        for (const auto& x : scratch) {
+            if (*x.p) cudaFree(*x.p);
+            *x.p = nullptr;
+            cudaError_t e = cudaMalloc((void**)x.p, np * x.per_slot * sizeof(float4));
             if (e != cudaSuccess) return fail(ENG_ENOMEM, std::string("device allocation failed: ") + cudaGetErrorString(e));
         }
         uint32_t** u[] = {&key_, &slot_, &perm_};
@@ -233,7 +233,8 @@ int Engine::ensure_capacity(uint64_t parts, uint64_t cells) {
         if (mask_) cudaFree(mask_);
         mask_ = nullptr;
         {
-            cudaError_t e = cudaMalloc((void**)&mask_, (size_t)SPH_MASK_ROWS * np * sizeof(uint32_t));
+            mask_stride_ = (np + 3) & ~(uint64_t)3;   // the density pass reads rows four slots at a time
+            cudaError_t e = cudaMalloc((void**)&mask_, (size_t)SPH_MASK_ROWS * mask_stride_ * sizeof(uint32_t));
             if (e != cudaSuccess) return fail(ENG_ENOMEM, std::string("device allocation failed: ") + cudaGetErrorString(e));
         }
         if (dbg_nbr_) { cudaFree(dbg_nbr_); dbg_nbr_ = nullptr; }
@@ -512,7 +513,7 @@ StepArgs Engine::args() const {
     a.particles = (uint32_t)total_particles();
     a.total_cells = total_cells_;
     a.P0 = P0_; a.V0 = V0_; a.A0 = A0_;
-    a.P1 = P1_; a.V1 = V1_; a.A1 = A1_;
+    a.G = G_; a.A1 = A1_;
     a.V2 = V2_; a.rho = rho_; a.N = N_;
     a.R = R_; a.okey = okey_; a.pend = pend_;
     a.count = count_; a.start = start_; a.scan_sums = scan_sums_;
@@ -524,7 +525,7 @@ StepArgs Engine::args() const {
     a.key = key_; a.slot = slot_; a.tmp = mask_; a.perm = perm_;
     a.status = status_;
     a.mask = mask_;
-    a.mask_stride = pcap_;
+    a.mask_stride = mask_stride_;
     a.maxdisp = scal_;
     a.block = exec_.tile;
     a.tile_ctr = exec_.persistent ? scal_ + 4 : nullptr;
@@ -1163,7 +1164,7 @@ int Engine::debug_get(int id, int field, void* host, uint64_t count) {
             if (!need(n)) return fail(ENG_EINVAL, "buffer too small");
             uint32_t* tmp = nullptr;
             ENG_CK(cudaMalloc((void**)&tmp, n * sizeof(uint32_t)), "debug alloc");
-            ENG_CK(launch_sorted_keys(d_params_ + s->table_index, P1_, n, pb, tmp, stream_), "sorted keys");
+            ENG_CK(launch_sorted_keys(d_params_ + s->table_index, G_, n, pb, tmp, stream_), "sorted keys");
             ENG_CK(cudaMemcpyAsync(host, tmp, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_), "debug copy");
             ENG_CK(cudaStreamSynchronize(stream_), "debug sync");
             cudaFree(tmp);
@@ -1234,9 +1235,11 @@ int Engine::debug_get(int id, int field, void* host, uint64_t count) {
         case F_ACC:
         case F_VEL_INT: {
             if (!need(3ull * n)) return fail(ENG_EINVAL, "buffer too small");
-            const float4* src = field == F_NORMAL ? N_ : field == F_POS_SORTED ? P1_ : field == F_ACC ? A0_ : V2_;
+            const float4* src = field == F_NORMAL ? N_ : field == F_POS_SORTED ? G_ : field == F_ACC ? A0_ : V2_;
+            const size_t per_slot = field == F_POS_SORTED ? 2 : 1;
             std::vector<float4> v(n);
-            ENG_CK(cudaMemcpy(v.data(), src + pb, n * sizeof(float4), cudaMemcpyDeviceToHost), "debug copy");
+            ENG_CK(cudaMemcpy2D(v.data(), sizeof(float4), src + per_slot * pb, per_slot * sizeof(float4),
+                                sizeof(float4), n, cudaMemcpyDeviceToHost), "debug copy");
             float* out = (float*)host;
             for (uint32_t i = 0; i < n; ++i) { out[3 * i] = v[i].x; out[3 * i + 1] = v[i].y; out[3 * i + 2] = v[i].z; }
             return ENG_OK;

@@ -221,7 +221,8 @@ private:
     std::map<uint32_t, uint32_t> free_;
     uint64_t pcap_ = 0, ccap_ = 0, slots_end_ = 0;
     // device arenas
-    float4 *P0_ = nullptr, *P1_ = nullptr, *V0_ = nullptr, *V1_ = nullptr, *V2_ = nullptr, *A0_ = nullptr,
+    float4 *P0_ = nullptr, *G_ = nullptr, *V0_ = nullptr, *V2_ = nullptr, *A0_ = nullptr,   // G_: two per slot
+          
            *A1_ = nullptr, *N_ = nullptr, *R_ = nullptr;   // R_: two per slot
     float* rho_ = nullptr;
     uint32_t *okey_ = nullptr;         // packed cells of the last substep (state order)
@@ -229,7 +230,8 @@ private:
     uint32_t *key_ = nullptr, *slot_ = nullptr, *perm_ = nullptr;
     uint32_t *count_ = nullptr, *start_ = nullptr, *scan_sums_ = nullptr, *status_ = nullptr;
     uint32_t *gate_ = nullptr;        // status word of the passes an export ran ahead (status_ + 1)
-    uint32_t *mask_ = nullptr;        // SPH_MASK_ROWS neighbour-mask words per slot
+    uint32_t *mask_ = nullptr;        // SPH_MASK_ROWS neighbour words per slot, rows of mask_stride_
+    size_t mask_stride_ = 0;
     uint32_t *scal_ = nullptr;        // per-substep scalars: [0] displacement max, [4..7] tile counters
     ExecConfig exec_;
     int sm_count_ = 1;

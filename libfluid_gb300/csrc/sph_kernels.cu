@@ -12,8 +12,13 @@
 //   P0,V0,A0  state between substeps (P0.w = density of the last substep)
 //   V2, okey  post-integration velocity and cell of the last substep, for a
 //             scene whose XSPH update is pending (pend[scene] != 0)
-//   P1,V1,A1  state gathered into cell order (with a pending update, V1.w
-//             holds the gathered okey bits)
+//   G, A1     state gathered into cell order: G holds two float4 per slot,
+//             P0 and the velocity (with a pending update, its w lane holds
+//             the gathered okey bits)
+//   X         the gathered positions again for the density pass's candidate
+//             scan, four slots at a time: their x, their y, their z, 48 bytes
+//             in all (they lie in rows of the neighbour words that the density
+//             pass does not write)
 //   rho       density per sorted slot
 //   R         neighbour record per sorted slot, 32 bytes, written by the
 //             density pass: (x, y, z, 1/rho) and (velocity with the pending
@@ -351,6 +356,9 @@ __global__ void __launch_bounds__(SPH_TILE) k_scatter(const DevScene* __restrict
 // post-integration velocities in V2 and its previous cells in okey: those
 // are gathered (the density pass applies the XSPH update); otherwise V0.
 // ---------------------------------------------------------------------------
+// Where slot f's x lies in the per-axis copies (its y 4, its z 8 floats further).
+__device__ __forceinline__ size_t axes_index(uint32_t f) { return 12 * (size_t)(f / 4u) + (f & 3u); }
+
 __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevScene* __restrict__ scenes,
                                                           const uint4* __restrict__ tiles,
                                                           const uint32_t* __restrict__ start,
@@ -362,7 +370,7 @@ __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevScene* __rest
                                                           const float4* __restrict__ V2,
                                                           const uint32_t* __restrict__ okey,
                                                           const uint32_t* __restrict__ pend,
-                                                          float4* __restrict__ P1, float4* __restrict__ V1,
+                                                          float4* __restrict__ G, float* __restrict__ X,
                                                           float4* __restrict__ A1,
                                                           uint32_t* __restrict__ perm,
                                                           uint32_t* __restrict__ status) {
@@ -385,12 +393,16 @@ __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevScene* __rest
     for (uint32_t m = b; m < e; ++m) rank += (__ldg(tmp + m) < i) ? 1u : 0u;
     const uint32_t f = b + rank;
     perm[f] = i;
-    P1[f] = P0[i];
+    const float4 p = P0[i];
+    float* xf = X + axes_index(f);
+    xf[0] = p.x;
+    xf[4] = p.y;
+    xf[8] = p.z;
     float4 v = pending ? V2[i] : V0[i];
     // the cell of the last substep travels with the velocity (w lane) to the
     // density pass's XSPH update, which loads both together
     if (pending) v.w = __uint_as_float(__ldg(okey + i));
-    V1[f] = v;
+    st_float4_pair(G + 2 * (size_t)f, p, v);
     A1[f] = A0[i];
 }
 
@@ -414,16 +426,16 @@ __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevScene* __rest
 // word per row of up to 32 candidates (SPH_MASK_SKIN).
 //
 // Deferred XSPH.  For a scene whose previous substep ended without its XSPH
-// update (pend[scene] != 0), P1 holds that substep's post-integration
-// positions (w = its densities), V1 its post-integration velocities with, in
-// the w lane, the cells the particles were sorted into then (okey bits).  The reference's update
+// update (pend[scene] != 0), G holds that substep's post-integration
+// positions (w = its densities) and its post-integration velocities with, in
+// their w lane, the cells the particles were sorted into then (okey bits).  The reference's update
 // (correctVelocityXSPH, fluidphysics.cu:355-409) sums over pairs with
 // r^2 <= h^2 at these positions whose previous cells are adjacent (its cell
 // lists were those of the previous sort); every such pair is within h now, so
 // phase 2 meets all of them, and the previous-cell test keeps exactly the
 // reference's pairs.  The poly6 weight is the one the density sum uses.  The
 // corrected velocity goes to the record R, which the force pass reads; without
-// a pending update it is V1's.
+// a pending update it is G's.
 //
 // The record.  All that a later pass needs of a neighbour sits in 32 bytes,
 // one sector, fetched by one 256-bit load: position, velocity, q = 1/rho and
@@ -457,9 +469,9 @@ k_density(const DevParams* __restrict__ params,
                                                       const DevScene* __restrict__ scenes,
                                                       const uint4* __restrict__ tiles,
                                                       const uint32_t* __restrict__ start,
-                                                      const float4* __restrict__ P1, float* __restrict__ rho_out,
+                                                      const float4* __restrict__ G, const float* __restrict__ X,
+                                                      float* __restrict__ rho_out,
                                                       uint32_t* __restrict__ mask, size_t mask_stride,
-                                                      const float4* __restrict__ V1,
                                                       const uint32_t* __restrict__ pend, float4* __restrict__ R,
                                                       uint32_t* __restrict__ nbr_out, uint32_t ntiles,
                                                       uint32_t* __restrict__ tile_ctr,
@@ -478,15 +490,16 @@ k_density(const DevParams* __restrict__ params,
     const uint32_t k = t.y + li;
     const DevScene sc = scenes[t.x];
     const DevParams& pp = params[t.x];
-    float4 p = make_float4(0.f, 0.f, 0.f, 0.f), vi = p;
-    if (act) {
-        p = P1[k];
-        vi = V1[k];
-    }
-    const int3 g = grid_of(pp, p.x, p.y, p.z);
+    // phase 1 needs the position alone; the rest of the particle's state is
+    // loaded after it (registers)
+    const float* xk = X + axes_index(k);
+    const float px = act ? xk[0] : 0.f, py = act ? xk[4] : 0.f, pz = act ? xk[8] : 0.f;
+    const int3 g = grid_of(pp, px, py, pz);
     const bool work = act && grid_inside(pp, g);
+    float4 p, vi;
     if (act && !work) {
         if (part == 0u) {
+            ld_float4_pair(G + 2 * (size_t)k, p, vi);
             rho_out[k] = 0.f;
             st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, 0.f), make_float4(vi.x, vi.y, vi.z, 0.f));
             if (nbr_out) nbr_out[k] = 0;
@@ -502,35 +515,40 @@ k_density(const DevParams* __restrict__ params,
     const uint32_t rs = blockDim.x;
     uint8_t* list = reinterpret_cast<uint8_t*>(s_list + SPH_NBR_ROWS * rs + threadIdx.x * SPH_NBR_LIST_WORDS);
     NbrHeader hd;
+    constexpr uint32_t kCap = SKIN ? SPH_NBR_CAP_SKIN : SPH_NBR_CAP;
 
     // ---- phase 1: distance test of every candidate ----
-    // A candidate's bit is the sign of h^2 - r^2 (set outside; the sign of a
-    // rounded difference is that of the exact one, so the test is r^2 <= h^2
-    // to the bit), shifted into the word: the first candidate of a chunk ends
-    // in its highest bit.
-    auto visit = [&](const float4& q, uint32_t& dm, uint32_t& sm) {
-        const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-        const float rr = dot3(dx, dy, dz, dx, dy, dz);
-        dm = __funnelshift_l(__float_as_uint(h2 - rr), dm, 1);
-        if (SKIN) sm = __funnelshift_l(__float_as_uint(skin2 - rr), sm, 1);
+    // Four candidates at a time from the per-axis copies, aligned to four
+    // slots (the up to three before a row's start and after its end are tested
+    // too and masked out: no loop for the ragged ends), with the packed FP32
+    // instructions of sm_100-class GPUs (add/mul/fma.rn.f32x2): each component
+    // is rounded exactly as the scalar operation, so r^2 (dot3's fusion order)
+    // is the same to the bit.  Two neighbouring floats of one axis are the
+    // register pair that these instructions take; positions of four floats
+    // each would be taken apart with two moves per pair and axis, and cost
+    // 64 instead of 48 bytes of L1 bandwidth, the other limit of this pass
+    // (238 -> 206 us on the 1M dam break, 1.80 -> 1.55 ms on the 8M scene, the
+    // sort 2 us more for the copies).
+    // A candidate's bit is the sign of r^2 - h2n, h2n the float after h^2 (the
+    // sign of a rounded difference is that of the exact one, so the test is
+    // r^2 <= h^2 to the bit), shifted into the word: the first candidate of a
+    // chunk ends in its highest bit.
+    const float2 mx = make_float2(-px, -px), my = make_float2(-py, -py), mz = make_float2(-pz, -pz);
+    const float nh = -__uint_as_float(__float_as_uint(h2) + 1u), ns = -__uint_as_float(__float_as_uint(skin2) + 1u);
+    const float2 nh2 = make_float2(nh, nh), ns2 = make_float2(ns, ns);
+    auto shift_in = [](const float2& x, uint32_t& m) {
+        m = __funnelshift_l(__float_as_uint(x.x), m, 1);
+        m = __funnelshift_l(__float_as_uint(x.y), m, 1);
     };
-    // Two candidates at once with the packed FP32 instructions of sm_100-class
-    // GPUs (add/mul/fma.rn.f32x2): each component is rounded exactly as the
-    // scalar operation, so r^2 (dot3's fusion order) is the same to the bit.
-    const float2 px2 = make_float2(p.x, p.x), py2 = make_float2(p.y, p.y), pz2 = make_float2(p.z, p.z);
-    const float2 h22 = make_float2(h2, h2);
-    auto visit2 = [&](const float4& q0, const float4& q1, uint32_t& dm, uint32_t& sm) {
-        const float2 dx = __fadd2_rn(px2, make_float2(-q0.x, -q1.x));
-        const float2 dy = __fadd2_rn(py2, make_float2(-q0.y, -q1.y));
-        const float2 dz = __fadd2_rn(pz2, make_float2(-q0.z, -q1.z));
+    auto visit2 = [&](const float2& x, const float2& y, const float2& z, uint32_t& dm, uint32_t& sm) {
+        const float2 dx = __fadd2_rn(x, mx), dy = __fadd2_rn(y, my), dz = __fadd2_rn(z, mz);
         const float2 rr = __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
-        const float2 x = __fadd2_rn(h22, make_float2(-rr.x, -rr.y));
-        dm = __funnelshift_l(__float_as_uint(x.x), dm, 1);
-        dm = __funnelshift_l(__float_as_uint(x.y), dm, 1);
-        if (SKIN) {
-            sm = __funnelshift_l(__float_as_uint(skin2 - rr.x), sm, 1);
-            sm = __funnelshift_l(__float_as_uint(skin2 - rr.y), sm, 1);
-        }
+        shift_in(__fadd2_rn(rr, nh2), dm);
+        if (SKIN) shift_in(__fadd2_rn(rr, ns2), sm);
+    };
+    auto visit4 = [&](const float4& x, const float4& y, const float4& z, uint32_t& dm, uint32_t& sm) {
+        visit2(make_float2(x.x, x.y), make_float2(y.x, y.y), make_float2(z.x, z.y), dm, sm);
+        visit2(make_float2(x.z, x.w), make_float2(y.z, y.w), make_float2(z.z, z.w), dm, sm);
     };
     // The row ranges of this thread, loaded together (18 independent loads):
     // starts into the row table, lengths (at most 255 kept: a longer row is
@@ -561,37 +579,35 @@ k_density(const DevParams* __restrict__ params,
             break;
         }
         bool first = true;
-        uint32_t c0 = 0u;   // offset of the chunk in the row
+        const uint32_t mis = jb0 & 3u, alen = len + mis;   // from the aligned slot on
+        uint32_t c0 = 0u, skw = 0u;                        // offset of the chunk there
         do {
-            const uint32_t cb = jb0 + c0, clen = min(len - c0, 32u), ce = cb + clen;
+            const uint32_t cb = jb0 - mis + c0, clen = min(alen - c0, 32u);
+            const float4* xp = reinterpret_cast<const float4*>(X) + 3 * (size_t)(cb / 4u);
             uint32_t dm = 0u, sm = 0u;
-            uint32_t jj = cb;
-            // from an even slot on, two candidates per 256-bit load
-            if ((jj & 1u) != 0u) {
-                visit(__ldg(P1 + jj), dm, sm);
-                ++jj;
+            const uint32_t nq = (clen + 3u) / 4u;
+            uint32_t q = 0u;
+            for (; q + 2u <= nq; q += 2u) {
+                const float4 x0 = __ldg(xp), y0 = __ldg(xp + 1), z0 = __ldg(xp + 2);
+                const float4 x1 = __ldg(xp + 3), y1 = __ldg(xp + 4), z1 = __ldg(xp + 5);
+                xp += 6;
+                visit4(x0, y0, z0, dm, sm);
+                visit4(x1, y1, z1, dm, sm);
             }
-            for (; jj + 4u <= ce; jj += 4u) {
-                float4 q0, q1, q2, q3;
-                ld_float4_pair(P1 + jj, q0, q1);
-                ld_float4_pair(P1 + jj + 2u, q2, q3);
-                visit2(q0, q1, dm, sm);
-                visit2(q2, q3, dm, sm);
-            }
-            if (jj + 2u <= ce) {
-                float4 q0, q1;
-                ld_float4_pair(P1 + jj, q0, q1);
-                visit2(q0, q1, dm, sm);
-                jj += 2u;
-            }
-            if (jj < ce) visit(__ldg(P1 + jj), dm, sm);
-            // candidate cb + b in bit 31 - b, the particle itself left out
+            if (q < nq) visit4(__ldg(xp), __ldg(xp + 1), __ldg(xp + 2), dm, sm);
+            // candidate cb + b in bit 31 - b, those outside the row and the
+            // particle itself left out
             const uint32_t so = k - cb;
-            const uint32_t notself = (so < 32u) ? ~(0x80000000u >> so) : ~0u;
-            uint32_t bits = (~dm << (32u - clen)) & notself;
-            if (SKIN && len <= 32u)
-                mask[(size_t)(SPH_MASK_SKIN + rr) * mask_stride + k] = __brev((~sm << (32u - clen)) & notself);
-            if (hd.n + (uint32_t)__popc(bits) > SPH_NBR_CAP) hd.over = true;
+            uint32_t in = ~0u << (32u - clen);
+            if (c0 == 0u) in &= ~0u >> mis;
+            if (so < 32u) in &= ~(0x80000000u >> so);
+            uint32_t bits = (dm << (32u - 4u * nq)) & in;
+            if (SKIN) {
+                const uint32_t v = __brev((sm << (32u - 4u * nq)) & in);
+                if (c0 == 0u) skw = v >> mis;
+                else if (mis != 0u) skw |= v << (32u - mis);   // (rows of up to 32: at most two chunks)
+            }
+            if (hd.n + (uint32_t)__popc(bits) > kCap) hd.over = true;
             if (bits && !hd.over) {
                 int b = __clz(bits);
                 if (first) {
@@ -599,16 +615,17 @@ k_density(const DevParams* __restrict__ params,
                     rows[nrows++ * rs] = jb0;
                     hd.live |= 1u << (r0 + rr);
                     bits &= ~(0x80000000u >> b);
-                    list[hd.n++] = (uint8_t)(c0 + b + SPH_NBR_NEW_ROW);
+                    list[hd.n++] = (uint8_t)(c0 - mis + b + SPH_NBR_NEW_ROW);
                 }
                 while (bits) {
                     b = __clz(bits);
                     bits &= ~(0x80000000u >> b);
-                    list[hd.n++] = (uint8_t)(c0 + b);
+                    list[hd.n++] = (uint8_t)(c0 - mis + b);
                 }
             }
             c0 += 32u;
-        } while (c0 < len && (SKIN || !hd.over));
+        } while (c0 < alen && (SKIN || !hd.over));
+        if (SKIN && len <= 32u) mask[(size_t)(SPH_MASK_SKIN + rr) * mask_stride + k] = skw;
         if (!SKIN && hd.over) break;
     }
 
@@ -624,7 +641,7 @@ k_density(const DevParams* __restrict__ params,
             const NbrHeader ho(w & ~(15u << 9));
             const uint8_t* from = reinterpret_cast<const uint8_t*>(
                 s_list + SPH_NBR_ROWS * rs + (li + o) * SPH_NBR_LIST_WORDS);
-            if (hd.n + ho.n > SPH_NBR_CAP) {
+            if (hd.n + ho.n > kCap) {
                 hd.over = true;
                 break;
             }
@@ -640,6 +657,7 @@ k_density(const DevParams* __restrict__ params,
     mask[k] = hd.pack();
 
     // ---- phase 2: the density pairs, in candidate order ----
+    ld_float4_pair(G + 2 * (size_t)k, p, vi);
     const float h = pp.h, mass = pp.mass, c6 = pp.poly6, two_m = pp.two_mass;
     float sum = 0.0f;
     uint32_t cnt = 0;
@@ -650,14 +668,12 @@ k_density(const DevParams* __restrict__ params,
     float2 axy = make_float2(0.f, 0.f);
     float az = 0.f;
     const float2 mvixy = make_float2(-vi.x, -vi.y);
-    // the pair's XSPH operands (velocity, and its last cell in the w lane) are
-    // loaded with its position, before any test, so that the latencies overlap
+    // position with the previous density, and the XSPH operands (velocity, and
+    // the last cell in the w lane): one 256-bit load
     struct Nbr { float4 q, v; };
     auto load = [&](uint32_t j) {
         Nbr n;
-        n.q = __ldg(P1 + j);
-        n.v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (xs) n.v = __ldg(V1 + j);
+        ld_float4_pair(G + 2 * (size_t)j, n.q, n.v);
         return n;
     };
     auto use = [&](const Nbr& n) {
@@ -1022,7 +1038,7 @@ __global__ void k_xsph(const DevParams* __restrict__ params,
                                                    const DevScene* __restrict__ scenes,
                                                    const uint4* __restrict__ tiles,
                                                    const uint32_t* __restrict__ start,
-                                                   const float4* __restrict__ P1,
+                                                   const float4* __restrict__ G,
                                                    const float4* __restrict__ P0,
                                                    const float4* __restrict__ V2,
                                                    const uint32_t* __restrict__ mask, size_t mask_stride,
@@ -1039,7 +1055,7 @@ __global__ void k_xsph(const DevParams* __restrict__ params,
     if (pp.flags & SPH_FLAG_DEFER_XSPH) return;   // the next density pass applies it
     if (threadIdx.x == 0) pend[t.x] = 0u;         // the update is applied here
     const float4 vi = V2[k];
-    const float4 old = P1[k];   // the cell this particle was sorted into
+    const float4 old = G[2 * (size_t)k];   // the cell this particle was sorted into
     const int3 g = grid_of(pp, old.x, old.y, old.z);
     if (!grid_inside(pp, g)) {
         V0[k] = vi;
@@ -1107,15 +1123,14 @@ __global__ void __launch_bounds__(SPH_TILE) k_unsort_vel(const uint4* __restrict
 
 // ---------------------------------------------------------------------------
 // Undo a force pass run ahead of the step that takes it: the state before it
-// is what the prefix gathered (P1, A1; V1 holds the post-integration
+// is what the prefix gathered (G, A1; G holds the post-integration
 // velocities of a scene whose XSPH update is pending, with its previous cells
 // in the w lane), scattered back to the slots it came from.  The force pass
 // writes no array the prefix wrote, so the prefix stays valid.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(SPH_TILE) k_undo_ahead(const uint4* __restrict__ tiles,
                                                          const uint32_t* __restrict__ perm,
-                                                         const float4* __restrict__ P1,
-                                                         const float4* __restrict__ V1,
+                                                         const float4* __restrict__ G,
                                                          const float4* __restrict__ A1, float4* __restrict__ P0,
                                                          float4* __restrict__ V2, float4* __restrict__ A0,
                                                          uint32_t* __restrict__ okey) {
@@ -1123,8 +1138,9 @@ __global__ void __launch_bounds__(SPH_TILE) k_undo_ahead(const uint4* __restrict
     if (threadIdx.x >= t.z) return;
     const uint32_t f = t.y + threadIdx.x;
     const uint32_t i = __ldg(perm + f);
-    const float4 v = V1[f];
-    P0[i] = P1[f];
+    float4 p, v;
+    ld_float4_pair(G + 2 * (size_t)f, p, v);
+    P0[i] = p;
     V2[i] = make_float4(v.x, v.y, v.z, 0.f);
     A0[i] = A1[f];
     okey[i] = __float_as_uint(v.w);
@@ -1199,14 +1215,14 @@ __global__ void k_lattice(LatticeSpec spec, uint32_t base, float4* __restrict__ 
 
 // Sorted hash for the debug tap: key of the particle now at each slot, with
 // the NULL bucket reported as NULL_HASH (m_Hash after the sort).
-__global__ void k_sorted_keys(const DevParams* __restrict__ params, const float4* __restrict__ P1, uint32_t n,
+__global__ void k_sorted_keys(const DevParams* __restrict__ params, const float4* __restrict__ G, uint32_t n,
                               uint32_t base, uint32_t* __restrict__ out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     // the cell of the position gathered into slot i by the last sort: the key
     // it was sorted by (the key array itself may already hold the next
     // substep's keys, written by the force pass)
-    const float4 p = P1[base + i];
+    const float4 p = G[2 * (size_t)(base + i)];
     const uint32_t k = cell_of(*params, p.x, p.y, p.z);
     out[i] = (k == params->ncells) ? SPH_NULL_HASH : k;
 }
@@ -1303,10 +1319,16 @@ cudaError_t launch_scan_raw(const uint32_t* counts, uint32_t n, uint32_t* tile_s
     k_scan_down<<<nt, SCAN_THREADS, 0, st>>>(counts, n, tile_sums, starts);
     return cudaGetLastError();
 }
+// The per-axis positions lie in three neighbour-word rows that the density pass
+// does not write: past the list, or where a skin pass needs the rows after it, in
+// the list's last three (which is then shorter).
+static float* axes(const StepArgs& a) {
+    return reinterpret_cast<float*>(a.mask + (a.skin_masks ? SPH_AXIS_ROWS_SKIN : SPH_MASK_SKIN) * a.mask_stride);
+}
 cudaError_t launch_sort(const StepArgs& a, cudaStream_t st) {
     k_scatter<<<a.ntiles, a.block, 0, st>>>(a.scenes, a.tiles, a.start, a.key, a.slot, a.tmp, a.status);
     k_rank_gather<<<a.ntiles, a.block, 0, st>>>(a.scenes, a.tiles, a.start, a.key, a.tmp, a.P0, a.V0, a.A0, a.V2,
-                                                a.okey, a.pend, a.P1, a.V1, a.A1, a.perm, a.status);
+                                                a.okey, a.pend, a.G, axes(a), a.A1, a.perm, a.status);
     return cudaGetLastError();
 }
 bool density_split(const StepArgs& a) {
@@ -1317,13 +1339,13 @@ cudaError_t launch_density(const StepArgs& a, cudaStream_t st) {
     const size_t smem = (size_t)SPH_NBR_SMEM_WORDS * a.block * sizeof(uint32_t);
     if (density_split(a)) {
         k_density<false, true><<<a.ntiles, 3u * a.block, 3u * smem, st>>>(
-            a.params, a.scenes, a.tiles, a.start, a.P1, a.rho, a.mask, a.mask_stride, a.V1, a.pend, a.R, a.dbg_nbr,
+            a.params, a.scenes, a.tiles, a.start, a.G, axes(a), a.rho, a.mask, a.mask_stride, a.pend, a.R, a.dbg_nbr,
             a.ntiles, nullptr, a.status);
         return cudaGetLastError();
     }
     auto kern = a.skin_masks ? k_density<true> : k_density<false>;
-    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.P1, a.rho, a.mask, a.mask_stride,
-                                            a.V1, a.pend, a.R, a.dbg_nbr, a.ntiles, ctr(a, 0), a.status);
+    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.G, axes(a), a.rho, a.mask, a.mask_stride,
+                                            a.pend, a.R, a.dbg_nbr, a.ntiles, ctr(a, 0), a.status);
     return cudaGetLastError();
 }
 cudaError_t launch_unsort_vel(const StepArgs& a, uint32_t first_tile, uint32_t ntiles, uint32_t base, uint32_t n,
@@ -1335,7 +1357,7 @@ cudaError_t launch_unsort_vel(const StepArgs& a, uint32_t first_tile, uint32_t n
 }
 cudaError_t launch_undo_ahead(const StepArgs& a, uint32_t first_tile, uint32_t ntiles, cudaStream_t st) {
     if (ntiles == 0) return cudaSuccess;
-    k_undo_ahead<<<ntiles, a.block, 0, st>>>(a.tiles + first_tile, a.perm, a.P1, a.V1, a.A1, a.P0, a.V2, a.A0,
+    k_undo_ahead<<<ntiles, a.block, 0, st>>>(a.tiles + first_tile, a.perm, a.G, a.A1, a.P0, a.V2, a.A0,
                                              a.okey);
     return cudaGetLastError();
 }
@@ -1357,7 +1379,7 @@ cudaError_t launch_force(const StepArgs& a, cudaStream_t st) {
 }
 cudaError_t launch_xsph(const StepArgs& a, cudaStream_t st) {
     auto kern = (a.variant & SPH_VARIANT_XSPH_ROWS) ? k_xsph<1> : k_xsph<0>;
-    kern<<<a.grid_nbr, a.block, 0, st>>>(a.params, a.scenes, a.tiles, a.start, a.P1, a.P0, a.V2, a.mask,
+    kern<<<a.grid_nbr, a.block, 0, st>>>(a.params, a.scenes, a.tiles, a.start, a.G, a.P0, a.V2, a.mask,
                                          a.mask_stride, a.maxdisp, a.V0, a.pend, a.ntiles, ctr(a, 3), a.status);
     return cudaGetLastError();
 }
@@ -1385,10 +1407,10 @@ cudaError_t launch_lattice(const LatticeSpec& spec, uint32_t base, float4* P0, f
     k_lattice<<<(n + 255) / 256, 256, 0, st>>>(spec, base, P0, V0, A0, rho);
     return cudaGetLastError();
 }
-cudaError_t launch_sorted_keys(const DevParams* params, const float4* P1, uint32_t n, uint32_t base,
+cudaError_t launch_sorted_keys(const DevParams* params, const float4* G, uint32_t n, uint32_t base,
                                uint32_t* out, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    k_sorted_keys<<<(n + 255) / 256, 256, 0, st>>>(params, P1, n, base, out);
+    k_sorted_keys<<<(n + 255) / 256, 256, 0, st>>>(params, G, n, base, out);
     return cudaGetLastError();
 }
 

@@ -15,11 +15,11 @@ struct StepArgs {
     uint32_t particles;        // particles the tiles hold
     uint32_t total_cells;      // packed cell arena size including NULL buckets
     float4 *P0, *V0, *A0;      // state
-    float4 *P1, *V1, *A1;      // cell-ordered state
+    float4 *G, *A1;            // cell-ordered state (G: position and velocity, two per slot)
     float4 *V2;                // post-integration velocity (before XSPH)
     float4 *R;                 // neighbour records, two per slot: (x, y, z, 1/rho), (velocity with any pending
                                // XSPH update applied, (rho/rho0)^gamma)
-    uint32_t *okey;            // each slot's cell in the last substep (packed; gathered into V1.w)
+    uint32_t *okey;            // each slot's cell in the last substep (packed; gathered into G's velocity w)
     uint32_t *pend;            // per scene: its last XSPH update is pending
     float *rho;                // density per sorted slot
     float4 *N;                 // normals
@@ -33,7 +33,7 @@ struct StepArgs {
     uint32_t *tmp;             // scatter list of the sort; shares the mask words, which the density pass writes later
     uint32_t *status;
     uint32_t *mask;            // SPH_MASK_ROWS neighbour words per slot, word m at mask[m*mask_stride + slot]
-    size_t mask_stride;
+    size_t mask_stride;        // (a multiple of 4: rows are read four slots at a time)
     uint32_t *maxdisp;         // largest (displacement/h)^2 of the substep, float bits
     uint32_t block;            // threads per block = particles per tile
     uint32_t grid_nbr;         // blocks of the neighbour passes (ntiles, or the persistent grid)
@@ -101,7 +101,7 @@ cudaError_t launch_pack(const float4* P0, const float4* V0, uint32_t n, uint32_t
                         float* pos, float* colour, float* vel, cudaStream_t st);
 cudaError_t launch_lattice(const LatticeSpec& spec, uint32_t base, float4* P0, float4* V0, float4* A0, float* rho,
                            cudaStream_t st);
-cudaError_t launch_sorted_keys(const DevParams* params, const float4* P1, uint32_t n, uint32_t base,
+cudaError_t launch_sorted_keys(const DevParams* params, const float4* G, uint32_t n, uint32_t base,
                                uint32_t* out, cudaStream_t st);
 
 }  // namespace sph

@@ -58,9 +58,12 @@ struct DevParams {
 // words, used only when some scene runs a per-substep XSPH pass.
 #define SPH_NBR_LIST       1u    // first list row; row 0 is the header
 #define SPH_NBR_LIST_WORDS 17u   // (odd: the threads' lists in shared memory start in different banks)
-#define SPH_MASK_SKIN      18u   // 9 rows: candidates within the skin radius (rows of <= 32)
+#define SPH_MASK_SKIN      18u   // 9 rows: candidates within the skin radius (rows of <= 32); without a skin pass
+                                 // the first three hold the per-axis positions of the candidate scan
+#define SPH_AXIS_ROWS_SKIN 15u   // with one, these three do
 #define SPH_MASK_ROWS      27u
 #define SPH_NBR_CAP        68u   // listed neighbours: four to a word
+#define SPH_NBR_CAP_SKIN   56u   // with a skin pass: the words before SPH_AXIS_ROWS_SKIN
 #define SPH_NBR_NEW_ROW    128u  // added to a row's first neighbour
 #define SPH_NBR_MAX_ROW    128u  // longest row whose offsets fit below that
 #define SPH_NBR_ROWS       10u   // row starts kept per thread: nine and one that is read ahead
