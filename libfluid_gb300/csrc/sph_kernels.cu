@@ -658,7 +658,9 @@ k_density(const DevParams* __restrict__ params,
 
     // ---- phase 2: the density pairs, in candidate order ----
     ld_float4_pair(G + 2 * (size_t)k, p, vi);
-    const float h = pp.h, mass = pp.mass, c6 = pp.poly6, two_m = pp.two_mass;
+    // Factors that are the same for every pair are left to the end: the sums
+    // hold (h^2 - r^2)^3, and for XSPH that over the densities' sum.
+    const float h = pp.h;
     float sum = 0.0f;
     uint32_t cnt = 0;
     // deferred XSPH of the previous substep (only for particles that had a cell then)
@@ -684,15 +686,14 @@ k_density(const DevParams* __restrict__ params,
         const float rr = dot3(dx, dy, dz, dx, dy, dz);
         // true for every listed neighbour of finite position; the test matters in the tail
         if (rr <= h2) {
-            const float rd = sqrtf(rr);
-            const float x = fmaf(-rd, rd, h2);
-            const float w = (rd >= h) ? 0.0f : c6 * (x * x * x);
-            sum = fmaf(mass, w, sum);
+            const float x = h2_minus_r2(rr, h, h2);
+            const float w = x * x * x;
+            sum += w;
             cnt++;
             if (xs) {
                 const float rs = p.w + q.w;   // the previous substep's densities
                 if (rs > eps && cells_adjacent_fast(oi, oj)) {
-                    const float coeff = w * __fdividef(two_m, rs);
+                    const float coeff = w * rcp_approx(rs);
                     axy = __ffma2_rn(make_float2(coeff, coeff), __fadd2_rn(make_float2(vj.x, vj.y), mvixy), axy);
                     az = fmaf(coeff, vj.z - vi.z, az);
                 }
@@ -710,6 +711,7 @@ k_density(const DevParams* __restrict__ params,
     if (hd.over)
         walk_tail(pp, start, sc.cell_base, delta, g, hd.n ? last + 1u : 0u,
                   [&](uint32_t j) { if (j != k) use(load(j)); });
+    sum = (pp.mass * pp.poly6) * sum;
     const float d = fabsf(sdf(pp, p.x, p.y, p.z));
     float corr = sum;
     if (d < pp.h) corr = fmaf(pp.rest_density, 1.0f - boundary_density(pp, d), corr);
@@ -719,9 +721,10 @@ k_density(const DevParams* __restrict__ params,
     const float e = (corr == 0.0f) ? -0.0f : powf(ratio, pp.gamma) + 0.0f;
     rho_out[k] = rho;
     if (xs) {
-        vi.x = fmaf(pp.xsph, axy.x, vi.x);
-        vi.y = fmaf(pp.xsph, axy.y, vi.y);
-        vi.z = fmaf(pp.xsph, az, vi.z);
+        const float cx = pp.xsph * (pp.poly6 * pp.two_mass);
+        vi.x = fmaf(cx, axy.x, vi.x);
+        vi.y = fmaf(cx, axy.y, vi.y);
+        vi.z = fmaf(cx, az, vi.z);
     }
     // a density the later passes skip as a neighbour's (rho <= eps) is marked by 0
     st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, rho > eps ? 1.0f / rho : 0.0f),
@@ -764,9 +767,8 @@ __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restric
     float sz = 0.f;
     const float2 pxy = make_float2(p.x, p.y);
     // m gradPoly6(r) rvec / (rho_j r) = m c (h^2 - r^2)^2 rvec / rho_j: the
-    // factor r of gradPoly6 cancels the 1/r; h^2 - r^2 is formed from the
-    // rounded root r as gradPoly6 forms it (it cancels near r = h)
-    const float mc = pp.mass * pp.grad_poly6;
+    // factor r of gradPoly6 cancels the 1/r; m c, the same for every pair, is
+    // left to the end
     const float h2 = pp.h2, eps = pp.eps, h = pp.h;
     extern __shared__ uint32_t s_rows[];
     walk_neighbours<kNormalsDepth>(
@@ -777,14 +779,14 @@ __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restric
             const float rx = rxy.x, ry = rxy.y, rz = p.z - q.z;
             const float r2 = dot3(rx, ry, rz, rx, ry, rz);
             if (r2 <= h2 && r2 > eps && q.w > 0.0f) {
-                const float r = sqrtf(r2);
-                const float x = fmaf(-r, r, h2);
-                const float s = (r >= h) ? 0.0f : mc * (x * x) * q.w;
+                const float x = h2_minus_r2(r2, h, h2);
+                const float s = (x * x) * q.w;
                 sxy = __ffma2_rn(make_float2(s, s), rxy, sxy);
                 sz = fmaf(s, rz, sz);
             }
         });
-    N[k] = make_float4(pp.h * sxy.x, pp.h * sxy.y, pp.h * sz, 0.f);
+    const float hc = pp.h * (pp.mass * pp.grad_poly6);
+    N[k] = make_float4(hc * sxy.x, hc * sxy.y, hc * sz, 0.f);
   });
 }
 
