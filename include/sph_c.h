@@ -222,16 +222,16 @@ int sph_debug_scan_fault(sph_system* s, uint32_t spin_limit, int withhold_first_
  * neighbour-mask skin in units of h, in (0, 1]; variant: SPH_VARIANT_* bits
  * choosing how the neighbour walks are scheduled.  Defaults: tile 128,
  * persistent 0, skin 0.1, variant 63 (per-row XSPH walk, 64-register force
- * build, the density scan split over three threads per particle in launches of
- * at most 49,152 particles).  Bits without an effect are accepted. */
-#define SPH_VARIANT_DENSITY_ROWS   0x1u  /* density: with DENSITY_SPLIT, the split scan */
+ * build, several lanes per particle in launches of few particles).  Bits
+ * without an effect are accepted. */
+#define SPH_VARIANT_DENSITY_ROWS   0x1u  /* no effect: one candidate scan is left */
 #define SPH_VARIANT_XSPH_ROWS      0x2u  /* XSPH: one loop per cell row */
 #define SPH_VARIANT_FORCE_OCC      0x4u  /* force: 64-register build, more resident warps */
 #define SPH_VARIANT_FORCE_TABLE    0x8u  /* no effect: forces and normals walk the neighbour list */
 #define SPH_VARIANT_NORMALS_TABLE  0x10u /* no effect */
-#define SPH_VARIANT_DENSITY_SPLIT  0x20u /* density: three threads per particle share the candidate
-                                            scan (with DENSITY_ROWS, one block per tile, no skin
-                                            words; launches of at most 49,152 particles) */
+#define SPH_VARIANT_DENSITY_SPLIT  0x20u /* neighbour passes: eight or four lanes per particle in launches of
+                                            at most 14,336 or 34,816 particles (40,960 or 61,440 of crowded
+                                            scenes), one block per tile */
 typedef struct sph_exec_config {
     uint32_t tile;
     uint32_t persistent;

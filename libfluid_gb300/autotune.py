@@ -31,16 +31,16 @@ TILES = (128, 256)
 PERSISTENT = (0, 2, 4)
 SKINS = (0.1, 0.15, 0.2, 0.3)
 VARIANTS = tuple(range(64))
-# Launches of at most this many particles take the split density scan
-# (SPH_VARIANT_DENSITY_SPLIT, bit 0x20; SPH_DENSITY_SPLIT_MAX in
+# Launches of at most this many particles run several lanes per particle in the
+# neighbour passes (SPH_VARIANT_DENSITY_SPLIT, bit 0x20; SPH_DENSITY_SPLIT_MAX in
 # csrc/sph_types.h); above it the bit changes nothing and is not swept.
-DENSITY_SPLIT_MAX = 49152
+DENSITY_SPLIT_MAX = 34816
 
 
 def variants_for(particles: int, persistent: int) -> tuple:
     """The variant values worth timing for a launch of `particles` particles:
-    all 64 where the split density scan can apply (one block per tile and a
-    small enough launch), else the 32 without its bit, which would change
+    all 64 where several lanes per particle can apply (one block per tile and
+    a small enough launch), else the 32 without that bit, which would change
     nothing there."""
     split = particles <= DENSITY_SPLIT_MAX and persistent == 0
     return VARIANTS if split else VARIANTS[:32]

@@ -511,6 +511,11 @@ StepArgs Engine::args() const {
     a.tiles = d_tiles_;
     a.ntiles = ntiles_;
     a.particles = (uint32_t)total_particles();
+    // neighbours at rest density: the particles in a sphere of radius h
+    double nbrs = 0.0;
+    for (const auto& s : scenes_)
+        nbrs += (double)s.n * (4.0 / 3.0 * 3.14159265 * s.dp.h * s.dp.h * s.dp.h * s.dp.rest_density / s.dp.mass);
+    a.crowded = nbrs >= (double)SPH_CROWDED_NBRS * a.particles ? 1u : 0u;
     a.total_cells = total_cells_;
     a.P0 = P0_; a.V0 = V0_; a.A0 = A0_;
     a.G = G_; a.A1 = A1_;

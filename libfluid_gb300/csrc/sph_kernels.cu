@@ -457,14 +457,80 @@ __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevScene* __rest
 // us at 250k), one in the force pass (two measured the same at 64 registers,
 // where they spill, and 5% slower at 80).
 constexpr int kDensityDepth = 2, kNormalsDepth = 2, kForceDepth = 1;
-// SPLIT (no SKIN, one block per tile): three threads per particle share phase
-// 1, thread q of the particle taking rows 3q..3q+2 and a list of its own;
-// after a barrier the first thread appends the others' lists to its own, which
-// gives the list one thread would have made, and runs phase 2.  A small
-// scene's pass lasts as long as one thread's walk, and the split shortens the
-// candidate scan's share of it threefold.
-template <bool SKIN, bool SPLIT = false>
-__global__ void __launch_bounds__(SPLIT ? 3 * SPH_TILE : SPH_TILE, SPLIT ? 1 : DENSITY_MINB)
+// Phase 1's distance test: four candidates at a time from the per-axis copies,
+// aligned to four slots (the up to three before a row's start and after its end
+// are tested too and masked out: no loop for the ragged ends), with the packed
+// FP32 instructions of sm_100-class GPUs (add/mul/fma.rn.f32x2): each component
+// is rounded exactly as the scalar operation, so r^2 (dot3's fusion order) is
+// the same to the bit.  Two neighbouring floats of one axis are the register
+// pair that these instructions take; positions of four floats each would be
+// taken apart with two moves per pair and axis, and cost 64 instead of 48 bytes
+// of L1 bandwidth, the other limit of this pass (238 -> 206 us on the 1M dam
+// break, 1.80 -> 1.55 ms on the 8M scene, the sort 2 us more for the copies).
+// A candidate's bit is the sign of r^2 - h2n, h2n the float after h^2 (the sign
+// of a rounded difference is that of the exact one, so the test is r^2 <= h^2
+// to the bit), shifted into the word: the first candidate ends in its highest
+// bit.
+template <bool SKIN>
+struct CandidateScan {
+    float2 mx, my, mz, nh2, ns2;
+    __device__ __forceinline__ CandidateScan(float px, float py, float pz, float h2, float skin2)
+        : mx(make_float2(-px, -px)), my(make_float2(-py, -py)), mz(make_float2(-pz, -pz)) {
+        const float nh = -__uint_as_float(__float_as_uint(h2) + 1u), ns = -__uint_as_float(__float_as_uint(skin2) + 1u);
+        nh2 = make_float2(nh, nh);
+        ns2 = make_float2(ns, ns);
+    }
+    static __device__ __forceinline__ void shift_in(const float2& x, uint32_t& m) {
+        m = __funnelshift_l(__float_as_uint(x.x), m, 1);
+        m = __funnelshift_l(__float_as_uint(x.y), m, 1);
+    }
+    __device__ __forceinline__ void visit2(const float2& x, const float2& y, const float2& z, uint32_t& dm,
+                                           uint32_t& sm) const {
+        const float2 dx = __fadd2_rn(x, mx), dy = __fadd2_rn(y, my), dz = __fadd2_rn(z, mz);
+        const float2 rr = __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
+        shift_in(__fadd2_rn(rr, nh2), dm);
+        if (SKIN) shift_in(__fadd2_rn(rr, ns2), sm);
+    }
+    __device__ __forceinline__ void visit4(const float4& x, const float4& y, const float4& z, uint32_t& dm,
+                                           uint32_t& sm) const {
+        visit2(make_float2(x.x, x.y), make_float2(y.x, y.y), make_float2(z.x, z.y), dm, sm);
+        visit2(make_float2(x.z, x.w), make_float2(y.z, y.w), make_float2(z.z, z.w), dm, sm);
+    }
+};
+
+// A particle outside the grid: no density, its velocity kept.
+__device__ __forceinline__ void density_outside(uint32_t k, const float4& p, const float4& v, float* rho_out, float4* R,
+                                                uint32_t* nbr_out) {
+    rho_out[k] = 0.f;
+    st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, 0.f), make_float4(v.x, v.y, v.z, 0.f));
+    if (nbr_out) nbr_out[k] = 0;
+}
+// The density, its equation of state and the record of slot k from the sums of
+// (h^2 - r^2)^3 and, with xs, of XSPH's (ax, ay, az).
+__device__ __forceinline__ void density_finish(const DevParams& pp, uint32_t k, float sum, bool xs, float ax, float ay,
+                                               float az, const float4& p, float4 vi, float* rho_out, float4* R) {
+    sum = (pp.mass * pp.poly6) * sum;
+    const float d = fabsf(sdf(pp, p.x, p.y, p.z));
+    float corr = sum;
+    if (d < pp.h) corr = fmaf(pp.rest_density, 1.0f - boundary_density(pp, d), corr);
+    const float rho = (sum == 0.0f) ? pp.rest_density : corr;
+    const float ratio = corr * pp.inv_rest_density;
+    // no density at all (corr 0) has pressure 0: marked by -0
+    const float e = (corr == 0.0f) ? -0.0f : powf(ratio, pp.gamma) + 0.0f;
+    rho_out[k] = rho;
+    if (xs) {
+        const float cx = pp.xsph * (pp.poly6 * pp.two_mass);
+        vi.x = fmaf(cx, ax, vi.x);
+        vi.y = fmaf(cx, ay, vi.y);
+        vi.z = fmaf(cx, az, vi.z);
+    }
+    // a density the later passes skip as a neighbour's (rho <= eps) is marked by 0
+    st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, rho > pp.eps ? 1.0f / rho : 0.0f),
+                   make_float4(vi.x, vi.y, vi.z, e));
+}
+
+template <bool SKIN>
+__global__ void __launch_bounds__(SPH_TILE, DENSITY_MINB)
 k_density(const DevParams* __restrict__ params,
                                                       const DevScene* __restrict__ scenes,
                                                       const uint4* __restrict__ tiles,
@@ -476,41 +542,28 @@ k_density(const DevParams* __restrict__ params,
                                                       uint32_t* __restrict__ nbr_out, uint32_t ntiles,
                                                       uint32_t* __restrict__ tile_ctr,
                                                       const uint32_t* __restrict__ status) {
-  static_assert(!SPLIT || !SKIN, "the split scan writes no skin words");
   extern __shared__ uint32_t s_list[];
   if (step_failed(status)) return;
-  for_each_tile(tiles, ntiles, tile_ctr, [&](const uint4 t) {
-    // particle li of the tile; with SPLIT, part q of its phase 1.  Every
-    // thread of a split block reaches the barrier after phase 1.
-    const uint32_t ts = SPLIT ? blockDim.x / 3u : blockDim.x;
-    const uint32_t part = SPLIT ? threadIdx.x / ts : 0u;
-    const uint32_t li = SPLIT ? threadIdx.x - part * ts : threadIdx.x;
-    if (!SPLIT && li >= t.z) return;
-    const bool act = !SPLIT || li < t.z;
-    const uint32_t k = t.y + li;
+  for_each_tile<1>(tiles, ntiles, tile_ctr, [&](const uint4 t) {
+    if (threadIdx.x >= t.z) return;
+    const uint32_t k = t.y + threadIdx.x;
     const DevScene sc = scenes[t.x];
     const DevParams& pp = params[t.x];
     // phase 1 needs the position alone; the rest of the particle's state is
     // loaded after it (registers)
     const float* xk = X + axes_index(k);
-    const float px = act ? xk[0] : 0.f, py = act ? xk[4] : 0.f, pz = act ? xk[8] : 0.f;
+    const float px = xk[0], py = xk[4], pz = xk[8];
     const int3 g = grid_of(pp, px, py, pz);
-    const bool work = act && grid_inside(pp, g);
     float4 p, vi;
-    if (act && !work) {
-        if (part == 0u) {
-            ld_float4_pair(G + 2 * (size_t)k, p, vi);
-            rho_out[k] = 0.f;
-            st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, 0.f), make_float4(vi.x, vi.y, vi.z, 0.f));
-            if (nbr_out) nbr_out[k] = 0;
-        }
-        if (!SPLIT) return;
+    if (!grid_inside(pp, g)) {
+        ld_float4_pair(G + 2 * (size_t)k, p, vi);
+        density_outside(k, p, vi, rho_out, R, nbr_out);
+        return;
     }
     const uint32_t delta = sc.part_base - __ldg(start + sc.cell_base);
     // the skin-radius words serve only the per-substep XSPH pass
     const float h2 = pp.h2, skin2 = SKIN ? pp.skin2 : pp.h2, eps = pp.eps;
-    // row starts in a column per thread, list words in a row per thread; a
-    // split block has one set per thread
+    // row starts in a column per thread, list words in a row per thread
     uint32_t* rows = s_list + threadIdx.x;
     const uint32_t rs = blockDim.x;
     uint8_t* list = reinterpret_cast<uint8_t*>(s_list + SPH_NBR_ROWS * rs + threadIdx.x * SPH_NBR_LIST_WORDS);
@@ -518,48 +571,17 @@ k_density(const DevParams* __restrict__ params,
     constexpr uint32_t kCap = SKIN ? SPH_NBR_CAP_SKIN : SPH_NBR_CAP;
 
     // ---- phase 1: distance test of every candidate ----
-    // Four candidates at a time from the per-axis copies, aligned to four
-    // slots (the up to three before a row's start and after its end are tested
-    // too and masked out: no loop for the ragged ends), with the packed FP32
-    // instructions of sm_100-class GPUs (add/mul/fma.rn.f32x2): each component
-    // is rounded exactly as the scalar operation, so r^2 (dot3's fusion order)
-    // is the same to the bit.  Two neighbouring floats of one axis are the
-    // register pair that these instructions take; positions of four floats
-    // each would be taken apart with two moves per pair and axis, and cost
-    // 64 instead of 48 bytes of L1 bandwidth, the other limit of this pass
-    // (238 -> 206 us on the 1M dam break, 1.80 -> 1.55 ms on the 8M scene, the
-    // sort 2 us more for the copies).
-    // A candidate's bit is the sign of r^2 - h2n, h2n the float after h^2 (the
-    // sign of a rounded difference is that of the exact one, so the test is
-    // r^2 <= h^2 to the bit), shifted into the word: the first candidate of a
-    // chunk ends in its highest bit.
-    const float2 mx = make_float2(-px, -px), my = make_float2(-py, -py), mz = make_float2(-pz, -pz);
-    const float nh = -__uint_as_float(__float_as_uint(h2) + 1u), ns = -__uint_as_float(__float_as_uint(skin2) + 1u);
-    const float2 nh2 = make_float2(nh, nh), ns2 = make_float2(ns, ns);
-    auto shift_in = [](const float2& x, uint32_t& m) {
-        m = __funnelshift_l(__float_as_uint(x.x), m, 1);
-        m = __funnelshift_l(__float_as_uint(x.y), m, 1);
-    };
-    auto visit2 = [&](const float2& x, const float2& y, const float2& z, uint32_t& dm, uint32_t& sm) {
-        const float2 dx = __fadd2_rn(x, mx), dy = __fadd2_rn(y, my), dz = __fadd2_rn(z, mz);
-        const float2 rr = __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
-        shift_in(__fadd2_rn(rr, nh2), dm);
-        if (SKIN) shift_in(__fadd2_rn(rr, ns2), sm);
-    };
-    auto visit4 = [&](const float4& x, const float4& y, const float4& z, uint32_t& dm, uint32_t& sm) {
-        visit2(make_float2(x.x, x.y), make_float2(y.x, y.y), make_float2(z.x, z.y), dm, sm);
-        visit2(make_float2(x.z, x.w), make_float2(y.z, y.w), make_float2(z.z, z.w), dm, sm);
-    };
+    // (CandidateScan)
+    const CandidateScan<SKIN> scan(px, py, pz, h2, skin2);
     // The row ranges of this thread, loaded together (18 independent loads):
     // starts into the row table, lengths (at most 255 kept: a longer row is
     // cut short as any above 128 is) packed into bytes.
-    constexpr int kRows = SPLIT ? 3 : 9;
-    const int r0 = SPLIT ? 3 * (int)part : 0;
+    constexpr int kRows = 9;
     uint32_t lens[(kRows + 3) / 4] = {};
 #pragma unroll
     for (int rr = 0; rr < kRows; ++rr) {
         uint32_t jb0, je0;
-        if ((!SPLIT || work) && row_range(pp, start, sc.cell_base, delta, g, r0 + rr, jb0, je0)) {
+        if (row_range(pp, start, sc.cell_base, delta, g, rr, jb0, je0)) {
             rows[rr * rs] = jb0;
             lens[rr / 4] |= min(je0 - jb0, 255u) << (8 * (rr % 4));
         }
@@ -591,10 +613,10 @@ k_density(const DevParams* __restrict__ params,
                 const float4 x0 = __ldg(xp), y0 = __ldg(xp + 1), z0 = __ldg(xp + 2);
                 const float4 x1 = __ldg(xp + 3), y1 = __ldg(xp + 4), z1 = __ldg(xp + 5);
                 xp += 6;
-                visit4(x0, y0, z0, dm, sm);
-                visit4(x1, y1, z1, dm, sm);
+                scan.visit4(x0, y0, z0, dm, sm);
+                scan.visit4(x1, y1, z1, dm, sm);
             }
-            if (q < nq) visit4(__ldg(xp), __ldg(xp + 1), __ldg(xp + 2), dm, sm);
+            if (q < nq) scan.visit4(__ldg(xp), __ldg(xp + 1), __ldg(xp + 2), dm, sm);
             // candidate cb + b in bit 31 - b, those outside the row and the
             // particle itself left out
             const uint32_t so = k - cb;
@@ -613,7 +635,7 @@ k_density(const DevParams* __restrict__ params,
                 if (first) {
                     first = false;
                     rows[nrows++ * rs] = jb0;
-                    hd.live |= 1u << (r0 + rr);
+                    hd.live |= 1u << rr;
                     bits &= ~(0x80000000u >> b);
                     list[hd.n++] = (uint8_t)(c0 - mis + b + SPH_NBR_NEW_ROW);
                 }
@@ -629,29 +651,6 @@ k_density(const DevParams* __restrict__ params,
         if (!SKIN && hd.over) break;
     }
 
-    if constexpr (SPLIT) {
-        // the first thread appends the lists of the other two
-        __shared__ uint32_t s_hd[3 * SPH_TILE];
-        s_hd[threadIdx.x] = hd.pack() | (nrows << 9);
-        __syncthreads();
-        if (part != 0u || !work) return;
-        for (uint32_t q = 1; q < 3u && !hd.over; ++q) {
-            const uint32_t o = q * ts;
-            const uint32_t w = s_hd[li + o];
-            const NbrHeader ho(w & ~(15u << 9));
-            const uint8_t* from = reinterpret_cast<const uint8_t*>(
-                s_list + SPH_NBR_ROWS * rs + (li + o) * SPH_NBR_LIST_WORDS);
-            if (hd.n + ho.n > kCap) {
-                hd.over = true;
-                break;
-            }
-            for (uint32_t m = 0; m < ho.n; ++m) list[hd.n + m] = from[m];
-            for (uint32_t r = 0; r < ((w >> 9) & 15u); ++r) rows[nrows++ * rs] = rows[r * rs + o];
-            hd.n += ho.n;
-            hd.live |= ho.live;
-            hd.over = ho.over;
-        }
-    }
     // the last word's padding: offset 0 of the current row (read, not used)
     for (uint32_t m = hd.n; m & 3u; ++m) list[m] = 0;
     mask[k] = hd.pack();
@@ -711,24 +710,185 @@ k_density(const DevParams* __restrict__ params,
     if (hd.over)
         walk_tail(pp, start, sc.cell_base, delta, g, hd.n ? last + 1u : 0u,
                   [&](uint32_t j) { if (j != k) use(load(j)); });
-    sum = (pp.mass * pp.poly6) * sum;
-    const float d = fabsf(sdf(pp, p.x, p.y, p.z));
-    float corr = sum;
-    if (d < pp.h) corr = fmaf(pp.rest_density, 1.0f - boundary_density(pp, d), corr);
-    const float rho = (sum == 0.0f) ? pp.rest_density : corr;
-    const float ratio = corr * pp.inv_rest_density;
-    // no density at all (corr 0) has pressure 0: marked by -0
-    const float e = (corr == 0.0f) ? -0.0f : powf(ratio, pp.gamma) + 0.0f;
-    rho_out[k] = rho;
-    if (xs) {
-        const float cx = pp.xsph * (pp.poly6 * pp.two_mass);
-        vi.x = fmaf(cx, axy.x, vi.x);
-        vi.y = fmaf(cx, axy.y, vi.y);
-        vi.z = fmaf(cx, az, vi.z);
+    density_finish(pp, k, sum, xs, axy.x, axy.y, az, p, vi, rho_out, R);
+    if (nbr_out) nbr_out[k] = cnt;
+  });
+}
+
+// Several lanes per particle (WideShared), for launches of few particles.
+template <int LANES>
+__global__ void __launch_bounds__(kWideBlock, 7)
+k_density_wide(const DevParams* __restrict__ params, const DevScene* __restrict__ scenes,
+               const uint4* __restrict__ tiles, const uint32_t* __restrict__ start, const float4* __restrict__ G,
+               const float* __restrict__ X, float* __restrict__ rho_out, uint32_t* __restrict__ mask,
+               size_t mask_stride, const uint32_t* __restrict__ pend, float4* __restrict__ R,
+               uint32_t* __restrict__ nbr_out, const uint32_t* __restrict__ status) {
+  extern __shared__ uint4 s_dyn[];
+  if (step_failed(status)) return;
+  for_each_tile<LANES>(tiles, 0u, nullptr, [&](const uint4 t) {
+    // every lane stays to the end of phase 2
+    const uint32_t li = tile_particle<LANES>();
+    const bool act = li < t.z;
+    uint32_t k = t.y + (act ? li : 0u);
+    const DevScene sc = scenes[t.x];
+    const DevParams& pp = params[t.x];
+    const bool pending = __ldg(pend + t.x) != 0u;
+    float4 p, vi;
+    ld_float4_pair(G + 2 * (size_t)k, p, vi);
+    const int3 g = grid_of(pp, p.x, p.y, p.z);
+    const bool work = act && grid_inside(pp, g);
+    if (act && !work) density_outside(k, p, vi, rho_out, R, nbr_out);   // (the same by every lane)
+    const uint32_t delta = sc.part_base - __ldg(start + sc.cell_base);
+    const float h2 = pp.h2, h = pp.h, eps = pp.eps;
+    const WideLanes<LANES> wl;
+    WideShared<LANES>& ws = reinterpret_cast<WideShared<LANES>*>(s_dyn)[threadIdx.x / LANES];
+
+    // ---- phase 1: the lanes test up to 32 candidates of a row, four at a time ----
+    wide_ranges(pp, start, sc.cell_base, delta, g, work, wl, ws);
+    const CandidateScan<false> scan(p.x, p.y, p.z, h2, h2);
+    constexpr uint32_t kQuads = 8u / LANES;   // fours of candidates per lane
+    struct Chunk { float4 x[kQuads], y[kQuads], z[kQuads]; };
+    auto fetch = [&](int r, uint32_t c) {
+        const uint32_t jb0 = ws.jb[r], mis = jb0 & 3u;
+        Chunk f = {};
+#pragma unroll
+        for (uint32_t q = 0u; q < kQuads; ++q) {
+            const uint32_t o = c + 4u * (wl.l + LANES * q);
+            if (o < ws.len[r] + mis) {
+                const float4* xp = reinterpret_cast<const float4*>(X) + 3 * (size_t)((jb0 - mis + o) / 4u);
+                f.x[q] = __ldg(xp);
+                f.y[q] = __ldg(xp + 1);
+                f.z[q] = __ldg(xp + 2);
+            }
+        }
+        return f;
+    };
+    // The hits of a chunk as a word, candidate b in bit 31 - b, without those
+    // outside the row and the particle itself.
+    auto step = [&](int r, uint32_t c, const Chunk& f) {
+        const uint32_t jb0 = ws.jb[r], mis = jb0 & 3u, len = ws.len[r], alen = len ? len + mis : 0u;
+        uint32_t w = 0u;
+#pragma unroll
+        for (uint32_t q = 0u; q < kQuads; ++q) {
+            uint32_t m = 0u, none = 0u;
+            scan.visit4(f.x[q], f.y[q], f.z[q], m, none);
+            w |= m << (28u - 4u * (wl.l + LANES * q));
+        }
+#pragma unroll
+        for (uint32_t d = 1u; d < LANES; d *= 2u) w |= __shfl_xor_sync(~0u, w, d);
+        const uint32_t left = alen > 32u * c ? alen - 32u * c : 0u;
+        if (left < 32u) w &= ~(~0u >> left);
+        if (c == 0u) w &= ~0u >> mis;
+        const uint32_t so = k - (jb0 - mis + 32u * c);
+        if (so < 32u) w &= ~(0x80000000u >> so);
+        if (wl.l == 0u && len <= SPH_NBR_MAX_ROW && left != 0u) ws.words[r][c] = w;
+        return (uint32_t)__popc(w);
+    };
+    // The list's rows: it ends before the first that does not fit.
+    NbrHeader hd;
+    uint32_t at[(8 + LANES) / LANES] = {};   // where this lane's rows begin in the list
+    auto row_done = [&](int r, uint32_t hits) {
+        hd.over = hd.over || ws.len[r] > SPH_NBR_MAX_ROW || hd.n + hits > SPH_NBR_CAP;
+        if (hd.over) return;
+        if (wl.l == (uint32_t)(r % LANES)) at[r / LANES] = hd.n;
+        if (hits) hd.live |= 1u << r;
+        hd.n += hits;
+    };
+#pragma unroll
+    for (int z = 0; z < 9; z += 3) {
+        const Chunk q[3] = {fetch(z, 0u), fetch(z + 1, 0u), fetch(z + 2, 0u)};   // loaded together
+#pragma unroll
+        for (int y = 0; y < 3; ++y) {
+            const int r = z + y;
+            uint32_t hits = step(r, 0u, q[y]);
+            const uint32_t len = ws.len[r];
+            const uint32_t most = __reduce_max_sync(~0u, len <= SPH_NBR_MAX_ROW ? len + (ws.jb[r] & 3u) : 0u);
+            for (uint32_t c = 1u; 32u * c < most; ++c) hits += step(r, c, fetch(r, 32u * c));
+            row_done(r, hits);
+        }
     }
-    // a density the later passes skip as a neighbour's (rho <= eps) is marked by 0
-    st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, rho > eps ? 1.0f / rho : 0.0f),
-                   make_float4(vi.x, vi.y, vi.z, e));
+    __syncwarp();
+    // Each lane writes its rows' bytes.
+#pragma unroll
+    for (uint32_t i = 0u; i < (8u + LANES) / LANES; ++i) {
+        const uint32_t r = wl.l + LANES * i;
+        if (r < 9u && ((hd.live >> r) & 1u)) {
+            const uint32_t jb0 = ws.jb[r], mis = jb0 & 3u;
+            ws.rows[__popc(hd.live & ((1u << r) - 1u))] = jb0;
+            uint32_t pos = at[i], flag = SPH_NBR_NEW_ROW;
+            for (uint32_t c = 0u; 32u * c < ws.len[r] + mis; ++c) {
+                uint32_t bits = ws.words[r][c];
+                while (bits) {
+                    const uint32_t b = (uint32_t)__clz(bits);
+                    bits &= ~(0x80000000u >> b);
+                    ws.list[pos++] = (uint8_t)(32u * c + b - mis + flag);
+                    flag = 0u;
+                }
+            }
+        }
+    }
+    if (wl.l < ((0u - hd.n) & 3u)) ws.list[hd.n + wl.l] = 0;
+    __syncwarp();
+    if (work) {
+        if (wl.l == 0u) mask[k] = hd.pack();
+        for (uint32_t w = wl.l; 4u * w < hd.n; w += LANES)
+            mask[(size_t)(SPH_NBR_LIST + w) * mask_stride + k] = reinterpret_cast<const uint32_t*>(ws.list)[w];
+    }
+
+    // ---- phase 2 ----
+    // Terms: w, the XSPH coefficient, the velocity difference, and ones.  Lane 0
+    // sums w times one, lanes 1 to 3 the coefficient times a component, each in
+    // list order: the sums one thread forms, to the bit.
+    uint32_t cnt = 0u;
+    const uint32_t oi = pending ? __float_as_uint(vi.w) : SPH_OKEY_NULL;
+    const bool xs = oi != SPH_OKEY_NULL;
+    float acc = 0.0f;
+    ws.terms[5][wl.l] = 1.0f;
+    const float* scale = ws.terms[wl.l == 0u ? 0 : 1];
+    const float* value = ws.terms[wl.l == 0u ? 5 : 1 + min(wl.l, 3u)];
+    struct Nbr { float4 q, v; };
+    auto load = [&](uint32_t j) {
+        Nbr n;
+        ld_float4_pair(G + 2 * (size_t)j, n.q, n.v);
+        return n;
+    };
+    auto term = [&](const Nbr& n, uint32_t j, bool on) {
+        float w = 0.f, c = 0.f;
+        float3 dv = make_float3(0.f, 0.f, 0.f);
+        const float dx = p.x - n.q.x, dy = p.y - n.q.y, dz = p.z - n.q.z;
+        const float rr = dot3(dx, dy, dz, dx, dy, dz);
+        on = on && rr <= h2 && j != k;
+        if (on) {
+            const float x = h2_minus_r2(rr, h, h2);
+            w = x * x * x;
+            const float rs = p.w + n.q.w;   // the previous substep's densities
+            if (xs && rs > eps && cells_adjacent_fast(oi, __float_as_uint(n.v.w))) {
+                c = w * rcp_approx(rs);
+                dv = make_float3(n.v.x - vi.x, n.v.y - vi.y, n.v.z - vi.z);
+            }
+        }
+        cnt += (uint32_t)__popc(wl.ballot(on));
+        ws.terms[0][wl.l] = w;
+        ws.terms[1][wl.l] = c;
+        ws.terms[2][wl.l] = dv.x;
+        ws.terms[3][wl.l] = dv.y;
+        ws.terms[4][wl.l] = dv.z;
+    };
+    auto add = [&]() { acc = wide_sum<LANES>(scale, value, acc); };
+    const uint32_t last = wide_list(wl, ws, work ? hd.n : 0u, load, term, add);
+    wide_tail(wl, ws, work && hd.over, hd.n ? last + 1u : 0u, load, term, add);
+
+    // ---- the rest is one thread's work per particle: the block's first threads ----
+    if (wl.l < 4u) ws.terms[0][wl.l] = acc;
+    if (wl.l == 0u) ws.words[0][0] = work ? cnt : SPH_OKEY_NULL;
+    if (!wide_handover<LANES>(t, k)) return;
+    const WideShared<LANES>& mine = reinterpret_cast<WideShared<LANES>*>(s_dyn)[threadIdx.x];
+    const float* sums = mine.terms[0];
+    cnt = mine.words[0][0];
+    if (cnt == SPH_OKEY_NULL) return;   // outside the grid
+    ld_float4_pair(G + 2 * (size_t)k, p, vi);
+    density_finish(pp, k, sums[0], pending && __float_as_uint(vi.w) != SPH_OKEY_NULL, sums[1], sums[2], sums[3], p, vi,
+                   rho_out, R);
     if (nbr_out) nbr_out[k] = cnt;
   });
 }
@@ -737,9 +897,11 @@ k_density(const DevParams* __restrict__ params,
 // Surface normals (computeNormals, fluidphysics.cu:154-210).  Only launched
 // for scenes with surface tension: with sigma == 0 the normals enter the
 // force only through sigma * (...), which is exactly zero.  Neighbours come
-// from the density pass's list, as in the force pass.
+// from the density pass's list, as in the force pass.  LANES > 1: several lanes
+// per particle (WideShared).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restrict__ params,
+template <int LANES>
+__global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(const DevParams* __restrict__ params,
                                                       const DevScene* __restrict__ scenes,
                                                       const uint4* __restrict__ tiles,
                                                       const uint32_t* __restrict__ start,
@@ -749,17 +911,22 @@ __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restric
                                                       uint32_t* __restrict__ tile_ctr,
                                                       const uint32_t* __restrict__ status) {
   if (step_failed(status)) return;
-  for_each_tile(tiles, ntiles, tile_ctr, [&](const uint4 t) {
+  extern __shared__ uint4 s_dyn[];
+  for_each_tile<LANES>(tiles, ntiles, tile_ctr, [&](const uint4 t) {
     const DevParams& pp = params[t.x];
     if (!(pp.flags & 1u)) return;
-    if (threadIdx.x >= t.z) return;
-    const uint32_t k = t.y + threadIdx.x;
+    const uint32_t li = tile_particle<LANES>();
+    if (LANES == 1 && li >= t.z) return;
+    const bool act = li < t.z;
+    const uint32_t k = t.y + (act ? li : 0u);
     const DevScene sc = scenes[t.x];
+    const WideEarly early = wide_early<LANES>(mask, mask_stride, k);
     const float4 p = R[2 * (size_t)k];
     const int3 g = grid_of(pp, p.x, p.y, p.z);
-    if (!grid_inside(pp, g)) {
+    const bool work = act && grid_inside(pp, g);
+    if (act && !work) {
         N[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        return;
+        if (LANES == 1) return;
     }
     const uint32_t delta = sc.part_base - __ldg(start + sc.cell_base);
     // x and y packed (f32x2, rounded per component as the scalar operations), z alone
@@ -770,21 +937,47 @@ __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restric
     // factor r of gradPoly6 cancels the 1/r; m c, the same for every pair, is
     // left to the end
     const float h2 = pp.h2, eps = pp.eps, h = pp.h;
-    extern __shared__ uint32_t s_rows[];
-    walk_neighbours<kNormalsDepth>(
-        pp, start, sc.cell_base, delta, g, mask, mask_stride, k, s_rows + threadIdx.x, blockDim.x,
-        [&](uint32_t j) { return __ldg(R + 2 * (size_t)j); },   // w = 1/rho_j, 0 where rho_j <= eps
-        [&](const float4& q) {
-            const float2 rxy = __fadd2_rn(pxy, make_float2(-q.x, -q.y));
-            const float rx = rxy.x, ry = rxy.y, rz = p.z - q.z;
-            const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-            if (r2 <= h2 && r2 > eps && q.w > 0.0f) {
-                const float x = h2_minus_r2(r2, h, h2);
-                const float s = (x * x) * q.w;
-                sxy = __ffma2_rn(make_float2(s, s), rxy, sxy);
-                sz = fmaf(s, rz, sz);
-            }
-        });
+    auto load = [&](uint32_t j) { return __ldg(R + 2 * (size_t)j); };   // w = 1/rho_j, 0 where rho_j <= eps
+    if constexpr (LANES > 1) {
+        const WideLanes<LANES> wl;
+        WideShared<LANES>& ws = reinterpret_cast<WideShared<LANES>*>(s_dyn)[threadIdx.x / LANES];
+        float acc = 0.f;   // lanes 0 to 2: the sum's components
+        const float* value = ws.terms[1 + min(wl.l, 2u)];
+        wide_neighbours(
+            pp, start, sc.cell_base, delta, g, mask, mask_stride, k, work, early, wl, ws, load,
+            [&](const float4& q, uint32_t, bool on) {
+                const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
+                const float r2 = dot3(rx, ry, rz, rx, ry, rz);
+                on = on && r2 <= h2 && r2 > eps && q.w > 0.0f;
+                float s = 0.f;
+                if (on) {
+                    const float x = h2_minus_r2(r2, h, h2);
+                    s = (x * x) * q.w;
+                }
+                ws.terms[0][wl.l] = s;
+                ws.terms[1][wl.l] = on ? rx : 0.f;
+                ws.terms[2][wl.l] = on ? ry : 0.f;
+                ws.terms[3][wl.l] = on ? rz : 0.f;
+            },
+            [&]() { acc = wide_sum<LANES>(ws.terms[0], value, acc); });
+        sxy = make_float2(wl.get(acc, 0), wl.get(acc, 1));
+        sz = wl.get(acc, 2);
+        if (!work || wl.l != 0u) return;
+    } else {
+        walk_neighbours<kNormalsDepth>(
+            pp, start, sc.cell_base, delta, g, mask, mask_stride, k,
+            reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load, [&](const float4& q) {
+                const float2 rxy = __fadd2_rn(pxy, make_float2(-q.x, -q.y));
+                const float rx = rxy.x, ry = rxy.y, rz = p.z - q.z;
+                const float r2 = dot3(rx, ry, rz, rx, ry, rz);
+                if (r2 <= h2 && r2 > eps && q.w > 0.0f) {
+                    const float x = h2_minus_r2(r2, h, h2);
+                    const float s = (x * x) * q.w;
+                    sxy = __ffma2_rn(make_float2(s, s), rxy, sxy);
+                    sz = fmaf(s, rz, sz);
+                }
+            });
+    }
     const float hc = pp.h * (pp.mass * pp.grad_poly6);
     N[k] = make_float4(hc * sxy.x, hc * sxy.y, hc * sz, 0.f);
   });
@@ -807,8 +1000,10 @@ __global__ void __launch_bounds__(SPH_TILE) k_normals(const DevParams* __restric
 // budget as resident blocks of 256 threads per SM: 3 (80 registers, no
 // spills) or 4 (64 registers, more warps per SM, a few spilled values in the
 // tension build).
-template <bool TENSION, int MINB>
-__global__ void __launch_bounds__(SPH_TILE, MINB)
+// LANES > 1: several lanes per particle through the pair sums (WideShared), then
+// one.
+template <bool TENSION, int MINB, int LANES = 1>
+__global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE, MINB)
 k_force_integrate(const DevParams* __restrict__ params,
                                                               const DevScene* __restrict__ scenes,
                                                               const uint4* __restrict__ tiles,
@@ -826,22 +1021,28 @@ k_force_integrate(const DevParams* __restrict__ params,
                                                               float4* __restrict__ dbg_forces, uint32_t ntiles,
                                                               uint32_t* __restrict__ tile_ctr) {
   if (step_failed(status)) return;
-  for_each_tile(tiles, ntiles, tile_ctr, [&](const uint4 t) {
-    // lanes holding a particle of this tile (taken before any divergence)
-    const unsigned lanes = __ballot_sync(0xffffffffu, threadIdx.x < t.z);
-    if (threadIdx.x >= t.z) return;
-    const uint32_t k = t.y + threadIdx.x;
+  extern __shared__ uint4 s_dyn[];
+  for_each_tile<LANES>(tiles, ntiles, tile_ctr, [&](const uint4 t) {
+    const uint32_t li = tile_particle<LANES>();
+    const bool act = li < t.z;
+    // lanes that integrate a particle of this tile (taken before any divergence)
+    unsigned lanes = __ballot_sync(0xffffffffu, act);
+    if (LANES == 1 && !act) return;
+    uint32_t k = t.y + (act ? li : 0u);
     const DevScene sc = scenes[t.x];
     const DevParams& pp = params[t.x];
     // the scene's XSPH update is now pending (applied by the next density
     // pass, or by k_xsph right after this pass)
     if (threadIdx.x == 0) pend[t.x] = 1u;
+    const WideEarly early = wide_early<LANES>(mask, mask_stride, k);
+    if (LANES > 1 && threadIdx.x < kWideBlock / LANES && blockIdx.x * (kWideBlock / LANES) + threadIdx.x < t.z)
+        prefetch_l1(A1 + t.y + blockIdx.x * (kWideBlock / LANES) + threadIdx.x);
     float4 pi, vi;
     ld_float4_pair(R + 2 * (size_t)k, pi, vi);
-    const float ri = rho[k];
-    const int3 g = grid_of(pp, pi.x, pi.y, pi.z);
+    float ri = rho[k];
+    int3 g = grid_of(pp, pi.x, pi.y, pi.z);
     const bool tension = TENSION && (pp.flags & 1u) != 0u;
-    const bool inside = grid_inside(pp, g);
+    bool inside = grid_inside(pp, g);
     float fpx = 0.f, fpy = 0.f, fpz = 0.f;   // pressure
     float fvx = 0.f, fvy = 0.f, fvz = 0.f;   // viscosity (the pressure is added after the sums)
     float ftx = 0.f, fty = 0.f, ftz = 0.f;   // tension
@@ -864,7 +1065,8 @@ k_force_integrate(const DevParams* __restrict__ params,
     // pairs.  Against one division, rounded root and pair of weighted vectors
     // per term this took 18 of 145 M warp instructions from the pass: 196 -> 189
     // us on the 1M dam break, 1.86 -> 1.69 ms on the 8M tension scene.
-    auto pair = [&](const float4& pj, const float4& vj, const float4& nj) {
+    // press(sp, sv, r) and tens(c, r, dn) take the terms.
+    auto pair = [&](const float4& pj, const float4& vj, const float4& nj, auto&& press, auto&& tens) {
         const float rx = pj.x - pi.x, ry = pj.y - pi.y, rz = pj.z - pi.z;
         const float r2 = dot3(rx, ry, rz, rx, ry, rz);
         if (r2 <= h2 && r2 > FLT_MIN && pj.w > 0.0f) {
@@ -881,34 +1083,83 @@ k_force_integrate(const DevParams* __restrict__ params,
             const float mid = fmaf(pri, pj.w * pj.w, eos_k * (vj.w - 1.0f) * inv_ri2);
             const float hr2 = hr * hr;
             const float sr = hr2 * inv_r;
-            const float sp = sr * mid, sv = sr * Pi;
-            fpx = fmaf(sp, rx, fpx); fpy = fmaf(sp, ry, fpy); fpz = fmaf(sp, rz, fpz);
-            fvx = fmaf(sv, rx, fvx); fvy = fmaf(sv, ry, fvy); fvz = fmaf(sv, rz, fvz);
+            const float3 rv = make_float3(rx, ry, rz);
+            press(sr * mid, sr * Pi, rv);
             if (tension) {
                 // Akinci cohesion + curvature (fluidphysics.cu:291-293), cohesion
                 // times 1/r, both over -sigma m.  With sigma == 0 the tension
                 // force is sigma * (finite sum) = 0, so the term is skipped.
                 const float t = hr2 * hr * r2;
-                const float c = coh * ((r > rsel) ? t : fmaf(2.0f, t, -(coh_near * inv_r)));
-                ftx = fmaf(c, rx, ftx) + (ni.x - nj.x);
-                fty = fmaf(c, ry, fty) + (ni.y - nj.y);
-                ftz = fmaf(c, rz, ftz) + (ni.z - nj.z);
+                tens(coh * ((r > rsel) ? t : fmaf(2.0f, t, -(coh_near * inv_r))), rv,
+                     make_float3(ni.x - nj.x, ni.y - nj.y, ni.z - nj.z));
             }
         }
     };
     struct Nbr { float4 p, v, n; };
-    if (inside) {
-        extern __shared__ uint32_t s_rows[];
-        walk_neighbours<kForceDepth>(
-            pp, start, sc.cell_base, delta, g, mask, mask_stride, k, s_rows + threadIdx.x, blockDim.x,
-            [&](uint32_t j) {
-                Nbr r;
-                ld_float4_pair(R + 2 * (size_t)j, r.p, r.v);
-                r.n = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (tension) r.n = __ldg(N + j);
-                return r;
+    auto load = [&](uint32_t j) {
+        Nbr r;
+        ld_float4_pair(R + 2 * (size_t)j, r.p, r.v);
+        r.n = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (tension) r.n = __ldg(N + j);
+        return r;
+    };
+    if constexpr (LANES > 1) {
+        // Terms: the two scales, rvec, then the cohesion's scale and the
+        // normals' difference.  Lanes 0 to 2 sum one component each, in list
+        // order.
+        const WideLanes<LANES> wl;
+        WideShared<LANES>& ws = reinterpret_cast<WideShared<LANES>*>(s_dyn)[threadIdx.x / LANES];
+        const uint32_t axis = min(wl.l, 2u);
+        float sum_p = 0.f, sum_v = 0.f, sum_t = 0.f;
+        wide_neighbours(
+            pp, start, sc.cell_base, delta, g, mask, mask_stride, k, act && inside, early, wl, ws, load,
+            [&](const Nbr& r, uint32_t, bool on) {
+                float o[9] = {};
+                if (on)
+                    pair(r.p, r.v, r.n,
+                         [&](float sp, float sv, const float3& d) {
+                             o[0] = sp; o[1] = sv; o[2] = d.x; o[3] = d.y; o[4] = d.z;
+                         },
+                         [&](float c, const float3&, const float3& dn) {
+                             o[5] = c; o[6] = dn.x; o[7] = dn.y; o[8] = dn.z;
+                         });
+#pragma unroll
+                for (int c = 0; c < (TENSION ? 9 : 5); ++c) ws.terms[c][wl.l] = o[c];
             },
-            [&](const Nbr& r) { pair(r.p, r.v, r.n); });
+            [&]() {
+                sum_p = wide_sum<LANES>(ws.terms[0], ws.terms[2u + axis], sum_p);
+                sum_v = wide_sum<LANES>(ws.terms[1], ws.terms[2u + axis], sum_v);
+                if (tension) sum_t = wide_sum<LANES>(ws.terms[5], ws.terms[2u + axis], sum_t, ws.terms[6u + axis]);
+            });
+        // the rest is one thread's work per particle: the block's first threads
+        ws.terms[0][wl.l] = sum_p;
+        ws.terms[1][wl.l] = sum_v;
+        ws.terms[2][wl.l] = sum_t;
+        if (!wide_handover<LANES>(t, k)) return;
+        lanes = ~0u >> (32u - min(kWideBlock / LANES, t.z - blockIdx.x * (kWideBlock / LANES)));
+        const WideShared<LANES>& w = reinterpret_cast<WideShared<LANES>*>(s_dyn)[threadIdx.x];
+        fpx = w.terms[0][0]; fpy = w.terms[0][1]; fpz = w.terms[0][2];
+        fvx = w.terms[1][0]; fvy = w.terms[1][1]; fvz = w.terms[1][2];
+        ftx = w.terms[2][0]; fty = w.terms[2][1]; ftz = w.terms[2][2];
+        ld_float4_pair(R + 2 * (size_t)k, pi, vi);
+        ri = rho[k];
+        g = grid_of(pp, pi.x, pi.y, pi.z);
+        inside = grid_inside(pp, g);
+    } else if (inside) {
+        walk_neighbours<kForceDepth>(
+            pp, start, sc.cell_base, delta, g, mask, mask_stride, k,
+            reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load, [&](const Nbr& r) {
+                pair(r.p, r.v, r.n,
+                     [&](float sp, float sv, const float3& d) {
+                         fpx = fmaf(sp, d.x, fpx); fpy = fmaf(sp, d.y, fpy); fpz = fmaf(sp, d.z, fpz);
+                         fvx = fmaf(sv, d.x, fvx); fvy = fmaf(sv, d.y, fvy); fvz = fmaf(sv, d.z, fvz);
+                     },
+                     [&](float c, const float3& d, const float3& dn) {
+                         ftx = fmaf(c, d.x, ftx) + dn.x;
+                         fty = fmaf(c, d.y, fty) + dn.y;
+                         ftz = fmaf(c, d.z, ftz) + dn.z;
+                     });
+            });
     }
     if (inside) {
         // the factors left out of the sums
@@ -1049,7 +1300,7 @@ __global__ void k_xsph(const DevParams* __restrict__ params,
                                                    uint32_t* __restrict__ tile_ctr,
                                                    const uint32_t* __restrict__ status) {
   if (step_failed(status)) return;
-  for_each_tile(tiles, ntiles, tile_ctr, [&](const uint4 t) {
+  for_each_tile<1>(tiles, ntiles, tile_ctr, [&](const uint4 t) {
     if (threadIdx.x >= t.z) return;
     const uint32_t k = t.y + threadIdx.x;
     const DevScene sc = scenes[t.x];
@@ -1273,17 +1524,14 @@ cudaError_t init_kernel_attributes() {
         {(const void*)k_force_integrate<true, 4>, SPH_ROWS_CARVEOUT_PCT},
         {(const void*)k_force_integrate<false, 3>, SPH_ROWS_CARVEOUT_PCT},
         {(const void*)k_force_integrate<false, 4>, SPH_ROWS_CARVEOUT_PCT},
-        {(const void*)k_normals, SPH_ROWS_CARVEOUT_PCT},
+        {(const void*)k_normals<1>, SPH_ROWS_CARVEOUT_PCT},
         {(const void*)k_density<false>, SPH_LIST_CARVEOUT_PCT},
-        {(const void*)k_density<true>, SPH_LIST_CARVEOUT_PCT},
-        {(const void*)k_density<false, true>, SPH_LIST_CARVEOUT_PCT}};
+        {(const void*)k_density<true>, SPH_LIST_CARVEOUT_PCT}};
     for (const auto& x : fns) {
         const cudaError_t e = cudaFuncSetAttribute(x.f, cudaFuncAttributePreferredSharedMemoryCarveout, x.pct);
         if (e != cudaSuccess) return e;
     }
-    // the split scan keeps three lists per particle: above 48 KB from 128-particle tiles on
-    return cudaFuncSetAttribute((const void*)k_density<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(3u * SPH_TILE * SPH_NBR_SMEM_WORDS * sizeof(uint32_t)));
+    return cudaSuccess;
 }
 
 // a.scan_sums holds at least nt + 2 64-bit words: the tile counter, then one
@@ -1333,18 +1581,28 @@ cudaError_t launch_sort(const StepArgs& a, cudaStream_t st) {
                                                 a.okey, a.pend, a.G, axes(a), a.A1, a.perm, a.status);
     return cudaGetLastError();
 }
-bool density_split(const StepArgs& a) {
-    return (a.variant & SPH_VARIANT_DENSITY_SPLIT) != 0u && (a.variant & SPH_VARIANT_DENSITY_ROWS) != 0u &&
-           !a.skin_masks && a.tile_ctr == nullptr && a.particles <= SPH_DENSITY_SPLIT_MAX;
+// Lanes per particle of the neighbour passes (WideShared).
+static int lanes(const StepArgs& a) {
+    if ((a.variant & SPH_VARIANT_DENSITY_SPLIT) == 0u || a.tile_ctr != nullptr || a.ntiles > 65535u) return 1;
+    if (a.particles <= (a.crowded ? SPH_CROWDED8_MAX : SPH_WIDE8_MAX)) return 8;
+    return a.particles <= (a.crowded ? SPH_CROWDED4_MAX : SPH_DENSITY_SPLIT_MAX) ? 4 : 1;
+}
+static dim3 wide_grid(const StepArgs& a, int lanes) {
+    return dim3((a.block * (uint32_t)lanes + kWideBlock - 1u) / kWideBlock, a.ntiles);
+}
+static size_t wide_smem(int lanes) {
+    return kWideBlock / lanes * (lanes == 8 ? sizeof(WideShared<8>) : sizeof(WideShared<4>));
 }
 cudaError_t launch_density(const StepArgs& a, cudaStream_t st) {
-    const size_t smem = (size_t)SPH_NBR_SMEM_WORDS * a.block * sizeof(uint32_t);
-    if (density_split(a)) {
-        k_density<false, true><<<a.ntiles, 3u * a.block, 3u * smem, st>>>(
-            a.params, a.scenes, a.tiles, a.start, a.G, axes(a), a.rho, a.mask, a.mask_stride, a.pend, a.R, a.dbg_nbr,
-            a.ntiles, nullptr, a.status);
+    const int l = a.skin_masks ? 1 : lanes(a);
+    if (l > 1) {
+        auto kern = l == 8 ? k_density_wide<8> : k_density_wide<4>;
+        kern<<<wide_grid(a, l), kWideBlock, wide_smem(l), st>>>(a.params, a.scenes, a.tiles, a.start, a.G, axes(a),
+                                                               a.rho, a.mask, a.mask_stride, a.pend, a.R, a.dbg_nbr,
+                                                               a.status);
         return cudaGetLastError();
     }
+    const size_t smem = (size_t)SPH_NBR_SMEM_WORDS * a.block * sizeof(uint32_t);
     auto kern = a.skin_masks ? k_density<true> : k_density<false>;
     kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.G, axes(a), a.rho, a.mask, a.mask_stride,
                                             a.pend, a.R, a.dbg_nbr, a.ntiles, ctr(a, 0), a.status);
@@ -1365,15 +1623,23 @@ cudaError_t launch_undo_ahead(const StepArgs& a, uint32_t first_tile, uint32_t n
 }
 static size_t rows_smem(const StepArgs& a) { return (size_t)SPH_NBR_ROWS * a.block * sizeof(uint32_t); }
 cudaError_t launch_normals(const StepArgs& a, cudaStream_t st) {
-    k_normals<<<a.grid_nbr, a.block, rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.mask,
+    const int l = lanes(a);
+    auto kern = l == 8 ? k_normals<8> : l == 4 ? k_normals<4> : k_normals<1>;
+    kern<<<l > 1 ? wide_grid(a, l) : dim3(a.grid_nbr), l > 1 ? kWideBlock : a.block,
+           l > 1 ? wide_smem(l) : rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.mask,
                                                          a.mask_stride, a.N, a.ntiles, ctr(a, 1), a.status);
     return cudaGetLastError();
 }
 cudaError_t launch_force(const StepArgs& a, cudaStream_t st) {
     const bool occ = (a.variant & SPH_VARIANT_FORCE_OCC) != 0u;
-    auto kern = a.any_tension ? (occ ? k_force_integrate<true, 4> : k_force_integrate<true, 3>)
-                              : (occ ? k_force_integrate<false, 4> : k_force_integrate<false, 3>);
-    kern<<<a.grid_nbr, a.block, rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.rho, a.A1, a.N,
+    const int l = lanes(a);
+    auto kern = l == 8   ? (a.any_tension ? k_force_integrate<true, 1, 8> : k_force_integrate<false, 1, 8>)
+                : l == 4 ? (a.any_tension ? k_force_integrate<true, 1, 4> : k_force_integrate<false, 1, 4>)
+                : a.any_tension ? (occ ? k_force_integrate<true, 4> : k_force_integrate<true, 3>)
+                                : (occ ? k_force_integrate<false, 4> : k_force_integrate<false, 3>);
+    kern<<<l > 1 ? wide_grid(a, l) : dim3(a.grid_nbr), l > 1 ? kWideBlock : a.block,
+           l > 1 ? wide_smem(l) : rows_smem(a), st>>>(
+                                                    a.params, a.scenes, a.tiles, a.start, a.R, a.rho, a.A1, a.N,
                                                     a.mask, a.mask_stride, a.P0, a.V2, a.A0,
                                                     a.skin_masks ? a.maxdisp : nullptr, a.okey, a.pend, a.count,
                                                     a.key, a.slot, a.status, a.dbg_forces, a.ntiles, ctr(a, 2));

@@ -72,23 +72,34 @@ struct DevParams {
 // Kernel variants (bits of the execution config's `variant`). All variants
 // visit neighbours in the same order and give identical results; they differ
 // only in how the walk is scheduled.
-#define SPH_VARIANT_DENSITY_ROWS  0x1u   // density: with DENSITY_SPLIT, the split scan (else no effect: one scan is left)
+#define SPH_VARIANT_DENSITY_ROWS  0x1u   // no effect: one candidate scan is left
 #define SPH_VARIANT_XSPH_ROWS     0x2u   // XSPH: one loop per cell row instead of one flattened walk
 #define SPH_VARIANT_FORCE_OCC     0x4u   // force: 64-register build (more resident warps)
 #define SPH_VARIANT_FORCE_TABLE   0x8u   // no effect: the force and normal passes walk the neighbour list
 #define SPH_VARIANT_NORMALS_TABLE 0x10u  // no effect
-#define SPH_VARIANT_DENSITY_SPLIT 0x20u  // density: three threads per particle share the candidate scan
-                                         // (launches of at most SPH_DENSITY_SPLIT_MAX particles)
+#define SPH_VARIANT_DENSITY_SPLIT 0x20u  // neighbour passes: several lanes per particle in small launches
+                                         // (at most SPH_DENSITY_SPLIT_MAX particles, more where crowded)
 #define SPH_VARIANT_MASK          0x3fu
-#define SPH_VARIANT_DEFAULT       0x3fu  // measured fastest on the 1M dam break, the 256-scene batch
-                                         // and the 8M tension scene (where the split scan does not
-                                         // apply), and on dam breaks of 8,000 to 32,768 particles
-// Largest launch (particles over all tiles) that the split scan serves: it
-// gained 6-9% per substep on dam breaks of 8,000 to 32,768 particles and lost
-// 10% at 64,000 (the blocks of three times the threads run fewer at once).
-#ifndef SPH_DENSITY_SPLIT_MAX
-#define SPH_DENSITY_SPLIT_MAX     49152u
+#define SPH_VARIANT_DEFAULT       0x3fu
+
+// Largest launches (particles over all tiles) that run eight and four lanes per
+// particle in the neighbour passes.  Measured on cubes of fluid at rest density
+// (33 neighbours), substep in us with eight lanes, four, one: 13,824 particles
+// 34.9, 36.7, 52.5; 21,952 45.9, 40.0, 52.2; 32,768 55.4, 46.1, 53.3; 35,937
+// with surface tension 75.0, 70.6, 67.2; 46,656 68.0, 60.9, 58.2.  A crowded
+// particle's walk is longer and the lanes shorten it by more: scenes of 92 to
+// 160 neighbours, 38,266 particles 507, 544, 865; 59,048 (92) 326, 322, 338;
+// 59,048 (160) 626, 623, 731; 119,168 855, 820, 532.  Crowded: at least
+// SPH_CROWDED_NBRS neighbours on average, from h, the rest density and the mass.
+#ifndef SPH_WIDE8_MAX
+#define SPH_WIDE8_MAX         14336u
 #endif
+#ifndef SPH_DENSITY_SPLIT_MAX
+#define SPH_DENSITY_SPLIT_MAX 34816u
+#endif
+#define SPH_CROWDED_NBRS      80u
+#define SPH_CROWDED8_MAX      40960u
+#define SPH_CROWDED4_MAX      61440u
 
 // Scene placement in the engine's arenas.
 struct DevScene {
