@@ -170,7 +170,7 @@ void Engine::free_all() {
     for (auto p : f4) { if (*p) cudaFree(*p); *p = nullptr; }
     if (rho_) cudaFree(rho_);
     rho_ = nullptr;
-    uint32_t** u[] = {&key_, &slot_, &perm_, &count_, &start_, &scan_sums_, &dbg_nbr_, &mask_,
+    uint32_t** u[] = {&key_, &slot_, &perm_, &count_, &start_, &scan_sums_, &dbg_nbr_, &mask_, &sums_,
                       &okey_, &pend_};
     for (auto p : u) { if (*p) cudaFree(*p); *p = nullptr; }
     if (stage_) cudaFree(stage_);
@@ -251,12 +251,14 @@ int Engine::ensure_capacity(uint64_t parts, uint64_t cells) {
         if (count_) cudaFree(count_);
         if (start_) cudaFree(start_);
         if (scan_sums_) cudaFree(scan_sums_);
-        count_ = start_ = scan_sums_ = nullptr;
+        if (sums_) cudaFree(sums_);
+        count_ = start_ = scan_sums_ = sums_ = nullptr;
         cudaError_t e1 = cudaMalloc((void**)&count_, nc * sizeof(uint32_t));
         cudaError_t e2 = cudaMalloc((void**)&start_, (nc + 1) * sizeof(uint32_t));
         // the scan's tile counter and look-back descriptors (64-bit words)
         cudaError_t e3 = cudaMalloc((void**)&scan_sums_, (nc / 4096 + 3) * sizeof(unsigned long long));
-        if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess)
+        cudaError_t e4 = cudaMalloc((void**)&sums_, (nc / kScanTileCells + 1) * sizeof(uint32_t));
+        if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess)
             return fail(ENG_ENOMEM, "device allocation of cell arrays failed");
         ccap_ = nc;
         graph_dirty_ = true;
@@ -521,7 +523,7 @@ StepArgs Engine::args() const {
     a.G = G_; a.A1 = A1_;
     a.V2 = V2_; a.rho = rho_; a.N = N_;
     a.R = R_; a.okey = okey_; a.pend = pend_;
-    a.count = count_; a.start = start_; a.scan_sums = scan_sums_;
+    a.count = count_; a.start = start_; a.sums = sums_; a.scan_sums = scan_sums_;
     a.scan_first = 0u;
     a.scan_cells = 0u;   // all cells
     a.scan_zeroes_counts = 1u;
@@ -551,8 +553,14 @@ int Engine::launch_prefix(bool profile) { return launch_prefix_args(args(), prof
 
 // The hash of the current positions, for when no force pass produced it (the
 // first substep, or after the state, the layout or the parameters changed).
+cudaError_t Engine::clear_counts() {
+    const uint32_t nt = (total_cells_ + kScanTileCells - 1u) / kScanTileCells;
+    cudaError_t e = cudaMemsetAsync(count_, 0, (size_t)total_cells_ * sizeof(uint32_t), stream_);
+    if (e == cudaSuccess) e = cudaMemsetAsync(sums_, 0, (size_t)nt * sizeof(uint32_t), stream_);
+    return e;
+}
 int Engine::launch_hash_standalone(const StepArgs& a) {
-    ENG_CK(cudaMemsetAsync(count_, 0, (size_t)total_cells_ * sizeof(uint32_t), stream_), "memset counts");
+    ENG_CK(clear_counts(), "memset counts");
     ENG_CK(launch_hash(a, stream_), "hash");
     return ENG_OK;
 }
@@ -564,7 +572,9 @@ int Engine::launch_prefix_args(const StepArgs& a, bool profile, bool hash) {
     cudaStream_t st = stream_;
     auto mark = [&](int i) { if (profile) cudaEventRecord(ev_[i], st); };
     mark(0);
-    ENG_CK(cudaMemsetAsync(scal_, 0, 8 * sizeof(uint32_t), st), "memset substep scalars");
+    // the displacement maximum of a per-substep XSPH pass, the tile counters of persistent launches
+    if (a.skin_masks || a.tile_ctr)
+        ENG_CK(cudaMemsetAsync(scal_, 0, 8 * sizeof(uint32_t), st), "memset substep scalars");
     if (hash) { int rc = launch_hash_standalone(a); if (rc) return rc; }
     mark(1);
     ENG_CK(launch_scan(a, st), "scan");
@@ -622,7 +632,7 @@ int Engine::settle() {
     cudaSetDevice(device_);
     const Scene& s = scenes_.front();
     ENG_CK(launch_undo_ahead(args(), s.tile_first, s.tile_count, stream_), "undo");
-    ENG_CK(cudaMemsetAsync(count_, 0, (size_t)total_cells_ * sizeof(uint32_t), stream_), "memset counts");
+    ENG_CK(clear_counts(), "memset counts");
     ENG_CK(cudaMemsetAsync(scal_, 0, 8 * sizeof(uint32_t), stream_), "memset substep scalars");
     hashed_ = false;
     // an export that follows waits for this event before it packs the state

@@ -179,6 +179,7 @@ private:
     int upload_params();
     int launch_prefix(bool profile);   // [memset, hash], scan, sort, density
     int launch_prefix_args(const StepArgs& a, bool profile, bool hash);
+    cudaError_t clear_counts();        // cell counts and their sums to zero
     int launch_hash_standalone(const StepArgs& a);
     int prefix_scene(const Scene& s, bool wait = true);  // the prefix over one scene's tiles
     int launch_suffix(bool profile);   // normals, force + integrator, [XSPH]
@@ -229,6 +230,7 @@ private:
     uint32_t *pend_ = nullptr;                      // per scene-table entry: XSPH update pending
     uint32_t *key_ = nullptr, *slot_ = nullptr, *perm_ = nullptr;
     uint32_t *count_ = nullptr, *start_ = nullptr, *scan_sums_ = nullptr, *status_ = nullptr;
+    uint32_t* sums_ = nullptr;         // the counts' sums per scan tile
     uint32_t *gate_ = nullptr;        // status word of the passes an export ran ahead (status_ + 1)
     uint32_t *mask_ = nullptr;        // SPH_MASK_ROWS neighbour words per slot, rows of mask_stride_
     size_t mask_stride_ = 0;

@@ -34,6 +34,30 @@
 
 namespace sph {
 
+// Adds the lanes in `mask` to their cells' counts and, with `sums`, to the sums
+// of the scan tiles (kScanTileCells cells) they lie in, from which every block of
+// the scan finds its own prefix.  Returns the lane's provisional slot in its
+// cell.  Equal cells share one atomic; the cells of a warp in cell order nearly
+// always lie in one tile and share that one too.
+__device__ __forceinline__ uint32_t count_cell(unsigned mask, uint32_t cell, uint32_t* __restrict__ count,
+                                               uint32_t* __restrict__ sums) {
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned peers = __match_any_sync(mask, cell);
+    const int leader = __ffs(peers) - 1;
+    if (sums) {
+        const uint32_t tile = cell / kScanTileCells;
+        const int first = __ffs(mask) - 1;
+        const uint32_t t0 = __shfl_sync(mask, tile, first);
+        const bool one_tile = __all_sync(mask, tile == t0);
+        if ((int)lane == (one_tile ? first : leader))
+            atomicAdd(sums + tile, (uint32_t)__popc(one_tile ? mask : peers));
+    }
+    uint32_t base = 0;
+    if ((int)lane == leader) base = atomicAdd(&count[cell], (uint32_t)__popc(peers));
+    base = __shfl_sync(mask, base, leader);
+    return base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+}
+
 // ---------------------------------------------------------------------------
 // Spatial hash + cell counts (hash.cu:10-27 and the fill at
 // fluidsystem.cu:304-306).  Equal keys inside a warp are combined with
@@ -51,6 +75,7 @@ __global__ void __launch_bounds__(SPH_TILE) k_hash(const DevParams* __restrict__
                                                    const uint32_t* __restrict__ pend, uint32_t* __restrict__ okey,
                                                    uint32_t* __restrict__ status) {
     const uint4 t = tiles[blockIdx.x];
+    const unsigned lanes = __ballot_sync(0xffffffffu, threadIdx.x < t.z);
     if (threadIdx.x >= t.z) return;
     const uint32_t i = t.y + threadIdx.x;
     const DevScene sc = scenes[t.x];
@@ -64,21 +89,15 @@ __global__ void __launch_bounds__(SPH_TILE) k_hash(const DevParams* __restrict__
         if (o != SPH_OKEY_NULL && (!inside || (o & ~SPH_OKEY_MOVED) != pack_cell(gc))) okey[i] = o | SPH_OKEY_MOVED;
     }
     if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) atomicOr(status, SPH_STATUS_NONFINITE);
-    const uint32_t gkey = sc.cell_base + local;
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned active = __activemask();
-    const unsigned peers = __match_any_sync(active, gkey);
-    const int leader = __ffs(peers) - 1;
-    uint32_t base = 0;
-    if ((int)lane == leader) base = atomicAdd(&count[gkey], (uint32_t)__popc(peers));
-    base = __shfl_sync(active, base, leader);
     key[i] = local;
-    slot[i] = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+    slot[i] = count_cell(lanes, sc.cell_base + local, count, nullptr);
 }
 
 // ---------------------------------------------------------------------------
-// Exclusive scan of cell counts -> cell starts (fluidsystem.cu:316).
-// Reduce-then-scan: 4096 counts per tile.
+// Exclusive scan of cell counts -> cell starts (fluidsystem.cu:316), 4096
+// counts per tile, in three forms: the substep's (k_scan_tiles), whose tile
+// sums the hash made; one pass over any range (k_scan_single); and reduce,
+// scan, down-sweep over caller's memory (launch_scan_raw).
 // ---------------------------------------------------------------------------
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 16;
@@ -179,7 +198,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t* __re
     }
 }
 
-// Single-pass form of the same scan, used by the substep: decoupled
+// Single-pass form of the same scan, for a range whose tile sums nobody made (one
+// scene's cells, when a single scene of many is read): decoupled
 // look-back (Merrill and Garland, "Single-pass Parallel Prefix Scan with
 // Decoupled Look-back", NVIDIA technical report NVR-2016-002).  Each tile
 // publishes its aggregate, then adds the aggregates of the tiles before it
@@ -190,9 +210,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t* __re
 // running and waits only on tiles before it; the waits are bounded all the
 // same (SPH_STATUS_SCAN_TIMEOUT, the outputs are then invalid).
 //
-// With `zero` set the kernel also leaves every count it read at zero: the
-// next substep's hash (fused into the force pass) adds into them, which
-// otherwise needs a memset of the whole count array.
+// With `zero` set the kernel also leaves every count it read at zero (as
+// k_scan_tiles does).
 constexpr unsigned long long SCAN_AGG = 1ull << 32;
 constexpr unsigned long long SCAN_PRE = 2ull << 32;
 constexpr uint32_t SCAN_SPIN_LIMIT = 1u << 22;   // the default limit (StepArgs.scan_spin_limit = 0)
@@ -315,6 +334,77 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_single(uint32_t* __restri
     }
 }
 
+// The substep's scan.  A tile's prefix is the sum of the tiles before it, which
+// the hash counted (count_cell) and every block reads for itself.  No block
+// waits for another and no descriptors are cleared: against the look-back the
+// substep of the 1M dam break (489 tiles) went from 379 to 372 us and that of
+// 1,728 particles from 27 to 25 us.  The sums' reads grow with the square of the
+// tiles, so from SPH_SCAN_SUM_TILES on (67 million cells; 0.1 ms of reads beside
+// 0.1 ms of scan) the look-back takes over.  The counts are left at zero: the next substep's hash (fused into
+// the force pass) adds into them, which otherwise needs a memset of the whole
+// array; k_scatter clears the sums.
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(uint32_t* __restrict__ in, uint32_t n,
+                                                             const uint32_t* __restrict__ sums,
+                                                             uint32_t* __restrict__ out) {
+    __shared__ uint32_t warp_tot[SCAN_THREADS / 32], warp_pre[SCAN_THREADS / 32];
+    const uint32_t tile = blockIdx.x, base = tile * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
+    const bool whole = base + SCAN_ITEMS <= n;
+    uint32_t v[SCAN_ITEMS];
+    if (whole) {
+        const uint4* p4 = reinterpret_cast<const uint4*>(in + base);
+#pragma unroll
+        for (int q = 0; q < SCAN_ITEMS / 4; ++q) {
+            const uint4 w = p4[q];
+            v[4 * q] = w.x; v[4 * q + 1] = w.y; v[4 * q + 2] = w.z; v[4 * q + 3] = w.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; ++k) v[k] = (base + k < n) ? in[base + k] : 0u;
+    }
+    uint32_t pre = 0u;
+    for (uint32_t i = threadIdx.x; i < tile; i += SCAN_THREADS) pre += __ldg(sums + i);
+    uint32_t s = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; ++k) s += v[k];
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t inc = warp_incl_scan(s);
+    pre = __reduce_add_sync(0xffffffffu, pre);
+    if (lane == 31) {
+        warp_tot[warp] = inc;
+        warp_pre[warp] = pre;
+    }
+    __syncthreads();
+    uint32_t run = inc - s;
+#pragma unroll
+    for (int w = 0; w < SCAN_THREADS / 32; ++w) run += warp_pre[w] + ((unsigned)w < warp ? warp_tot[w] : 0u);
+    if (whole) {
+        uint4* o4 = reinterpret_cast<uint4*>(out + base);
+        uint4* z4 = reinterpret_cast<uint4*>(in + base);
+#pragma unroll
+        for (int q = 0; q < SCAN_ITEMS / 4; ++q) {
+            uint4 w;
+            w.x = run; run += v[4 * q];
+            w.y = run; run += v[4 * q + 1];
+            w.z = run; run += v[4 * q + 2];
+            w.w = run; run += v[4 * q + 3];
+            o4[q] = w;
+            z4[q] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        if (base + SCAN_ITEMS == n) out[n] = run;   // total after the last cell
+    } else {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; ++k) {
+            const uint32_t idx = base + k;
+            if (idx < n) {
+                out[idx] = run;
+                in[idx] = 0u;
+            }
+            run += v[k];
+            if (idx + 1 == n) out[n] = run;
+        }
+    }
+}
+
 // The cell starts are invalid once a wait of the scan ran out, and the cell
 // order is incomplete once the rank pass met a cell of more than
 // SPH_MAX_CELL_OCC particles (it writes no slot of that cell): every pass
@@ -327,15 +417,18 @@ __device__ __forceinline__ bool step_failed(const uint32_t* status) {
 }
 
 // ---------------------------------------------------------------------------
-// Scatter: provisional slot of each particle in cell order.
+// Scatter: provisional slot of each particle in cell order.  The scan's tile
+// sums (nsums of them) are left at zero for the next hash.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(SPH_TILE) k_scatter(const DevScene* __restrict__ scenes,
                                                       const uint4* __restrict__ tiles,
                                                       const uint32_t* __restrict__ start,
                                                       const uint32_t* __restrict__ key,
                                                       const uint32_t* __restrict__ slot,
-                                                      uint32_t* __restrict__ tmp,
+                                                      uint32_t* __restrict__ tmp, uint32_t* __restrict__ sums,
+                                                      uint32_t nsums,
                                                       const uint32_t* __restrict__ status) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nsums; i += gridDim.x * blockDim.x) sums[i] = 0u;
     if (step_failed(status)) return;
     const uint4 t = tiles[blockIdx.x];
     if (threadIdx.x >= t.z) return;
@@ -1016,7 +1109,9 @@ k_force_integrate(const DevParams* __restrict__ params,
                                                               float4* __restrict__ P0, float4* __restrict__ V2,
                                                               float4* __restrict__ A0, uint32_t* __restrict__ maxdisp,
                                                               uint32_t* __restrict__ okey, uint32_t* __restrict__ pend,
-                                                              uint32_t* __restrict__ count, uint32_t* __restrict__ key,
+                                                              uint32_t* __restrict__ count,
+                                                              uint32_t* __restrict__ sums,
+                                                              uint32_t* __restrict__ key,
                                                               uint32_t* __restrict__ slot, uint32_t* __restrict__ status,
                                                               float4* __restrict__ dbg_forces, uint32_t ntiles,
                                                               uint32_t* __restrict__ tile_ctr) {
@@ -1229,17 +1324,8 @@ k_force_integrate(const DevParams* __restrict__ params,
     const bool inside_new = grid_inside(pp, gn);
     if (!(isfinite(px) && isfinite(py) && isfinite(pz))) atomicOr(status, SPH_STATUS_NONFINITE);
     const uint32_t local = inside_new ? (uint32_t)gn.x + (uint32_t)gn.y * pp.gx + (uint32_t)gn.z * pp.gxy : pp.ncells;
-    {
-        const uint32_t gkey = sc.cell_base + local;
-        const unsigned lane = threadIdx.x & 31u;
-        const unsigned peers = __match_any_sync(lanes, gkey);
-        const int leader = __ffs(peers) - 1;
-        uint32_t base = 0;
-        if ((int)lane == leader) base = atomicAdd(&count[gkey], (uint32_t)__popc(peers));
-        base = __shfl_sync(peers, base, leader);
-        key[k] = local;
-        slot[k] = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-    }
+    key[k] = local;
+    slot[k] = count_cell(lanes, sc.cell_base + local, count, sums);
     okey[k] = grid_inside(pp, g)
                   ? (pack_cell(g) | ((inside_new && pack_cell(gn) == pack_cell(g)) ? 0u : SPH_OKEY_MOVED))
                   : SPH_OKEY_NULL;
@@ -1507,9 +1593,12 @@ cudaError_t launch_build_tiles(const DevScene* scenes, const uint32_t* tile_firs
     k_build_tiles<<<nscenes, 128, 0, st>>>(scenes, tile_first, tile, tiles);
     return cudaGetLastError();
 }
+static uint32_t scan_tiles(uint32_t cells) { return (cells + SCAN_TILE - 1) / SCAN_TILE; }
 cudaError_t launch_hash(const StepArgs& a, cudaStream_t st) {
     k_hash<<<a.ntiles, a.block, 0, st>>>(a.params, a.scenes, a.tiles, a.P0, a.count, a.key, a.slot, a.pend, a.okey,
                                          a.status);
+    // an unsorted state's warps are spread over the tiles: their sums from the counts
+    k_scan_reduce<<<scan_tiles(a.total_cells), SCAN_THREADS, 0, st>>>(a.count, a.total_cells, a.sums);
     return cudaGetLastError();
 }
 static inline uint32_t* ctr(const StepArgs& a, int k) { return a.tile_ctr ? a.tile_ctr + k : nullptr; }
@@ -1534,6 +1623,10 @@ cudaError_t init_kernel_attributes() {
     return cudaSuccess;
 }
 
+// Whether this scan covers every scene's cells and consumes the counts: the
+// tile sums are then this scan's, and cleared after it.
+static bool whole_scan(const StepArgs& a) { return a.scan_cells == 0u && a.scan_zeroes_counts != 0u; }
+
 // a.scan_sums holds at least nt + 2 64-bit words: the tile counter, then one
 // look-back descriptor per tile; they start at zero.  With scan_withhold the
 // counter starts at 1 instead: the blocks take tiles 1..nt, no block takes
@@ -1544,6 +1637,11 @@ cudaError_t init_kernel_attributes() {
 cudaError_t launch_scan(const StepArgs& a, cudaStream_t st) {
     const uint32_t n = a.scan_cells ? a.scan_cells : a.total_cells;
     if (n == 0) return cudaErrorInvalidValue;
+    if (whole_scan(a) && scan_tiles(n) <= SPH_SCAN_SUM_TILES && !a.scan_spin_limit && !a.scan_withhold) {
+        // (the test controls are the look-back's)
+        k_scan_tiles<<<scan_tiles(n), SCAN_THREADS, 0, st>>>(a.count, n, a.sums, a.start);
+        return cudaGetLastError();
+    }
     uint32_t* counts = a.count + a.scan_first;
     uint32_t* starts = a.start + a.scan_first;
     const uint32_t vec_ok = ((reinterpret_cast<uintptr_t>(counts) | reinterpret_cast<uintptr_t>(starts)) & 15u) == 0u;
@@ -1576,7 +1674,8 @@ static float* axes(const StepArgs& a) {
     return reinterpret_cast<float*>(a.mask + (a.skin_masks ? SPH_AXIS_ROWS_SKIN : SPH_MASK_SKIN) * a.mask_stride);
 }
 cudaError_t launch_sort(const StepArgs& a, cudaStream_t st) {
-    k_scatter<<<a.ntiles, a.block, 0, st>>>(a.scenes, a.tiles, a.start, a.key, a.slot, a.tmp, a.status);
+    k_scatter<<<a.ntiles, a.block, 0, st>>>(a.scenes, a.tiles, a.start, a.key, a.slot, a.tmp, a.sums,
+                                            whole_scan(a) ? scan_tiles(a.total_cells) : 0u, a.status);
     k_rank_gather<<<a.ntiles, a.block, 0, st>>>(a.scenes, a.tiles, a.start, a.key, a.tmp, a.P0, a.V0, a.A0, a.V2,
                                                 a.okey, a.pend, a.G, axes(a), a.A1, a.perm, a.status);
     return cudaGetLastError();
@@ -1641,7 +1740,7 @@ cudaError_t launch_force(const StepArgs& a, cudaStream_t st) {
            l > 1 ? wide_smem(l) : rows_smem(a), st>>>(
                                                     a.params, a.scenes, a.tiles, a.start, a.R, a.rho, a.A1, a.N,
                                                     a.mask, a.mask_stride, a.P0, a.V2, a.A0,
-                                                    a.skin_masks ? a.maxdisp : nullptr, a.okey, a.pend, a.count,
+                                                    a.skin_masks ? a.maxdisp : nullptr, a.okey, a.pend, a.count, a.sums,
                                                     a.key, a.slot, a.status, a.dbg_forces, a.ntiles, ctr(a, 2));
     return cudaGetLastError();
 }

@@ -24,7 +24,9 @@ struct StepArgs {
     uint32_t *pend;            // per scene: its last XSPH update is pending
     float *rho;                // density per sorted slot
     float4 *N;                 // normals
-    uint32_t *count, *start, *scan_sums;
+    uint32_t *count, *start;
+    uint32_t *sums;                // the counts' sums per scan tile (kScanTileCells cells), zero where the counts are
+    uint32_t *scan_sums;           // look-back descriptors
     uint32_t scan_first;           // the scan covers cells [scan_first, scan_first + scan_cells) (one scene's
     uint32_t scan_cells;           // range for a single scene's prefix; else 0 and total_cells)
     uint32_t scan_zeroes_counts;   // nonzero: the scan leaves every count it read at zero for the next hash
@@ -66,9 +68,13 @@ cudaError_t launch_build_tiles(const DevScene* scenes, const uint32_t* tile_firs
                                uint4* tiles, cudaStream_t st);
 cudaError_t launch_hash(const StepArgs& a, cudaStream_t st);
 cudaError_t launch_scan(const StepArgs& a, cudaStream_t st);
-// Cells per scan tile, and the most tiles launch_scan_raw takes (k_scan_top
-// scans them in one block of 1024 threads, 32 sums each).
-constexpr uint32_t kScanTileCells = 4096u;
+constexpr uint32_t kScanTileCells = 4096u;   // cells per scan tile
+// Most tiles whose scan adds up the tile sums before each tile (k_scan_tiles).
+#ifndef SPH_SCAN_SUM_TILES
+#define SPH_SCAN_SUM_TILES 16384u
+#endif
+// The most tiles launch_scan_raw takes (k_scan_top scans them in one block of
+// 1024 threads, 32 sums each).
 constexpr uint32_t kScanRawMaxTiles = 1024u * 32u;
 // Exclusive scan of counts[0,n) into starts[0,n] with caller-provided tile
 // sums (ceil(n/kScanTileCells) entries, at most kScanRawMaxTiles).
