@@ -135,7 +135,7 @@ int sph_batch_sync(sph_batch* b) {
 
 int sph_batch_get_state(sph_batch* b, int scene_id, float* pos, float* colour, float* vel, uint32_t n) {
     if (!b) return SPH_EINVAL;
-    return berr(b, b->eng->get_state(scene_id, pos, colour, vel, n));
+    return berr(b, b->eng->get_state(scene_id, pos, colour, vel, n, false, true));
 }
 
 int sph_batch_snapshot(sph_batch* b, int scene_id, void* buf, uint64_t cap, uint64_t* written) {

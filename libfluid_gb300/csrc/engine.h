@@ -73,7 +73,11 @@ public:
     int set_state(int id, const float* pos, const float* vel, uint32_t n, bool from_device = false);
     int set_positions(int id, uint32_t first, const float* pos, uint32_t count);
     int generate_lattice(int id, const LatticeSpec& spec, uint32_t first);
-    int get_state(int id, float* pos, float* colour, float* vel, uint32_t n, bool to_device = false);
+    // With `many`, the caller reads several scenes between steps: from the
+    // second read on, one prefix over all scenes (which the next step then
+    // starts from) serves them instead of one prefix per scene.
+    int get_state(int id, float* pos, float* colour, float* vel, uint32_t n, bool to_device = false,
+                  bool many = false);
     // Exact state (3n float4 on the host: positions, velocities,
     // accelerations, in slot order, w lanes included) for snapshot/resume.
     int save_state(int id, float4* host, uint32_t n);
@@ -250,6 +254,10 @@ private:
     // host mirrors
     DevParams* h_params_ = nullptr;    // pinned
     uint32_t* h_status_ = nullptr;     // pinned
+    // Pinned landing place of small exports (kSmallExport bytes): the kernels
+    // write into it directly and the host copies from there.
+    float* h_small_ = nullptr;
+    uint32_t reads_ = 0;               // scene reads since the last step or change (get_state with `many`)
     std::vector<DevScene> h_scenes_;
     std::vector<uint32_t> h_tile_first_;   // per scene: its first tile (the tiles are built on the device)
     uint32_t ntiles_ = 0;

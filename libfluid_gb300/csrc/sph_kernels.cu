@@ -1437,8 +1437,10 @@ __global__ void __launch_bounds__(SPH_TILE) k_unsort_vel(const uint4* __restrict
                                                          float* __restrict__ out, float4* __restrict__ V0,
                                                          uint32_t* __restrict__ pend,
                                                          const uint32_t* __restrict__ status,
-                                                         uint32_t* __restrict__ gate, uint32_t n) {
+                                                         uint32_t* __restrict__ gate, uint32_t n,
+                                                         uint32_t* __restrict__ status_out) {
     const uint4 t = tiles[blockIdx.x];
+    if (status_out && blockIdx.x == 0 && threadIdx.x == 0) *status_out = __ldcg(status);
     // the status word of a force pass run ahead (launch_unsort_vel): it
     // starts failed, so that pass does nothing, when the prefix reported an error
     if (gate && blockIdx.x == 0 && threadIdx.x == 0) *gate = __ldcg(status) != 0u ? SPH_STATUS_SCAN_TIMEOUT : 0u;
@@ -1708,10 +1710,11 @@ cudaError_t launch_density(const StepArgs& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 cudaError_t launch_unsort_vel(const StepArgs& a, uint32_t first_tile, uint32_t ntiles, uint32_t base, uint32_t n,
-                              float* out, float4* V0, bool clear_pending, cudaStream_t st, uint32_t* gate) {
+                              float* out, float4* V0, bool clear_pending, cudaStream_t st, uint32_t* gate,
+                              uint32_t* status_out) {
     if (ntiles == 0) return cudaSuccess;
     k_unsort_vel<<<ntiles, a.block, 0, st>>>(a.tiles + first_tile, a.perm, a.R, base, out, V0,
-                                             clear_pending ? a.pend : nullptr, a.status, gate, n);
+                                             clear_pending ? a.pend : nullptr, a.status, gate, n, status_out);
     return cudaGetLastError();
 }
 cudaError_t launch_undo_ahead(const StepArgs& a, uint32_t first_tile, uint32_t ntiles, cudaStream_t st) {

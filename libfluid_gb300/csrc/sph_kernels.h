@@ -90,9 +90,11 @@ cudaError_t launch_xsph(const StepArgs& a, cudaStream_t st);
 // slot - base) and/or into V0; optionally clears the scene's pending flag.
 // Does nothing after a failed prefix.  With `gate`, also
 // sets that word up as the status word of a force pass run ahead: failed (the
-// pass does nothing) when a.status reports an error.
+// pass does nothing) when a.status reports an error.  With `status_out` (which
+// may be pinned host memory), leaves the status word there.
 cudaError_t launch_unsort_vel(const StepArgs& a, uint32_t first_tile, uint32_t ntiles, uint32_t base, uint32_t n,
-                              float* out, float4* V0, bool clear_pending, cudaStream_t st, uint32_t* gate = nullptr);
+                              float* out, float4* V0, bool clear_pending, cudaStream_t st, uint32_t* gate = nullptr,
+                              uint32_t* status_out = nullptr);
 // Undo a force pass run ahead (one scene whose XSPH update was pending, over
 // its tiles): P0, V2, A0 and okey back from the prefix's gathered copies.
 cudaError_t launch_undo_ahead(const StepArgs& a, uint32_t first_tile, uint32_t ntiles, cudaStream_t st);
