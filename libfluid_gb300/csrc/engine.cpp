@@ -76,7 +76,6 @@ bool derive_params(const SceneConfig& c, DevParams& d, std::string* err) {
     d.gamma = c.gamma;
     const float inv_gamma = (c.gamma == 0.0f) ? 1.0f : 1.0f / c.gamma;
     d.eos_k = c.gas_constant * c.rest_density * inv_gamma;
-    d.cs_k = c.gas_constant / d.inv_rest_density;
     d.mass = c.mass;
     d.two_mass = 2.0f * c.mass;
     d.particle_size = c.particle_size;
@@ -106,7 +105,7 @@ bool derive_params(const SceneConfig& c, DevParams& d, std::string* err) {
     return true;
 }
 
-// six float4 arrays, the gathered state and the records of two each; key, slot, perm, okey and rho
+// six float4 arrays, the gathered state and the records of two each; key, slot, perm, okey and C2
 // (the sort's scatter list shares the mask words)
 uint64_t Engine::bytes_per_particle() { return 6 * 16 + 2 * 32 + 5 * 4 + SPH_MASK_ROWS * 4; }
 uint64_t Engine::bytes_per_cell() { return 2 * 4 + 1; }
@@ -174,8 +173,8 @@ int Engine::cuda_fail(cudaError_t e, const char* what) {
 void Engine::free_all() {
     float4** f4[] = {&P0_, &G_, &V0_, &V2_, &A0_, &A1_, &N_, &R_, &dbg_forces_};
     for (auto p : f4) { if (*p) cudaFree(*p); *p = nullptr; }
-    if (rho_) cudaFree(rho_);
-    rho_ = nullptr;
+    if (C2_) cudaFree(C2_);
+    C2_ = nullptr;
     uint32_t** u[] = {&key_, &slot_, &perm_, &count_, &start_, &scan_sums_, &dbg_nbr_, &mask_, &sums_,
                       &okey_, &pend_};
     for (auto p : u) { if (*p) cudaFree(*p); *p = nullptr; }
@@ -204,11 +203,11 @@ int Engine::ensure_capacity(uint64_t parts, uint64_t cells) {
         if (np >= (1ull << 31)) return fail(ENG_ENOMEM, "particle capacity exceeds 2^31");
         // state between substeps: P0, V0, A0, and for scenes with a pending
         // XSPH update their post-integration velocities V2 and cells; and the
-        // fields of the last substep that the debug taps read (rho, R)
+        // fields of the last substep that the debug taps read (C2, R)
         struct Kept { void** p; size_t entry; };
         const Kept state[] = {{(void**)&P0_, sizeof(float4)}, {(void**)&V0_, sizeof(float4)},
                               {(void**)&A0_, sizeof(float4)}, {(void**)&V2_, sizeof(float4)},
-                              {(void**)&R_, 2 * sizeof(float4)}, {(void**)&rho_, sizeof(float)},
+                              {(void**)&R_, 2 * sizeof(float4)}, {(void**)&C2_, sizeof(float)},
                               {(void**)&okey_, sizeof(uint32_t)}};
         struct { float4** p; uint64_t per_slot; } scratch[] = {{&G_, 2}, {&A1_, 1}, {&N_, 1}};
         for (const Kept& k : state) {
@@ -527,7 +526,7 @@ StepArgs Engine::args() const {
     a.total_cells = total_cells_;
     a.P0 = P0_; a.V0 = V0_; a.A0 = A0_;
     a.G = G_; a.A1 = A1_;
-    a.V2 = V2_; a.rho = rho_; a.N = N_;
+    a.V2 = V2_; a.C2 = C2_; a.N = N_;
     a.R = R_; a.okey = okey_; a.pend = pend_;
     a.count = count_; a.start = start_; a.sums = sums_; a.scan_sums = scan_sums_;
     a.scan_first = 0u;
@@ -951,7 +950,7 @@ int Engine::set_state(int id, const float* pos, const float* vel, uint32_t n, bo
         }
     }
     clear_pending(*s);
-    ENG_CK(launch_unpack(dpos, dvel, n, s->part_base, P0_, V0_, A0_, rho_, stream_), "unpack");
+    ENG_CK(launch_unpack(dpos, dvel, n, s->part_base, P0_, V0_, A0_, C2_, R_, stream_), "unpack");
     ENG_CK(cudaStreamSynchronize(stream_), "upload sync");
     return ENG_OK;
 }
@@ -987,7 +986,7 @@ int Engine::generate_lattice(int id, const LatticeSpec& spec, uint32_t first) {
     if (s->pending) { int rc = materialize(*s); if (rc) return rc; }
     prefix_valid_ = false;
     hashed_ = false;
-    ENG_CK(launch_lattice(spec, s->part_base + first, P0_, V0_, A0_, rho_, stream_), "lattice");
+    ENG_CK(launch_lattice(spec, s->part_base + first, P0_, V0_, A0_, C2_, R_, stream_), "lattice");
     return ENG_OK;
 }
 
@@ -1180,7 +1179,8 @@ int Engine::load_state(int id, const float4* host, uint32_t n) {
     ENG_CK(cudaMemcpyAsync(V0_ + s->part_base, host + n, bytes, cudaMemcpyHostToDevice, stream_), "restore");
     ENG_CK(cudaMemcpyAsync(A0_ + s->part_base, host + 2 * (size_t)n, bytes, cudaMemcpyHostToDevice, stream_),
            "restore");
-    ENG_CK(cudaMemsetAsync(rho_ + s->part_base, 0, n * sizeof(float), stream_), "restore");
+    ENG_CK(cudaMemsetAsync(C2_ + s->part_base, 0, n * sizeof(float), stream_), "restore");
+    ENG_CK(cudaMemsetAsync(R_ + 2 * (size_t)s->part_base, 0, 2 * bytes, stream_), "restore");
     ENG_CK(cudaStreamSynchronize(stream_), "restore sync");
     return ENG_OK;
 }
@@ -1249,22 +1249,13 @@ int Engine::debug_get(int id, int field, void* host, uint64_t count) {
         case F_PRESSURE:
         case F_SOUNDSPEED: {
             if (!need(n)) return fail(ENG_EINVAL, "buffer too small");
-            float* out = (float*)host;
-            ENG_CK(cudaMemcpy(out, rho_ + pb, n * sizeof(float), cudaMemcpyDeviceToHost), "debug copy");
-            if (field == F_DENSITY) return ENG_OK;
-            // pressure and squared sound speed from the record's (rho/rho0)^gamma;
-            // both are zero outside the grid (rho 0) and where the summed
-            // density is zero (-0 in the record)
-            std::vector<float4> v((size_t)n * 2);
-            ENG_CK(cudaMemcpy(v.data(), R_ + 2 * (size_t)pb, (size_t)n * 2 * sizeof(float4), cudaMemcpyDeviceToHost),
-                   "debug copy");
-            const DevParams& d = s->dp;
-            for (uint32_t i = 0; i < n; ++i) {
-                const float e = v[2 * (size_t)i + 1].w;
-                const bool none = out[i] == 0.0f || (e == 0.0f && std::signbit(e));
-                if (field == F_PRESSURE) out[i] = none ? 0.0f : d.eos_k * (e - 1.0f);
-                else out[i] = none ? 0.0f : d.gas_constant * std::pow(std::fabs(e), (d.gamma - 1.0f) / d.gamma);
+            if (field == F_SOUNDSPEED) {
+                ENG_CK(cudaMemcpy(host, C2_ + pb, n * sizeof(float), cudaMemcpyDeviceToHost), "debug copy");
+                return ENG_OK;
             }
+            // the w lanes of the records
+            ENG_CK(cudaMemcpy2D(host, sizeof(float), (const float*)(R_ + 2 * (size_t)pb) + (field == F_DENSITY ? 3 : 7),
+                                2 * sizeof(float4), sizeof(float), n, cudaMemcpyDeviceToHost), "debug copy");
             return ENG_OK;
         }
         case F_FPRESSURE:

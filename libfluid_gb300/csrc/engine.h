@@ -229,7 +229,7 @@ private:
     float4 *P0_ = nullptr, *G_ = nullptr, *V0_ = nullptr, *V2_ = nullptr, *A0_ = nullptr,   // G_: two per slot
           
            *A1_ = nullptr, *N_ = nullptr, *R_ = nullptr;   // R_: two per slot
-    float* rho_ = nullptr;
+    float* C2_ = nullptr;
     uint32_t *okey_ = nullptr;         // packed cells of the last substep (state order)
     uint32_t *pend_ = nullptr;                      // per scene-table entry: XSPH update pending
     uint32_t *key_ = nullptr, *slot_ = nullptr, *perm_ = nullptr;

@@ -19,11 +19,11 @@
 //             scan, four slots at a time: their x, their y, their z, 48 bytes
 //             in all (they lie in rows of the neighbour words that the density
 //             pass does not write)
-//   rho       density per sorted slot
 //   R         neighbour record per sorted slot, 32 bytes, written by the
-//             density pass: (x, y, z, 1/rho) and (velocity with the pending
-//             XSPH update applied, (rho/rho0)^gamma); see density_record
-//   N         surface normals (only when a scene has surface tension)
+//             density pass: (x, y, z, rho) and (velocity with the pending
+//             XSPH update applied, pressure)
+//   C2        squared sound speed per sorted slot
+//   N         surface normals, w: C2 again (only when a scene has surface tension)
 #include <cfloat>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -530,17 +530,12 @@ __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevScene* __rest
 // corrected velocity goes to the record R, which the force pass reads; without
 // a pending update it is G's.
 //
-// The record.  All that a later pass needs of a neighbour sits in 32 bytes,
-// one sector, fetched by one 256-bit load: position, velocity, q = 1/rho and
-// e = (rho/rho0)^gamma.  Pressure, squared sound speed and 1/rho^2 follow as
-// eos_k (e - 1), cs_k e q and q^2 (a few multiplications per pair against a
-// third and half of a second gather).  e is stored instead of the pressure
-// because the sound speed of a thin spray ((rho/rho0)^7 near 0) would cancel
-// in p + eos_k.
-// Measured against separate gathers of position, (rho, p, c^2, 1/rho^2) and
-// velocity (48 bytes in three requests): force pass 230 -> 196 us on the 1M
-// dam break, 2.19 -> 1.86 ms on the 8M tension scene, whose normal pass (one
-// 16-byte gather instead of two) went from 1.16 to 1.09 ms.
+// The record.  Position, density, velocity and pressure of a neighbour sit in 32
+// bytes, one sector, fetched by one 256-bit load; the squared sound speed comes
+// from C2, or with surface tension from the normal's w lane, and 1/rho^2 is
+// formed per pair (rcp_exact).  Against separate gathers of position, (rho, p,
+// c^2, 1/rho^2) and velocity (48 bytes in three requests) the force pass of the
+// 1M dam break went from 230 to 196 us, before the neighbour lists.
 // ---------------------------------------------------------------------------
 #ifndef DENSITY_MINB
 #define DENSITY_MINB 4
@@ -592,34 +587,29 @@ struct CandidateScan {
 };
 
 // A particle outside the grid: no density, its velocity kept.
-__device__ __forceinline__ void density_outside(uint32_t k, const float4& p, const float4& v, float* rho_out, float4* R,
+__device__ __forceinline__ void density_outside(uint32_t k, const float4& p, const float4& v, float* C2, float4* R,
                                                 uint32_t* nbr_out) {
-    rho_out[k] = 0.f;
+    C2[k] = 0.f;
     st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, 0.f), make_float4(v.x, v.y, v.z, 0.f));
     if (nbr_out) nbr_out[k] = 0;
 }
-// The density, its equation of state and the record of slot k from the sums of
-// (h^2 - r^2)^3 and, with xs, of XSPH's (ax, ay, az).
+// The density, its equation of state and the record of slot k from the pair
+// sums (with xs, XSPH's too).
 __device__ __forceinline__ void density_finish(const DevParams& pp, uint32_t k, float sum, bool xs, float ax, float ay,
-                                               float az, const float4& p, float4 vi, float* rho_out, float4* R) {
-    sum = (pp.mass * pp.poly6) * sum;
+                                               float az, const float4& p, float4 vi, float* C2, float4* R) {
     const float d = fabsf(sdf(pp, p.x, p.y, p.z));
     float corr = sum;
     if (d < pp.h) corr = fmaf(pp.rest_density, 1.0f - boundary_density(pp, d), corr);
     const float rho = (sum == 0.0f) ? pp.rest_density : corr;
     const float ratio = corr * pp.inv_rest_density;
-    // no density at all (corr 0) has pressure 0: marked by -0
-    const float e = (corr == 0.0f) ? -0.0f : powf(ratio, pp.gamma) + 0.0f;
-    rho_out[k] = rho;
+    const float prs = (corr == 0.0f) ? 0.0f : pp.eos_k * (powf(ratio, pp.gamma) - 1.0f);
+    C2[k] = pp.gas_constant * powf(ratio, pp.gamma - 1.0f);
     if (xs) {
-        const float cx = pp.xsph * (pp.poly6 * pp.two_mass);
-        vi.x = fmaf(cx, ax, vi.x);
-        vi.y = fmaf(cx, ay, vi.y);
-        vi.z = fmaf(cx, az, vi.z);
+        vi.x = fmaf(pp.xsph, ax, vi.x);
+        vi.y = fmaf(pp.xsph, ay, vi.y);
+        vi.z = fmaf(pp.xsph, az, vi.z);
     }
-    // a density the later passes skip as a neighbour's (rho <= eps) is marked by 0
-    st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, rho > pp.eps ? 1.0f / rho : 0.0f),
-                   make_float4(vi.x, vi.y, vi.z, e));
+    st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, rho), make_float4(vi.x, vi.y, vi.z, prs));
 }
 
 template <bool SKIN>
@@ -629,7 +619,7 @@ k_density(const DevParams* __restrict__ params,
                                                       const uint4* __restrict__ tiles,
                                                       const uint32_t* __restrict__ start,
                                                       const float4* __restrict__ G, const float* __restrict__ X,
-                                                      float* __restrict__ rho_out,
+                                                      float* __restrict__ C2,
                                                       uint32_t* __restrict__ mask, size_t mask_stride,
                                                       const uint32_t* __restrict__ pend, float4* __restrict__ R,
                                                       uint32_t* __restrict__ nbr_out, uint32_t ntiles,
@@ -650,7 +640,7 @@ k_density(const DevParams* __restrict__ params,
     float4 p, vi;
     if (!grid_inside(pp, g)) {
         ld_float4_pair(G + 2 * (size_t)k, p, vi);
-        density_outside(k, p, vi, rho_out, R, nbr_out);
+        density_outside(k, p, vi, C2, R, nbr_out);
         return;
     }
     const uint32_t delta = sc.part_base - __ldg(start + sc.cell_base);
@@ -750,9 +740,7 @@ k_density(const DevParams* __restrict__ params,
 
     // ---- phase 2: the density pairs, in candidate order ----
     ld_float4_pair(G + 2 * (size_t)k, p, vi);
-    // Factors that are the same for every pair are left to the end: the sums
-    // hold (h^2 - r^2)^3, and for XSPH that over the densities' sum.
-    const float h = pp.h;
+    const float h = pp.h, mass = pp.mass, c6 = pp.poly6, two_m = pp.two_mass;
     float sum = 0.0f;
     uint32_t cnt = 0;
     // deferred XSPH of the previous substep (only for particles that had a cell then)
@@ -778,14 +766,13 @@ k_density(const DevParams* __restrict__ params,
         const float rr = dot3(dx, dy, dz, dx, dy, dz);
         // true for every listed neighbour of finite position; the test matters in the tail
         if (rr <= h2) {
-            const float x = h2_minus_r2(rr, h, h2);
-            const float w = x * x * x;
-            sum += w;
+            const float w = poly6_r2(rr, h, h2, c6);
+            sum = fmaf(mass, w, sum);
             cnt++;
             if (xs) {
                 const float rs = p.w + q.w;   // the previous substep's densities
                 if (rs > eps && cells_adjacent_fast(oi, oj)) {
-                    const float coeff = w * rcp_approx(rs);
+                    const float coeff = w * div_approx(two_m, rs);
                     axy = __ffma2_rn(make_float2(coeff, coeff), __fadd2_rn(make_float2(vj.x, vj.y), mvixy), axy);
                     az = fmaf(coeff, vj.z - vi.z, az);
                 }
@@ -803,7 +790,7 @@ k_density(const DevParams* __restrict__ params,
     if (hd.over)
         walk_tail(pp, start, sc.cell_base, delta, g, hd.n ? last + 1u : 0u,
                   [&](uint32_t j) { if (j != k) use(load(j)); });
-    density_finish(pp, k, sum, xs, axy.x, axy.y, az, p, vi, rho_out, R);
+    density_finish(pp, k, sum, xs, axy.x, axy.y, az, p, vi, C2, R);
     if (nbr_out) nbr_out[k] = cnt;
   });
 }
@@ -813,7 +800,7 @@ template <int LANES>
 __global__ void __launch_bounds__(kWideBlock, 7)
 k_density_wide(const DevParams* __restrict__ params, const DevScene* __restrict__ scenes,
                const uint4* __restrict__ tiles, const uint32_t* __restrict__ start, const float4* __restrict__ G,
-               const float* __restrict__ X, float* __restrict__ rho_out, uint32_t* __restrict__ mask,
+               const float* __restrict__ X, float* __restrict__ C2, uint32_t* __restrict__ mask,
                size_t mask_stride, const uint32_t* __restrict__ pend, float4* __restrict__ R,
                uint32_t* __restrict__ nbr_out, const uint32_t* __restrict__ status) {
   extern __shared__ uint4 s_dyn[];
@@ -830,7 +817,7 @@ k_density_wide(const DevParams* __restrict__ params, const DevScene* __restrict_
     ld_float4_pair(G + 2 * (size_t)k, p, vi);
     const int3 g = grid_of(pp, p.x, p.y, p.z);
     const bool work = act && grid_inside(pp, g);
-    if (act && !work) density_outside(k, p, vi, rho_out, R, nbr_out);   // (the same by every lane)
+    if (act && !work) density_outside(k, p, vi, C2, R, nbr_out);   // (the same by every lane)
     const uint32_t delta = sc.part_base - __ldg(start + sc.cell_base);
     const float h2 = pp.h2, h = pp.h, eps = pp.eps;
     const WideLanes<LANES> wl;
@@ -929,14 +916,15 @@ k_density_wide(const DevParams* __restrict__ params, const DevScene* __restrict_
     }
 
     // ---- phase 2 ----
-    // Terms: w, the XSPH coefficient, the velocity difference, and ones.  Lane 0
-    // sums w times one, lanes 1 to 3 the coefficient times a component, each in
+    // Terms: w, the XSPH coefficient, the velocity difference, and the mass.  Lane 0
+    // sums w times the mass, lanes 1 to 3 the coefficient times a component, each in
     // list order: the sums one thread forms, to the bit.
     uint32_t cnt = 0u;
     const uint32_t oi = pending ? __float_as_uint(vi.w) : SPH_OKEY_NULL;
     const bool xs = oi != SPH_OKEY_NULL;
     float acc = 0.0f;
-    ws.terms[5][wl.l] = 1.0f;
+    const float c6 = pp.poly6, two_m = pp.two_mass;
+    ws.terms[5][wl.l] = pp.mass;
     const float* scale = ws.terms[wl.l == 0u ? 0 : 1];
     const float* value = ws.terms[wl.l == 0u ? 5 : 1 + min(wl.l, 3u)];
     struct Nbr { float4 q, v; };
@@ -952,11 +940,10 @@ k_density_wide(const DevParams* __restrict__ params, const DevScene* __restrict_
         const float rr = dot3(dx, dy, dz, dx, dy, dz);
         on = on && rr <= h2 && j != k;
         if (on) {
-            const float x = h2_minus_r2(rr, h, h2);
-            w = x * x * x;
+            w = poly6_r2(rr, h, h2, c6);
             const float rs = p.w + n.q.w;   // the previous substep's densities
             if (xs && rs > eps && cells_adjacent_fast(oi, __float_as_uint(n.v.w))) {
-                c = w * rcp_approx(rs);
+                c = w * div_approx(two_m, rs);
                 dv = make_float3(n.v.x - vi.x, n.v.y - vi.y, n.v.z - vi.z);
             }
         }
@@ -981,7 +968,7 @@ k_density_wide(const DevParams* __restrict__ params, const DevScene* __restrict_
     if (cnt == SPH_OKEY_NULL) return;   // outside the grid
     ld_float4_pair(G + 2 * (size_t)k, p, vi);
     density_finish(pp, k, sums[0], pending && __float_as_uint(vi.w) != SPH_OKEY_NULL, sums[1], sums[2], sums[3], p, vi,
-                   rho_out, R);
+                   C2, R);
     if (nbr_out) nbr_out[k] = cnt;
   });
 }
@@ -998,7 +985,7 @@ __global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(c
                                                       const DevScene* __restrict__ scenes,
                                                       const uint4* __restrict__ tiles,
                                                       const uint32_t* __restrict__ start,
-                                                      const float4* __restrict__ R,
+                                                      const float4* __restrict__ R, const float* __restrict__ C2,
                                                       const uint32_t* __restrict__ mask, size_t mask_stride,
                                                       float4* __restrict__ N, uint32_t ntiles,
                                                       uint32_t* __restrict__ tile_ctr,
@@ -1027,10 +1014,17 @@ __global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(c
     float sz = 0.f;
     const float2 pxy = make_float2(p.x, p.y);
     // m gradPoly6(r) rvec / (rho_j r) = m c (h^2 - r^2)^2 rvec / rho_j: the
-    // factor r of gradPoly6 cancels the 1/r; m c, the same for every pair, is
-    // left to the end
+    // factor r of gradPoly6 cancels the 1/r; h^2 - r^2 is formed from the
+    // rounded root r as gradPoly6 forms it (it cancels near r = h)
+    const float mc = pp.mass * pp.grad_poly6;
     const float h2 = pp.h2, eps = pp.eps, h = pp.h;
-    auto load = [&](uint32_t j) { return __ldg(R + 2 * (size_t)j); };   // w = 1/rho_j, 0 where rho_j <= eps
+    auto load = [&](uint32_t j) { return __ldg(R + 2 * (size_t)j); };   // w = rho_j
+    // the pair's factor of rvec
+    auto grad = [&](float r2, float rhoj) {
+        const float r = sqrt_exact(r2, rsqrt_approx(r2));
+        const float x = fmaf(-r, r, h2);
+        return (r >= h) ? 0.0f : div_approx(mc * (x * x), rhoj);
+    };
     if constexpr (LANES > 1) {
         const WideLanes<LANES> wl;
         WideShared<LANES>& ws = reinterpret_cast<WideShared<LANES>*>(s_dyn)[threadIdx.x / LANES];
@@ -1041,12 +1035,9 @@ __global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(c
             [&](const float4& q, uint32_t, bool on) {
                 const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
                 const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-                on = on && r2 <= h2 && r2 > eps && q.w > 0.0f;
+                on = on && r2 <= h2 && r2 > eps && q.w > eps;
                 float s = 0.f;
-                if (on) {
-                    const float x = h2_minus_r2(r2, h, h2);
-                    s = (x * x) * q.w;
-                }
+                if (on) s = grad(r2, q.w);
                 ws.terms[0][wl.l] = s;
                 ws.terms[1][wl.l] = on ? rx : 0.f;
                 ws.terms[2][wl.l] = on ? ry : 0.f;
@@ -1059,20 +1050,20 @@ __global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(c
     } else {
         walk_neighbours<kNormalsDepth>(
             pp, start, sc.cell_base, delta, g, mask, mask_stride, k,
-            reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load, [&](const float4& q) {
+            reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load,
+            [&](const float4&) { return true; }, [&](const float4& q) {
                 const float2 rxy = __fadd2_rn(pxy, make_float2(-q.x, -q.y));
                 const float rx = rxy.x, ry = rxy.y, rz = p.z - q.z;
                 const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-                if (r2 <= h2 && r2 > eps && q.w > 0.0f) {
-                    const float x = h2_minus_r2(r2, h, h2);
-                    const float s = (x * x) * q.w;
+                if (r2 <= h2 && r2 > eps && q.w > eps) {
+                    const float s = grad(r2, q.w);
                     sxy = __ffma2_rn(make_float2(s, s), rxy, sxy);
                     sz = fmaf(s, rz, sz);
                 }
             });
     }
-    const float hc = pp.h * (pp.mass * pp.grad_poly6);
-    N[k] = make_float4(hc * sxy.x, hc * sxy.y, hc * sz, 0.f);
+    // w: the squared sound speed, so that the force pass gathers it with the normal
+    N[k] = make_float4(pp.h * sxy.x, pp.h * sxy.y, pp.h * sz, C2[k]);
   });
 }
 
@@ -1080,7 +1071,7 @@ __global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(c
 // Forces (computeAllForces, fluidphysics.cu:215-352) fused with the leapfrog
 // integrator and box boundary (LeapfrogIntegratorOperator,
 // fluidintegrator.cu:11-70).  Reads cell-order state (the density pass's
-// records R and densities, A1, N), writes the integrated state to P0 (w =
+// records R, C2, A1, N), writes the integrated state to P0 (w =
 // density), V2,
 // A0, each particle's cell to okey, and the next substep's hash of the new
 // positions (key, slot, cell counts), so that substep needs no hash pass.
@@ -1088,6 +1079,14 @@ __global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(c
 // force buffers in the reference's order, which after the swapped arguments
 // at fluidsystem.cu:352-364 is ((pressure + tension) + viscosity) + adhesion.
 // ---------------------------------------------------------------------------
+// Every operation and its rounding are those of the plain formulas in
+// fluidphysics.cu (as the oracle writes them), whatever form computes it: a
+// particle that rests against a wall takes the contact branch or not by its
+// last bit, so results stay comparable over many substeps only if all of them
+// agree to the bit.  Leaving the constant factors to the end of the sums and
+// h - r as (h^2 - r^2)/(h + r) measured 139 against 145 us (1M dam break) and
+// 1.22 against 1.33 ms (8M tension scene), but moved such particles.
+//
 // TENSION = false is the build for launches where no scene has surface
 // tension (the tension terms are then compiled out).  MINB is the register
 // budget as resident blocks of 256 threads per SM: 3 (80 registers, no
@@ -1102,7 +1101,7 @@ k_force_integrate(const DevParams* __restrict__ params,
                                                               const uint4* __restrict__ tiles,
                                                               const uint32_t* __restrict__ start,
                                                               const float4* __restrict__ R,
-                                                              const float* __restrict__ rho,
+                                                              const float* __restrict__ C2,
                                                               const float4* __restrict__ A1,
                                                               const float4* __restrict__ N,
                                                               const uint32_t* __restrict__ mask, size_t mask_stride,
@@ -1134,59 +1133,56 @@ k_force_integrate(const DevParams* __restrict__ params,
         prefetch_l1(A1 + t.y + blockIdx.x * (kWideBlock / LANES) + threadIdx.x);
     float4 pi, vi;
     ld_float4_pair(R + 2 * (size_t)k, pi, vi);
-    float ri = rho[k];
     int3 g = grid_of(pp, pi.x, pi.y, pi.z);
     const bool tension = TENSION && (pp.flags & 1u) != 0u;
     bool inside = grid_inside(pp, g);
     float fpx = 0.f, fpy = 0.f, fpz = 0.f;   // pressure
-    float fvx = 0.f, fvy = 0.f, fvz = 0.f;   // viscosity (the pressure is added after the sums)
+    float fvx = 0.f, fvy = 0.f, fvz = 0.f;   // "viscosity" (pressure re-added)
     float ftx = 0.f, fty = 0.f, ftz = 0.f;   // tension
     float fax = 0.f, fay = 0.f, faz = 0.f;   // adhesion
     const uint32_t delta = sc.part_base - __ldg(start + sc.cell_base);
     float4 ni = make_float4(0.f, 0.f, 0.f, 0.f);
     if (tension && inside) ni = N[k];
-    const float h2 = pp.h2, hh = pp.h, visc_eps = pp.visc_eps;
-    const float inv_ri2 = 1.0f / (ri * ri), eos_k = pp.eos_k, pri = eos_k * (vi.w - 1.0f), eqi = vi.w * pi.w;
-    // r > rsel selects the cohesion branch (never, were the coefficient 0)
-    const float coh = pp.mass / pp.surface_tension, rsel = pp.cohesion != 0.0f ? pp.halfh : INFINITY;
-    const float coh_near = pp.h6 * 0.0156f;
-    // One pair: neighbour j with its record and normal.  Every factor that is
-    // the same for all pairs is left to the end of the sums (it would cost an
-    // instruction per pair and a register), and each scalar is formed once:
-    // with s = (h - r)^2 / r (the spiky gradient over r without its
-    // coefficient), the pressure sum takes s mid rvec and the viscosity sum,
-    // which has the pressure in it again, only s Pi rvec (the pressure sum is
-    // added at the end).  j == k has r^2 = 0 and drops out with the coincident
-    // pairs.  Against one division, rounded root and pair of weighted vectors
-    // per term this took 18 of 145 M warp instructions from the pass: 196 -> 189
-    // us on the 1M dam break, 1.86 -> 1.69 ms on the 8M tension scene.
-    // press(sp, sv, r) and tens(c, r, dn) take the terms.
+    const float ri = pi.w, pri = vi.w, csi = C2[k], inv_ri2 = 1.0f / (ri * ri);
+    // 2 rho0 / (rho_i + rho_i) of the tension sum (fluidphysics.cu:293), once per particle
+    const float tden = (2.0f * pp.rest_density) / (ri + ri);
+    // per-scene constants of the pair loop, held in registers
+    const float h2 = pp.h2, hh = pp.h, visc_eps = pp.visc_eps, visc = -pp.viscosity;
+    const float mass = pp.mass, gsp = pp.grad_spiky;
+    const float sm = -pp.surface_tension * mass;
+    const Cohesion coh(pp);
+    // One pair: neighbour j with its record, and its normal with the squared
+    // sound speed.  press(mid, mp, c) takes the pressure and viscosity terms'
+    // scales and the spiky gradient along rvec; tens(t) the tension term.  Listed
+    // neighbours lie within h; those of the tail are tested by the caller (dist2).
+    // r is the correctly rounded root: h - r cancels, and pairs at r ~ h must see
+    // the reference's r; 1/r and the quotients only scale (approximate).  At
+    // r = h the gradient and the cohesion vanish with h - r.  j == k has r^2 = 0
+    // and drops out with the coincident pairs.
+    auto dist2 = [&](const float4& pj) {
+        const float rx = pj.x - pi.x, ry = pj.y - pi.y, rz = pj.z - pi.z;
+        return dot3(rx, ry, rz, rx, ry, rz);
+    };
     auto pair = [&](const float4& pj, const float4& vj, const float4& nj, auto&& press, auto&& tens) {
         const float rx = pj.x - pi.x, ry = pj.y - pi.y, rz = pj.z - pi.z;
         const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-        if (r2 <= h2 && r2 > FLT_MIN && pj.w > 0.0f) {
-            const float inv_r = rsqrt_approx(r2), r = r2 * inv_r;
-            const float hr = h_minus_r(r2, r, hh, h2);
+        if (r2 > FLT_MIN && pj.w > FLT_MIN) {
+            const float inv_r = rsqrt_approx(r2), r = sqrt_exact(r2, inv_r);
             // artificial viscosity -visc (cs_i + cs_j) mu / (rho_i + rho_j),
-            // mu = h ux / (r^2 + 0.01 h^2), only for approaching pairs (ux < 0),
-            // over -visc h cs_k; 1/(rho_i + rho_j) = q_j / (rho_i q_j + 1)
-            const float ux = dot3(vj.x - vi.x, vj.y - vi.y, vj.z - vi.z, rx, ry, rz);
-            const float den = pj.w * rcp_approx((r2 + visc_eps) * fmaf(ri, pj.w, 1.0f));
-            const float Pi = fminf(ux, 0.0f) * fmaf(vj.w, pj.w, eqi) * den;
-            // p_j/rho_i^2 + p_i/rho_j^2, p_j formed first: where rho is next to
-            // nothing, the terms overflow exactly where the reference's do
-            const float mid = fmaf(pri, pj.w * pj.w, eos_k * (vj.w - 1.0f) * inv_ri2);
-            const float hr2 = hr * hr;
-            const float sr = hr2 * inv_r;
-            const float3 rv = make_float3(rx, ry, rz);
-            press(sr * mid, sr * Pi, rv);
+            // mu = h ux / (r^2 + 0.01 h^2), only for approaching pairs (ux < 0)
+            const float ux = fminf(dot3(vj.x - vi.x, vj.y - vi.y, vj.z - vi.z, rx, ry, rz), 0.0f);
+            const float Pi = div_approx((visc * (csi + nj.w)) * (hh * ux), (r2 + visc_eps) * (ri + pj.w));
+            const float mid = vj.w * inv_ri2 + pri * rcp_exact(pj.w * pj.w);
+            const float hr = hh - r;
+            const float sr = (mass * ((gsp * hr) * hr)) * inv_r;
+            press(mid, mid + Pi, make_float3(sr * rx, sr * ry, sr * rz));
             if (tension) {
-                // Akinci cohesion + curvature (fluidphysics.cu:291-293), cohesion
-                // times 1/r, both over -sigma m.  With sigma == 0 the tension
-                // force is sigma * (finite sum) = 0, so the term is skipped.
-                const float t = hr2 * hr * r2;
-                tens(coh * ((r > rsel) ? t : fmaf(2.0f, t, -(coh_near * inv_r))), rv,
-                     make_float3(ni.x - nj.x, ni.y - nj.y, ni.z - nj.z));
+                // Akinci cohesion + curvature (fluidphysics.cu:291-293).  With
+                // sigma == 0 the tension force is sigma * (finite sum) = 0, so
+                // the term is skipped.
+                const float sc2 = (-mass * mass) * coh(r, hr) * inv_r;
+                tens(make_float3(sc2 * rx + sm * (ni.x - nj.x), sc2 * ry + sm * (ni.y - nj.y),
+                                 sc2 * rz + sm * (ni.z - nj.z)));
             }
         }
     };
@@ -1196,12 +1192,12 @@ k_force_integrate(const DevParams* __restrict__ params,
         ld_float4_pair(R + 2 * (size_t)j, r.p, r.v);
         r.n = make_float4(0.f, 0.f, 0.f, 0.f);
         if (tension) r.n = __ldg(N + j);
+        else r.n.w = __ldg(C2 + j);
         return r;
     };
     if constexpr (LANES > 1) {
-        // Terms: the two scales, rvec, then the cohesion's scale and the
-        // normals' difference.  Lanes 0 to 2 sum one component each, in list
-        // order.
+        // Terms: the two scales, the gradient, then the tension and its factor.
+        // Lanes 0 to 2 sum one component each, in list order.
         const WideLanes<LANES> wl;
         WideShared<LANES>& ws = reinterpret_cast<WideShared<LANES>*>(s_dyn)[threadIdx.x / LANES];
         const uint32_t axis = min(wl.l, 2u);
@@ -1209,22 +1205,20 @@ k_force_integrate(const DevParams* __restrict__ params,
         wide_neighbours(
             pp, start, sc.cell_base, delta, g, mask, mask_stride, k, act && inside, early, wl, ws, load,
             [&](const Nbr& r, uint32_t, bool on) {
-                float o[9] = {};
-                if (on)
+                float o[9] = {};   // (zeros for lanes without a pair, the tension's factor too: it may be infinite)
+                if (on && dist2(r.p) <= h2)
                     pair(r.p, r.v, r.n,
-                         [&](float sp, float sv, const float3& d) {
-                             o[0] = sp; o[1] = sv; o[2] = d.x; o[3] = d.y; o[4] = d.z;
+                         [&](float mid, float mp, const float3& c) {
+                             o[0] = mid; o[1] = mp; o[2] = c.x; o[3] = c.y; o[4] = c.z;
                          },
-                         [&](float c, const float3&, const float3& dn) {
-                             o[5] = c; o[6] = dn.x; o[7] = dn.y; o[8] = dn.z;
-                         });
+                         [&](const float3& t) { o[5] = t.x; o[6] = t.y; o[7] = t.z; o[8] = tden; });
 #pragma unroll
                 for (int c = 0; c < (TENSION ? 9 : 5); ++c) ws.terms[c][wl.l] = o[c];
             },
             [&]() {
                 sum_p = wide_sum<LANES>(ws.terms[0], ws.terms[2u + axis], sum_p);
                 sum_v = wide_sum<LANES>(ws.terms[1], ws.terms[2u + axis], sum_v);
-                if (tension) sum_t = wide_sum<LANES>(ws.terms[5], ws.terms[2u + axis], sum_t, ws.terms[6u + axis]);
+                if (tension) sum_t = wide_sum<LANES>(ws.terms[8], ws.terms[5u + axis], sum_t);
             });
         // the rest is one thread's work per particle: the block's first threads
         ws.terms[0][wl.l] = sum_p;
@@ -1237,43 +1231,31 @@ k_force_integrate(const DevParams* __restrict__ params,
         fvx = w.terms[1][0]; fvy = w.terms[1][1]; fvz = w.terms[1][2];
         ftx = w.terms[2][0]; fty = w.terms[2][1]; ftz = w.terms[2][2];
         ld_float4_pair(R + 2 * (size_t)k, pi, vi);
-        ri = rho[k];
         g = grid_of(pp, pi.x, pi.y, pi.z);
         inside = grid_inside(pp, g);
     } else if (inside) {
         walk_neighbours<kForceDepth>(
             pp, start, sc.cell_base, delta, g, mask, mask_stride, k,
-            reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load, [&](const Nbr& r) {
+            reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load,
+            [&](const Nbr& r) { return dist2(r.p) <= h2; }, [&](const Nbr& r) {
                 pair(r.p, r.v, r.n,
-                     [&](float sp, float sv, const float3& d) {
-                         fpx = fmaf(sp, d.x, fpx); fpy = fmaf(sp, d.y, fpy); fpz = fmaf(sp, d.z, fpz);
-                         fvx = fmaf(sv, d.x, fvx); fvy = fmaf(sv, d.y, fvy); fvz = fmaf(sv, d.z, fvz);
+                     [&](float mid, float mp, const float3& c) {
+                         fpx = fmaf(c.x, mid, fpx); fpy = fmaf(c.y, mid, fpy); fpz = fmaf(c.z, mid, fpz);
+                         fvx = fmaf(c.x, mp, fvx); fvy = fmaf(c.y, mp, fvy); fvz = fmaf(c.z, mp, fvz);
                      },
-                     [&](float c, const float3& d, const float3& dn) {
-                         ftx = fmaf(c, d.x, ftx) + dn.x;
-                         fty = fmaf(c, d.y, fty) + dn.y;
-                         ftz = fmaf(c, d.z, ftz) + dn.z;
+                     [&](const float3& t) {
+                         ftx = fmaf(tden, t.x, ftx); fty = fmaf(tden, t.y, fty); ftz = fmaf(tden, t.z, ftz);
                      });
             });
     }
     if (inside) {
-        // the factors left out of the sums
-        const float sp = pp.mass * pp.grad_spiky, sv = -pp.viscosity * hh * pp.cs_k * sp;
-        fpx = sp * fpx; fpy = sp * fpy; fpz = sp * fpz;
-        fvx = pp.viscosity * fmaf(sv, fvx, fpx);
-        fvy = pp.viscosity * fmaf(sv, fvy, fpy);
-        fvz = pp.viscosity * fmaf(sv, fvz, fpz);
-        if (tension) {
-            // sigma, -sigma m, and 2 rho0 / (rho_i + rho_i) of the tension sum (fluidphysics.cu:293)
-            const float st = pp.surface_tension * ((2.0f * pp.rest_density) / (ri + ri)) *
-                             (-pp.surface_tension * pp.mass);
-            ftx = st * ftx; fty = st * fty; ftz = st * ftz;
-        }
+        fvx = pp.viscosity * fvx; fvy = pp.viscosity * fvy; fvz = pp.viscosity * fvz;
+        ftx = pp.surface_tension * ftx; fty = pp.surface_tension * fty; ftz = pp.surface_tension * ftz;
         const float z = -fminf(sdf(pp, pi.x, pi.y, pi.z), 0.0f) * 0.25f * pp.inv_particle_size;
         if (z < 1.0f) {
             const float3 nb = sdf_normal(pp, pi.x, pi.y, pi.z);
             const float denom = 1.0f / powf(1.0f - z, 3.0f);
-            const float a = pp.adhesion * ri * pp.inv_rest_density * denom;
+            const float a = pp.adhesion * pi.w * pp.inv_rest_density * denom;
             fax = a * nb.x; fay = a * nb.y; faz = a * nb.z;
         }
     }
@@ -1313,7 +1295,7 @@ k_force_integrate(const DevParams* __restrict__ params,
         const float kk = (1.0f + pp.vdamp) * dot3(nb.x, nb.y, nb.z, vx, vy, vz);
         vx = fmaf(-kk, nb.x, vx); vy = fmaf(-kk, nb.y, vy); vz = fmaf(-kk, nb.z, vz);
     }
-    P0[k] = make_float4(px, py, pz, ri);
+    P0[k] = make_float4(px, py, pz, pi.w);
     V2[k] = make_float4(vx, vy, vz, 0.f);
     A0[k] = make_float4(anx, any, anz, 0.f);
     // The next substep's hash (k_hash's work, on the position just written):
@@ -1492,14 +1474,17 @@ __global__ void __launch_bounds__(SPH_TILE) k_undo_ahead(const uint4* __restrict
 // ---------------------------------------------------------------------------
 __global__ void k_unpack_state(const float* __restrict__ pos, const float* __restrict__ vel, uint32_t n,
                                uint32_t base, float4* __restrict__ P0, float4* __restrict__ V0,
-                               float4* __restrict__ A0, float* __restrict__ rho) {
+                               float4* __restrict__ A0, float* __restrict__ C2,
+                               float4* __restrict__ R) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t s = base + i;
     P0[s] = make_float4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], 0.f);
     V0[s] = vel ? make_float4(vel[3 * i], vel[3 * i + 1], vel[3 * i + 2], 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
     A0[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-    rho[s] = 0.f;
+    C2[s] = 0.f;
+    R[2 * (size_t)s].w = 0.f;
+    R[2 * (size_t)s + 1].w = 0.f;
 }
 
 // Overwrite positions of slots [base, base+n) keeping the rest of the state
@@ -1534,7 +1519,8 @@ __global__ void k_pack_state(const float4* __restrict__ P0, const float4* __rest
 // Lattice block with seeded jitter; site (ix,iy,iz) -> particle
 // (ix*ny + iy)*nz + iz.  Coordinate: lo + (i + 0.5)*spacing + (2u-1)*jitter.
 __global__ void k_lattice(LatticeSpec spec, uint32_t base, float4* __restrict__ P0, float4* __restrict__ V0,
-                          float4* __restrict__ A0, float* __restrict__ rho) {
+                          float4* __restrict__ A0, float* __restrict__ C2,
+                               float4* __restrict__ R) {
     const uint32_t n = spec.nx * spec.ny * spec.nz;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -1551,7 +1537,9 @@ __global__ void k_lattice(LatticeSpec spec, uint32_t base, float4* __restrict__ 
     P0[s] = make_float4(c[0], c[1], c[2], 0.f);
     V0[s] = make_float4(spec.vel[0], spec.vel[1], spec.vel[2], 0.f);
     A0[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-    rho[s] = 0.f;
+    C2[s] = 0.f;
+    R[2 * (size_t)s].w = 0.f;
+    R[2 * (size_t)s + 1].w = 0.f;
 }
 
 // Sorted hash for the debug tap: key of the particle now at each slot, with
@@ -1699,13 +1687,13 @@ cudaError_t launch_density(const StepArgs& a, cudaStream_t st) {
     if (l > 1) {
         auto kern = l == 8 ? k_density_wide<8> : k_density_wide<4>;
         kern<<<wide_grid(a, l), kWideBlock, wide_smem(l), st>>>(a.params, a.scenes, a.tiles, a.start, a.G, axes(a),
-                                                               a.rho, a.mask, a.mask_stride, a.pend, a.R, a.dbg_nbr,
+                                                               a.C2, a.mask, a.mask_stride, a.pend, a.R, a.dbg_nbr,
                                                                a.status);
         return cudaGetLastError();
     }
     const size_t smem = (size_t)SPH_NBR_SMEM_WORDS * a.block * sizeof(uint32_t);
     auto kern = a.skin_masks ? k_density<true> : k_density<false>;
-    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.G, axes(a), a.rho, a.mask, a.mask_stride,
+    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.G, axes(a), a.C2, a.mask, a.mask_stride,
                                             a.pend, a.R, a.dbg_nbr, a.ntiles, ctr(a, 0), a.status);
     return cudaGetLastError();
 }
@@ -1728,7 +1716,7 @@ cudaError_t launch_normals(const StepArgs& a, cudaStream_t st) {
     const int l = lanes(a);
     auto kern = l == 8 ? k_normals<8> : l == 4 ? k_normals<4> : k_normals<1>;
     kern<<<l > 1 ? wide_grid(a, l) : dim3(a.grid_nbr), l > 1 ? kWideBlock : a.block,
-           l > 1 ? wide_smem(l) : rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.mask,
+           l > 1 ? wide_smem(l) : rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.C2, a.mask,
                                                          a.mask_stride, a.N, a.ntiles, ctr(a, 1), a.status);
     return cudaGetLastError();
 }
@@ -1741,7 +1729,7 @@ cudaError_t launch_force(const StepArgs& a, cudaStream_t st) {
                                 : (occ ? k_force_integrate<false, 4> : k_force_integrate<false, 3>);
     kern<<<l > 1 ? wide_grid(a, l) : dim3(a.grid_nbr), l > 1 ? kWideBlock : a.block,
            l > 1 ? wide_smem(l) : rows_smem(a), st>>>(
-                                                    a.params, a.scenes, a.tiles, a.start, a.R, a.rho, a.A1, a.N,
+                                                    a.params, a.scenes, a.tiles, a.start, a.R, a.C2, a.A1, a.N,
                                                     a.mask, a.mask_stride, a.P0, a.V2, a.A0,
                                                     a.skin_masks ? a.maxdisp : nullptr, a.okey, a.pend, a.count, a.sums,
                                                     a.key, a.slot, a.status, a.dbg_forces, a.ntiles, ctr(a, 2));
@@ -1754,9 +1742,9 @@ cudaError_t launch_xsph(const StepArgs& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 cudaError_t launch_unpack(const float* pos, const float* vel, uint32_t n, uint32_t base, float4* P0, float4* V0,
-                          float4* A0, float* rho, cudaStream_t st) {
+                          float4* A0, float* C2, float4* R, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    k_unpack_state<<<(n + 255) / 256, 256, 0, st>>>(pos, vel, n, base, P0, V0, A0, rho);
+    k_unpack_state<<<(n + 255) / 256, 256, 0, st>>>(pos, vel, n, base, P0, V0, A0, C2, R);
     return cudaGetLastError();
 }
 cudaError_t launch_set_positions(const float* pos, uint32_t n, uint32_t base, float4* P0, cudaStream_t st) {
@@ -1770,11 +1758,11 @@ cudaError_t launch_pack(const float4* P0, const float4* V0, uint32_t n, uint32_t
     k_pack_state<<<(n + 255) / 256, 256, 0, st>>>(P0, V0, n, base, inv_rest_density, pos, colour, vel);
     return cudaGetLastError();
 }
-cudaError_t launch_lattice(const LatticeSpec& spec, uint32_t base, float4* P0, float4* V0, float4* A0, float* rho,
-                           cudaStream_t st) {
+cudaError_t launch_lattice(const LatticeSpec& spec, uint32_t base, float4* P0, float4* V0, float4* A0, float* C2,
+                           float4* R, cudaStream_t st) {
     const uint32_t n = spec.nx * spec.ny * spec.nz;
     if (n == 0) return cudaSuccess;
-    k_lattice<<<(n + 255) / 256, 256, 0, st>>>(spec, base, P0, V0, A0, rho);
+    k_lattice<<<(n + 255) / 256, 256, 0, st>>>(spec, base, P0, V0, A0, C2, R);
     return cudaGetLastError();
 }
 cudaError_t launch_sorted_keys(const DevParams* params, const float4* G, uint32_t n, uint32_t base,

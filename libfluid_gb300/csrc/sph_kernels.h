@@ -18,11 +18,11 @@ struct StepArgs {
     float4 *P0, *V0, *A0;      // state
     float4 *G, *A1;            // cell-ordered state (G: position and velocity, two per slot)
     float4 *V2;                // post-integration velocity (before XSPH)
-    float4 *R;                 // neighbour records, two per slot: (x, y, z, 1/rho), (velocity with any pending
-                               // XSPH update applied, (rho/rho0)^gamma)
+    float4 *R;                 // neighbour records, two per slot: (x, y, z, rho), (velocity with any pending
+                               // XSPH update applied, pressure)
     uint32_t *okey;            // each slot's cell in the last substep (packed; gathered into G's velocity w)
     uint32_t *pend;            // per scene: its last XSPH update is pending
-    float *rho;                // density per sorted slot
+    float *C2;                 // squared sound speed per sorted slot
     float4 *N;                 // normals
     uint32_t *count, *start;
     uint32_t *sums;                // the counts' sums per scan tile (kScanTileCells cells), zero where the counts are
@@ -100,12 +100,12 @@ cudaError_t launch_unsort_vel(const StepArgs& a, uint32_t first_tile, uint32_t n
 cudaError_t launch_undo_ahead(const StepArgs& a, uint32_t first_tile, uint32_t ntiles, cudaStream_t st);
 
 cudaError_t launch_unpack(const float* pos, const float* vel, uint32_t n, uint32_t base, float4* P0, float4* V0,
-                          float4* A0, float* rho, cudaStream_t st);
+                          float4* A0, float* C2, float4* R, cudaStream_t st);
 cudaError_t launch_set_positions(const float* pos, uint32_t n, uint32_t base, float4* P0, cudaStream_t st);
 cudaError_t launch_pack(const float4* P0, const float4* V0, uint32_t n, uint32_t base, float inv_rest_density,
                         float* pos, float* colour, float* vel, cudaStream_t st);
-cudaError_t launch_lattice(const LatticeSpec& spec, uint32_t base, float4* P0, float4* V0, float4* A0, float* rho,
-                           cudaStream_t st);
+cudaError_t launch_lattice(const LatticeSpec& spec, uint32_t base, float4* P0, float4* V0, float4* A0, float* C2,
+                           float4* R, cudaStream_t st);
 cudaError_t launch_sorted_keys(const DevParams* params, const float4* G, uint32_t n, uint32_t base,
                                uint32_t* out, cudaStream_t st);
 

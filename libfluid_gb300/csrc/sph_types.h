@@ -43,8 +43,7 @@ struct DevParams {
     float inv_h2;                 // 1/h^2, normalises displacements for the XSPH mask check
     float xsph_disp_limit2;       // (skin/2)^2 * 0.98: largest (displacement/h)^2 XSPH may accept
     float sphere_r;               // sphere boundary (flags bit2): radius about the box centre
-    float cs_k;                   // gas_constant * rho0: squared sound speed = cs_k (rho/rho0)^gamma / rho
-    uint32_t pad_;
+    uint32_t pad_[2];
 };
 
 // The skin words are built with radius (1 + skin) h (default skin below).

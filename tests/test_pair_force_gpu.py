@@ -2,14 +2,12 @@
 FP32 oracle.
 
 One pair per site, sites 4 h apart, so that each force is a single pair's
-term and nothing averages its error.  The distances cover both forms of h - r
-(the rounded root within h^2/256 of r = h, the quotient below), their line,
-both branches of the cohesion kernel, and pairs at and beyond h.
+term and nothing averages its error.  The distances cover both branches of the
+cohesion kernel, pairs near r = h, where h - r is a few ulp of r, and pairs
+beyond it.
 
-Tolerance: the two forms of h - r differ by half an ulp of r, at most 3e-5 of
-h - r where they meet (h - r = h/512), 6e-5 in its square; 1e-4 of the pair's
-own magnitude, the bar of every force test, covers it and the roundings of
-the few other factors.
+Tolerance: 1e-4 of the pair's own magnitude, the bar of every force test; half
+an ulp of r would be 3e-5 of h - r at r = h (1 - 2^-9).
 """
 import numpy as np
 import pytest
