@@ -826,49 +826,25 @@ k_density_wide(const DevParams* __restrict__ params, const DevScene* __restrict_
     // ---- phase 1: the lanes test up to 32 candidates of a row, four at a time ----
     wide_ranges(pp, start, sc.cell_base, delta, g, work, wl, ws);
     const CandidateScan<false> scan(p.x, p.y, p.z, h2, h2);
-    constexpr uint32_t kQuads = 8u / LANES;   // fours of candidates per lane
-    struct Chunk { float4 x[kQuads], y[kQuads], z[kQuads]; };
+    using Chunk = WideChunk<LANES>;
     auto fetch = [&](int r, uint32_t c) {
-        const uint32_t jb0 = ws.jb[r], mis = jb0 & 3u;
-        Chunk f = {};
-#pragma unroll
-        for (uint32_t q = 0u; q < kQuads; ++q) {
-            const uint32_t o = c + 4u * (wl.l + LANES * q);
-            if (o < ws.len[r] + mis) {
-                const float4* xp = reinterpret_cast<const float4*>(X) + 3 * (size_t)((jb0 - mis + o) / 4u);
-                f.x[q] = __ldg(xp);
-                f.y[q] = __ldg(xp + 1);
-                f.z[q] = __ldg(xp + 2);
-            }
-        }
+        const uint32_t jb0 = ws.jb[r];
+        Chunk f;
+        f.fetch(X, wl, (jb0 & ~3u) + c, jb0 + ws.len[r]);
         return f;
     };
-    // The hits of a chunk as a word, candidate b in bit 31 - b, without those
-    // outside the row and the particle itself.
+    // The hits of a row's chunk c.
     auto step = [&](int r, uint32_t c, const Chunk& f) {
-        const uint32_t jb0 = ws.jb[r], mis = jb0 & 3u, len = ws.len[r], alen = len ? len + mis : 0u;
-        uint32_t w = 0u;
-#pragma unroll
-        for (uint32_t q = 0u; q < kQuads; ++q) {
-            uint32_t m = 0u, none = 0u;
-            scan.visit4(f.x[q], f.y[q], f.z[q], m, none);
-            w |= m << (28u - 4u * (wl.l + LANES * q));
-        }
-#pragma unroll
-        for (uint32_t d = 1u; d < LANES; d *= 2u) w |= __shfl_xor_sync(~0u, w, d);
-        const uint32_t left = alen > 32u * c ? alen - 32u * c : 0u;
-        if (left < 32u) w &= ~(~0u >> left);
-        if (c == 0u) w &= ~0u >> mis;
-        const uint32_t so = k - (jb0 - mis + 32u * c);
-        if (so < 32u) w &= ~(0x80000000u >> so);
-        if (wl.l == 0u && len <= SPH_NBR_MAX_ROW && left != 0u) ws.words[r][c] = w;
+        const uint32_t jb0 = ws.jb[r], len = ws.len[r], first = (jb0 & ~3u) + 32u * c;
+        const uint32_t w = f.hits(scan, wl, first, jb0, jb0 + len, k);
+        if (wl.l == 0u && len <= SPH_NBR_MAX_ROW && first < jb0 + len) ws.words[r][c] = w;
         return (uint32_t)__popc(w);
     };
     // The list's rows: it ends before the first that does not fit.
     NbrHeader hd;
     uint32_t at[(8 + LANES) / LANES] = {};   // where this lane's rows begin in the list
     auto row_done = [&](int r, uint32_t hits) {
-        hd.over = hd.over || ws.len[r] > SPH_NBR_MAX_ROW || hd.n + hits > SPH_NBR_CAP;
+        hd.over = hd.over || ws.len[r] > SPH_NBR_MAX_ROW || hd.n + hits > SPH_NBR_CAP_WIDE;
         if (hd.over) return;
         if (wl.l == (uint32_t)(r % LANES)) at[r / LANES] = hd.n;
         if (hits) hd.live |= 1u << r;
@@ -876,6 +852,7 @@ k_density_wide(const DevParams* __restrict__ params, const DevScene* __restrict_
     };
 #pragma unroll
     for (int z = 0; z < 9; z += 3) {
+        if (z != 0 && __all_sync(~0u, hd.over || !work)) break;   // (wide_tail tests the rest)
         const Chunk q[3] = {fetch(z, 0u), fetch(z + 1, 0u), fetch(z + 2, 0u)};   // loaded together
 #pragma unroll
         for (int y = 0; y < 3; ++y) {
@@ -956,7 +933,7 @@ k_density_wide(const DevParams* __restrict__ params, const DevScene* __restrict_
     };
     auto add = [&]() { acc = wide_sum<LANES>(scale, value, acc); };
     const uint32_t last = wide_list(wl, ws, work ? hd.n : 0u, load, term, add);
-    wide_tail(wl, ws, work && hd.over, hd.n ? last + 1u : 0u, load, term, add);
+    wide_tail(wl, ws, work && hd.over, hd.n ? last + 1u : 0u, k, X, scan, load, term, add);
 
     // ---- the rest is one thread's work per particle: the block's first threads ----
     if (wl.l < 4u) ws.terms[0][wl.l] = acc;
@@ -986,6 +963,7 @@ __global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(c
                                                       const uint4* __restrict__ tiles,
                                                       const uint32_t* __restrict__ start,
                                                       const float4* __restrict__ R, const float* __restrict__ C2,
+                                                      const float* __restrict__ X,
                                                       const uint32_t* __restrict__ mask, size_t mask_stride,
                                                       float4* __restrict__ N, uint32_t ntiles,
                                                       uint32_t* __restrict__ tile_ctr,
@@ -1031,7 +1009,8 @@ __global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(c
         float acc = 0.f;   // lanes 0 to 2: the sum's components
         const float* value = ws.terms[1 + min(wl.l, 2u)];
         wide_neighbours(
-            pp, start, sc.cell_base, delta, g, mask, mask_stride, k, work, early, wl, ws, load,
+            pp, start, sc.cell_base, delta, g, mask, mask_stride, k, work, early, wl, ws, X,
+            CandidateScan<false>(p.x, p.y, p.z, h2, h2), load,
             [&](const float4& q, uint32_t, bool on) {
                 const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
                 const float r2 = dot3(rx, ry, rz, rx, ry, rz);
@@ -1104,6 +1083,7 @@ k_force_integrate(const DevParams* __restrict__ params,
                                                               const float* __restrict__ C2,
                                                               const float4* __restrict__ A1,
                                                               const float4* __restrict__ N,
+                                                              const float* __restrict__ X,
                                                               const uint32_t* __restrict__ mask, size_t mask_stride,
                                                               float4* __restrict__ P0, float4* __restrict__ V2,
                                                               float4* __restrict__ A0, uint32_t* __restrict__ maxdisp,
@@ -1203,7 +1183,8 @@ k_force_integrate(const DevParams* __restrict__ params,
         const uint32_t axis = min(wl.l, 2u);
         float sum_p = 0.f, sum_v = 0.f, sum_t = 0.f;
         wide_neighbours(
-            pp, start, sc.cell_base, delta, g, mask, mask_stride, k, act && inside, early, wl, ws, load,
+            pp, start, sc.cell_base, delta, g, mask, mask_stride, k, act && inside, early, wl, ws, X,
+            CandidateScan<false>(pi.x, pi.y, pi.z, h2, h2), load,
             [&](const Nbr& r, uint32_t, bool on) {
                 float o[9] = {};   // (zeros for lanes without a pair, the tension's factor too: it may be infinite)
                 if (on && dist2(r.p) <= h2)
@@ -1661,7 +1642,7 @@ cudaError_t launch_scan_raw(const uint32_t* counts, uint32_t n, uint32_t* tile_s
 // does not write: past the list, or where a skin pass needs the rows after it, in
 // the list's last three (which is then shorter).
 static float* axes(const StepArgs& a) {
-    return reinterpret_cast<float*>(a.mask + (a.skin_masks ? SPH_AXIS_ROWS_SKIN : SPH_MASK_SKIN) * a.mask_stride);
+    return reinterpret_cast<float*>(a.mask + (a.skin_masks ? SPH_AXIS_ROWS_SKIN : SPH_AXIS_ROWS) * a.mask_stride);
 }
 cudaError_t launch_sort(const StepArgs& a, cudaStream_t st) {
     k_scatter<<<a.ntiles, a.block, 0, st>>>(a.scenes, a.tiles, a.start, a.key, a.slot, a.tmp, a.sums,
@@ -1674,7 +1655,7 @@ cudaError_t launch_sort(const StepArgs& a, cudaStream_t st) {
 static int lanes(const StepArgs& a) {
     if ((a.variant & SPH_VARIANT_DENSITY_SPLIT) == 0u || a.tile_ctr != nullptr || a.ntiles > 65535u) return 1;
     if (a.particles <= (a.crowded ? SPH_CROWDED8_MAX : SPH_WIDE8_MAX)) return 8;
-    return a.particles <= (a.crowded ? SPH_CROWDED4_MAX : SPH_DENSITY_SPLIT_MAX) ? 4 : 1;
+    return a.particles <= SPH_DENSITY_SPLIT_MAX ? 4 : 1;
 }
 static dim3 wide_grid(const StepArgs& a, int lanes) {
     return dim3((a.block * (uint32_t)lanes + kWideBlock - 1u) / kWideBlock, a.ntiles);
@@ -1716,21 +1697,21 @@ cudaError_t launch_normals(const StepArgs& a, cudaStream_t st) {
     const int l = lanes(a);
     auto kern = l == 8 ? k_normals<8> : l == 4 ? k_normals<4> : k_normals<1>;
     kern<<<l > 1 ? wide_grid(a, l) : dim3(a.grid_nbr), l > 1 ? kWideBlock : a.block,
-           l > 1 ? wide_smem(l) : rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.C2, a.mask,
+           l > 1 ? wide_smem(l) : rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.C2, axes(a), a.mask,
                                                          a.mask_stride, a.N, a.ntiles, ctr(a, 1), a.status);
     return cudaGetLastError();
 }
 cudaError_t launch_force(const StepArgs& a, cudaStream_t st) {
     const bool occ = (a.variant & SPH_VARIANT_FORCE_OCC) != 0u;
     const int l = lanes(a);
-    auto kern = l == 8   ? (a.any_tension ? k_force_integrate<true, 1, 8> : k_force_integrate<false, 1, 8>)
-                : l == 4 ? (a.any_tension ? k_force_integrate<true, 1, 4> : k_force_integrate<false, 1, 4>)
+    auto kern = l == 8   ? (a.any_tension ? k_force_integrate<true, 5, 8> : k_force_integrate<false, 6, 8>)
+                : l == 4 ? (a.any_tension ? k_force_integrate<true, 5, 4> : k_force_integrate<false, 7, 4>)
                 : a.any_tension ? (occ ? k_force_integrate<true, 4> : k_force_integrate<true, 3>)
                                 : (occ ? k_force_integrate<false, 4> : k_force_integrate<false, 3>);
     kern<<<l > 1 ? wide_grid(a, l) : dim3(a.grid_nbr), l > 1 ? kWideBlock : a.block,
            l > 1 ? wide_smem(l) : rows_smem(a), st>>>(
                                                     a.params, a.scenes, a.tiles, a.start, a.R, a.C2, a.A1, a.N,
-                                                    a.mask, a.mask_stride, a.P0, a.V2, a.A0,
+                                                    axes(a), a.mask, a.mask_stride, a.P0, a.V2, a.A0,
                                                     a.skin_masks ? a.maxdisp : nullptr, a.okey, a.pend, a.count, a.sums,
                                                     a.key, a.slot, a.status, a.dbg_forces, a.ntiles, ctr(a, 2));
     return cudaGetLastError();

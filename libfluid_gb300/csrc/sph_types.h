@@ -57,12 +57,13 @@ struct DevParams {
 // words, used only when some scene runs a per-substep XSPH pass.
 #define SPH_NBR_LIST       1u    // first list row; row 0 is the header
 #define SPH_NBR_LIST_WORDS 17u   // (odd: the threads' lists in shared memory start in different banks)
-#define SPH_MASK_SKIN      18u   // 9 rows: candidates within the skin radius (rows of <= 32); without a skin pass
-                                 // the first three hold the per-axis positions of the candidate scan
-#define SPH_AXIS_ROWS_SKIN 15u   // with one, these three do
+#define SPH_MASK_SKIN      18u   // 9 rows: candidates within the skin radius (rows of <= 32)
+#define SPH_AXIS_ROWS      24u   // 3 rows: the per-axis positions of the candidate scan
+#define SPH_AXIS_ROWS_SKIN 15u   // with a skin pass, whose words take those
 #define SPH_MASK_ROWS      27u
 #define SPH_NBR_CAP        68u   // listed neighbours: four to a word
 #define SPH_NBR_CAP_SKIN   56u   // with a skin pass: the words before SPH_AXIS_ROWS_SKIN
+#define SPH_NBR_CAP_WIDE   92u   // several lanes per particle: all words before SPH_AXIS_ROWS
 #define SPH_NBR_NEW_ROW    128u  // added to a row's first neighbour
 #define SPH_NBR_MAX_ROW    128u  // longest row whose offsets fit below that
 #define SPH_NBR_ROWS       10u   // row starts kept per thread: nine and one that is read ahead
@@ -86,10 +87,11 @@ struct DevParams {
 // (33 neighbours), substep in us with eight lanes, four, one: 13,824 particles
 // 34.9, 36.7, 52.5; 21,952 45.9, 40.0, 52.2; 32,768 55.4, 46.1, 53.3; 35,937
 // with surface tension 75.0, 70.6, 67.2; 46,656 68.0, 60.9, 58.2.  A crowded
-// particle's walk is longer and the lanes shorten it by more: scenes of 92 to
-// 160 neighbours, 38,266 particles 507, 544, 865; 59,048 (92) 326, 322, 338;
-// 59,048 (160) 626, 623, 731; 119,168 855, 820, 532.  Crowded: at least
-// SPH_CROWDED_NBRS neighbours on average, from h, the rest density and the mass.
+// particle's walk is longer and the lanes shorten it by more: two collapsing
+// columns of (neighbours on average) 38,266 particles (200) 323, 389, 897;
+// 59,048 (158) 403, 459, 757; 59,048 (91) 170, 164, 351; 119,168 (116) 561,
+// 574, 559.  Crowded: at least SPH_CROWDED_NBRS neighbours on average, from h,
+// the rest density and the mass.
 #ifndef SPH_WIDE8_MAX
 #define SPH_WIDE8_MAX         14336u
 #endif
@@ -97,8 +99,7 @@ struct DevParams {
 #define SPH_DENSITY_SPLIT_MAX 34816u
 #endif
 #define SPH_CROWDED_NBRS      80u
-#define SPH_CROWDED8_MAX      40960u
-#define SPH_CROWDED4_MAX      61440u
+#define SPH_CROWDED8_MAX      61440u
 
 // Scene placement in the engine's arenas.
 struct DevScene {

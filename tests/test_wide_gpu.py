@@ -48,7 +48,7 @@ def test_lanes_at_other_tiles(tile):
     _same([_block(9, 10, 11, 0.03), _block(26, 27, 25, 0.0, seed=6)], tile)
 
 
-# about 113 neighbours: eight lanes to 40,960 particles, four to 61,440
+# about 113 neighbours: eight lanes to 61,440 particles
 @pytest.mark.parametrize("dims", [(20, 20, 20), (35, 36, 34)])
 def test_crowded_lanes(dims):
     _same([_block(*dims, 0.04, spacing=0.00667)])
@@ -56,3 +56,38 @@ def test_crowded_lanes(dims):
 
 def test_batch_of_small_scenes():
     _same([_block(3 + k, 4, 5, 0.01 * (k % 2), seed=k) for k in range(40)])
+
+
+# neighbours of an inner particle around the 92 that a list built by several lanes
+# holds, far above, and with cell rows past its offsets (of 128): the rest is found
+# by testing candidates again, in the same order
+@pytest.mark.parametrize("spacing", [0.0078, 0.00714, 0.0066, 0.006, 0.005, 0.0042])
+def test_past_the_list(spacing):
+    _same([_block(13, 14, 15, 0.04, spacing=spacing)])
+
+
+def test_past_the_list_at_the_limit():
+    _same([_block(39, 39, 40, 0.03, spacing=0.0064)])      # 60,840 particles
+    _same([_block(40, 40, 39, 0.03, spacing=0.0064)])      # 62,400: one thread each
+
+
+def test_past_the_list_for_some():
+    """Particles of one warp whose lists end early and not."""
+    _same([_block(2 + k, 3, 5, 0.02, spacing=0.005 if k % 2 else 0.01, seed=k) for k in range(20)]
+          + [_block(20, 20, 20, 0.0, spacing=0.005)])
+
+
+@pytest.mark.parametrize("spacing", [0.00714, 0.005])
+def test_past_the_list_with_a_pass_per_substep(spacing):
+    """XSPH by its own pass: a shorter list, the axis copies in other rows."""
+    out = []
+    for variant in (31, 63):
+        b = Batch(0)
+        b.set_exec(tile=128, variant=variant)
+        b.set_deferred_xsph(False)
+        sid = b.add_scene(_block(13, 14, 15, 0.04, spacing=spacing))
+        b.step(3)
+        out.append(b.get_state(sid))
+        b.close()
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
