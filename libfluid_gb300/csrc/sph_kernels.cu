@@ -419,9 +419,14 @@ __device__ __forceinline__ bool step_failed(const uint32_t* status) {
 // ---------------------------------------------------------------------------
 // Scatter: provisional slot of each particle in cell order.  The scan's tile
 // sums (nsums of them) are left at zero for the next hash.
+// A thread's chain of loads (tile, scene, key, start) is all there is to it, so
+// a block takes kScatterTiles tiles and has their loads in flight together: with
+// one, two, four and eight tiles the sort (this and the rank pass) of 1M
+// particles took 33.0, 30.6, 28.7 and 31.2 us, of 8M 212, 189, 178 and 187.
 // ---------------------------------------------------------------------------
+constexpr uint32_t kScatterTiles = 4u;
 __global__ void __launch_bounds__(SPH_TILE) k_scatter(const DevScene* __restrict__ scenes,
-                                                      const uint4* __restrict__ tiles,
+                                                      const uint4* __restrict__ tiles, uint32_t ntiles,
                                                       const uint32_t* __restrict__ start,
                                                       const uint32_t* __restrict__ key,
                                                       const uint32_t* __restrict__ slot,
@@ -430,13 +435,27 @@ __global__ void __launch_bounds__(SPH_TILE) k_scatter(const DevScene* __restrict
                                                       const uint32_t* __restrict__ status) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nsums; i += gridDim.x * blockDim.x) sums[i] = 0u;
     if (step_failed(status)) return;
-    const uint4 t = tiles[blockIdx.x];
-    if (threadIdx.x >= t.z) return;
-    const uint32_t i = t.y + threadIdx.x;
-    const DevScene sc = scenes[t.x];
-    const uint32_t s0 = __ldg(start + sc.cell_base);
-    const uint32_t c = sc.cell_base + key[i];
-    tmp[sc.part_base + (__ldg(start + c) - s0) + slot[i]] = i;
+    bool on[kScatterTiles];
+    uint32_t i[kScatterTiles], c[kScatterTiles], to[kScatterTiles];
+#pragma unroll
+    for (uint32_t q = 0u; q < kScatterTiles; ++q) {
+        const uint32_t b = blockIdx.x * kScatterTiles + q;
+        const uint4 t = b < ntiles ? tiles[b] : make_uint4(0u, 0u, 0u, 0u);
+        on[q] = threadIdx.x < t.z;
+        i[q] = t.y + threadIdx.x;
+        c[q] = to[q] = 0u;
+        if (on[q]) {
+            const DevScene sc = scenes[t.x];
+            c[q] = sc.cell_base + key[i[q]];
+            to[q] = sc.part_base - __ldg(start + sc.cell_base) + slot[i[q]];
+        }
+    }
+#pragma unroll
+    for (uint32_t q = 0u; q < kScatterTiles; ++q)
+        if (on[q]) to[q] += __ldg(start + c[q]);
+#pragma unroll
+    for (uint32_t q = 0u; q < kScatterTiles; ++q)
+        if (on[q]) tmp[to[q]] = i[q];
 }
 
 // ---------------------------------------------------------------------------
@@ -1645,8 +1664,9 @@ static float* axes(const StepArgs& a) {
     return reinterpret_cast<float*>(a.mask + (a.skin_masks ? SPH_AXIS_ROWS_SKIN : SPH_AXIS_ROWS) * a.mask_stride);
 }
 cudaError_t launch_sort(const StepArgs& a, cudaStream_t st) {
-    k_scatter<<<a.ntiles, a.block, 0, st>>>(a.scenes, a.tiles, a.start, a.key, a.slot, a.tmp, a.sums,
-                                            whole_scan(a) ? scan_tiles(a.total_cells) : 0u, a.status);
+    k_scatter<<<(a.ntiles + kScatterTiles - 1u) / kScatterTiles, a.block, 0, st>>>(
+        a.scenes, a.tiles, a.ntiles, a.start, a.key, a.slot, a.tmp, a.sums,
+        whole_scan(a) ? scan_tiles(a.total_cells) : 0u, a.status);
     k_rank_gather<<<a.ntiles, a.block, 0, st>>>(a.scenes, a.tiles, a.start, a.key, a.tmp, a.P0, a.V0, a.A0, a.V2,
                                                 a.okey, a.pend, a.G, axes(a), a.A1, a.perm, a.status);
     return cudaGetLastError();
