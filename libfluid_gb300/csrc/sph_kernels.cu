@@ -607,15 +607,17 @@ struct CandidateScan {
 
 // A particle outside the grid: no density, its velocity kept.
 __device__ __forceinline__ void density_outside(uint32_t k, const float4& p, const float4& v, float* C2, float4* R,
-                                                uint32_t* nbr_out) {
+                                                uint32_t* nbr_out, float4* D = nullptr) {
     C2[k] = 0.f;
+    if (D) D[k] = make_float4(p.x, p.y, p.z, 0.f);
     st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, 0.f), make_float4(v.x, v.y, v.z, 0.f));
     if (nbr_out) nbr_out[k] = 0;
 }
 // The density, its equation of state and the record of slot k from the pair
 // sums (with xs, XSPH's too).
 __device__ __forceinline__ void density_finish(const DevParams& pp, uint32_t k, float sum, bool xs, float ax, float ay,
-                                               float az, const float4& p, float4 vi, float* C2, float4* R) {
+                                               float az, const float4& p, float4 vi, float* C2, float4* R,
+                                               float4* D = nullptr) {
     const float d = fabsf(sdf(pp, p.x, p.y, p.z));
     float corr = sum;
     if (d < pp.h) corr = fmaf(pp.rest_density, 1.0f - boundary_density(pp, d), corr);
@@ -629,6 +631,7 @@ __device__ __forceinline__ void density_finish(const DevParams& pp, uint32_t k, 
         vi.z = fmaf(pp.xsph, az, vi.z);
     }
     st_float4_pair(R + 2 * (size_t)k, make_float4(p.x, p.y, p.z, rho), make_float4(vi.x, vi.y, vi.z, prs));
+    if (D) D[k] = make_float4(p.x, p.y, p.z, rho);
 }
 
 template <bool SKIN>
@@ -641,7 +644,8 @@ k_density(const DevParams* __restrict__ params,
                                                       float* __restrict__ C2,
                                                       uint32_t* __restrict__ mask, size_t mask_stride,
                                                       const uint32_t* __restrict__ pend, float4* __restrict__ R,
-                                                      uint32_t* __restrict__ nbr_out, uint32_t ntiles,
+                                                      float4* __restrict__ D, uint32_t* __restrict__ nbr_out,
+                                                      uint32_t ntiles,
                                                       uint32_t* __restrict__ tile_ctr,
                                                       const uint32_t* __restrict__ status) {
   extern __shared__ uint32_t s_list[];
@@ -659,7 +663,7 @@ k_density(const DevParams* __restrict__ params,
     float4 p, vi;
     if (!grid_inside(pp, g)) {
         ld_float4_pair(G + 2 * (size_t)k, p, vi);
-        density_outside(k, p, vi, C2, R, nbr_out);
+        density_outside(k, p, vi, C2, R, nbr_out, D);
         return;
     }
     const uint32_t delta = sc.part_base - __ldg(start + sc.cell_base);
@@ -809,7 +813,7 @@ k_density(const DevParams* __restrict__ params,
     if (hd.over)
         walk_tail(pp, start, sc.cell_base, delta, g, hd.n ? last + 1u : 0u,
                   [&](uint32_t j) { if (j != k) use(load(j)); });
-    density_finish(pp, k, sum, xs, axy.x, axy.y, az, p, vi, C2, R);
+    density_finish(pp, k, sum, xs, axy.x, axy.y, az, p, vi, C2, R, D);
     if (nbr_out) nbr_out[k] = cnt;
   });
 }
@@ -975,14 +979,20 @@ k_density_wide(const DevParams* __restrict__ params, const DevScene* __restrict_
 // force only through sigma * (...), which is exactly zero.  Neighbours come
 // from the density pass's list, as in the force pass.  LANES > 1: several lanes
 // per particle (WideShared).
+//
+// A gather takes the L1 pipe a cycle for each 128-byte line its lanes touch, and
+// the pass little else.  D holds position and density 16 bytes a slot where
+// there is room for it (eight neighbours to a line): 528 us for 8M particles,
+// 622 from the records (dstride 2), for 2.5 us of the density pass, which writes
+// it.
 // ---------------------------------------------------------------------------
 template <int LANES>
 __global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(const DevParams* __restrict__ params,
                                                       const DevScene* __restrict__ scenes,
                                                       const uint4* __restrict__ tiles,
                                                       const uint32_t* __restrict__ start,
-                                                      const float4* __restrict__ R, const float* __restrict__ C2,
-                                                      const float* __restrict__ X,
+                                                      const float4* __restrict__ D, uint32_t dstride,
+                                                      const float* __restrict__ C2, const float* __restrict__ X,
                                                       const uint32_t* __restrict__ mask, size_t mask_stride,
                                                       float4* __restrict__ N, uint32_t ntiles,
                                                       uint32_t* __restrict__ tile_ctr,
@@ -998,7 +1008,7 @@ __global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(c
     const uint32_t k = t.y + (act ? li : 0u);
     const DevScene sc = scenes[t.x];
     const WideEarly early = wide_early<LANES>(mask, mask_stride, k);
-    const float4 p = R[2 * (size_t)k];
+    const float4 p = D[dstride * (size_t)k];
     const int3 g = grid_of(pp, p.x, p.y, p.z);
     const bool work = act && grid_inside(pp, g);
     if (act && !work) {
@@ -1015,7 +1025,7 @@ __global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(c
     // rounded root r as gradPoly6 forms it (it cancels near r = h)
     const float mc = pp.mass * pp.grad_poly6;
     const float h2 = pp.h2, eps = pp.eps, h = pp.h;
-    auto load = [&](uint32_t j) { return __ldg(R + 2 * (size_t)j); };   // w = rho_j
+    auto load = [&](uint32_t j) { return __ldg(D + dstride * (size_t)j); };   // w = rho_j
     // the pair's factor of rvec
     auto grad = [&](float r2, float rhoj) {
         const float r = sqrt_exact(r2, rsqrt_approx(r2));
@@ -1683,6 +1693,12 @@ static dim3 wide_grid(const StepArgs& a, int lanes) {
 static size_t wide_smem(int lanes) {
     return kWideBlock / lanes * (lanes == 8 ? sizeof(WideShared<8>) : sizeof(WideShared<4>));
 }
+// Position and density once more, 16 bytes a slot, where the normal pass runs
+// and the neighbour words leave room (long lists and skin words do not).
+static float4* dense(const StepArgs& a) {
+    if (!a.any_tension || a.skin_masks || lanes(a) > 1) return nullptr;
+    return reinterpret_cast<float4*>(a.mask + SPH_DENSE_ROWS * a.mask_stride);
+}
 cudaError_t launch_density(const StepArgs& a, cudaStream_t st) {
     const int l = a.skin_masks ? 1 : lanes(a);
     if (l > 1) {
@@ -1694,8 +1710,9 @@ cudaError_t launch_density(const StepArgs& a, cudaStream_t st) {
     }
     const size_t smem = (size_t)SPH_NBR_SMEM_WORDS * a.block * sizeof(uint32_t);
     auto kern = a.skin_masks ? k_density<true> : k_density<false>;
-    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.G, axes(a), a.C2, a.mask, a.mask_stride,
-                                            a.pend, a.R, a.dbg_nbr, a.ntiles, ctr(a, 0), a.status);
+    kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.G, axes(a), a.C2, a.mask,
+                                            a.mask_stride, a.pend, a.R, dense(a), a.dbg_nbr, a.ntiles, ctr(a, 0),
+                                            a.status);
     return cudaGetLastError();
 }
 cudaError_t launch_unsort_vel(const StepArgs& a, uint32_t first_tile, uint32_t ntiles, uint32_t base, uint32_t n,
@@ -1716,8 +1733,9 @@ static size_t rows_smem(const StepArgs& a) { return (size_t)SPH_NBR_ROWS * a.blo
 cudaError_t launch_normals(const StepArgs& a, cudaStream_t st) {
     const int l = lanes(a);
     auto kern = l == 8 ? k_normals<8> : l == 4 ? k_normals<4> : k_normals<1>;
+    const float4* D = dense(a);
     kern<<<l > 1 ? wide_grid(a, l) : dim3(a.grid_nbr), l > 1 ? kWideBlock : a.block,
-           l > 1 ? wide_smem(l) : rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, a.R, a.C2, axes(a), a.mask,
+           l > 1 ? wide_smem(l) : rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, D ? D : a.R, D ? 1u : 2u, a.C2, axes(a), a.mask,
                                                          a.mask_stride, a.N, a.ntiles, ctr(a, 1), a.status);
     return cudaGetLastError();
 }

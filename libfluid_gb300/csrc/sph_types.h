@@ -58,6 +58,7 @@ struct DevParams {
 #define SPH_NBR_LIST       1u    // first list row; row 0 is the header
 #define SPH_NBR_LIST_WORDS 17u   // (odd: the threads' lists in shared memory start in different banks)
 #define SPH_MASK_SKIN      18u   // 9 rows: candidates within the skin radius (rows of <= 32)
+#define SPH_DENSE_ROWS     18u   // 4 rows: position and density again, for the normal pass (one thread per particle)
 #define SPH_AXIS_ROWS      24u   // 3 rows: the per-axis positions of the candidate scan
 #define SPH_AXIS_ROWS_SKIN 15u   // with a skin pass, whose words take those
 #define SPH_MASK_ROWS      27u

@@ -5,6 +5,8 @@ without surface tension, and for a batch of scenes that share a launch."""
 import numpy as np
 import pytest
 
+from helpers import configure_gpu
+from libfluid_gb300 import FluidSystem
 from libfluid_gb300 import workloads as W
 from libfluid_gb300.batch import Batch
 
@@ -91,3 +93,25 @@ def test_past_the_list_with_a_pass_per_substep(spacing):
         b.close()
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("dims", [(9, 10, 11), (33, 34, 33)])
+def test_lanes_switched_between_steps(dims):
+    """A blocking step leaves the next substep's density pass done; one that follows
+    with other lanes does not read what that pass stored for its own."""
+    spec = _block(*dims, 0.05)
+    out = []
+    for variants in ((31, 31, 31), (63, 31, 63), (31, 63, 31)):
+        fs = FluidSystem(0)
+        configure_gpu(fs, spec)
+        for v in variants:
+            fs.setExec(tile=128, variant=v)
+            fs.advance(spec.dt, 1)
+        n = spec.n
+        got = [np.zeros((n, 3), np.float32) for _ in range(3)]
+        fs.exportToData(*got)
+        out.append(got)
+        fs.close()
+    for got in out[1:]:
+        for x, y in zip(out[0], got):
+            assert np.array_equal(x, y)
