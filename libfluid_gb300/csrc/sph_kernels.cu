@@ -25,6 +25,7 @@
 //   C2        squared sound speed per sorted slot
 //   N         surface normals, w: C2 again (only when a scene has surface tension)
 #include <cfloat>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -471,7 +472,25 @@ __global__ void __launch_bounds__(SPH_TILE) k_scatter(const DevScene* __restrict
 // Where slot f's x lies in the per-axis copies (its y 4, its z 8 floats further).
 __device__ __forceinline__ size_t axes_index(uint32_t f) { return 12 * (size_t)(f / 4u) + (f & 3u); }
 
-__global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevScene* __restrict__ scenes,
+// The same for HalfScan: a position in its cell's terms, in half precision.  x is
+// kept modulo four cells, in [-2, 2), twice: from cell 0 and from cell 2, so that
+// any three neighbouring cells lie in order in one of the two; y and z as their
+// place in the cell, in [-1/2, 1/2).  Four slots to 32 bytes: x, x from cell 2, y, z.
+__device__ __forceinline__ size_t half_index(uint32_t f) { return 16 * (size_t)(f / 4u) + (f & 3u); }
+__device__ __forceinline__ void half_axes(__half* H, uint32_t f, const float4& p, float inv_cell) {
+    const float ux = p.x * inv_cell, uy = p.y * inv_cell, uz = p.z * inv_cell;
+    const float cx = floorf(ux);
+    const int c = __float2int_rz(cx);
+    H += half_index(f);
+    H[0] = __float2half_rn((ux - cx) + (float)((c & 3) - 2));
+    H[4] = __float2half_rn((ux - cx) + (float)(((c + 2) & 3) - 2));
+    H[8] = __float2half_rn((uy - floorf(uy)) - 0.5f);
+    H[12] = __float2half_rn((uz - floorf(uz)) - 0.5f);
+}
+
+template <bool HALF>
+__global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevParams* __restrict__ params,
+                                                          const DevScene* __restrict__ scenes,
                                                           const uint4* __restrict__ tiles,
                                                           const uint32_t* __restrict__ start,
                                                           const uint32_t* __restrict__ key,
@@ -506,10 +525,14 @@ __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevScene* __rest
     const uint32_t f = b + rank;
     perm[f] = i;
     const float4 p = P0[i];
-    float* xf = X + axes_index(f);
-    xf[0] = p.x;
-    xf[4] = p.y;
-    xf[8] = p.z;
+    if (HALF) {
+        half_axes(reinterpret_cast<__half*>(X), f, p, params[t.x].inv_cell);
+    } else {
+        float* xf = X + axes_index(f);
+        xf[0] = p.x;
+        xf[4] = p.y;
+        xf[8] = p.z;
+    }
     float4 v = pending ? V2[i] : V0[i];
     // the cell of the last substep travels with the velocity (w lane) to the
     // density pass's XSPH update, which loads both together
@@ -522,13 +545,14 @@ __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevScene* __rest
 // Density + Tait EOS (computeDensity, fluidphysics.cu:8-84), in two phases.
 //
 // Phase 1 scans the candidates of the 27 cells with the distance test alone,
-// 32 at a time, and appends those within h (j != i) to the particle's
+// 32 at a time, and appends those within h (j != i), and with HalfScan a few
+// just beyond, to the particle's
 // neighbour list in shared memory (NbrList).  Phase 2 walks that list, does
 // the kernel arithmetic for the pairs (about one candidate in six), so a warp
 // does not run it on every candidate that any of its lanes accepts, and
 // stores the list for the normal and force passes.  Coincident pairs
 // (r^2 <= eps) stay in the list: the density sum and XSPH take them, the other
-// passes drop them with their own r^2 > eps test.  Neighbours past the list's
+// passes drop them with their own r^2 > eps test, and all drop those beyond h.  Neighbours past the list's
 // end are found again by testing the remaining candidates (walk_tail).  Both
 // forms visit neighbours in the same order (rows z outer, then y, then slots,
 // the row's cells x ascending); the reference's loop runs the cells x outer
@@ -573,7 +597,8 @@ constexpr int kDensityDepth = 2, kNormalsDepth = 2, kForceDepth = 1;
 // pair that these instructions take; positions of four floats each would be
 // taken apart with two moves per pair and axis, and cost 64 instead of 48 bytes
 // of L1 bandwidth, the other limit of this pass (238 -> 206 us on the 1M dam
-// break, 1.80 -> 1.55 ms on the 8M scene, the sort 2 us more for the copies).
+// break, 1.80 -> 1.55 ms on the 8M scene, with one thread per particle; HalfScan
+// has taken its place there).
 // A candidate's bit is the sign of r^2 - h2n, h2n the float after h^2 (the sign
 // of a rounded difference is that of the exact one, so the test is r^2 <= h^2
 // to the bit), shifted into the word: the first candidate ends in its highest
@@ -602,6 +627,54 @@ struct CandidateScan {
                                            uint32_t& sm) const {
         visit2(make_float2(x.x, x.y), make_float2(y.x, y.y), make_float2(z.x, z.y), dm, sm);
         visit2(make_float2(x.z, x.w), make_float2(y.z, y.w), make_float2(z.z, z.w), dm, sm);
+    }
+};
+
+// The same test in half precision, which finds every candidate within h and one
+// in a hundred or so beyond (DevParams::near2); whoever uses the list tests each
+// pair exactly.  A candidate is 6 bytes to load instead of 12: each lane's bytes
+// pass through the L1 pipe, however many lanes load the same ones, and that pipe
+// was busy 80% of the pass, 43% of it with the scan's loads.  Density pass 205 ->
+// 185 us (1M dam break), 1.550 -> 1.386 ms (8M tension scene), 71 -> 59 us
+// (250,000 particles); the force pass tests pairs it did not before, 145 -> 147
+// us and 1.331 -> 1.350 ms.  With several lanes per particle the loads are shared
+// out and the longer lists would cost more than they save.
+struct HalfScan {
+    __half2 nx, ny, nz, nt;   // minus the particle's place in the row's terms; minus the threshold
+    float fy, fz;             // its place in its cell
+    uint32_t copy;            // which x it compares with: from cell 0 or from cell 2
+    __device__ __forceinline__ HalfScan(const DevParams& P, const float4& p, const int3& g) {
+        const float fx = p.x * P.inv_cell - (float)g.x;
+        fy = p.y * P.inv_cell - (float)g.y;
+        fz = p.z * P.inv_cell - (float)g.z;
+        // cells g.x - 1 to g.x + 1 in order: g.x is the second or third of the four
+        const bool second = ((g.x - 1) & 2) != 0;
+        copy = second ? 1u : 0u;
+        nx = __float2half2_rn(-(fx + (float)(((g.x + (second ? 2 : 0)) & 3) - 2)));
+        nt = __half2half2(__float2half_rd(-P.near2));
+        ny = nz = nt;
+    }
+    // Row r = 3 (1 + its z - the particle's) + 1 + its y - the particle's.
+    __device__ __forceinline__ void row(int r) {
+        ny = __float2half2_rn((float)(r % 3) - 0.5f - fy);
+        nz = __float2half2_rn((float)(r / 3) - 0.5f - fz);
+    }
+    static __device__ __forceinline__ uint32_t bits(const __half2& x) {
+        return *reinterpret_cast<const uint32_t*>(&x);
+    }
+    static __device__ __forceinline__ __half2 half2(uint32_t x) { return *reinterpret_cast<const __half2*>(&x); }
+    // r^2 - threshold of two candidates: negative where near
+    __device__ __forceinline__ uint32_t two(uint32_t x, uint32_t y, uint32_t z) const {
+        const __half2 dx = __hadd2(half2(x), nx), dy = __hadd2(half2(y), ny), dz = __hadd2(half2(z), nz);
+        return bits(__hfma2(dz, dz, __hfma2(dy, dy, __hfma2(dx, dx, nt))));
+    }
+    // A four's hits into the low bits of m: the signs spread over a byte each, then
+    // minus one times minus 8, 4, 2, 1.
+    __device__ __forceinline__ void visit4(const uint2& x, const uint4& yz, uint32_t& m) const {
+        const uint32_t a = two(x.x, yz.x, yz.z), b = two(x.y, yz.y, yz.w);
+        uint32_t s;
+        asm("prmt.b32 %0, %1, %2, 0xFDB9;" : "=r"(s) : "r"(a), "r"(b));
+        m = (uint32_t)__dp4a((int)s, (int)0xFFFEFCF8, (int)(m << 4));
     }
 };
 
@@ -657,10 +730,14 @@ k_density(const DevParams* __restrict__ params,
     const DevParams& pp = params[t.x];
     // phase 1 needs the position alone; the rest of the particle's state is
     // loaded after it (registers)
-    const float* xk = X + axes_index(k);
-    const float px = xk[0], py = xk[4], pz = xk[8];
-    const int3 g = grid_of(pp, px, py, pz);
     float4 p, vi;
+    if (SKIN) {
+        const float* xk = X + axes_index(k);
+        p = make_float4(xk[0], xk[4], xk[8], 0.f);
+    } else {
+        p = G[2 * (size_t)k];
+    }
+    const int3 g = grid_of(pp, p.x, p.y, p.z);
     if (!grid_inside(pp, g)) {
         ld_float4_pair(G + 2 * (size_t)k, p, vi);
         density_outside(k, p, vi, C2, R, nbr_out, D);
@@ -677,8 +754,9 @@ k_density(const DevParams* __restrict__ params,
     constexpr uint32_t kCap = SKIN ? SPH_NBR_CAP_SKIN : SPH_NBR_CAP;
 
     // ---- phase 1: distance test of every candidate ----
-    // (CandidateScan)
-    const CandidateScan<SKIN> scan(px, py, pz, h2, skin2);
+    // (CandidateScan; HalfScan without the skin words)
+    const CandidateScan<SKIN> scan(p.x, p.y, p.z, h2, skin2);
+    HalfScan half(pp, p, g);
     // The row ranges of this thread, loaded together (18 independent loads):
     // starts into the row table, lengths (at most 255 kept: a longer row is
     // cut short as any above 128 is) packed into bytes.
@@ -706,6 +784,7 @@ k_density(const DevParams* __restrict__ params,
             if (SKIN) continue;   // later rows still get their skin words
             break;
         }
+        if (!SKIN) half.row(rr);
         bool first = true;
         const uint32_t mis = jb0 & 3u, alen = len + mis;   // from the aligned slot on
         uint32_t c0 = 0u, skw = 0u;                        // offset of the chunk there
@@ -715,6 +794,34 @@ k_density(const DevParams* __restrict__ params,
             uint32_t dm = 0u, sm = 0u;
             const uint32_t nq = (clen + 3u) / 4u;
             uint32_t q = 0u;
+            if constexpr (!SKIN) {
+                const uint2* hp = reinterpret_cast<const uint2*>(X) + 4 * (size_t)(cb / 4u);
+                const uint2* hx = hp + half.copy;
+                for (; q + 4u <= nq; q += 4u) {
+                    const uint2 x0 = __ldg(hx), x1 = __ldg(hx + 4), x2 = __ldg(hx + 8), x3 = __ldg(hx + 12);
+                    const uint4 v0 = __ldg(reinterpret_cast<const uint4*>(hp + 2));
+                    const uint4 v1 = __ldg(reinterpret_cast<const uint4*>(hp + 6));
+                    const uint4 v2 = __ldg(reinterpret_cast<const uint4*>(hp + 10));
+                    const uint4 v3 = __ldg(reinterpret_cast<const uint4*>(hp + 14));
+                    hx += 16;
+                    hp += 16;
+                    half.visit4(x0, v0, dm);
+                    half.visit4(x1, v1, dm);
+                    half.visit4(x2, v2, dm);
+                    half.visit4(x3, v3, dm);
+                }
+                for (; q + 2u <= nq; q += 2u) {
+                    const uint2 x0 = __ldg(hx), x1 = __ldg(hx + 4);
+                    const uint4 v0 = __ldg(reinterpret_cast<const uint4*>(hp + 2));
+                    const uint4 v1 = __ldg(reinterpret_cast<const uint4*>(hp + 6));
+                    hx += 8;
+                    hp += 8;
+                    half.visit4(x0, v0, dm);
+                    half.visit4(x1, v1, dm);
+                }
+                if (q < nq) half.visit4(__ldg(hx), __ldg(reinterpret_cast<const uint4*>(hp + 2)), dm);
+                q = nq;
+            }
             for (; q + 2u <= nq; q += 2u) {
                 const float4 x0 = __ldg(xp), y0 = __ldg(xp + 1), z0 = __ldg(xp + 2);
                 const float4 x1 = __ldg(xp + 3), y1 = __ldg(xp + 4), z1 = __ldg(xp + 5);
@@ -1059,7 +1166,7 @@ __global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(c
         walk_neighbours<kNormalsDepth>(
             pp, start, sc.cell_base, delta, g, mask, mask_stride, k,
             reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load,
-            [&](const float4&) { return true; }, [&](const float4& q) {
+            [&](const float4& q) {
                 const float2 rxy = __fadd2_rn(pxy, make_float2(-q.x, -q.y));
                 const float rx = rxy.x, ry = rxy.y, rz = p.z - q.z;
                 const float r2 = dot3(rx, ry, rz, rx, ry, rz);
@@ -1168,14 +1275,10 @@ k_force_integrate(const DevParams* __restrict__ params,
     // the reference's r; 1/r and the quotients only scale (approximate).  At
     // r = h the gradient and the cohesion vanish with h - r.  j == k has r^2 = 0
     // and drops out with the coincident pairs.
-    auto dist2 = [&](const float4& pj) {
-        const float rx = pj.x - pi.x, ry = pj.y - pi.y, rz = pj.z - pi.z;
-        return dot3(rx, ry, rz, rx, ry, rz);
-    };
     auto pair = [&](const float4& pj, const float4& vj, const float4& nj, auto&& press, auto&& tens) {
         const float rx = pj.x - pi.x, ry = pj.y - pi.y, rz = pj.z - pi.z;
         const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-        if (r2 > FLT_MIN && pj.w > FLT_MIN) {
+        if (r2 <= h2 && r2 > FLT_MIN && pj.w > FLT_MIN) {
             const float inv_r = rsqrt_approx(r2), r = sqrt_exact(r2, inv_r);
             // artificial viscosity -visc (cs_i + cs_j) mu / (rho_i + rho_j),
             // mu = h ux / (r^2 + 0.01 h^2), only for approaching pairs (ux < 0)
@@ -1216,7 +1319,7 @@ k_force_integrate(const DevParams* __restrict__ params,
             CandidateScan<false>(pi.x, pi.y, pi.z, h2, h2), load,
             [&](const Nbr& r, uint32_t, bool on) {
                 float o[9] = {};   // (zeros for lanes without a pair, the tension's factor too: it may be infinite)
-                if (on && dist2(r.p) <= h2)
+                if (on)
                     pair(r.p, r.v, r.n,
                          [&](float mid, float mp, const float3& c) {
                              o[0] = mid; o[1] = mp; o[2] = c.x; o[3] = c.y; o[4] = c.z;
@@ -1247,7 +1350,7 @@ k_force_integrate(const DevParams* __restrict__ params,
         walk_neighbours<kForceDepth>(
             pp, start, sc.cell_base, delta, g, mask, mask_stride, k,
             reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load,
-            [&](const Nbr& r) { return dist2(r.p) <= h2; }, [&](const Nbr& r) {
+            [&](const Nbr& r) {
                 pair(r.p, r.v, r.n,
                      [&](float mid, float mp, const float3& c) {
                          fpx = fmaf(c.x, mid, fpx); fpy = fmaf(c.y, mid, fpy); fpz = fmaf(c.z, mid, fpz);
@@ -1673,19 +1776,22 @@ cudaError_t launch_scan_raw(const uint32_t* counts, uint32_t n, uint32_t* tile_s
 static float* axes(const StepArgs& a) {
     return reinterpret_cast<float*>(a.mask + (a.skin_masks ? SPH_AXIS_ROWS_SKIN : SPH_AXIS_ROWS) * a.mask_stride);
 }
-cudaError_t launch_sort(const StepArgs& a, cudaStream_t st) {
-    k_scatter<<<(a.ntiles + kScatterTiles - 1u) / kScatterTiles, a.block, 0, st>>>(
-        a.scenes, a.tiles, a.ntiles, a.start, a.key, a.slot, a.tmp, a.sums,
-        whole_scan(a) ? scan_tiles(a.total_cells) : 0u, a.status);
-    k_rank_gather<<<a.ntiles, a.block, 0, st>>>(a.scenes, a.tiles, a.start, a.key, a.tmp, a.P0, a.V0, a.A0, a.V2,
-                                                a.okey, a.pend, a.G, axes(a), a.A1, a.perm, a.status);
-    return cudaGetLastError();
-}
 // Lanes per particle of the neighbour passes (WideShared).
 static int lanes(const StepArgs& a) {
     if ((a.variant & SPH_VARIANT_DENSITY_SPLIT) == 0u || a.tile_ctr != nullptr || a.ntiles > 65535u) return 1;
     if (a.particles <= (a.crowded ? SPH_CROWDED8_MAX : SPH_WIDE8_MAX)) return 8;
     return a.particles <= SPH_DENSITY_SPLIT_MAX ? 4 : 1;
+}
+// Whether the candidate scan is HalfScan's.
+static bool half_scan(const StepArgs& a) { return !a.skin_masks && lanes(a) == 1; }
+cudaError_t launch_sort(const StepArgs& a, cudaStream_t st) {
+    k_scatter<<<(a.ntiles + kScatterTiles - 1u) / kScatterTiles, a.block, 0, st>>>(
+        a.scenes, a.tiles, a.ntiles, a.start, a.key, a.slot, a.tmp, a.sums,
+        whole_scan(a) ? scan_tiles(a.total_cells) : 0u, a.status);
+    auto rank = half_scan(a) ? k_rank_gather<true> : k_rank_gather<false>;
+    rank<<<a.ntiles, a.block, 0, st>>>(a.params, a.scenes, a.tiles, a.start, a.key, a.tmp, a.P0, a.V0, a.A0, a.V2,
+                                                a.okey, a.pend, a.G, axes(a), a.A1, a.perm, a.status);
+    return cudaGetLastError();
 }
 static dim3 wide_grid(const StepArgs& a, int lanes) {
     return dim3((a.block * (uint32_t)lanes + kWideBlock - 1u) / kWideBlock, a.ntiles);

@@ -43,7 +43,8 @@ struct DevParams {
     float inv_h2;                 // 1/h^2, normalises displacements for the XSPH mask check
     float xsph_disp_limit2;       // (skin/2)^2 * 0.98: largest (displacement/h)^2 XSPH may accept
     float sphere_r;               // sphere boundary (flags bit2): radius about the box centre
-    uint32_t pad_[2];
+    float near2;                  // threshold of the half-precision candidate test (HalfScan), in cells squared
+    uint32_t pad_;
 };
 
 // The skin words are built with radius (1 + skin) h (default skin below).
@@ -59,7 +60,8 @@ struct DevParams {
 #define SPH_NBR_LIST_WORDS 17u   // (odd: the threads' lists in shared memory start in different banks)
 #define SPH_MASK_SKIN      18u   // 9 rows: candidates within the skin radius (rows of <= 32)
 #define SPH_DENSE_ROWS     18u   // 4 rows: position and density again, for the normal pass (one thread per particle)
-#define SPH_AXIS_ROWS      24u   // 3 rows: the per-axis positions of the candidate scan
+#define SPH_AXIS_ROWS      24u   // 3 rows: the per-axis positions of the candidate scan, of which the
+                                 // half-precision ones (one thread per particle) take 2
 #define SPH_AXIS_ROWS_SKIN 15u   // with a skin pass, whose words take those
 #define SPH_MASK_ROWS      27u
 #define SPH_NBR_CAP        68u   // listed neighbours: four to a word
