@@ -580,9 +580,6 @@ __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevParams* __res
 // c^2, 1/rho^2) and velocity (48 bytes in three requests) the force pass of the
 // 1M dam break went from 230 to 196 us, before the neighbour lists.
 // ---------------------------------------------------------------------------
-#ifndef DENSITY_MINB
-#define DENSITY_MINB 4
-#endif
 // Neighbour loads in flight per list step: two where the registers hold them
 // (density 239.5 against 246.5 us on the 1M dam break, normals 26.7 against 30.7
 // us at 250k), one in the force pass (two measured the same at 64 registers,
@@ -707,8 +704,14 @@ __device__ __forceinline__ void density_finish(const DevParams& pp, uint32_t k, 
     if (D) D[k] = make_float4(p.x, p.y, p.z, rho);
 }
 
+// Registers: with 56 nine blocks of 128 threads share an SM (as many as the lists
+// in shared memory allow beside L1), with 64 eight, and a few values spill either
+// way.  Loads of three fours in flight with 56, of four with 64: 180 and 185 us
+// (1M dam break), 1.334 and 1.387 ms (8M tension scene), 59.6 and 59.2 us (250,000
+// particles); four with 56 183 us and 1.361 ms, three with 64 194 us and 1.439 ms,
+// 72 (no spills) 192 us, 48 225 us.
 template <bool SKIN>
-__global__ void __launch_bounds__(SPH_TILE, DENSITY_MINB)
+__global__ void __maxnreg__(SKIN ? 64 : 56)
 k_density(const DevParams* __restrict__ params,
                                                       const DevScene* __restrict__ scenes,
                                                       const uint4* __restrict__ tiles,
@@ -797,29 +800,20 @@ k_density(const DevParams* __restrict__ params,
             if constexpr (!SKIN) {
                 const uint2* hp = reinterpret_cast<const uint2*>(X) + 4 * (size_t)(cb / 4u);
                 const uint2* hx = hp + half.copy;
-                for (; q + 4u <= nq; q += 4u) {
-                    const uint2 x0 = __ldg(hx), x1 = __ldg(hx + 4), x2 = __ldg(hx + 8), x3 = __ldg(hx + 12);
+                // six fours or seven make a row at rest density
+                for (; q + 3u <= nq; q += 3u) {
+                    const uint2 x0 = __ldg(hx), x1 = __ldg(hx + 4), x2 = __ldg(hx + 8);
                     const uint4 v0 = __ldg(reinterpret_cast<const uint4*>(hp + 2));
                     const uint4 v1 = __ldg(reinterpret_cast<const uint4*>(hp + 6));
                     const uint4 v2 = __ldg(reinterpret_cast<const uint4*>(hp + 10));
-                    const uint4 v3 = __ldg(reinterpret_cast<const uint4*>(hp + 14));
-                    hx += 16;
-                    hp += 16;
+                    hx += 12;
+                    hp += 12;
                     half.visit4(x0, v0, dm);
                     half.visit4(x1, v1, dm);
                     half.visit4(x2, v2, dm);
-                    half.visit4(x3, v3, dm);
                 }
-                for (; q + 2u <= nq; q += 2u) {
-                    const uint2 x0 = __ldg(hx), x1 = __ldg(hx + 4);
-                    const uint4 v0 = __ldg(reinterpret_cast<const uint4*>(hp + 2));
-                    const uint4 v1 = __ldg(reinterpret_cast<const uint4*>(hp + 6));
-                    hx += 8;
-                    hp += 8;
-                    half.visit4(x0, v0, dm);
-                    half.visit4(x1, v1, dm);
-                }
-                if (q < nq) half.visit4(__ldg(hx), __ldg(reinterpret_cast<const uint4*>(hp + 2)), dm);
+                for (; q < nq; ++q, hx += 4, hp += 4)
+                    half.visit4(__ldg(hx), __ldg(reinterpret_cast<const uint4*>(hp + 2)), dm);
                 q = nq;
             }
             for (; q + 2u <= nq; q += 2u) {
