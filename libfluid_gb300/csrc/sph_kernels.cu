@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
+#include <type_traits>
 #include "sph_types.h"
 #include "sph_device.cuh"
 #include "sph_kernels.h"
@@ -580,11 +581,14 @@ __global__ void __launch_bounds__(SPH_TILE) k_rank_gather(const DevParams* __res
 // c^2, 1/rho^2) and velocity (48 bytes in three requests) the force pass of the
 // 1M dam break went from 230 to 196 us, before the neighbour lists.
 // ---------------------------------------------------------------------------
-// Neighbour loads in flight per list step: two where the registers hold them
-// (density 239.5 against 246.5 us on the 1M dam break, normals 26.7 against 30.7
-// us at 250k), one in the force pass (two measured the same at 64 registers,
-// where they spill, and 5% slower at 80).
-constexpr int kDensityDepth = 2, kNormalsDepth = 2, kForceDepth = 1;
+// Neighbour loads in flight per list step, as many as the registers hold.  Where
+// occupancy decides: density two (239.5 against 246.5 us with one, 1M dam break),
+// force one (two measured the same at 64 registers, where they spill), normals
+// four with 48 registers (502 us for 8M particles; two with 48 507, two with 56
+// 533, four with 64 539).  FEW: launches of one wave (SPH_ONE_WAVE_THREADS).
+template <bool FEW> constexpr int kDensityDepth = FEW ? 4 : 2;
+template <int MINB> constexpr int kForceDepth = MINB <= 3 ? 2 : 1;
+constexpr int kNormalsDepth = 4;
 // Phase 1's distance test: four candidates at a time from the per-axis copies,
 // aligned to four slots (the up to three before a row's start and after its end
 // are tested too and masked out: no loop for the ragged ends), with the packed
@@ -709,9 +713,9 @@ __device__ __forceinline__ void density_finish(const DevParams& pp, uint32_t k, 
 // way.  Loads of three fours in flight with 56, of four with 64: 180 and 185 us
 // (1M dam break), 1.334 and 1.387 ms (8M tension scene), 59.6 and 59.2 us (250,000
 // particles); four with 56 183 us and 1.361 ms, three with 64 194 us and 1.439 ms,
-// 72 (no spills) 192 us, 48 225 us.
-template <bool SKIN>
-__global__ void __maxnreg__(SKIN ? 64 : 56)
+// 72 (no spills) 192 us, 48 225 us.  FEW: SPH_ONE_WAVE_THREADS.
+template <bool SKIN, bool FEW>
+__global__ void __maxnreg__(FEW ? 80 : SKIN ? 64 : 56)
 k_density(const DevParams* __restrict__ params,
                                                       const DevScene* __restrict__ scenes,
                                                       const uint4* __restrict__ tiles,
@@ -800,20 +804,32 @@ k_density(const DevParams* __restrict__ params,
             if constexpr (!SKIN) {
                 const uint2* hp = reinterpret_cast<const uint2*>(X) + 4 * (size_t)(cb / 4u);
                 const uint2* hx = hp + half.copy;
-                // six fours or seven make a row at rest density
-                for (; q + 3u <= nq; q += 3u) {
-                    const uint2 x0 = __ldg(hx), x1 = __ldg(hx + 4), x2 = __ldg(hx + 8);
-                    const uint4 v0 = __ldg(reinterpret_cast<const uint4*>(hp + 2));
-                    const uint4 v1 = __ldg(reinterpret_cast<const uint4*>(hp + 6));
-                    const uint4 v2 = __ldg(reinterpret_cast<const uint4*>(hp + 10));
-                    hx += 12;
-                    hp += 12;
-                    half.visit4(x0, v0, dm);
-                    half.visit4(x1, v1, dm);
-                    half.visit4(x2, v2, dm);
+                // (at rest density a row is six fours or seven)
+                auto fours = [&](auto count) {
+                    constexpr uint32_t n = decltype(count)::value;
+                    for (; q + n <= nq; q += n) {
+                        uint2 x[n];
+                        uint4 yz[n];
+#pragma unroll
+                        for (uint32_t i = 0u; i < n; ++i) {
+                            x[i] = __ldg(hx + 4 * i);
+                            yz[i] = __ldg(reinterpret_cast<const uint4*>(hp + 4 * i + 2));
+                        }
+                        hx += 4 * n;
+                        hp += 4 * n;
+#pragma unroll
+                        for (uint32_t i = 0u; i < n; ++i) half.visit4(x[i], yz[i], dm);
+                    }
+                };
+                if constexpr (FEW) {
+                    fours(std::integral_constant<uint32_t, 4u>());
+                    fours(std::integral_constant<uint32_t, 2u>());
+                    fours(std::integral_constant<uint32_t, 1u>());
+                } else {
+                    fours(std::integral_constant<uint32_t, 3u>());
+                    for (; q < nq; ++q, hx += 4, hp += 4)
+                        half.visit4(__ldg(hx), __ldg(reinterpret_cast<const uint4*>(hp + 2)), dm);
                 }
-                for (; q < nq; ++q, hx += 4, hp += 4)
-                    half.visit4(__ldg(hx), __ldg(reinterpret_cast<const uint4*>(hp + 2)), dm);
                 q = nq;
             }
             for (; q + 2u <= nq; q += 2u) {
@@ -909,7 +925,7 @@ k_density(const DevParams* __restrict__ params,
     for (uint32_t m = 0; m < hd.n; m += 4u) {
         const uint32_t w = words[m >> 2];
         mask[(size_t)(SPH_NBR_LIST + (m >> 2)) * mask_stride + k] = w;
-        last = visit_word<kDensityDepth>(w, hd.n - m, table, load, use);
+        last = visit_word<kDensityDepth<FEW>>(w, hd.n - m, table, load, use);
     }
     if (hd.over)
         walk_tail(pp, start, sc.cell_base, delta, g, hd.n ? last + 1u : 0u,
@@ -1087,8 +1103,8 @@ k_density_wide(const DevParams* __restrict__ params, const DevScene* __restrict_
 // 622 from the records (dstride 2), for 2.5 us of the density pass, which writes
 // it.
 // ---------------------------------------------------------------------------
-template <int LANES>
-__global__ void __launch_bounds__(LANES > 1 ? kWideBlock : SPH_TILE) k_normals(const DevParams* __restrict__ params,
+template <int LANES, bool FEW = false>
+__global__ void __maxnreg__(LANES > 1 ? 40 : FEW ? 64 : 48) k_normals(const DevParams* __restrict__ params,
                                                       const DevScene* __restrict__ scenes,
                                                       const uint4* __restrict__ tiles,
                                                       const uint32_t* __restrict__ start,
@@ -1341,7 +1357,7 @@ k_force_integrate(const DevParams* __restrict__ params,
         g = grid_of(pp, pi.x, pi.y, pi.z);
         inside = grid_inside(pp, g);
     } else if (inside) {
-        walk_neighbours<kForceDepth>(
+        walk_neighbours<kForceDepth<MINB>>(
             pp, start, sc.cell_base, delta, g, mask, mask_stride, k,
             reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load,
             [&](const Nbr& r) {
@@ -1710,9 +1726,11 @@ cudaError_t init_kernel_attributes() {
         {(const void*)k_force_integrate<true, 4>, SPH_ROWS_CARVEOUT_PCT},
         {(const void*)k_force_integrate<false, 3>, SPH_ROWS_CARVEOUT_PCT},
         {(const void*)k_force_integrate<false, 4>, SPH_ROWS_CARVEOUT_PCT},
-        {(const void*)k_normals<1>, SPH_ROWS_CARVEOUT_PCT},
-        {(const void*)k_density<false>, SPH_LIST_CARVEOUT_PCT},
-        {(const void*)k_density<true>, SPH_LIST_CARVEOUT_PCT}};
+        {(const void*)k_normals<1, false>, SPH_ROWS_CARVEOUT_PCT},
+        {(const void*)k_normals<1, true>, SPH_ROWS_CARVEOUT_PCT},
+        {(const void*)k_density<false, false>, SPH_LIST_CARVEOUT_PCT},
+        {(const void*)k_density<false, true>, SPH_LIST_CARVEOUT_PCT},
+        {(const void*)k_density<true, false>, SPH_LIST_CARVEOUT_PCT}};
     for (const auto& x : fns) {
         const cudaError_t e = cudaFuncSetAttribute(x.f, cudaFuncAttributePreferredSharedMemoryCarveout, x.pct);
         if (e != cudaSuccess) return e;
@@ -1776,6 +1794,10 @@ static int lanes(const StepArgs& a) {
     if (a.particles <= (a.crowded ? SPH_CROWDED8_MAX : SPH_WIDE8_MAX)) return 8;
     return a.particles <= SPH_DENSITY_SPLIT_MAX ? 4 : 1;
 }
+// Whether a launch of one thread per particle fits the GPU at 80 registers.
+static bool one_wave(const StepArgs& a) {
+    return a.tile_ctr == nullptr && (uint64_t)a.ntiles * a.block <= SPH_ONE_WAVE_THREADS;
+}
 // Whether the candidate scan is HalfScan's.
 static bool half_scan(const StepArgs& a) { return !a.skin_masks && lanes(a) == 1; }
 cudaError_t launch_sort(const StepArgs& a, cudaStream_t st) {
@@ -1809,7 +1831,7 @@ cudaError_t launch_density(const StepArgs& a, cudaStream_t st) {
         return cudaGetLastError();
     }
     const size_t smem = (size_t)SPH_NBR_SMEM_WORDS * a.block * sizeof(uint32_t);
-    auto kern = a.skin_masks ? k_density<true> : k_density<false>;
+    auto kern = a.skin_masks ? k_density<true, false> : one_wave(a) ? k_density<false, true> : k_density<false, false>;
     kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.G, axes(a), a.C2, a.mask,
                                             a.mask_stride, a.pend, a.R, dense(a), a.dbg_nbr, a.ntiles, ctr(a, 0),
                                             a.status);
@@ -1832,7 +1854,9 @@ cudaError_t launch_undo_ahead(const StepArgs& a, uint32_t first_tile, uint32_t n
 static size_t rows_smem(const StepArgs& a) { return (size_t)SPH_NBR_ROWS * a.block * sizeof(uint32_t); }
 cudaError_t launch_normals(const StepArgs& a, cudaStream_t st) {
     const int l = lanes(a);
-    auto kern = l == 8 ? k_normals<8> : l == 4 ? k_normals<4> : k_normals<1>;
+    auto kern = l == 8   ? k_normals<8>
+                : l == 4 ? k_normals<4>
+                         : one_wave(a) ? k_normals<1, true> : k_normals<1, false>;
     const float4* D = dense(a);
     kern<<<l > 1 ? wide_grid(a, l) : dim3(a.grid_nbr), l > 1 ? kWideBlock : a.block,
            l > 1 ? wide_smem(l) : rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, D ? D : a.R, D ? 1u : 2u, a.C2, axes(a), a.mask,
@@ -1840,7 +1864,7 @@ cudaError_t launch_normals(const StepArgs& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 cudaError_t launch_force(const StepArgs& a, cudaStream_t st) {
-    const bool occ = (a.variant & SPH_VARIANT_FORCE_OCC) != 0u;
+    const bool occ = (a.variant & SPH_VARIANT_FORCE_OCC) != 0u && !one_wave(a);
     const int l = lanes(a);
     auto kern = l == 8   ? (a.any_tension ? k_force_integrate<true, 5, 8> : k_force_integrate<false, 6, 8>)
                 : l == 4 ? (a.any_tension ? k_force_integrate<true, 5, 4> : k_force_integrate<false, 7, 4>)
