@@ -515,7 +515,7 @@ def measure_batched(dist, num_scenes: int, steps: int, warmup: int, clocks_csv=N
     b.close()
     # the plain step, one scene at a time: each scene in its own engine, the
     # same warm-up, then the same substeps timed (graph replay).  A scene
-    # alone is small enough for the split density scan (variant bit 0x20),
+    # alone is small enough for several lanes per particle (variant bit 0x20),
     # which the batch's own launches are too large to take.
     plain_exe = dict(exe)
     plain_exe["variant"] = exe.get("variant", 63) | 0x20

@@ -230,7 +230,7 @@ int sph_debug_scan_fault(sph_system* s, uint32_t spin_limit, int withhold_first_
 #define SPH_VARIANT_FORCE_TABLE    0x8u  /* no effect: forces and normals walk the neighbour list */
 #define SPH_VARIANT_NORMALS_TABLE  0x10u /* no effect */
 #define SPH_VARIANT_DENSITY_SPLIT  0x20u /* neighbour passes: eight or four lanes per particle in launches of
-                                            at most 14,336 or 34,816 particles (40,960 or 61,440 of crowded
+                                            at most 14,336 or 34,816 particles (eight to 61,440 of crowded
                                             scenes), one block per tile */
 typedef struct sph_exec_config {
     uint32_t tile;

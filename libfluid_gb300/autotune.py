@@ -4,11 +4,9 @@ Sweeps, on a GPU, the execution choices that do not change results (every
 choice computes bit-identical values; tests/test_exec_configs_gpu.py checks
 it): particles per tile (= threads per block), persistent blocks per SM for
 the neighbour passes (0 = one block per tile), the neighbour-mask skin, and
-then, on the best of those, the kernel-variant bits (per-row density and XSPH
-walks, the force kernel's register budget, row-table walks of the force and
-normal passes, and for launches small enough to take it the density scan
-split over three threads per particle, which sets how many particles a warp
-scans: 32, or about 10).  Each candidate is timed with CUDA events over graph-replayed
+then, on the best of those, the kernel-variant bits (the per-row walk of the
+per-substep XSPH pass, the force kernel's register budget, and for launches small
+enough to take them several lanes per particle; the other bits have no effect).  Each candidate is timed with CUDA events over graph-replayed
 substeps after warm-up.  The best configuration per workload is written to
 tuned.json next to this file; the engine's compiled-in defaults (ExecConfig
 in csrc/engine.h) follow that record.

@@ -17,8 +17,10 @@
 //             the gathered okey bits)
 //   X         the gathered positions again for the density pass's candidate
 //             scan, four slots at a time: their x, their y, their z, 48 bytes
-//             in all (they lie in rows of the neighbour words that the density
-//             pass does not write)
+//             in all, or with one thread per particle cell-relative halves, 32
+//             bytes (HalfScan); they lie in rows of the neighbour words that the
+//             density pass does not write
+//   D         position and density again for the normal pass, in such rows too
 //   R         neighbour record per sorted slot, 32 bytes, written by the
 //             density pass: (x, y, z, rho) and (velocity with the pending
 //             XSPH update applied, pressure)

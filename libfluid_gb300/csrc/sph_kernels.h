@@ -51,8 +51,8 @@ struct StepArgs {
 // Shared-memory carveouts (percent of the SM's maximum) requested for the
 // density pass (lists and row starts of 9 blocks of 128 threads) and for the
 // normal and force passes (row starts of 8), so that L1 keeps the rest.
-// Measured on the 1M dam break: 50 and 18 give 237.7 and 138.0 us, 58 and 25
-// 239.5 and 139.3, 44 and 10 237.9 and 191.8 (too few blocks fit).
+// Measured on the 1M dam break: density 183.0 us with 50, 184.3 with 58; force
+// 138.0 with 18, 139.3 with 25, 191.8 with 10 (too few blocks fit).
 #ifndef SPH_LIST_CARVEOUT_PCT
 #define SPH_LIST_CARVEOUT_PCT 50
 #endif
