@@ -342,7 +342,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_single(uint32_t* __restri
 // the hash counted (count_cell) and every block reads for itself.  No block
 // waits for another and no descriptors are cleared: against the look-back the
 // substep of the 1M dam break (489 tiles) went from 379 to 372 us and that of
-// 1,728 particles from 27 to 25 us.  The sums' reads grow with the square of the
+// 1,728 particles from 27 to 25 us.  Lanes take fours of cells side by side, so
+// that a warp's loads and stores cover whole lines (13.0 -> 9.7 us by events around
+// the pass at 1M, against 16 cells in a row per lane).  The sums' reads grow with the square of the
 // tiles, so from SPH_SCAN_SUM_TILES on (67 million cells; 0.1 ms of reads beside
 // 0.1 ms of scan) the look-back takes over.  The counts are left at zero: the next substep's hash (fused into
 // the force pass) adds into them, which otherwise needs a memset of the whole
@@ -350,61 +352,60 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_single(uint32_t* __restri
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(uint32_t* __restrict__ in, uint32_t n,
                                                              const uint32_t* __restrict__ sums,
                                                              uint32_t* __restrict__ out) {
+    constexpr uint32_t kFours = SCAN_ITEMS / 4u;
     __shared__ uint32_t warp_tot[SCAN_THREADS / 32], warp_pre[SCAN_THREADS / 32];
-    const uint32_t tile = blockIdx.x, base = tile * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
-    const bool whole = base + SCAN_ITEMS <= n;
-    uint32_t v[SCAN_ITEMS];
-    if (whole) {
-        const uint4* p4 = reinterpret_cast<const uint4*>(in + base);
+    const uint32_t tile = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    // a warp's lanes take fours side by side, kFours times
+    const uint32_t base = tile * SCAN_TILE + warp * (32u * SCAN_ITEMS) + 4u * lane;
+    uint4 v[kFours];
 #pragma unroll
-        for (int q = 0; q < SCAN_ITEMS / 4; ++q) {
-            const uint4 w = p4[q];
-            v[4 * q] = w.x; v[4 * q + 1] = w.y; v[4 * q + 2] = w.z; v[4 * q + 3] = w.w;
+    for (uint32_t q = 0u; q < kFours; ++q) {
+        const uint32_t c = base + 128u * q;
+        if (c + 4u <= n) {
+            v[q] = *reinterpret_cast<const uint4*>(in + c);
+        } else {
+            v[q].x = c < n ? in[c] : 0u;
+            v[q].y = c + 1u < n ? in[c + 1u] : 0u;
+            v[q].z = c + 2u < n ? in[c + 2u] : 0u;
+            v[q].w = 0u;
         }
-    } else {
-#pragma unroll
-        for (int k = 0; k < SCAN_ITEMS; ++k) v[k] = (base + k < n) ? in[base + k] : 0u;
     }
     uint32_t pre = 0u;
     for (uint32_t i = threadIdx.x; i < tile; i += SCAN_THREADS) pre += __ldg(sums + i);
-    uint32_t s = 0;
+    uint32_t run[kFours], tot = 0u;   // cells before each four in the warp
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) s += v[k];
-    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t inc = warp_incl_scan(s);
+    for (uint32_t q = 0u; q < kFours; ++q) {
+        const uint32_t s = v[q].x + v[q].y + v[q].z + v[q].w, inc = warp_incl_scan(s);
+        run[q] = tot + inc - s;
+        tot += __shfl_sync(0xffffffffu, inc, 31);
+    }
     pre = __reduce_add_sync(0xffffffffu, pre);
-    if (lane == 31) {
-        warp_tot[warp] = inc;
+    if (lane == 0u) {
+        warp_tot[warp] = tot;
         warp_pre[warp] = pre;
     }
     __syncthreads();
-    uint32_t run = inc - s;
+    uint32_t before = 0u;
 #pragma unroll
-    for (int w = 0; w < SCAN_THREADS / 32; ++w) run += warp_pre[w] + ((unsigned)w < warp ? warp_tot[w] : 0u);
-    if (whole) {
-        uint4* o4 = reinterpret_cast<uint4*>(out + base);
-        uint4* z4 = reinterpret_cast<uint4*>(in + base);
+    for (uint32_t w = 0u; w < SCAN_THREADS / 32u; ++w) before += warp_pre[w] + (w < warp ? warp_tot[w] : 0u);
 #pragma unroll
-        for (int q = 0; q < SCAN_ITEMS / 4; ++q) {
-            uint4 w;
-            w.x = run; run += v[4 * q];
-            w.y = run; run += v[4 * q + 1];
-            w.z = run; run += v[4 * q + 2];
-            w.w = run; run += v[4 * q + 3];
-            o4[q] = w;
-            z4[q] = make_uint4(0u, 0u, 0u, 0u);
-        }
-        if (base + SCAN_ITEMS == n) out[n] = run;   // total after the last cell
-    } else {
-#pragma unroll
-        for (int k = 0; k < SCAN_ITEMS; ++k) {
-            const uint32_t idx = base + k;
-            if (idx < n) {
-                out[idx] = run;
-                in[idx] = 0u;
-            }
-            run += v[k];
-            if (idx + 1 == n) out[n] = run;
+    for (uint32_t q = 0u; q < kFours; ++q) {
+        const uint32_t c = base + 128u * q;
+        uint4 o;
+        o.x = before + run[q];
+        o.y = o.x + v[q].x;
+        o.z = o.y + v[q].y;
+        o.w = o.z + v[q].z;
+        if (c + 4u <= n) {
+            *reinterpret_cast<uint4*>(out + c) = o;
+            *reinterpret_cast<uint4*>(in + c) = make_uint4(0u, 0u, 0u, 0u);
+            if (c + 4u == n) out[n] = o.w + v[q].w;   // total after the last cell
+        } else if (c < n) {
+            out[c] = o.x;
+            in[c] = 0u;
+            if (c + 1u < n) { out[c + 1u] = o.y; in[c + 1u] = 0u; }
+            if (c + 2u < n) { out[c + 2u] = o.z; in[c + 2u] = 0u; }
+            out[n] = c + 1u == n ? o.y : c + 2u == n ? o.z : o.w;
         }
     }
 }
