@@ -682,6 +682,59 @@ struct HalfScan {
     }
 };
 
+// Candidates from slot `from` on, in row order; f(j) tests the distance.  The
+// density pass's: walk_tail there costs its list's loop registers (180 -> 207 us at
+// 1M).
+template <class F>
+__device__ __forceinline__ void walk_rows(const DevParams& P, const uint32_t* __restrict__ start, uint32_t cell_base,
+                                          uint32_t delta, int3 g, uint32_t from, F&& f) {
+#pragma unroll 1
+    for (int r = 0; r < 9; ++r) {
+        uint32_t jb, je;
+        if (!row_range(P, start, cell_base, delta, g, r, jb, je)) continue;
+        for (uint32_t j = max(jb, from); j < je; ++j) f(j);
+    }
+}
+// The same without k, in the normal and force passes.  With H (HalfScan's
+// positions) those that it finds, 32 tested before the first is visited: visiting
+// each candidate to test it runs the pair arithmetic on almost every one, as one
+// lane in 32 that accepts is enough.  Without H all of them; f(j) tests the
+// distance itself.  66,560 particles compressed until most lists end early: substep
+// 185 -> 151 us.
+template <class F>
+__device__ __forceinline__ void walk_tail(const DevParams& P, const uint32_t* __restrict__ start, uint32_t cell_base,
+                                          uint32_t delta, int3 g, const float4& p, uint32_t k, uint32_t from,
+                                          const float* __restrict__ H, F&& f) {
+    HalfScan half(P, p, g);
+#pragma unroll 1
+    for (int r = 0; r < 9; ++r) {
+        uint32_t jb, je;
+        if (!row_range(P, start, cell_base, delta, g, r, jb, je)) continue;
+        jb = max(jb, from);
+        half.row(r);
+#pragma unroll 1
+        for (uint32_t c = jb & ~3u; c < je; c += 32u) {
+            const uint32_t left = je - c, nq = (min(left, 32u) + 3u) / 4u;
+            uint32_t bits = ~0u;
+            if (H) {
+                const uint2* hp = reinterpret_cast<const uint2*>(H) + 4 * (size_t)(c / 4u);
+                uint32_t dm = 0u;
+                for (uint32_t q = 0u; q < nq; ++q, hp += 4)
+                    half.visit4(__ldg(hp + half.copy), __ldg(reinterpret_cast<const uint4*>(hp + 2)), dm);
+                bits = dm << (32u - 4u * nq);
+            }
+            if (left < 32u) bits &= ~(~0u >> left);
+            if (c < jb) bits &= ~0u >> (jb - c);
+            if (k - c < 32u) bits &= ~(0x80000000u >> (k - c));
+            while (bits) {
+                const uint32_t b = (uint32_t)__clz(bits);
+                bits &= ~(0x80000000u >> b);
+                f(c + b);
+            }
+        }
+    }
+}
+
 // A particle outside the grid: no density, its velocity kept.
 __device__ __forceinline__ void density_outside(uint32_t k, const float4& p, const float4& v, float* C2, float4* R,
                                                 uint32_t* nbr_out, float4* D = nullptr) {
@@ -833,16 +886,16 @@ k_density(const DevParams* __restrict__ params,
                     for (; q < nq; ++q, hx += 4, hp += 4)
                         half.visit4(__ldg(hx), __ldg(reinterpret_cast<const uint4*>(hp + 2)), dm);
                 }
-                q = nq;
+            } else {
+                for (; q + 2u <= nq; q += 2u) {
+                    const float4 x0 = __ldg(xp), y0 = __ldg(xp + 1), z0 = __ldg(xp + 2);
+                    const float4 x1 = __ldg(xp + 3), y1 = __ldg(xp + 4), z1 = __ldg(xp + 5);
+                    xp += 6;
+                    scan.visit4(x0, y0, z0, dm, sm);
+                    scan.visit4(x1, y1, z1, dm, sm);
+                }
+                if (q < nq) scan.visit4(__ldg(xp), __ldg(xp + 1), __ldg(xp + 2), dm, sm);
             }
-            for (; q + 2u <= nq; q += 2u) {
-                const float4 x0 = __ldg(xp), y0 = __ldg(xp + 1), z0 = __ldg(xp + 2);
-                const float4 x1 = __ldg(xp + 3), y1 = __ldg(xp + 4), z1 = __ldg(xp + 5);
-                xp += 6;
-                scan.visit4(x0, y0, z0, dm, sm);
-                scan.visit4(x1, y1, z1, dm, sm);
-            }
-            if (q < nq) scan.visit4(__ldg(xp), __ldg(xp + 1), __ldg(xp + 2), dm, sm);
             // candidate cb + b in bit 31 - b, those outside the row and the
             // particle itself left out
             const uint32_t so = k - cb;
@@ -931,7 +984,7 @@ k_density(const DevParams* __restrict__ params,
         last = visit_word<kDensityDepth<FEW>>(w, hd.n - m, table, load, use);
     }
     if (hd.over)
-        walk_tail(pp, start, sc.cell_base, delta, g, hd.n ? last + 1u : 0u,
+        walk_rows(pp, start, sc.cell_base, delta, g, hd.n ? last + 1u : 0u,
                   [&](uint32_t j) { if (j != k) use(load(j)); });
     density_finish(pp, k, sum, xs, axy.x, axy.y, az, p, vi, C2, R, D);
     if (nbr_out) nbr_out[k] = cnt;
@@ -1113,6 +1166,7 @@ __global__ void __maxnreg__(LANES > 1 ? 40 : FEW ? 64 : 48) k_normals(const DevP
                                                       const uint32_t* __restrict__ start,
                                                       const float4* __restrict__ D, uint32_t dstride,
                                                       const float* __restrict__ C2, const float* __restrict__ X,
+                                                      bool half_x,
                                                       const uint32_t* __restrict__ mask, size_t mask_stride,
                                                       float4* __restrict__ N, uint32_t ntiles,
                                                       uint32_t* __restrict__ tile_ctr,
@@ -1176,18 +1230,23 @@ __global__ void __maxnreg__(LANES > 1 ? 40 : FEW ? 64 : 48) k_normals(const DevP
         sz = wl.get(acc, 2);
         if (!work || wl.l != 0u) return;
     } else {
+        auto pair = [&](const float4& q) {
+            const float2 rxy = __fadd2_rn(pxy, make_float2(-q.x, -q.y));
+            const float rx = rxy.x, ry = rxy.y, rz = p.z - q.z;
+            const float r2 = dot3(rx, ry, rz, rx, ry, rz);
+            if (r2 <= h2 && r2 > eps && q.w > eps) {
+                const float s = grad(r2, q.w);
+                sxy = __ffma2_rn(make_float2(s, s), rxy, sxy);
+                sz = fmaf(s, rz, sz);
+            }
+        };
         walk_neighbours<kNormalsDepth>(
             pp, start, sc.cell_base, delta, g, mask, mask_stride, k,
             reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load,
-            [&](const float4& q) {
-                const float2 rxy = __fadd2_rn(pxy, make_float2(-q.x, -q.y));
-                const float rx = rxy.x, ry = rxy.y, rz = p.z - q.z;
-                const float r2 = dot3(rx, ry, rz, rx, ry, rz);
-                if (r2 <= h2 && r2 > eps && q.w > eps) {
-                    const float s = grad(r2, q.w);
-                    sxy = __ffma2_rn(make_float2(s, s), rxy, sxy);
-                    sz = fmaf(s, rz, sz);
-                }
+            pair,
+            [&](uint32_t from) {
+                walk_tail(pp, start, sc.cell_base, delta, g, p, k, from, half_x ? X : nullptr,
+                          [&](uint32_t j) { pair(load(j)); });
             });
     }
     // w: the squared sound speed, so that the force pass gathers it with the normal
@@ -1232,7 +1291,7 @@ k_force_integrate(const DevParams* __restrict__ params,
                                                               const float* __restrict__ C2,
                                                               const float4* __restrict__ A1,
                                                               const float4* __restrict__ N,
-                                                              const float* __restrict__ X,
+                                                              const float* __restrict__ X, bool half_x,
                                                               const uint32_t* __restrict__ mask, size_t mask_stride,
                                                               float4* __restrict__ P0, float4* __restrict__ V2,
                                                               float4* __restrict__ A0, uint32_t* __restrict__ maxdisp,
@@ -1360,18 +1419,22 @@ k_force_integrate(const DevParams* __restrict__ params,
         g = grid_of(pp, pi.x, pi.y, pi.z);
         inside = grid_inside(pp, g);
     } else if (inside) {
+        auto visit = [&](const Nbr& r) {
+            pair(r.p, r.v, r.n,
+                 [&](float mid, float mp, const float3& c) {
+                     fpx = fmaf(c.x, mid, fpx); fpy = fmaf(c.y, mid, fpy); fpz = fmaf(c.z, mid, fpz);
+                     fvx = fmaf(c.x, mp, fvx); fvy = fmaf(c.y, mp, fvy); fvz = fmaf(c.z, mp, fvz);
+                 },
+                 [&](const float3& t) {
+                     ftx = fmaf(tden, t.x, ftx); fty = fmaf(tden, t.y, fty); ftz = fmaf(tden, t.z, ftz);
+                 });
+        };
         walk_neighbours<kForceDepth<MINB>>(
             pp, start, sc.cell_base, delta, g, mask, mask_stride, k,
             reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load,
-            [&](const Nbr& r) {
-                pair(r.p, r.v, r.n,
-                     [&](float mid, float mp, const float3& c) {
-                         fpx = fmaf(c.x, mid, fpx); fpy = fmaf(c.y, mid, fpy); fpz = fmaf(c.z, mid, fpz);
-                         fvx = fmaf(c.x, mp, fvx); fvy = fmaf(c.y, mp, fvy); fvz = fmaf(c.z, mp, fvz);
-                     },
-                     [&](const float3& t) {
-                         ftx = fmaf(tden, t.x, ftx); fty = fmaf(tden, t.y, fty); ftz = fmaf(tden, t.z, ftz);
-                     });
+            visit, [&](uint32_t from) {
+                walk_tail(pp, start, sc.cell_base, delta, g, pi, k, from, half_x ? X : nullptr,
+                          [&](uint32_t j) { visit(load(j)); });
             });
     }
     if (inside) {
@@ -1862,7 +1925,8 @@ cudaError_t launch_normals(const StepArgs& a, cudaStream_t st) {
                          : one_wave(a) ? k_normals<1, true> : k_normals<1, false>;
     const float4* D = dense(a);
     kern<<<l > 1 ? wide_grid(a, l) : dim3(a.grid_nbr), l > 1 ? kWideBlock : a.block,
-           l > 1 ? wide_smem(l) : rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, D ? D : a.R, D ? 1u : 2u, a.C2, axes(a), a.mask,
+           l > 1 ? wide_smem(l) : rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, D ? D : a.R, D ? 1u : 2u, a.C2, axes(a),
+                                                         half_scan(a), a.mask,
                                                          a.mask_stride, a.N, a.ntiles, ctr(a, 1), a.status);
     return cudaGetLastError();
 }
@@ -1876,7 +1940,7 @@ cudaError_t launch_force(const StepArgs& a, cudaStream_t st) {
     kern<<<l > 1 ? wide_grid(a, l) : dim3(a.grid_nbr), l > 1 ? kWideBlock : a.block,
            l > 1 ? wide_smem(l) : rows_smem(a), st>>>(
                                                     a.params, a.scenes, a.tiles, a.start, a.R, a.C2, a.A1, a.N,
-                                                    axes(a), a.mask, a.mask_stride, a.P0, a.V2, a.A0,
+                                                    axes(a), half_scan(a), a.mask, a.mask_stride, a.P0, a.V2, a.A0,
                                                     a.skin_masks ? a.maxdisp : nullptr, a.okey, a.pend, a.count, a.sums,
                                                     a.key, a.slot, a.status, a.dbg_forces, a.ntiles, ctr(a, 2));
     return cudaGetLastError();
