@@ -525,18 +525,34 @@ int Engine::upload_params() {
     return ENG_OK;
 }
 
+LaunchForm Engine::form_of(uint32_t particles, uint32_t ntiles, bool persistent) const {
+    return launch_form(particles, ntiles, exec_.tile, persistent, exec_.variant, crowded_, !all_defer_, any_tension_);
+}
+
+// The passes launched outside the graphs (an export's, ahead) follow captured ones
+// and the other way round, so a new form invalidates both the graphs and the prefix.
+void Engine::update_form() {
+    const uint64_t n = total_particles();
+    // neighbours at rest density: the particles in a sphere of radius h
+    double nbrs = 0.0;
+    for (const auto& s : scenes_)
+        nbrs += (double)s.n * (4.0 / 3.0 * 3.14159265 * s.dp.h * s.dp.h * s.dp.h * s.dp.rest_density / s.dp.mass);
+    crowded_ = nbrs >= (double)SPH_CROWDED_NBRS * n;
+    const LaunchForm f = form_of((uint32_t)n, ntiles_, exec_.persistent != 0u);
+    if (f != form_) {
+        form_ = f;
+        graph_dirty_ = true;
+        prefix_valid_ = false;
+    }
+}
+
 StepArgs Engine::args() const {
     StepArgs a;
     a.params = d_params_;
     a.scenes = d_scenes_;
     a.tiles = d_tiles_;
     a.ntiles = ntiles_;
-    a.particles = (uint32_t)total_particles();
-    // neighbours at rest density: the particles in a sphere of radius h
-    double nbrs = 0.0;
-    for (const auto& s : scenes_)
-        nbrs += (double)s.n * (4.0 / 3.0 * 3.14159265 * s.dp.h * s.dp.h * s.dp.h * s.dp.rest_density / s.dp.mass);
-    a.crowded = nbrs >= (double)SPH_CROWDED_NBRS * a.particles ? 1u : 0u;
+    a.form = form_;
     a.total_cells = total_cells_;
     a.P0 = P0_; a.V0 = V0_; a.A0 = A0_;
     a.G = G_; a.A1 = A1_;
@@ -671,7 +687,7 @@ int Engine::prepare() {
 int Engine::prepare_work() {
     if (layout_dirty_ || params_dirty_) hashed_ = false;
     if (layout_dirty_) { int rc = rebuild_layout(); if (rc) return rc; }
-    if (params_dirty_) { int rc = upload_params(); if (rc) return rc; }
+    if (params_dirty_) { int rc = upload_params(); if (rc) return rc; update_form(); }
     const bool graph = use_graph_ && !profiling_;
     if (graph && (graph_dirty_ || !exec_pre_ || !exec_suf_ || !exec_full_)) {
         // Re-capture; when only launch sizes and arguments changed (scenes
@@ -839,7 +855,7 @@ int Engine::prefix_scene(const Scene& sc, bool wait) {
     StepArgs a = args();
     a.tiles = d_tiles_ + sc.tile_first;
     a.ntiles = sc.tile_count;
-    a.particles = sc.n;
+    a.form = form_of(sc.n, sc.tile_count, false);
     a.grid_nbr = sc.tile_count;
     a.tile_ctr = nullptr;
     a.scan_zeroes_counts = 0u;   // keep the counts for the full prefix that follows

@@ -181,6 +181,8 @@ private:
     int ensure_capacity(uint64_t parts, uint64_t cells);
     int rebuild_layout();
     int upload_params();
+    LaunchForm form_of(uint32_t particles, uint32_t ntiles, bool persistent) const;
+    void update_form();                // form_ from the layout and parameters in force
     int launch_prefix(bool profile);   // [memset, hash], scan, sort, density
     int launch_prefix_args(const StepArgs& a, bool profile, bool hash);
     cudaError_t clear_counts();        // cell counts and their sums to zero
@@ -266,6 +268,8 @@ private:
     std::vector<uint32_t> cell_base_;
     uint32_t total_cells_ = 0;
     bool any_tension_ = false;
+    LaunchForm form_;                  // of every substep launch over all scenes
+    bool crowded_ = false;             // SPH_CROWDED_NBRS neighbours or more on average, at rest density
     bool layout_dirty_ = true, params_dirty_ = true, graph_dirty_ = true;
     bool debug_ = false, use_graph_ = true, profiling_ = false;
     bool stepped_ = false;

@@ -1854,23 +1854,11 @@ cudaError_t launch_scan_raw(const uint32_t* counts, uint32_t n, uint32_t* tile_s
 static float* axes(const StepArgs& a) {
     return reinterpret_cast<float*>(a.mask + (a.skin_masks ? SPH_AXIS_ROWS_SKIN : SPH_AXIS_ROWS) * a.mask_stride);
 }
-// Lanes per particle of the neighbour passes (WideShared).
-static int lanes(const StepArgs& a) {
-    if ((a.variant & SPH_VARIANT_DENSITY_SPLIT) == 0u || a.tile_ctr != nullptr || a.ntiles > 65535u) return 1;
-    if (a.particles <= (a.crowded ? SPH_CROWDED8_MAX : SPH_WIDE8_MAX)) return 8;
-    return a.particles <= SPH_DENSITY_SPLIT_MAX ? 4 : 1;
-}
-// Whether a launch of one thread per particle fits the GPU at 80 registers.
-static bool one_wave(const StepArgs& a) {
-    return a.tile_ctr == nullptr && (uint64_t)a.ntiles * a.block <= SPH_ONE_WAVE_THREADS;
-}
-// Whether the candidate scan is HalfScan's.
-static bool half_scan(const StepArgs& a) { return !a.skin_masks && lanes(a) == 1; }
 cudaError_t launch_sort(const StepArgs& a, cudaStream_t st) {
     k_scatter<<<(a.ntiles + kScatterTiles - 1u) / kScatterTiles, a.block, 0, st>>>(
         a.scenes, a.tiles, a.ntiles, a.start, a.key, a.slot, a.tmp, a.sums,
         whole_scan(a) ? scan_tiles(a.total_cells) : 0u, a.status);
-    auto rank = half_scan(a) ? k_rank_gather<true> : k_rank_gather<false>;
+    auto rank = a.form.half ? k_rank_gather<true> : k_rank_gather<false>;
     rank<<<a.ntiles, a.block, 0, st>>>(a.params, a.scenes, a.tiles, a.start, a.key, a.tmp, a.P0, a.V0, a.A0, a.V2,
                                                 a.okey, a.pend, a.G, axes(a), a.A1, a.perm, a.status);
     return cudaGetLastError();
@@ -1881,15 +1869,14 @@ static dim3 wide_grid(const StepArgs& a, int lanes) {
 static size_t wide_smem(int lanes) {
     return kWideBlock / lanes * (lanes == 8 ? sizeof(WideShared<8>) : sizeof(WideShared<4>));
 }
-// Position and density once more, 16 bytes a slot, where the normal pass runs
-// and the neighbour words leave room (long lists and skin words do not).
+// Position and density once more, 16 bytes a slot.
 static float4* dense(const StepArgs& a) {
-    if (!a.any_tension || a.skin_masks || lanes(a) > 1) return nullptr;
+    if (!a.form.dense) return nullptr;
     return reinterpret_cast<float4*>(a.mask + SPH_DENSE_ROWS * a.mask_stride);
 }
 cudaError_t launch_density(const StepArgs& a, cudaStream_t st) {
-    const int l = a.skin_masks ? 1 : lanes(a);
-    if (l > 1) {
+    const int l = (int)a.form.lanes;
+    if (a.form.density_wide) {
         auto kern = l == 8 ? k_density_wide<8> : k_density_wide<4>;
         kern<<<wide_grid(a, l), kWideBlock, wide_smem(l), st>>>(a.params, a.scenes, a.tiles, a.start, a.G, axes(a),
                                                                a.C2, a.mask, a.mask_stride, a.pend, a.R, a.dbg_nbr,
@@ -1897,7 +1884,7 @@ cudaError_t launch_density(const StepArgs& a, cudaStream_t st) {
         return cudaGetLastError();
     }
     const size_t smem = (size_t)SPH_NBR_SMEM_WORDS * a.block * sizeof(uint32_t);
-    auto kern = a.skin_masks ? k_density<true, false> : one_wave(a) ? k_density<false, true> : k_density<false, false>;
+    auto kern = a.skin_masks ? k_density<true, false> : a.form.one_wave ? k_density<false, true> : k_density<false, false>;
     kern<<<a.grid_nbr, a.block, smem, st>>>(a.params, a.scenes, a.tiles, a.start, a.G, axes(a), a.C2, a.mask,
                                             a.mask_stride, a.pend, a.R, dense(a), a.dbg_nbr, a.ntiles, ctr(a, 0),
                                             a.status);
@@ -1919,20 +1906,20 @@ cudaError_t launch_undo_ahead(const StepArgs& a, uint32_t first_tile, uint32_t n
 }
 static size_t rows_smem(const StepArgs& a) { return (size_t)SPH_NBR_ROWS * a.block * sizeof(uint32_t); }
 cudaError_t launch_normals(const StepArgs& a, cudaStream_t st) {
-    const int l = lanes(a);
+    const int l = (int)a.form.lanes;
     auto kern = l == 8   ? k_normals<8>
                 : l == 4 ? k_normals<4>
-                         : one_wave(a) ? k_normals<1, true> : k_normals<1, false>;
+                         : a.form.one_wave ? k_normals<1, true> : k_normals<1, false>;
     const float4* D = dense(a);
     kern<<<l > 1 ? wide_grid(a, l) : dim3(a.grid_nbr), l > 1 ? kWideBlock : a.block,
            l > 1 ? wide_smem(l) : rows_smem(a), st>>>(a.params, a.scenes, a.tiles, a.start, D ? D : a.R, D ? 1u : 2u, a.C2, axes(a),
-                                                         half_scan(a), a.mask,
+                                                         a.form.half, a.mask,
                                                          a.mask_stride, a.N, a.ntiles, ctr(a, 1), a.status);
     return cudaGetLastError();
 }
 cudaError_t launch_force(const StepArgs& a, cudaStream_t st) {
-    const bool occ = (a.variant & SPH_VARIANT_FORCE_OCC) != 0u && !one_wave(a);
-    const int l = lanes(a);
+    const bool occ = (a.variant & SPH_VARIANT_FORCE_OCC) != 0u && !a.form.one_wave;
+    const int l = (int)a.form.lanes;
     auto kern = l == 8   ? (a.any_tension ? k_force_integrate<true, 5, 8> : k_force_integrate<false, 6, 8>)
                 : l == 4 ? (a.any_tension ? k_force_integrate<true, 5, 4> : k_force_integrate<false, 7, 4>)
                 : a.any_tension ? (occ ? k_force_integrate<true, 4> : k_force_integrate<true, 3>)
@@ -1940,7 +1927,7 @@ cudaError_t launch_force(const StepArgs& a, cudaStream_t st) {
     kern<<<l > 1 ? wide_grid(a, l) : dim3(a.grid_nbr), l > 1 ? kWideBlock : a.block,
            l > 1 ? wide_smem(l) : rows_smem(a), st>>>(
                                                     a.params, a.scenes, a.tiles, a.start, a.R, a.C2, a.A1, a.N,
-                                                    axes(a), half_scan(a), a.mask, a.mask_stride, a.P0, a.V2, a.A0,
+                                                    axes(a), a.form.half, a.mask, a.mask_stride, a.P0, a.V2, a.A0,
                                                     a.skin_masks ? a.maxdisp : nullptr, a.okey, a.pend, a.count, a.sums,
                                                     a.key, a.slot, a.status, a.dbg_forces, a.ntiles, ctr(a, 2));
     return cudaGetLastError();

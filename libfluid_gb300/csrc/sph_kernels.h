@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "launch_form.h"
 #include "sph_types.h"
 
 namespace sph {
@@ -12,8 +13,7 @@ struct StepArgs {
     const DevScene* scenes;
     const uint4* tiles;        // (scene, first slot, count, 0)
     uint32_t ntiles;
-    uint32_t particles;        // particles the tiles hold
-    uint32_t crowded;          // nonzero when they have SPH_CROWDED_NBRS neighbours or more on average
+    LaunchForm form;           // of the sort and the neighbour passes; the same for all passes of a substep
     uint32_t total_cells;      // packed cell arena size including NULL buckets
     float4 *P0, *V0, *A0;      // state
     float4 *G, *A1;            // cell-ordered state (G: position and velocity, two per slot)

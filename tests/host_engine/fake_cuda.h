@@ -1,0 +1,40 @@
+// The engine (csrc/engine.cpp) on the host: the CUDA runtime calls it makes work
+// on host memory, a captured graph is a list of recorded calls, and every launch
+// only notes what it was given.  For tests of what the engine launches, in which
+// form and after which failures; nothing is computed.
+#pragma once
+#include <functional>
+#include <set>
+#include <vector>
+#include "engine.h"
+
+namespace fake {
+
+// What the passes of one substep have to agree on.
+struct Key {
+    sph::LaunchForm form;
+    uint32_t skin = 0, tension = 0, block = 0, ntiles = 0;
+    const void *tiles = nullptr, *mask = nullptr;
+    size_t stride = 0;
+    bool operator==(const Key& o) const {
+        return form == o.form && skin == o.skin && tension == o.tension && block == o.block && ntiles == o.ntiles &&
+               tiles == o.tiles && mask == o.mask && stride == o.stride;
+    }
+};
+
+struct State {
+    Key sorted, written;           // the last sort's and density pass's
+    uint64_t densities = 0;        // density passes run
+    uint64_t substeps = 0, mixed = 0;   // force passes; passes whose key was not that of the pass before
+    std::set<uint32_t> lanes;      // lanes that force passes ran with
+    std::set<const void*> crowded_cells;   // scenes (by their first slot's P0) with a cell of too many particles
+    size_t pinned_limit = ~(size_t)0;      // larger pinned allocations fail
+    cudaError_t last_error = cudaSuccess;
+    uint64_t null_writes = 0;      // packs and unsorts into a null or unknown buffer
+};
+extern State st;
+// Velocity that an unsort writes for every component.
+constexpr float kVelocity = 7.0f;
+constexpr float kPosition = 3.0f;
+
+}  // namespace fake

@@ -1,0 +1,103 @@
+"""The form in which the engine launches its passes (csrc/launch_form.h): the
+passes of one substep, from captured graphs or not, always share one.  The engine
+runs on a stand-in of the CUDA runtime, so nothing here touches a GPU.
+
+A parameter change (mass, rest density) moves a scene of some ten thousand
+particles across the line between one and eight lanes per particle, which store
+positions, lists and copies differently; an export's passes run ahead are launched
+outside the graphs."""
+import pytest
+
+from host_engine import run_driver
+
+DRIVER = r"""
+#include "fake_cuda.h"
+#include <cstdio>
+#include <cstdlib>
+#include <random>
+using namespace sph;
+
+static SceneConfig config(bool crowded, bool tension) {
+    SceneConfig c;
+    c.box_mode = 1;
+    c.lx = c.ly = c.lz = 1.f;
+    c.h = 0.1f;
+    c.rest_density = 1000.f;
+    c.mass = 1000.f * 4.19e-3f / (crowded ? 200.f : 33.f);   // neighbours at rest density
+    c.surface_tension = tension ? 0.05f : 0.f;
+    return c;
+}
+static void frame(Engine& e, int id, uint32_t n) {
+    std::vector<float> pos(3 * n), vel(3 * n);
+    e.step(1);
+    e.get_state(id, pos.data(), nullptr, vel.data(), n);
+}
+// Frames with the mass changed between them; the passes run ahead are taken.
+static void frames(uint32_t n, bool tension) {
+    Engine e(0);
+    int id = 0;
+    e.add_scene(config(true, tension), n, &id);
+    for (int i = 0; i < 12; ++i) {
+        frame(e, id, n);
+        if (i % 3 == 2) e.set_config(id, config((i / 3) % 2 != 0, tension));
+    }
+}
+// Any calls in any order.
+static void calls(uint32_t n, uint32_t seed) {
+    std::mt19937 rng(seed);
+    Engine e(0);
+    std::vector<int> ids(1);
+    bool crowded = false, tension = false;
+    e.add_scene(config(false, false), n, &ids[0]);
+    std::vector<float> a(3 * n), b(3 * n);
+    std::vector<float4> state(3 * n);
+    for (int i = 0; i < 300; ++i) {
+        const int id = ids[rng() % ids.size()];
+        const uint32_t m = e.scene(id)->n;
+        switch (rng() % 13) {
+            case 0: case 1: e.step(1); break;
+            case 2: e.step(3); break;
+            case 3: case 4: case 5: e.get_state(id, a.data(), nullptr, b.data(), m, false, rng() % 2 == 0); break;
+            case 6: crowded = !crowded; e.set_config(id, config(crowded, tension)); break;
+            case 7: tension = rng() % 2; e.set_config(id, config(crowded, tension)); break;
+            case 8: {
+                ExecConfig x = e.exec();
+                x.variant = rng() % 4 ? SPH_VARIANT_DEFAULT : 31u;
+                x.tile = 64u << (rng() % 3);
+                x.persistent = rng() % 4 ? 0u : 2u;
+                e.set_exec(x);
+                break;
+            }
+            case 9: e.set_use_graph(rng() % 4 != 0); break;
+            case 10: e.set_profiling(rng() % 4 == 0); break;
+            case 11: e.set_deferred_xsph(rng() % 4 != 0); break;
+            case 12:
+                if (ids.size() > 1 && rng() % 2) {
+                    e.remove_scene(ids.back());
+                    ids.pop_back();
+                } else if (ids.size() < 4) {
+                    ids.push_back(0);
+                    e.add_scene(config(crowded, tension), 1u + rng() % n, &ids.back());
+                } else {
+                    e.save_state(id, state.data(), m);
+                }
+        }
+    }
+}
+int main(int, char** argv) {
+    const uint32_t n = (uint32_t)std::atoi(argv[1]);
+    frames(n, false);
+    frames(n, true);
+    for (uint32_t s = 0; s < 20; ++s) calls(n, s);
+    std::printf("%llu %llu %zu %llu\n", (unsigned long long)fake::st.substeps, (unsigned long long)fake::st.mixed,
+                fake::st.lanes.size(), (unsigned long long)fake::st.null_writes);
+}
+"""
+
+
+# particles that the change takes from one to eight lanes and back; from four to eight; always eight
+@pytest.mark.parametrize("n, forms", [(40_000, 2), (20_000, 2), (2_000, 2)])
+def test_passes_of_a_substep_share_one_form(tmp_path, n, forms):
+    substeps, mixed, lanes, bad = map(int, run_driver(tmp_path, DRIVER, n).split())
+    assert substeps > 1000 and lanes >= forms
+    assert mixed == 0 and bad == 0
