@@ -728,6 +728,7 @@ int Engine::step(uint32_t substeps, bool sync) {
     cudaSetDevice(device_);
     if (scenes_.empty()) return ENG_OK;
     reads_ = 0u;
+    shared_failed_ = false;
     // no substeps: bring the layout, parameters and graphs up to date only
     // (a caller can then time substeps without the host work of a change)
     if (substeps == 0) {
@@ -948,6 +949,7 @@ int Engine::get_pass_times(double* ms_out, int cap, uint64_t* launches) {
 void Engine::clear_pending(Scene& s) {
     s.pending = false;
     reads_ = 0u;
+    shared_failed_ = false;
     hashed_ = false;
     if (!layout_dirty_ && pend_ && s.table_index < pend_cap_) cudaMemsetAsync(pend_ + s.table_index, 0, sizeof(uint32_t), stream_);
     prefix_valid_ = false;
@@ -1031,12 +1033,18 @@ int Engine::get_state(int id, float* pos, float* colour, float* vel, uint32_t n,
     // is not changed, so reading never alters the trajectory.
     const bool pend = s->pending && vel;
     // one scene of several, and no full prefix at hand: that scene's prefix
-    // only, unless the caller is reading scene after scene
+    // only, unless the caller is reading scene after scene.  A shared prefix that
+    // fails (for one scene's crowded cell, say) is not tried again before the next
+    // step or change: each read then answers for its own scene alone.
     auto run_prefix = [&](bool wait) {
         if (layout_dirty_ || params_dirty_) prefix_valid_ = false;
-        const bool all = prefix_valid_ || scenes_.size() == 1 || (many && reads_ >= 1u);
-        ++reads_;
-        return all ? ensure_prefix(wait) : prefix_scene(*s, wait);
+        if (prefix_valid_ || scenes_.size() == 1) return ensure_prefix(wait);
+        if (many && reads_++ >= 1u && !shared_failed_) {
+            const int rc = ensure_prefix(true);
+            if (rc != ENG_ECELL && rc != ENG_ETIMEOUT && rc != ENG_ENAN) return rc;
+            shared_failed_ = true;
+        }
+        return prefix_scene(*s, wait);
     };
     auto unsort = [&](float* out, uint32_t* gate, uint32_t* status_out) {
         return launch_unsort_vel(args(), s->tile_first, s->tile_count, s->part_base, s->n, out, nullptr, false, stream_,

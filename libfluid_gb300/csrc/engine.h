@@ -260,6 +260,7 @@ private:
     // write into it directly and the host copies from there.
     float* h_small_ = nullptr;
     uint32_t reads_ = 0;               // scene reads since the last step or change (get_state with `many`)
+    bool shared_failed_ = false;       // the prefix over all scenes that those reads share has failed
     std::vector<DevScene> h_scenes_;
     std::vector<uint32_t> h_tile_first_;   // per scene: its first tile (the tiles are built on the device)
     uint32_t ntiles_ = 0;

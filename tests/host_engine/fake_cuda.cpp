@@ -141,15 +141,15 @@ cudaError_t launch_sort(const StepArgs& a, cudaStream_t) {
     run([a] {
         if (fake::failed(a.status)) return;
         st.sorted = fake::key(a);
+        st.sorts.push_back(a.ntiles);
         for (uint32_t i = 0; i < a.ntiles; ++i)
-            if (st.crowded_cells.count(a.P0 + a.scenes[a.tiles[i].x].part_base)) *a.status |= SPH_STATUS_CELL_OVERFLOW;
+            if (st.crowded.count(a.scenes[a.tiles[i].x].part_base)) *a.status |= SPH_STATUS_CELL_OVERFLOW;
     });
     return fake::last();
 }
 cudaError_t launch_density(const StepArgs& a, cudaStream_t) {
     run([a] {
         if (fake::failed(a.status)) return;
-        ++st.densities;
         if (!(st.sorted == fake::key(a))) ++st.mixed;
         st.written = fake::key(a);
     });

@@ -24,10 +24,10 @@ struct Key {
 
 struct State {
     Key sorted, written;           // the last sort's and density pass's
-    uint64_t densities = 0;        // density passes run
     uint64_t substeps = 0, mixed = 0;   // force passes; passes whose key was not that of the pass before
     std::set<uint32_t> lanes;      // lanes that force passes ran with
-    std::set<const void*> crowded_cells;   // scenes (by their first slot's P0) with a cell of too many particles
+    std::set<uint32_t> crowded;    // scenes (by their first slot) that have a cell of too many particles
+    std::vector<uint32_t> sorts;   // tiles of each sort
     size_t pinned_limit = ~(size_t)0;      // larger pinned allocations fail
     cudaError_t last_error = cudaSuccess;
     uint64_t null_writes = 0;      // packs and unsorts into a null or unknown buffer
