@@ -136,7 +136,10 @@ Engine::Engine(int device) {
     cudaEventCreateWithFlags(&pack_ev_, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&vel_ev_, cudaEventDisableTiming);
     cudaMallocHost((void**)&h_status_, sizeof(uint32_t));
-    cudaMallocHost((void**)&h_small_, kSmallExport);
+    if (cudaMallocHost((void**)&h_small_, kSmallExport) != cudaSuccess) {
+        h_small_ = nullptr;   // small exports then take the way of the large ones
+        cudaGetLastError();
+    }
     cudaMalloc((void**)&status_, 2 * sizeof(uint32_t));
     cudaMemsetAsync(status_, 0, 2 * sizeof(uint32_t), stream_);
     gate_ = status_ + 1;
@@ -1066,7 +1069,7 @@ int Engine::get_state(int id, float* pos, float* colour, float* vel, uint32_t n,
     // device memory and copied: writing 36 MB over the host link from the
     // kernels measured twice as slow as the copy engine.
     const size_t bytes = (size_t)n * 3 * sizeof(float);
-    const bool small = 3 * bytes <= kSmallExport;
+    const bool small = h_small_ && 3 * bytes <= kSmallExport;
     float* st = h_small_;
     if (!small) { int rc = staging(3 * bytes, &st); if (rc) return rc; }
     float* dp = pos ? st : nullptr;

@@ -258,7 +258,7 @@ private:
     uint32_t* h_status_ = nullptr;     // pinned
     // Pinned landing place of small exports (kSmallExport bytes): the kernels
     // write into it directly and the host copies from there.
-    float* h_small_ = nullptr;
+    float* h_small_ = nullptr;         // (null: pinned memory was refused)
     uint32_t reads_ = 0;               // scene reads since the last step or change (get_state with `many`)
     bool shared_failed_ = false;       // the prefix over all scenes that those reads share has failed
     std::vector<DevScene> h_scenes_;

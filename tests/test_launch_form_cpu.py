@@ -97,7 +97,7 @@ int main(int, char** argv) {
 
 # particles that the change takes from one to eight lanes and back; from four to eight; always eight
 @pytest.mark.parametrize("n, forms", [(40_000, 2), (20_000, 2), (2_000, 2)])
-def test_passes_of_a_substep_share_one_form(tmp_path, n, forms):
-    substeps, mixed, lanes, bad = map(int, run_driver(tmp_path, DRIVER, n).split())
+def test_passes_of_a_substep_share_one_form(n, forms):
+    substeps, mixed, lanes, bad = map(int, run_driver(DRIVER, n).split())
     assert substeps > 1000 and lanes >= forms
     assert mixed == 0 and bad == 0
