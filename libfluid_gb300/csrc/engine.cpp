@@ -1075,10 +1075,14 @@ int Engine::get_state(int id, float* pos, float* colour, float* vel, uint32_t n,
     float* dp = pos ? st : nullptr;
     float* dc = colour ? st + (size_t)n * 3 : nullptr;
     float* dv = vel ? st + (size_t)n * 6 : nullptr;
-    auto hand_over = [&]() {
+    // Positions and colours are the state's, whatever became of the prefix; a
+    // pending update's velocities are there only if the unsort (launched: it has
+    // left the status word) found a complete one.
+    auto hand_over = [&](bool launched) {
         if (pos) std::memcpy(pos, dp, bytes);
         if (colour) std::memcpy(colour, dc, bytes);
-        if (vel) std::memcpy(vel, dv, bytes);
+        const uint32_t incomplete = SPH_STATUS_SCAN_TIMEOUT | SPH_STATUS_CELL_OVERFLOW;
+        if (vel && (!pend || (launched && (*h_status_ & incomplete) == 0u))) std::memcpy(vel, dv, bytes);
     };
     auto copy = [&](float* to, const float* from, cudaStream_t on) {
         return to ? cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, on) : cudaSuccess;
@@ -1120,7 +1124,7 @@ int Engine::get_state(int id, float* pos, float* colour, float* vel, uint32_t n,
         if (small) {
             ENG_CK(cudaEventSynchronize(pack_ev_), "export sync");
             if (pend) ENG_CK(cudaEventSynchronize(vel_ev_), "export sync");
-            hand_over();
+            hand_over(true);
         } else {
             ENG_CK(copy(pos, dp, copy_stream_), "download");
             ENG_CK(copy(colour, dc, copy_stream_), "download");
@@ -1147,18 +1151,15 @@ int Engine::get_state(int id, float* pos, float* colour, float* vel, uint32_t n,
     ENG_CK(launch_pack(P0_, V0_, n, s->part_base, s->dp.inv_rest_density, dp, dc, pend ? nullptr : dv, stream_),
            "pack");
     if (small) {
-        if (pend) {
-            const int rc = run_prefix(false);
-            if (rc) return rc;
-            ENG_CK(unsort(dv, nullptr, h_status_), "unsort");
-        }
+        int rc = pend ? run_prefix(false) : ENG_OK;
+        if (pend && rc == ENG_OK) ENG_CK(unsort(dv, nullptr, h_status_), "unsort");
         ENG_CK(cudaStreamSynchronize(stream_), "download sync");
-        if (pend && *h_status_ != 0u) {
-            const int rc = read_status();
-            if (rc) { prefix_valid_ = false; return rc; }
+        hand_over(rc == ENG_OK);
+        if (pend && rc == ENG_OK && *h_status_ != 0u) {
+            rc = read_status();
+            if (rc) prefix_valid_ = false;
         }
-        hand_over();
-        return ENG_OK;
+        return rc;
     }
     if (!pend) {
         ENG_CK(copy(pos, dp, stream_), "download");

@@ -165,6 +165,7 @@ cudaError_t launch_force(const StepArgs& a, cudaStream_t) {
         ++st.substeps;
         st.lanes.insert(a.form.lanes);
         if (!(st.written == fake::key(a))) ++st.mixed;
+        if (st.after_force) st.after_force();
     });
     return fake::last();
 }

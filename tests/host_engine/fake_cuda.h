@@ -27,6 +27,7 @@ struct State {
     uint64_t substeps = 0, mixed = 0;   // force passes; passes whose key was not that of the pass before
     std::set<uint32_t> lanes;      // lanes that force passes ran with
     std::set<uint32_t> crowded;    // scenes (by their first slot) that have a cell of too many particles
+    std::function<void()> after_force;     // called after each force pass
     std::vector<uint32_t> sorts;   // tiles of each sort
     size_t pinned_limit = ~(size_t)0;      // larger pinned allocations fail
     cudaError_t last_error = cudaSuccess;
