@@ -102,16 +102,16 @@ bool derive_params(const SceneConfig& c, DevParams& d, std::string* err) {
     d.skin2 = rs * rs;
     d.inv_h2 = 1.0f / d.h2;
     {
-        // HalfScan accepts every pair within h.  In units of a cell, a coordinate
-        // of a difference that matters (at most h) is off by less than e: the two
-        // positions' rounding to half (2^-11 where they reach 2 or 3/2, 2^-12 or
-        // 2^-13 where 1 or 1/2), the difference's (2^-12 up to 1) and that of the
-        // cell coordinates in float.  By Cauchy-Schwarz r^2 is then off by less
-        // than 2 r sqrt(3) e + 3 e^2.  The two sums before the last lie between
-        // minus the threshold and zero, 2^-11 of it each; the last is near zero.
+        // HalfScan accepts every pair within h, which is one cell up to rounding.  In
+        // units of a cell, a coordinate of a difference that matters (at most h) is
+        // off by less than e: the two positions' rounding to half (2^-11 where they
+        // reach 2 or 3/2, 2^-12 or 2^-13 where 1 or 1/2), the difference's (2^-12 up
+        // to 1) and that of the cell coordinates in float.  By Cauchy-Schwarz r^2 is
+        // then off by less than 2 r sqrt(3) e + 3 e^2.  The two sums before the last
+        // lie between minus the threshold and zero, 2^-11 of it each; the last is
+        // near zero.
         const double hc = (double)h * d.inv_cell, cells = std::max(d.gx, std::max(d.gy, d.gz));
-        const double e = std::ldexp(1.0, -11) + std::ldexp(1.0, -12) + std::ldexp(hc > 1.001 ? 2.0 * hc : 1.0, -12)
-                         + (cells + 4.0) * std::ldexp(1.0, -22);
+        const double e = std::ldexp(1.0, -11) + 2.0 * std::ldexp(1.0, -12) + (cells + 4.0) * std::ldexp(1.0, -22);
         const double t = hc * hc * (1.0 + 0.0011) + 3.4642 * hc * e + 3.0 * e * e + 1e-5;
         d.near2 = (float)std::fmin(t, 16.0);   // (the 27 cells reach to 12)
     }
