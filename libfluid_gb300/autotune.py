@@ -6,10 +6,10 @@ it): particles per tile (= threads per block), persistent blocks per SM for
 the neighbour passes (0 = one block per tile), the neighbour-mask skin, and
 then, on the best of those, the kernel-variant bits (the per-row walk of the
 per-substep XSPH pass, the force kernel's register budget, and for launches small
-enough to take them several lanes per particle; the other bits have no effect).  Each candidate is timed with CUDA events over graph-replayed
-substeps after warm-up.  The best configuration per workload is written to
-tuned.json next to this file; the engine's compiled-in defaults (ExecConfig
-in csrc/engine.h) follow that record.
+enough to take them several lanes per particle; the other bits have no effect).
+Each candidate is timed with CUDA events over graph-replayed substeps after
+warm-up.  The best configuration per workload is written to tuned.json next to
+this file.
 
     python -m libfluid_gb300.autotune [--workload batched|dam_break_1m|large_tension|all]
                                       [--steps 20] [--variants-only]
@@ -19,6 +19,7 @@ from __future__ import annotations
 import argparse
 import itertools
 import json
+import math
 import os
 import time
 
@@ -31,16 +32,28 @@ SKINS = (0.1, 0.15, 0.2, 0.3)
 VARIANTS = tuple(range(64))
 # Launches of at most this many particles run several lanes per particle in the
 # neighbour passes (SPH_VARIANT_DENSITY_SPLIT, bit 0x20; SPH_DENSITY_SPLIT_MAX in
-# csrc/sph_types.h); above it the bit changes nothing and is not swept.
+# csrc/sph_types.h), crowded ones up to the second limit (SPH_CROWDED8_MAX, from
+# SPH_CROWDED_NBRS neighbours on average on); above it the bit changes nothing and
+# is not swept.
 DENSITY_SPLIT_MAX = 34816
+CROWDED_MAX = 61440
+CROWDED_NEIGHBOURS = 80
 
 
-def variants_for(particles: int, persistent: int) -> tuple:
+def crowded(scenes) -> bool:
+    """Whether the scenes' particles have CROWDED_NEIGHBOURS neighbours or more on
+    average at rest density, as the engine counts them."""
+    neighbours = sum(s.n * 4.0 / 3.0 * math.pi * (1.0 / s.unit_cube_res if s.unit_cube_res else s.h) ** 3
+                     * s.rest_density / s.mass for s in scenes)
+    return neighbours >= CROWDED_NEIGHBOURS * sum(s.n for s in scenes)
+
+
+def variants_for(particles: int, persistent: int, is_crowded: bool = False) -> tuple:
     """The variant values worth timing for a launch of `particles` particles:
     all 64 where several lanes per particle can apply (one block per tile and
     a small enough launch), else the 32 without that bit, which would change
     nothing there."""
-    split = particles <= DENSITY_SPLIT_MAX and persistent == 0
+    split = particles <= (CROWDED_MAX if is_crowded else DENSITY_SPLIT_MAX) and persistent == 0
     return VARIANTS if split else VARIANTS[:32]
 
 
@@ -94,7 +107,7 @@ def tune(workload: str, steps: int = 20, device: int = 0, variants_only: bool = 
         trials.append({"tile": tile, "persistent": pers, "skin": skin, "variant": 0, "ms_per_step": ms,
                        "particle_steps_per_s": n / (ms * 1e-3)})
     best = min(trials, key=lambda t: t["ms_per_step"])
-    for v in variants_for(n, best["persistent"])[1:]:
+    for v in variants_for(n, best["persistent"], crowded(scenes))[1:]:
         ms = time_config(scenes, best["tile"], best["persistent"], best["skin"], steps, device=device, variant=v)
         trials.append({"tile": best["tile"], "persistent": best["persistent"], "skin": best["skin"], "variant": v,
                        "ms_per_step": ms, "particle_steps_per_s": n / (ms * 1e-3)})
