@@ -529,7 +529,8 @@ int Engine::upload_params() {
 }
 
 LaunchForm Engine::form_of(uint32_t particles, uint32_t ntiles, bool persistent) const {
-    return launch_form(particles, ntiles, exec_.tile, persistent, exec_.variant, crowded_, !all_defer_, any_tension_);
+    return launch_form(particles, ntiles, exec_.tile, persistent, exec_.variant, crowded_, !all_defer_, any_tension_,
+                       (uint32_t)sm_count_);
 }
 
 // The passes launched outside the graphs (an export's, ahead) follow captured ones

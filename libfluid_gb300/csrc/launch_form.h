@@ -24,11 +24,11 @@ struct LaunchForm {
     bool operator!=(const LaunchForm& o) const { return !(*this == o); }
 };
 
-// particles in ntiles tiles of `tile` threads; crowded: SPH_CROWDED_NBRS neighbours
+// particles in ntiles tiles of `tile` threads, on a GPU of `sms` SMs; crowded: SPH_CROWDED_NBRS neighbours
 // or more on average; skin: some scene runs a per-substep XSPH pass; tension: some
 // scene runs the normal pass.
 inline LaunchForm launch_form(uint32_t particles, uint32_t ntiles, uint32_t tile, bool persistent, uint32_t variant,
-                              bool crowded, bool skin, bool tension) {
+                              bool crowded, bool skin, bool tension, uint32_t sms) {
     LaunchForm f;
     if ((variant & SPH_VARIANT_DENSITY_SPLIT) != 0u && !persistent && ntiles <= 65535u) {   // (tiles are the grid's y)
         if (particles <= (crowded ? SPH_CROWDED8_MAX : SPH_WIDE8_MAX)) f.lanes = 8u;
@@ -37,7 +37,7 @@ inline LaunchForm launch_form(uint32_t particles, uint32_t ntiles, uint32_t tile
     f.density_wide = f.lanes > 1u && !skin;
     f.half = f.lanes == 1u && !skin;
     f.dense = f.half && tension;   // (long lists and skin words leave no room)
-    f.one_wave = !persistent && (uint64_t)ntiles * tile <= SPH_ONE_WAVE_THREADS;
+    f.one_wave = !persistent && (uint64_t)ntiles * tile <= (uint64_t)SPH_ONE_WAVE_THREADS * sms;
     return f;
 }
 

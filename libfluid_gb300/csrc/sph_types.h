@@ -101,14 +101,14 @@ struct DevParams {
 #ifndef SPH_DENSITY_SPLIT_MAX
 #define SPH_DENSITY_SPLIT_MAX 34816u
 #endif
-// Threads that the GPU holds at once with 80 registers each (152 SMs, six blocks
-// of 128): a launch of one thread per particle that is no larger gains nothing
+// Threads that an SM holds at once with 80 registers each (six blocks of 128; the
+// GPU with 152 SMs 116,736): a launch of one thread per particle that is no larger gains nothing
 // from smaller register budgets, and runs builds that have more loads in flight
 // instead.  Density, normals, force of 82,484 particles 32.5, 14.3, 27.5 -> 30.6,
 // 13.8, 24.6 us, of 97,336 (no normals) 33.3, -, 24.4 -> 31.5, -, 20.6; a launch
 // that takes a second wave is slower with them (125,000 particles 37.6, -, 26.6
 // -> 42.8, -, 30.6).
-#define SPH_ONE_WAVE_THREADS  116736u
+#define SPH_ONE_WAVE_THREADS  768u
 #define SPH_CROWDED_NBRS      80u
 #define SPH_CROWDED8_MAX      61440u
 

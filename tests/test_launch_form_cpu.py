@@ -101,3 +101,20 @@ def test_passes_of_a_substep_share_one_form(n, forms):
     substeps, mixed, lanes, bad = map(int, run_driver(DRIVER, n).split())
     assert substeps > 1000 and lanes >= forms
     assert mixed == 0 and bad == 0
+
+
+ONE_WAVE = r"""
+#include "launch_form.h"
+#include <cstdio>
+int main() {
+    for (uint32_t sms : {152u, 148u, 1u})
+        for (uint32_t tiles : {sms * 6u, sms * 6u + 1u})
+            for (bool persistent : {false, true})
+                std::printf("%d ", sph::launch_form(tiles * 128u, tiles, 128u, persistent, 31u, false, false, false, sms).one_wave);
+}
+"""
+
+
+def test_one_wave_follows_the_gpu():
+    """Six blocks of 128 threads to an SM, and one block more; not when persistent."""
+    assert run_driver(ONE_WAVE).split() == ["1", "0", "0", "0"] * 3
