@@ -106,6 +106,7 @@ def test_passes_of_a_substep_share_one_form(n, forms):
 ONE_WAVE = r"""
 #include "launch_form.h"
 #include <cstdio>
+#include <initializer_list>
 int main() {
     for (uint32_t sms : {152u, 148u, 1u})
         for (uint32_t tiles : {sms * 6u, sms * 6u + 1u})
