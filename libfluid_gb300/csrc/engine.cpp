@@ -528,8 +528,8 @@ int Engine::upload_params() {
     return ENG_OK;
 }
 
-LaunchForm Engine::form_of(uint32_t particles, uint32_t ntiles, bool persistent) const {
-    return launch_form(particles, ntiles, exec_.tile, persistent, exec_.variant, crowded_, !all_defer_, any_tension_,
+LaunchForm Engine::form_of(uint32_t ntiles, bool persistent) const {
+    return launch_form(ntiles, exec_.tile, persistent, exec_.variant, crowded_, !all_defer_, any_tension_,
                        (uint32_t)sm_count_);
 }
 
@@ -542,7 +542,7 @@ void Engine::update_form() {
     for (const auto& s : scenes_)
         nbrs += (double)s.n * (4.0 / 3.0 * 3.14159265 * s.dp.h * s.dp.h * s.dp.h * s.dp.rest_density / s.dp.mass);
     crowded_ = nbrs >= (double)SPH_CROWDED_NBRS * n;
-    const LaunchForm f = form_of((uint32_t)n, ntiles_, exec_.persistent != 0u);
+    const LaunchForm f = form_of(ntiles_, exec_.persistent != 0u);
     if (f != form_) {
         form_ = f;
         graph_dirty_ = true;
@@ -860,7 +860,7 @@ int Engine::prefix_scene(const Scene& sc, bool wait) {
     StepArgs a = args();
     a.tiles = d_tiles_ + sc.tile_first;
     a.ntiles = sc.tile_count;
-    a.form = form_of(sc.n, sc.tile_count, false);
+    a.form = form_of(sc.tile_count, false);
     a.grid_nbr = sc.tile_count;
     a.tile_ctr = nullptr;
     a.scan_zeroes_counts = 0u;   // keep the counts for the full prefix that follows

@@ -181,7 +181,7 @@ private:
     int ensure_capacity(uint64_t parts, uint64_t cells);
     int rebuild_layout();
     int upload_params();
-    LaunchForm form_of(uint32_t particles, uint32_t ntiles, bool persistent) const;
+    LaunchForm form_of(uint32_t ntiles, bool persistent) const;
     void update_form();                // form_ from the layout and parameters in force
     int launch_prefix(bool profile);   // [memset, hash], scan, sort, density
     int launch_prefix_args(const StepArgs& a, bool profile, bool hash);

@@ -81,11 +81,11 @@ struct DevParams {
 #define SPH_VARIANT_FORCE_TABLE   0x8u   // no effect: the force and normal passes walk the neighbour list
 #define SPH_VARIANT_NORMALS_TABLE 0x10u  // no effect
 #define SPH_VARIANT_DENSITY_SPLIT 0x20u  // neighbour passes: several lanes per particle in small launches
-                                         // (at most SPH_DENSITY_SPLIT_MAX particles, more where crowded)
+                                         // (at most SPH_DENSITY_SPLIT_MAX threads of tiles, more where crowded)
 #define SPH_VARIANT_MASK          0x3fu
 #define SPH_VARIANT_DEFAULT       0x3fu
 
-// Largest launches (particles over all tiles) that run eight and four lanes per
+// Largest launches (threads of all tiles) that run eight and four lanes per
 // particle in the neighbour passes.  Measured on cubes of fluid at rest density
 // (33 neighbours), substep in us with eight lanes, four, one: 13,824 particles
 // 34.9, 36.7, 52.5; 21,952 45.9, 40.0, 52.2; 32,768 55.4, 46.1, 53.3; 35,937
@@ -101,10 +101,9 @@ struct DevParams {
 #ifndef SPH_DENSITY_SPLIT_MAX
 #define SPH_DENSITY_SPLIT_MAX 34816u
 #endif
-// Threads that an SM holds at once with 80 registers each (six blocks of 128; the
-// GPU with 152 SMs 116,736): a launch of one thread per particle that is no larger gains nothing
-// from smaller register budgets, and runs builds that have more loads in flight
-// instead.  Density, normals, force of 82,484 particles 32.5, 14.3, 27.5 -> 30.6,
+// Threads that an SM holds at once with 80 registers each (six blocks of 128; 152 SMs
+// 116,736): a launch of one thread per particle that is no larger gains nothing from
+// smaller register budgets, and runs builds that have more loads in flight instead.  Density, normals, force of 82,484 particles 32.5, 14.3, 27.5 -> 30.6,
 // 13.8, 24.6 us, of 97,336 (no normals) 33.3, -, 24.4 -> 31.5, -, 20.6; a launch
 // that takes a second wave is slower with them (125,000 particles 37.6, -, 26.6
 // -> 42.8, -, 30.6).

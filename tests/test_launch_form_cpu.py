@@ -111,7 +111,7 @@ int main() {
     for (uint32_t sms : {152u, 148u, 1u})
         for (uint32_t tiles : {sms * 6u, sms * 6u + 1u})
             for (bool persistent : {false, true})
-                std::printf("%d ", sph::launch_form(tiles * 128u, tiles, 128u, persistent, 31u, false, false, false, sms).one_wave);
+                std::printf("%d ", sph::launch_form(tiles, 128u, persistent, 31u, false, false, false, sms).one_wave);
 }
 """
 
@@ -119,3 +119,29 @@ int main() {
 def test_one_wave_follows_the_gpu():
     """Six blocks of 128 threads to an SM, and one block more; not when persistent."""
     assert run_driver(ONE_WAVE).split() == ["1", "0", "0", "0"] * 3
+
+
+LANES = r"""
+#include "engine.h"
+#include <cstdio>
+#include <initializer_list>
+int main() {
+    using namespace sph;
+    auto lanes = [](uint32_t scenes, uint32_t n, uint32_t tile, bool crowded, uint32_t variant = SPH_VARIANT_DEFAULT) {
+        const uint32_t tiles = scenes * ((n + tile - 1u) / tile);
+        std::printf("%u ", launch_form(tiles, tile, false, variant, crowded, false, false, 152u).lanes);
+    };
+    for (uint32_t tile : {64u, 128u, 256u})   // one scene at the limits
+        for (uint32_t n : {1u, 14336u, 14337u, 34816u, 34817u}) lanes(1, n, tile, false);
+    for (uint32_t n : {34817u, 61440u, 61441u}) lanes(1, n, 128, true);
+    lanes(1, 100, 128, false, 31);
+    for (uint32_t scenes : {112u, 113u, 272u, 273u, 14000u, 100000u}) lanes(scenes, 1, 128, false);
+}
+"""
+
+
+def test_lanes_go_by_the_tiles():
+    """A scene alone by its particles; many tiny scenes by the threads launched for
+    them (one lane where most blocks would have no particle)."""
+    assert run_driver(LANES).split() == ["8", "8", "4", "4", "1"] * 3 + ["8", "8", "1"] + ["1"] + [
+        "8", "4", "4", "1", "1", "1"]
