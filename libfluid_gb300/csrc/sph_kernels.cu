@@ -695,16 +695,17 @@ __device__ __forceinline__ void walk_rows(const DevParams& P, const uint32_t* __
         for (uint32_t j = max(jb, from); j < je; ++j) f(j);
     }
 }
-// The same without k, in the normal and force passes.  With H (HalfScan's
-// positions) those that it finds, 32 tested before the first is visited: visiting
-// each candidate to test it runs the pair arithmetic on almost every one, as one
-// lane in 32 that accepts is enough.  Without H all of them; f(j) tests the
-// distance itself.  66,560 particles compressed until most lists end early: substep
-// 185 -> 151 us.
+// The same without k, in the normal and force passes: those that the candidate scan
+// finds (HalfScan with `half_x`, else CandidateScan, of X's positions), 32 tested
+// before the first is visited: visiting each candidate to test it runs the pair
+// arithmetic on almost every one, as one lane in 32 that accepts is enough.  f(j)
+// tests the distance itself.  66,560 particles compressed until most lists end
+// early: substep 185 -> 151 us; 64,000 of 260 neighbours with an XSPH pass per
+// substep (lists of 56, positions as floats) 1057 -> 865, 250,000 2266 -> 1992.
 template <class F>
 __device__ __forceinline__ void walk_tail(const DevParams& P, const uint32_t* __restrict__ start, uint32_t cell_base,
                                           uint32_t delta, int3 g, const float4& p, uint32_t k, uint32_t from,
-                                          const float* __restrict__ H, F&& f) {
+                                          const float* __restrict__ X, bool half_x, F&& f) {
     HalfScan half(P, p, g);
 #pragma unroll 1
     for (int r = 0; r < 9; ++r) {
@@ -715,14 +716,20 @@ __device__ __forceinline__ void walk_tail(const DevParams& P, const uint32_t* __
 #pragma unroll 1
         for (uint32_t c = jb & ~3u; c < je; c += 32u) {
             const uint32_t left = je - c, nq = (min(left, 32u) + 3u) / 4u;
-            uint32_t bits = ~0u;
-            if (H) {
-                const uint2* hp = reinterpret_cast<const uint2*>(H) + 4 * (size_t)(c / 4u);
-                uint32_t dm = 0u;
+            uint32_t dm = 0u;
+            if (half_x) {
+                const uint2* hp = reinterpret_cast<const uint2*>(X) + 4 * (size_t)(c / 4u);
                 for (uint32_t q = 0u; q < nq; ++q, hp += 4)
                     half.visit4(__ldg(hp + half.copy), __ldg(reinterpret_cast<const uint4*>(hp + 2)), dm);
-                bits = dm << (32u - 4u * nq);
+            } else {
+                const CandidateScan<false> scan(p.x, p.y, p.z, P.h2, P.h2);
+                const float4* xp = reinterpret_cast<const float4*>(X) + 3 * (size_t)(c / 4u);
+                uint32_t none = 0u;
+#pragma unroll 1
+                for (uint32_t q = 0u; q < nq; ++q, xp += 3)
+                    scan.visit4(__ldg(xp), __ldg(xp + 1), __ldg(xp + 2), dm, none);
             }
+            uint32_t bits = dm << (32u - 4u * nq);
             if (left < 32u) bits &= ~(~0u >> left);
             if (c < jb) bits &= ~0u >> (jb - c);
             if (k - c < 32u) bits &= ~(0x80000000u >> (k - c));
@@ -1245,7 +1252,7 @@ __global__ void __maxnreg__(LANES > 1 ? 40 : FEW ? 64 : 48) k_normals(const DevP
             reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load,
             pair,
             [&](uint32_t from) {
-                walk_tail(pp, start, sc.cell_base, delta, g, p, k, from, half_x ? X : nullptr,
+                walk_tail(pp, start, sc.cell_base, delta, g, p, k, from, X, half_x,
                           [&](uint32_t j) { pair(load(j)); });
             });
     }
@@ -1477,7 +1484,7 @@ k_force_integrate(const DevParams* __restrict__ params,
             pp, start, sc.cell_base, delta, g, mask, mask_stride, k,
             reinterpret_cast<uint32_t*>(s_dyn) + threadIdx.x, blockDim.x, load,
             visit, [&](uint32_t from) {
-                walk_tail(pp, start, sc.cell_base, delta, g, pi, k, from, half_x ? X : nullptr,
+                walk_tail(pp, start, sc.cell_base, delta, g, pi, k, from, X, half_x,
                           [&](uint32_t j) { visit(load(j)); });
             });
     }
