@@ -26,9 +26,8 @@ struct SceneConfig {
     int boundary = 0;                 // 0: the box; 1: the sphere of radius min half extent about its centre
 };
 
-// Execution choices of the substep.  Defaults are the autotuner's choice
-// (libfluid_gb300/autotune.py, recorded in libfluid_gb300/tuned.json) for the
-// 1M dam break and the 256-scene batch alike.
+// Execution choices of the substep.  libfluid_gb300/autotune.py sweeps them; its
+// record (tuned.json) is of an earlier build, the defaults are this build's.
 struct ExecConfig {
     uint32_t tile = 128;              // particles per tile = threads per block (64, 128 or 256)
     uint32_t persistent = 0;          // 0: one block per tile; k > 0: k blocks per SM pull tiles
@@ -228,9 +227,8 @@ private:
     std::map<uint32_t, uint32_t> free_;
     uint64_t pcap_ = 0, ccap_ = 0, slots_end_ = 0;
     // device arenas
-    float4 *P0_ = nullptr, *G_ = nullptr, *V0_ = nullptr, *V2_ = nullptr, *A0_ = nullptr,   // G_: two per slot
-          
-           *A1_ = nullptr, *N_ = nullptr, *R_ = nullptr;   // R_: two per slot
+    float4 *P0_ = nullptr, *V0_ = nullptr, *V2_ = nullptr, *A0_ = nullptr, *A1_ = nullptr, *N_ = nullptr;
+    float4 *G_ = nullptr, *R_ = nullptr;   // two per slot
     float* C2_ = nullptr;
     uint32_t *okey_ = nullptr;         // packed cells of the last substep (state order)
     uint32_t *pend_ = nullptr;                      // per scene-table entry: XSPH update pending

@@ -967,7 +967,8 @@ k_density(const DevParams* __restrict__ params,
         const float2 dxy = __fadd2_rn(make_float2(p.x, p.y), make_float2(-q.x, -q.y));
         const float dx = dxy.x, dy = dxy.y, dz = p.z - q.z;
         const float rr = dot3(dx, dy, dz, dx, dy, dz);
-        // true for every listed neighbour of finite position; the test matters in the tail
+        // the exact test: HalfScan's lists hold pairs just beyond h too, and past the
+        // list's end every candidate comes here
         if (rr <= h2) {
             const float w = poly6_r2(rr, h, h2, c6);
             sum = fmaf(mass, w, sum);
@@ -1392,8 +1393,9 @@ k_force_integrate(const DevParams* __restrict__ params,
     const Cohesion coh(pp);
     // One pair: neighbour j with its record, and its normal with the squared
     // sound speed.  press(mid, mp, c) takes the pressure and viscosity terms'
-    // scales and the spiky gradient along rvec; tens(t) the tension term.  Listed
-    // neighbours lie within h; those of the tail are tested by the caller (dist2).
+    // scales and the spiky gradient along rvec; tens(t) the tension term.  The test
+    // r^2 <= h^2 decides what counts: lists hold pairs just beyond h too (HalfScan),
+    // and what is found past their end may lie there as well.
     // r is the correctly rounded root: h - r cancels, and pairs at r ~ h must see
     // the reference's r; 1/r and the quotients only scale (approximate).  At
     // r = h the gradient and the cohesion vanish with h - r.  j == k has r^2 = 0
