@@ -136,10 +136,6 @@ Engine::Engine(int device) {
     cudaEventCreateWithFlags(&pack_ev_, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&vel_ev_, cudaEventDisableTiming);
     cudaMallocHost((void**)&h_status_, sizeof(uint32_t));
-    if (cudaMallocHost((void**)&h_small_, kSmallExport) != cudaSuccess) {
-        h_small_ = nullptr;   // small exports then take the way of the large ones
-        cudaGetLastError();
-    }
     cudaMalloc((void**)&status_, 2 * sizeof(uint32_t));
     cudaMemsetAsync(status_, 0, 2 * sizeof(uint32_t), stream_);
     gate_ = status_ + 1;
@@ -338,6 +334,27 @@ int Engine::staging(size_t bytes, float** out) {
     }
     *out = stage_;
     return ENG_OK;
+}
+
+// Pinned memory for an export of `bytes`; false where it is too large for that way
+// or was refused (it then takes the way of the large ones).  Made for the first such
+// export and as large as it needs to be: the driver gives it out of slabs of 2 MB,
+// and an engine that opens one pays 0.1 ms, and as much again when it closes it.
+bool Engine::small_landing(size_t bytes) {
+    if (bytes > kSmallExport || small_refused_) return false;
+    if (bytes > small_bytes_) {
+        if (h_small_) cudaFreeHost(h_small_);   // (no export is under way)
+        small_bytes_ = std::max<size_t>(32u << 10, std::min(kSmallExport, 2 * small_bytes_));
+        while (small_bytes_ < bytes) small_bytes_ = std::min(kSmallExport, 2 * small_bytes_);
+        if (cudaMallocHost((void**)&h_small_, small_bytes_) != cudaSuccess) {
+            h_small_ = nullptr;
+            small_bytes_ = 0;
+            small_refused_ = true;
+            cudaGetLastError();
+            return false;
+        }
+    }
+    return true;
 }
 
 uint64_t Engine::total_particles() const {
@@ -1070,7 +1087,7 @@ int Engine::get_state(int id, float* pos, float* colour, float* vel, uint32_t n,
     // device memory and copied: writing 36 MB over the host link from the
     // kernels measured twice as slow as the copy engine.
     const size_t bytes = (size_t)n * 3 * sizeof(float);
-    const bool small = h_small_ && 3 * bytes <= kSmallExport;
+    const bool small = small_landing(3 * bytes);
     float* st = h_small_;
     if (!small) { int rc = staging(3 * bytes, &st); if (rc) return rc; }
     float* dp = pos ? st : nullptr;

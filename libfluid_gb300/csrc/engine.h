@@ -211,6 +211,7 @@ private:
     uint32_t alloc_slots(uint32_t n);
     void free_slots(uint32_t base, uint32_t n);
     int staging(size_t bytes, float** out);
+    bool small_landing(size_t bytes);
     StepArgs args() const;
 
     int device_ = 0;
@@ -254,9 +255,11 @@ private:
     // host mirrors
     DevParams* h_params_ = nullptr;    // pinned
     uint32_t* h_status_ = nullptr;     // pinned
-    // Pinned landing place of small exports (kSmallExport bytes): the kernels
+    // Pinned landing place of small exports (up to kSmallExport bytes): the kernels
     // write into it directly and the host copies from there.
-    float* h_small_ = nullptr;         // (null: pinned memory was refused)
+    float* h_small_ = nullptr;
+    size_t small_bytes_ = 0;
+    bool small_refused_ = false;       // pinned memory was refused
     uint32_t reads_ = 0;               // scene reads since the last step or change (get_state with `many`)
     bool shared_failed_ = false;       // the prefix over all scenes that those reads share has failed
     std::vector<DevScene> h_scenes_;

@@ -70,10 +70,14 @@ cudaError_t cudaMallocHost(void** p, size_t n) {
         *p = nullptr;
         return fake::st.last_error = cudaErrorMemoryAllocation;
     }
+    fake::st.pinned += n;
     return take(p, n);
 }
 cudaError_t cudaFree(void* p) { return give(p); }
-cudaError_t cudaFreeHost(void* p) { return give(p); }
+cudaError_t cudaFreeHost(void* p) {
+    fake::st.pinned -= fake::blocks[(const char*)p];
+    return give(p);
+}
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { std::memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
     run([=] { std::memcpy(d, s, n); });

@@ -30,6 +30,7 @@ struct State {
     std::function<void()> after_force;     // called after each force pass
     std::vector<uint32_t> sorts;   // tiles of each sort
     size_t pinned_limit = ~(size_t)0;      // larger pinned allocations fail
+    size_t pinned = 0;                     // bytes pinned now
     cudaError_t last_error = cudaSuccess;
     uint64_t null_writes = 0;      // packs and unsorts into a null or unknown buffer
 };

@@ -78,3 +78,36 @@ def test_export_after_a_failed_prefix(blocking, many, ahead):
     """The error comes with the state's positions and colours, and the caller's
     velocities are left alone: none were computed."""
     assert run_driver(FAILED, blocking, many, ahead).split() == ["0", "7", "0"] * 2
+
+
+PINNED = r"""
+#include "fake_cuda.h"
+#include <cstdio>
+using namespace sph;
+int main() {
+    SceneConfig c;
+    c.box_mode = 1;
+    c.h = 0.1f;
+    {
+        Engine e(0);
+        int id[4];
+        const uint32_t n[] = {300, 1000, 10922, 10923};
+        for (int i = 0; i < 4; ++i) e.add_scene(c, n[i], &id[i]);
+        std::vector<float> p(3 * 10923), v(3 * 10923);
+        e.step(1);
+        const size_t before = fake::st.pinned;
+        for (int i : {3, 0, 1, 2, 0}) {
+            e.get_state(id[i], p.data(), nullptr, v.data(), n[i]);
+            std::printf("%zu ", fake::st.pinned - before);
+        }
+        std::printf("%d ", before < 4096u);
+    }
+    std::printf("%zu", fake::st.pinned);
+}
+"""
+
+
+def test_pinned_memory_as_needed():
+    """Nothing for a system that exports nothing small; then as much as the largest
+    needs, given back with the system."""
+    assert run_driver(PINNED).split() == ["0", "32768", "65536", "393216", "393216", "1", "0"]
