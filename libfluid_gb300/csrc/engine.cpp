@@ -174,6 +174,7 @@ int Engine::fail(int code, const std::string& msg) {
     return code;
 }
 int Engine::cuda_fail(cudaError_t e, const char* what) {
+    cudaGetLastError();   // reported here; the next launch does not report it again
     err_ = std::string(what) + ": " + cudaGetErrorString(e);
     return ENG_ECUDA;
 }
@@ -204,6 +205,72 @@ void Engine::free_all() {
     dev_bytes_ = 0;
 }
 
+// `*p` in a new device array of that size with the first `keep` bytes of the old
+// one; the old one stays where there is no memory.
+bool Engine::regrow(void** p, size_t bytes, size_t keep) {
+    void* q = nullptr;
+    if (cudaMalloc(&q, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (*p) {
+        if (keep) cudaMemcpyAsync(q, *p, keep, cudaMemcpyDeviceToDevice, stream_);
+        cudaStreamSynchronize(stream_);
+        cudaFree(*p);
+    }
+    *p = q;
+    return true;
+}
+
+// The arrays that hold nothing from one substep to the next, for the capacities in
+// force.
+struct Engine::Scratch { void** p; size_t bytes; };
+std::vector<Engine::Scratch> Engine::slot_scratch() {
+    const size_t n = pcap_;
+    mask_stride_ = (n + 3) & ~(size_t)3;   // the density pass reads rows four slots at a time
+    std::vector<Scratch> v = {{(void**)&G_, 2 * n * sizeof(float4)}, {(void**)&A1_, n * sizeof(float4)},
+                              {(void**)&N_, n * sizeof(float4)}, {(void**)&key_, n * sizeof(uint32_t)},
+                              {(void**)&slot_, n * sizeof(uint32_t)}, {(void**)&perm_, n * sizeof(uint32_t)},
+                              {(void**)&mask_, SPH_MASK_ROWS * mask_stride_ * sizeof(uint32_t)}};
+    if (debug_) {
+        v.push_back({(void**)&dbg_nbr_, n * sizeof(uint32_t)});
+        v.push_back({(void**)&dbg_forces_, n * 4 * sizeof(float4)});
+    }
+    return v;
+}
+std::vector<Engine::Scratch> Engine::cell_scratch() {
+    const size_t n = ccap_;
+    return {{(void**)&count_, n * sizeof(uint32_t)},
+            {(void**)&start_, (n + 1) * sizeof(uint32_t)},
+            // the scan's tile counter and look-back descriptors (64-bit words)
+            {(void**)&scan_sums_, (n / kScanTileCells + 3) * sizeof(unsigned long long)},
+            {(void**)&sums_, (n / kScanTileCells + 1) * sizeof(uint32_t)}};
+}
+bool Engine::alloc_scratch(const std::vector<Scratch>& arrays) {
+    for (const Scratch& x : arrays)
+        if (!*x.p && !regrow(x.p, x.bytes, 0)) return false;
+    return true;
+}
+void Engine::free_scratch(const std::vector<Scratch>& arrays) {
+    for (const Scratch& x : arrays) {
+        if (*x.p) cudaFree(*x.p);
+        *x.p = nullptr;
+    }
+}
+// `cap` (pcap_ or ccap_) raised to `to`, with the scratch arrays that follow it.  They
+// are freed first: the old and new ones together may not fit.  Without memory for the
+// new ones the old ones come back, now or before the next substep (prepare).
+bool Engine::grow_scratch(uint64_t& cap, uint64_t to, std::vector<Scratch> (Engine::*arrays)()) {
+    const uint64_t old = cap;
+    free_scratch((this->*arrays)());
+    cap = to;
+    if (alloc_scratch((this->*arrays)())) return true;
+    free_scratch((this->*arrays)());
+    cap = old;
+    if (old != 0 && !alloc_scratch((this->*arrays)())) scratch_lost_ = true;
+    return false;
+}
+
 // Grow the particle and cell arenas, preserving live particle state.
 int Engine::ensure_capacity(uint64_t parts, uint64_t cells) {
     cudaSetDevice(device_);
@@ -211,77 +278,30 @@ int Engine::ensure_capacity(uint64_t parts, uint64_t cells) {
     const ArenaPlan plan = plan_arena(parts, cells, pcap_, ccap_, byte_limit_, bytes_per_particle());
     if (plan.status == kArenaOverBudget) return fail(ENG_ENOMEM, "arena would exceed the memory budget");
     if (plan.status == kArenaAtBudget) return fail(ENG_ENOMEM, "arena at its memory budget");
+    if (plan.parts >= (1ull << 31)) return fail(ENG_ENOMEM, "particle capacity exceeds 2^31");
+    if (plan.parts > pcap_ || plan.cells > ccap_) {
+        // arrays move, whether all of them can grow or not: the graphs, a prefix at
+        // hand and the last hash are of the old ones
+        graph_dirty_ = true;
+        prefix_valid_ = false;
+        hashed_ = false;
+    }
     if (plan.parts > pcap_) {
         const uint64_t np = plan.parts;
-        if (np >= (1ull << 31)) return fail(ENG_ENOMEM, "particle capacity exceeds 2^31");
         // state between substeps: P0, V0, A0, and for scenes with a pending
         // XSPH update their post-integration velocities V2 and cells; and the
         // fields of the last substep that the debug taps read (C2, R)
-        struct Kept { void** p; size_t entry; };
-        const Kept state[] = {{(void**)&P0_, sizeof(float4)}, {(void**)&V0_, sizeof(float4)},
-                              {(void**)&A0_, sizeof(float4)}, {(void**)&V2_, sizeof(float4)},
-                              {(void**)&R_, 2 * sizeof(float4)}, {(void**)&C2_, sizeof(float)},
-                              {(void**)&okey_, sizeof(uint32_t)}};
-        struct { float4** p; uint64_t per_slot; } scratch[] = {{&G_, 2}, {&A1_, 1}, {&N_, 1}};
-        for (const Kept& k : state) {
-            void* q = nullptr;
-            cudaError_t e = cudaMalloc(&q, np * k.entry);
-            if (e != cudaSuccess) return fail(ENG_ENOMEM, std::string("device allocation failed: ") + cudaGetErrorString(e));
-            if (*k.p) {
-                ENG_CK(cudaMemcpyAsync(q, *k.p, pcap_ * k.entry, cudaMemcpyDeviceToDevice, stream_), "grow copy");
-                ENG_CK(cudaStreamSynchronize(stream_), "grow sync");
-                cudaFree(*k.p);
-            }
-            *k.p = q;
-        }
-        prefix_valid_ = false;
-        for (const auto& x : scratch) {
-            if (*x.p) cudaFree(*x.p);
-            *x.p = nullptr;
-            cudaError_t e = cudaMalloc((void**)x.p, np * x.per_slot * sizeof(float4));
-            if (e != cudaSuccess) return fail(ENG_ENOMEM, std::string("device allocation failed: ") + cudaGetErrorString(e));
-        }
-        uint32_t** u[] = {&key_, &slot_, &perm_};
-        for (auto p : u) {
-            if (*p) cudaFree(*p);
-            *p = nullptr;
-            cudaError_t e = cudaMalloc((void**)p, np * sizeof(uint32_t));
-            if (e != cudaSuccess) return fail(ENG_ENOMEM, std::string("device allocation failed: ") + cudaGetErrorString(e));
-        }
-        if (mask_) cudaFree(mask_);
-        mask_ = nullptr;
-        {
-            mask_stride_ = (np + 3) & ~(uint64_t)3;   // the density pass reads rows four slots at a time
-            cudaError_t e = cudaMalloc((void**)&mask_, (size_t)SPH_MASK_ROWS * mask_stride_ * sizeof(uint32_t));
-            if (e != cudaSuccess) return fail(ENG_ENOMEM, std::string("device allocation failed: ") + cudaGetErrorString(e));
-        }
-        if (dbg_nbr_) { cudaFree(dbg_nbr_); dbg_nbr_ = nullptr; }
-        if (dbg_forces_) { cudaFree(dbg_forces_); dbg_forces_ = nullptr; }
-        if (debug_) {
-            ENG_CK(cudaMalloc((void**)&dbg_nbr_, np * sizeof(uint32_t)), "debug alloc");
-            ENG_CK(cudaMalloc((void**)&dbg_forces_, np * 4 * sizeof(float4)), "debug alloc");
-        }
-        pcap_ = np;
-        graph_dirty_ = true;
+        struct { void** p; size_t entry; } state[] = {
+            {(void**)&P0_, sizeof(float4)}, {(void**)&V0_, sizeof(float4)}, {(void**)&A0_, sizeof(float4)},
+            {(void**)&V2_, sizeof(float4)}, {(void**)&R_, 2 * sizeof(float4)}, {(void**)&C2_, sizeof(float)},
+            {(void**)&okey_, sizeof(uint32_t)}};
+        for (const auto& k : state)
+            if (!regrow(k.p, np * k.entry, pcap_ * k.entry)) return fail(ENG_ENOMEM, "device allocation failed");
+        if (!debug_) free_scratch({{(void**)&dbg_nbr_, 0}, {(void**)&dbg_forces_, 0}});   // (of an earlier size)
+        if (!grow_scratch(pcap_, np, &Engine::slot_scratch)) return fail(ENG_ENOMEM, "device allocation failed");
     }
-    if (plan.cells > ccap_) {
-        const uint64_t nc = plan.cells;
-        if (count_) cudaFree(count_);
-        if (start_) cudaFree(start_);
-        if (scan_sums_) cudaFree(scan_sums_);
-        if (sums_) cudaFree(sums_);
-        count_ = start_ = scan_sums_ = sums_ = nullptr;
-        cudaError_t e1 = cudaMalloc((void**)&count_, nc * sizeof(uint32_t));
-        cudaError_t e2 = cudaMalloc((void**)&start_, (nc + 1) * sizeof(uint32_t));
-        // the scan's tile counter and look-back descriptors (64-bit words)
-        cudaError_t e3 = cudaMalloc((void**)&scan_sums_, (nc / 4096 + 3) * sizeof(unsigned long long));
-        cudaError_t e4 = cudaMalloc((void**)&sums_, (nc / kScanTileCells + 1) * sizeof(uint32_t));
-        if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess)
-            return fail(ENG_ENOMEM, "device allocation of cell arrays failed");
-        ccap_ = nc;
-        graph_dirty_ = true;
-        prefix_valid_ = false;
-    }
+    if (plan.cells > ccap_ && !grow_scratch(ccap_, plan.cells, &Engine::cell_scratch))
+        return fail(ENG_ENOMEM, "device allocation of cell arrays failed");
     dev_bytes_ = pcap_ * bytes_per_particle() + ccap_ * 8;
     return ENG_OK;
 }
@@ -486,35 +506,30 @@ int Engine::rebuild_layout() {
     total_cells_ = (uint32_t)cb;
     int rc = ensure_capacity(slots_end_, cb);
     if (rc) return rc;
+    // the tables, each with its own capacity: what a launch is given is never a
+    // freed array, whether the new ones can be had or not
+    graph_dirty_ = true;
+    auto table = [&](uint64_t& cap, uint64_t need, std::initializer_list<Scratch> arrays) {
+        if (need <= cap) return true;
+        const uint64_t to = std::max<uint64_t>(need, cap * 2);
+        for (const Scratch& x : arrays)
+            if (!regrow(x.p, to * x.bytes, 0)) return false;   // (bytes: per entry)
+        cap = to;
+        return true;
+    };
     if (ns > scene_cap_) {
-        if (d_scenes_) cudaFree(d_scenes_);
-        if (d_params_) cudaFree(d_params_);
+        DevParams* q = nullptr;
+        ENG_CK(cudaMallocHost((void**)&q, std::max<uint64_t>(ns, scene_cap_ * 2) * sizeof(DevParams)), "param staging");
         if (h_params_) cudaFreeHost(h_params_);
-        scene_cap_ = std::max<uint64_t>(ns, scene_cap_ * 2);
-        ENG_CK(cudaMalloc((void**)&d_scenes_, scene_cap_ * sizeof(DevScene)), "scene table");
-        ENG_CK(cudaMalloc((void**)&d_params_, scene_cap_ * sizeof(DevParams)), "param table");
-        ENG_CK(cudaMallocHost((void**)&h_params_, scene_cap_ * sizeof(DevParams)), "param staging");
-        graph_dirty_ = true;
+        h_params_ = q;
     }
-    if (ns > tile_first_cap_) {
-        if (d_tile_first_) cudaFree(d_tile_first_);
-        tile_first_cap_ = std::max<uint64_t>(ns, tile_first_cap_ * 2);
-        ENG_CK(cudaMalloc((void**)&d_tile_first_, tile_first_cap_ * sizeof(uint32_t)), "tile offsets");
-    }
-    if (ns > pend_cap_) {
-        if (pend_) cudaFree(pend_);
-        pend_cap_ = std::max<uint64_t>(ns, pend_cap_ * 2);
-        ENG_CK(cudaMalloc((void**)&pend_, pend_cap_ * sizeof(uint32_t)), "pending flags");
-        graph_dirty_ = true;
-    }
+    if (!table(scene_cap_, ns, {{(void**)&d_scenes_, sizeof(DevScene)}, {(void**)&d_params_, sizeof(DevParams)}}) ||
+        !table(tile_first_cap_, ns, {{(void**)&d_tile_first_, sizeof(uint32_t)}}) ||
+        !table(pend_cap_, ns, {{(void**)&pend_, sizeof(uint32_t)}}) ||
+        !table(tile_cap_, ntiles_, {{(void**)&d_tiles_, sizeof(uint4)}}))
+        return fail(ENG_ENOMEM, "device allocation of scene tables failed");
     if (ns) ENG_CK(cudaMemcpyAsync(pend_, h_pend.data(), ns * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_),
                    "pending flags upload");
-    if (ntiles_ > tile_cap_) {
-        if (d_tiles_) cudaFree(d_tiles_);
-        tile_cap_ = std::max<uint64_t>(ntiles_, tile_cap_ * 2);
-        ENG_CK(cudaMalloc((void**)&d_tiles_, tile_cap_ * sizeof(uint4)), "tile table");
-        graph_dirty_ = true;
-    }
     if (ns) ENG_CK(cudaMemcpyAsync(d_scenes_, h_scenes_.data(), ns * sizeof(DevScene), cudaMemcpyHostToDevice, stream_), "scene upload");
     if (ns) {
         ENG_CK(cudaMemcpyAsync(d_tile_first_, h_tile_first_.data(), ns * sizeof(uint32_t), cudaMemcpyHostToDevice,
@@ -525,7 +540,6 @@ int Engine::rebuild_layout() {
     ENG_CK(cudaStreamSynchronize(stream_), "layout sync");
     layout_dirty_ = false;
     params_dirty_ = true;
-    graph_dirty_ = true;
     return ENG_OK;
 }
 
@@ -698,7 +712,7 @@ int Engine::settle() {
 
 // Layout, parameters and (in graph mode) the two captured graphs up to date.
 int Engine::prepare() {
-    if (!layout_dirty_ && !params_dirty_ && !graph_dirty_ && exec_pre_ && exec_suf_ && exec_full_) return ENG_OK;
+    if (!layout_dirty_ && !params_dirty_ && !graph_dirty_ && !scratch_lost_ && exec_pre_ && exec_suf_ && exec_full_) return ENG_OK;
     const auto t0 = std::chrono::steady_clock::now();
     const int rc = prepare_work();
     prep_seconds_ += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -706,6 +720,12 @@ int Engine::prepare() {
 }
 
 int Engine::prepare_work() {
+    if (scratch_lost_) {   // (a growth that failed)
+        if (!alloc_scratch(slot_scratch()) || !alloc_scratch(cell_scratch()))
+            return fail(ENG_ENOMEM, "device allocation failed");
+        scratch_lost_ = false;
+        graph_dirty_ = true;
+    }
     if (layout_dirty_ || params_dirty_) hashed_ = false;
     if (layout_dirty_) { int rc = rebuild_layout(); if (rc) return rc; }
     if (params_dirty_) { int rc = upload_params(); if (rc) return rc; update_form(); }
@@ -1268,6 +1288,7 @@ int Engine::debug_get(int id, int field, void* host, uint64_t count) {
     const Scene* s = scene(id);
     if (!s) return fail(ENG_EINVAL, "unknown scene id");
     if (!stepped_) return fail(ENG_EINVAL, "no substep has run yet");
+    if (scratch_lost_) return fail(ENG_ENOMEM, "the last substep's fields were lost to a growth that failed");
     size_t k = 0;
     for (; k < scenes_.size(); ++k) if (scenes_[k].id == id) break;
     const uint32_t n = s->n, nc = s->dp.ncells, cb = cell_base_[k], pb = s->part_base;

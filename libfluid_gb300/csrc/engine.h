@@ -178,6 +178,13 @@ private:
     int fail(int code, const std::string& msg);
     int cuda_fail(cudaError_t e, const char* what);
     int ensure_capacity(uint64_t parts, uint64_t cells);
+    struct Scratch;
+    bool regrow(void** p, size_t bytes, size_t keep);
+    std::vector<Scratch> slot_scratch();
+    std::vector<Scratch> cell_scratch();
+    bool alloc_scratch(const std::vector<Scratch>& arrays);
+    void free_scratch(const std::vector<Scratch>& arrays);
+    bool grow_scratch(uint64_t& cap, uint64_t to, std::vector<Scratch> (Engine::*arrays)());
     int rebuild_layout();
     int upload_params();
     LaunchForm form_of(uint32_t ntiles, bool persistent) const;
@@ -250,6 +257,7 @@ private:
     DevScene* d_scenes_ = nullptr;
     uint4* d_tiles_ = nullptr;
     uint64_t scene_cap_ = 0, tile_cap_ = 0;
+    bool scratch_lost_ = false;        // a growth failed and the old arrays did not come back either
     uint64_t dev_bytes_ = 0;
     uint64_t byte_limit_ = 0;
     // host mirrors

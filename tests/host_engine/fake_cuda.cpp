@@ -1,4 +1,5 @@
 #include "fake_cuda.h"
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -51,6 +52,31 @@ static Key key(const sph::StepArgs& a) {
     k.stride = a.mask_stride;
     return k;
 }
+// Every array that the substep's passes index, for the slots and cells they reach.
+static void check(const sph::StepArgs& a) {
+    bool ok = inside(a.tiles, a.ntiles * sizeof(uint4)) && inside(a.status, 4);
+    size_t slots = 0, scenes = 0;
+    for (uint32_t i = 0; ok && i < a.ntiles; ++i) {
+        slots = std::max<size_t>(slots, a.tiles[i].y + a.tiles[i].z);
+        scenes = std::max<size_t>(scenes, a.tiles[i].x + 1u);
+    }
+    for (const void* p : {(const void*)a.P0, (const void*)a.V0, (const void*)a.A0, (const void*)a.A1,
+                          (const void*)a.V2, (const void*)a.N})
+        ok = ok && inside(p, slots * sizeof(float4));
+    for (const void* p : {(const void*)a.G, (const void*)a.R}) ok = ok && inside(p, 2 * slots * sizeof(float4));
+    for (const void* p : {(const void*)a.okey, (const void*)a.key, (const void*)a.slot, (const void*)a.perm,
+                          (const void*)a.C2})
+        ok = ok && inside(p, slots * sizeof(uint32_t));
+    ok = ok && a.mask_stride >= slots && inside(a.mask, SPH_MASK_ROWS * a.mask_stride * sizeof(uint32_t)) &&
+         inside(a.count, a.total_cells * sizeof(uint32_t)) && inside(a.start, (a.total_cells + 1) * sizeof(uint32_t)) &&
+         inside(a.sums, (a.total_cells + 4095) / 4096 * sizeof(uint32_t)) &&
+         inside(a.scan_sums, ((a.total_cells + 4095) / 4096 + 2) * sizeof(uint64_t)) &&
+         inside(a.params, scenes * sizeof(DevParams)) && inside(a.scenes, scenes * sizeof(DevScene)) &&
+         inside(a.pend, scenes * sizeof(uint32_t)) &&
+         (!a.dbg_nbr || inside(a.dbg_nbr, slots * sizeof(uint32_t))) &&
+         (!a.dbg_forces || inside(a.dbg_forces, 4 * slots * sizeof(float4)));
+    if (!ok) ++st.bad_arrays;
+}
 static bool failed(const uint32_t* s) { return (*s & (SPH_STATUS_SCAN_TIMEOUT | SPH_STATUS_CELL_OVERFLOW)) != 0u; }
 }  // namespace fake
 
@@ -64,7 +90,12 @@ cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 152; return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "fake"; }
 cudaError_t cudaGetLastError() { return fake::last(); }
-cudaError_t cudaMalloc(void** p, size_t n) { return take(p, n); }
+cudaError_t cudaMalloc(void** p, size_t n) {
+    const long k = (long)fake::st.mallocs++;
+    if (fake::st.fail_from >= 0 && k >= fake::st.fail_from && k < (long)fake::st.fail_from + fake::st.fail_count)
+        return fake::st.last_error = cudaErrorMemoryAllocation;
+    return take(p, n);
+}
 cudaError_t cudaMallocHost(void** p, size_t n) {
     if (n > fake::st.pinned_limit) {
         *p = nullptr;
@@ -139,10 +170,14 @@ cudaError_t launch_build_tiles(const DevScene* scenes, const uint32_t* tile_firs
             tiles[tile_first[s] + i] = make_uint4(s, scenes[s].part_base + f, std::min(tile, scenes[s].n - f), 0u);
     return fake::last();
 }
-cudaError_t launch_hash(const StepArgs&, cudaStream_t) { return fake::last(); }
+cudaError_t launch_hash(const StepArgs& a, cudaStream_t) {
+    run([a] { fake::check(a); });
+    return fake::last();
+}
 cudaError_t launch_scan(const StepArgs&, cudaStream_t) { return fake::last(); }
 cudaError_t launch_sort(const StepArgs& a, cudaStream_t) {
     run([a] {
+        fake::check(a);
         if (fake::failed(a.status)) return;
         st.sorted = fake::key(a);
         st.sorts.push_back(a.ntiles);
@@ -153,6 +188,7 @@ cudaError_t launch_sort(const StepArgs& a, cudaStream_t) {
 }
 cudaError_t launch_density(const StepArgs& a, cudaStream_t) {
     run([a] {
+        fake::check(a);
         if (fake::failed(a.status)) return;
         if (!(st.sorted == fake::key(a))) ++st.mixed;
         st.written = fake::key(a);
@@ -165,6 +201,7 @@ cudaError_t launch_normals(const StepArgs& a, cudaStream_t) {
 }
 cudaError_t launch_force(const StepArgs& a, cudaStream_t) {
     run([a] {
+        fake::check(a);
         if (fake::failed(a.status)) return;
         ++st.substeps;
         st.lanes.insert(a.form.lanes);

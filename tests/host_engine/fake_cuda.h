@@ -31,6 +31,9 @@ struct State {
     std::vector<uint32_t> sorts;   // tiles of each sort
     size_t pinned_limit = ~(size_t)0;      // larger pinned allocations fail
     size_t pinned = 0;                     // bytes pinned now
+    int fail_from = -1, fail_count = 0;    // device allocations from the fail_from-th on fail, fail_count of them
+    uint64_t mallocs = 0;                  // device allocations asked for
+    uint64_t bad_arrays = 0;               // launches given an array that is freed, null or too short
     cudaError_t last_error = cudaSuccess;
     uint64_t null_writes = 0;      // packs and unsorts into a null or unknown buffer
 };
